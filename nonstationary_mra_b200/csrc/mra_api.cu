@@ -58,6 +58,9 @@ struct mra_ctx {
     std::vector<DevBuf> bufs;
     size_t bytes = 0;
     cudaStream_t stream = nullptr;
+    cudaStream_t side = nullptr;           // heavy finest regions, beside the small ones
+    cudaEvent_t fork = nullptr, join = nullptr;
+    std::vector<int> heavy_blocks;         // 64-wide block columns of each heavy finest region, largest first
     cudaEvent_t ev[8]{};
     cudaEvent_t tev[2 * MRA_MAX_TIMED]{};  // start/stop of every launch
     // start/stop of each covariance-block launch of the prior levels, and the
@@ -131,6 +134,9 @@ struct mra_ctx {
             if (e) cudaEventDestroy(e);
         for (auto& e : cev)
             if (e) cudaEventDestroy(e);
+        if (fork) cudaEventDestroy(fork);
+        if (join) cudaEventDestroy(join);
+        if (side) cudaStreamDestroy(side);
         if (stream) cudaStreamDestroy(stream);
         for (auto& b : bufs) cudaFree(b.p);
     }
@@ -176,8 +182,10 @@ mra_status upload(void* dst, const void* src, size_t bytes, cudaStream_t st) {
 // Host-side description of the tree used for sizing, scheduling and FLOP counts.
 struct HostTree {
     std::vector<int64_t> nfin, npred, obs_off, pred_off, fin_anc, pred_order, lsig_off, pc_off;
-    std::vector<int64_t> child_lo, child_hi, par_order, sub_lo, sub_hi, dslot, post_order;
+    std::vector<int64_t> child_lo, child_hi, fin_items, heavy, sub_lo, sub_hi, dslot, post_order;
     std::vector<int8_t> factored;
+    std::vector<FinChunk> chunks;
+    std::vector<HeavyTile> heavy_tiles;
 };
 
 // Algorithmic multiply-adds of the region kernels as run here (symmetric
@@ -329,8 +337,18 @@ mra_status run_eval(mra_ctx* c, bool predict) {
                     }
                     launched += 3;
                 }
-                if (mixed && c->mixed_finest32) launched += launch_finest_group<float>(c->geom, tf, c->grid, predict, st);
-                else launched += launch_finest_group<double>(c->geom, td, c->grid, predict, st);
+                {
+                    const FinestFork fk{c->side, c->fork, c->join, c->heavy_blocks.data()};
+                    if (mixed && c->mixed_finest32) {
+                        launched += launch_finest<float>(c->geom, tf, c->grid, st, fk);
+                    } else {
+                        launched += launch_finest<double>(c->geom, td, c->grid, st, fk);
+                        if (td.fuse_post) {
+                            launch_posterior_level<double>(c->geom, td, c->M - 2, c->grid, predict, st);
+                            launched += 1;
+                        }
+                    }
+                }
                 break;
             case MRA_KERNEL_CONVERT:
                 if (c->mixed_prior32 && c->mixed_finest32) {
@@ -436,7 +454,9 @@ mra_status finish_eval(mra_ctx* c) {
 // Allocates the typed buffers of one precision and fills its DevTree.
 // Shared FP64 vectors and bookkeeping used by both trees.
 struct Shared {
-    double *yt, *ldprior, *vpost, *dpost, *dfin, *mean, *var;
+    double *yt, *ldprior, *vpost, *dpost, *dchild, *dfin, *heavy_inv, *mean, *var;
+    const FinChunk* chunks;
+    const HeavyTile* heavy_tiles;
     int *queue, *err;
     int8_t* factored;
 };
@@ -455,11 +475,18 @@ mra_status setup_tree(mra_ctx* c, DevTree<T>& t, const HostTree& h, const PointS
     t.pts = pts;
     t.y = y;
     t.obs_off = idx[0]; t.pred_off = idx[1]; t.fin_anc = idx[2]; t.pred_order = idx[3]; t.lsig_off = idx[4];
-    t.pc_off = idx[5]; t.child_lo = idx[6]; t.child_hi = idx[7]; t.par_order = idx[8]; t.sub_lo = idx[9];
+    t.pc_off = idx[5]; t.child_lo = idx[6]; t.child_hi = idx[7]; t.fin_items = idx[8]; t.sub_lo = idx[9];
     t.sub_hi = idx[10];
     t.dslot = idx[11];
     t.post_order = idx[12];
-    t.n_fin_items = (long)h.par_order.size();
+    t.n_fin_items = (long)h.fin_items.size();
+    t.heavy = idx[13];
+    t.n_heavy = (long)h.heavy.size();
+    t.chunks = sh.chunks;
+    t.n_chunks = (long)h.chunks.size();
+    t.heavy_tiles = sh.heavy_tiles;
+    t.n_heavy_tiles = (long)h.heavy_tiles.size();
+    t.heavy_inv = sh.heavy_inv;
     // sizes of the level-parity buffers
     size_t aout_sz[2] = {1, 1}, wout_sz[2] = {1, 1}, F_sz[2] = {1, 1}, f_sz[2] = {1, 1};
     for (int m = 1; m <= M - 2; ++m) {
@@ -481,8 +508,8 @@ mra_status setup_tree(mra_ctx* c, DevTree<T>& t, const HostTree& h, const PointS
     }
     t.ws_stride = post_part ? std::max((long)r * c->tf + 2L * c->tf * c->tf, n_slices(M - 1) * rr + (long)(M - 2) * rr + rr) + 64
                             : 64;
-    // prior: V of one conditioning step (r x r); finest: the inverse of a
-    // child's L_Sigma (n x n, n <= 64), or a whole sibling group's conditional
+    // prior: V of one conditioning step (r x r); finest: the inverse of a small
+    // region's L_Sigma (n x n, n <= 64), or a whole sibling group's conditional
     // covariance and block-diagonal inverse (2 x 64 x 64)
     if (prior_part) t.ws_stride = std::max(t.ws_stride, std::max(rr, 2L * 64 * 64) + 64);
     t.wsd_stride = post_part ? (long)(M - 1) * r + c->tf + 64 : 64;
@@ -551,6 +578,7 @@ mra_status setup_tree(mra_ctx* c, DevTree<T>& t, const HostTree& h, const PointS
     t.ldprior = sh.ldprior;
     t.vpost = sh.vpost;
     t.dpost = sh.dpost;
+    t.dchild = sh.dchild;
     t.dfin = sh.dfin;
     t.mean = sh.mean;
     t.var = sh.var;
@@ -658,8 +686,19 @@ mra_status mra_create(const mra_structure* s, const mra_model* m, int32_t precis
     c->have_pred = have_pred_arr && n_pred > 0;
     c->tf = 2 * r;
     if (const char* e = std::getenv("MRA_FACTORED_MAX")) c->tf = std::max(0, std::atoi(e));
+    if (precision == MRA_PRECISION_MIXED) {
+        if (const char* e = std::getenv("MRA_MIXED_FP32")) {
+            const std::string v(e);
+            c->mixed_prior32 = v.find("prior") != std::string::npos;
+            c->mixed_finest32 = v.find("finest") != std::string::npos;
+        }
+    }
     c->geom = make_geom(m);
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess)
+        return bail(fail(MRA_ERR_CUDA, "stream creation failed"));
+    if (cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->join, cudaEventDisableTiming) != cudaSuccess)
         return bail(fail(MRA_ERR_CUDA, "stream creation failed"));
     if (cudaError_t pe = prepare_kernels(); pe != cudaSuccess)
         return bail(fail(MRA_ERR_CUDA, std::string("kernel attributes: ") + cudaGetErrorString(pe)));
@@ -769,41 +808,64 @@ mra_status mra_create(const mra_structure* s, const mra_model* m, int32_t precis
         std::stable_sort(h.post_order.begin() + s0, h.post_order.begin() + s0 + cnt,
                          [&](int64_t a, int64_t b) { return cost[a] > cost[b]; });
     }
-    // work items of the finest kernel: a level M-3 region with its J sibling
-    // groups when it holds at most 64 J observations (conditioning shared by
-    // the groups), else each of its groups alone (load balance); for M = 2 the
-    // single level-0 group.  Most expensive first.
+    // finest level, conditioning: runs of at most 64 observations below one
+    // level M-3 region (the root when M = 2).  Every run walks the same chain of
+    // products whatever its width, so wider runs cost less per observation; they
+    // are narrowed only while there are fewer runs than two per SM.
     {
-        const long n_units = M >= 3 ? level_count(J, M - 3) : 0;
+        const long n_units = M >= 3 ? level_count(J, M - 3) : 1;
         const long lvl3 = M >= 3 ? level_start(J, M - 3) : 0;
-        long unit_max = 64L * J;  // observations of a unit processed as one item
-        if (const char* e = std::getenv("MRA_UNIT_OBS_MAX")) unit_max = std::max(0L, std::atol(e));
-        auto group_cost = [&](long gl) {
-            const double n = (double)(h.sub_hi[lvl2 + gl] - h.sub_lo[lvl2 + gl]);
-            return n * (n + 64.0 * L);
-        };
-        std::vector<std::pair<double, int64_t>> items;
-        if (M >= 3) {
+        long width = 64;
+        auto build = [&]() {
+            h.chunks.clear();
             for (long u = 0; u < n_units; ++u) {
-                const long nu = h.sub_hi[lvl3 + u] - h.sub_lo[lvl3 + u];
-                if (nu <= unit_max) {
-                    double c = 0.0;
-                    for (long gl = u * J; gl < u * J + J; ++gl) c += group_cost(gl);
-                    items.push_back({c, (int64_t)u});
-                } else {
-                    for (long gl = u * J; gl < u * J + J; ++gl)
-                        items.push_back({group_cost(gl), (int64_t)(n_units + gl)});
-                }
+                const long lo = h.sub_lo[lvl3 + u], nu = h.sub_hi[lvl3 + u] - lo;
+                if (nu <= 0) continue;
+                const long k = (nu + width - 1) / width;             // runs of this region, of equal size
+                const long w = (((nu + k - 1) / k) + 7) & ~7L;       // in whole fragments of 8
+                for (long o = 0; o < nu; o += w)
+                    h.chunks.push_back({(int64_t)(lo + o), (int32_t)std::min(w, nu - o), (int32_t)u});
             }
-        } else {
-            items.push_back({group_cost(0), 0});
+        };
+        for (build(); width > 16 && (long)h.chunks.size() < 2L * c->sms; build()) width /= 2;
+    }
+    // finest level, small regions: a sibling group whose children hold at most
+    // kChildMax observations each and kGroupMax together is one item (FP64), any
+    // other region of at most kFinTile is its own; most expensive first.  FP64
+    // regions beyond that are factored tile by tile.
+    {
+        const bool fp64 = !(precision == MRA_PRECISION_MIXED && c->mixed_finest32);
+        std::vector<std::pair<double, int64_t>> items, heavy;
+        for (long q = 0; q < cnt2; ++q) {
+            const long clo = h.child_lo[q], chi = h.child_hi[q];
+            const long np = h.obs_off[chi] - h.obs_off[clo];
+            if (np == 0) continue;
+            long nmax = 0;
+            for (long k = clo; k < chi; ++k) nmax = std::max<long>(nmax, h.nfin[k]);
+            if (fp64 && nmax <= kChildMax && np <= kGroupMax && chi - clo <= kThreads / 32) {
+                items.push_back({(double)np * (np + L * r), (int64_t)q});
+                continue;
+            }
+            for (long k = clo; k < chi; ++k) {
+                const double n = (double)h.nfin[k];
+                if (n == 0) continue;
+                if (fp64 && n > kFinTile) heavy.push_back({n, (int64_t)k});
+                else items.push_back({n * n * (n + 2.0 * L * r) + 64.0 * n * L * r, (int64_t)(cnt2 + k)});
+            }
         }
-        std::stable_sort(items.begin(), items.end(),
-                         [](const std::pair<double, int64_t>& x, const std::pair<double, int64_t>& y) {
-                             return x.first > y.first;
-                         });
-        h.par_order.resize(items.size());
-        for (size_t q = 0; q < items.size(); ++q) h.par_order[q] = items[q].second;
+        auto more = [](const std::pair<double, int64_t>& x, const std::pair<double, int64_t>& y) {
+            return x.first > y.first;
+        };
+        std::stable_sort(items.begin(), items.end(), more);
+        std::stable_sort(heavy.begin(), heavy.end(), more);
+        for (const auto& it : items) h.fin_items.push_back(it.second);
+        for (size_t q = 0; q < heavy.size(); ++q) {
+            h.heavy.push_back(heavy[q].second);
+            const int nb = (int)((h.nfin[heavy[q].second] + kFinTile - 1) / kFinTile);
+            c->heavy_blocks.push_back(nb);
+            for (int bi = 0; bi < nb; ++bi)
+                for (int bj = 0; bj <= bi; ++bj) h.heavy_tiles.push_back({(int32_t)q, (uint16_t)bi, (uint16_t)bj});
+        }
     }
     int64_t u_total = 0;
     for (int mm = 0; mm <= M - 2; ++mm) u_total += level_count(J, mm) * (int64_t)mm * r * r;
@@ -821,11 +883,11 @@ mra_status mra_create(const mra_structure* s, const mra_model* m, int32_t precis
     }
     double* y = c->alloc<double>(n_obs, &ce);
     if (ce) return bail(fail(MRA_ERR_OOM, "device allocation failed: y"));
-    const std::vector<int64_t>* tabs[13] = {&h.obs_off, &h.pred_off, &h.fin_anc, &h.pred_order, &h.lsig_off,
-                                            &h.pc_off, &h.child_lo, &h.child_hi, &h.par_order, &h.sub_lo, &h.sub_hi,
-                                            &h.dslot, &h.post_order};
-    int64_t* idx[13];
-    for (int q = 0; q < 13; ++q) {
+    const std::vector<int64_t>* tabs[14] = {&h.obs_off, &h.pred_off, &h.fin_anc, &h.pred_order, &h.lsig_off,
+                                            &h.pc_off, &h.child_lo, &h.child_hi, &h.fin_items, &h.sub_lo, &h.sub_hi,
+                                            &h.dslot, &h.post_order, &h.heavy};
+    int64_t* idx[14];
+    for (int q = 0; q < 14; ++q) {
         idx[q] = c->alloc<int64_t>(tabs[q]->size(), &ce);
         if (ce) return bail(fail(MRA_ERR_OOM, "device allocation failed: index tables"));
         mra_status u = upload(idx[q], tabs[q]->data(), tabs[q]->size() * sizeof(int64_t), c->stream);
@@ -860,7 +922,13 @@ mra_status mra_create(const mra_structure* s, const mra_model* m, int32_t precis
     if (!ce) sh.ldprior = c->alloc<double>(n_int, &ce);
     if (!ce) sh.vpost = c->alloc<double>(n_int * r, &ce);
     if (!ce) sh.dpost = c->alloc<double>(n_int, &ce);
+    if (!ce) sh.dchild = c->alloc<double>(n_fin, &ce);
     if (!ce) sh.dfin = c->alloc<double>(cnt2, &ce);
+    if (!ce) sh.heavy_inv = c->alloc<double>(h.heavy.size() * 64 * 64, &ce);
+    FinChunk* chunks = nullptr;
+    HeavyTile* heavy_tiles = nullptr;
+    if (!ce) sh.chunks = chunks = c->alloc<FinChunk>(h.chunks.size(), &ce);
+    if (!ce) sh.heavy_tiles = heavy_tiles = c->alloc<HeavyTile>(h.heavy_tiles.size(), &ce);
     if (!ce) sh.mean = c->alloc<double>(n_pred, &ce);
     if (!ce) sh.var = c->alloc<double>(n_pred, &ce);
     if (!ce) sh.queue = c->alloc<int>(kQueueCounters, &ce);
@@ -869,17 +937,15 @@ mra_status mra_create(const mra_structure* s, const mra_model* m, int32_t precis
     if (ce) return bail(fail(MRA_ERR_OOM, "device allocation failed: shared vectors"));
     {
         mra_status u = upload(sh.factored, h.factored.data(), n_int * sizeof(int8_t), c->stream);
+        if (!u) u = upload(chunks, h.chunks.data(), h.chunks.size() * sizeof(FinChunk), c->stream);
+        if (!u) u = upload(heavy_tiles, h.heavy_tiles.data(), h.heavy_tiles.size() * sizeof(HeavyTile), c->stream);
         if (u) return bail(u);
         CU(cudaMemsetAsync(sh.dpost, 0, n_int * sizeof(double), c->stream));
+        CU(cudaMemsetAsync(sh.dchild, 0, n_fin * sizeof(double), c->stream));
     }
     c->u_total = u_total;
     mra_status st;
     if (precision == MRA_PRECISION_MIXED) {
-        if (const char* e = std::getenv("MRA_MIXED_FP32")) {
-            const std::string v(e);
-            c->mixed_prior32 = v.find("prior") != std::string::npos;
-            c->mixed_finest32 = v.find("finest") != std::string::npos;
-        }
         const bool both = c->mixed_prior32 && c->mixed_finest32;
         st = setup_tree<float>(c, c->tf32, h, pts, y, idx, u_total, sh, true, false, c->have_pred);
         if (!st) st = setup_tree<double>(c, c->td, h, pts, y, idx, u_total, sh, !both, true, false);
@@ -1237,6 +1303,7 @@ mra_status mra_autotune(mra_ctx* c, int32_t evals, int32_t* choice_out, double* 
     int ib = 0;
     for (int k = 0; k < nc; ++k) {
         CU(set_gemm_tiles(cand[k]));
+        CU(set_gemm_tiles_finest(cand[k]));
         double d, ll, ms = 0.0;
         mra_status st = mra_loglik(c, &d, &ll);  // warm-up with this choice
         if (st != MRA_OK) return st;
@@ -1251,6 +1318,7 @@ mra_status mra_autotune(mra_ctx* c, int32_t evals, int32_t* choice_out, double* 
         if (ms < best) best = ms, ib = k;
     }
     CU(set_gemm_tiles(cand[ib]));
+    CU(set_gemm_tiles_finest(cand[ib]));
     if (choice_out)
         for (int b = 0; b < 3; ++b) choice_out[b] = cand[ib][b];
     if (ms_out) *ms_out = best / evals;

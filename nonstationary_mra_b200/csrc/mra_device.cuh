@@ -445,6 +445,86 @@ __device__ inline void fill_cov(const Geom& g, const PointSet& P, long a0, int n
     fill_cov_blocks<T>(g, P, &a0, 1, na, b0, nb, self, out, ld, 0, sm);
 }
 
+constexpr int kCovThreads = 256;
+constexpr int kCovChunk = 64;  // column points staged per chunk (7 x 64 doubles of shared memory)
+
+// The straight-line nonstationary FP64 block: one row point per thread with its
+// parameters in registers, the column points staged in chunks, entries of
+// cov_fast_entry (the same arithmetic as fill_row_fast).
+template <typename T, int NU, int PREF>
+__device__ __forceinline__ void cov_block_fast(const PointSet& P, long a0, int nr, long b0, int nc, bool self,
+                                               T* __restrict__ out, long ld, double ih2, double ihs2,
+                                               double* stage) {
+    double* sx = stage;
+    double* sy = sx + kCovChunk;
+    double* sz = sy + kCovChunk;
+    double* sg = sz + kCovChunk;
+    double* s4 = sg + kCovChunk;  // sqrt(s2) b (PREF 1) or sqrt(s2) (PREF 0)
+    double* s5 = s4 + kCovChunk;  // b (PREF 0)
+    const int tid = threadIdx.x, nt = blockDim.x;
+    const int rows = nr < nt ? nr : nt;
+    const int cols = nt / rows;
+    const bool worker = tid < rows * cols;
+    const int tr = tid % rows, tc = tid / rows;
+    for (int q0 = 0; q0 < nc; q0 += kCovChunk) {
+        const int qn = nc - q0 < kCovChunk ? nc - q0 : kCovChunk;
+        __syncthreads();
+        for (int e = tid; e < qn; e += nt) {
+            const long ib = b0 + q0 + e;
+            const double bb = P.beta[ib], ssq = sqrt(P.s2[ib]);
+            sx[e] = P.c0[ib];
+            sy[e] = P.c1[ib];
+            sz[e] = P.c2[ib];
+            sg[e] = bb * bb * ih2;
+            s4[e] = PREF == 1 ? ssq * bb : ssq;
+            s5[e] = bb;
+        }
+        __syncthreads();
+        if (!worker) continue;
+        for (int t = tr; t < nr; t += rows) {
+            const long ia = a0 + t;
+            const double pc0 = P.c0[ia], pc1 = P.c1[ia], pc2 = P.c2[ia], sa = P.s2[ia], ba = P.beta[ia];
+            const double ssa = sqrt(sa), ga = ba * ba * ih2, ca = ssa * ba * ihs2, ba_h = ba * ihs2;
+            const double diag = self ? sa + P.t2[ia] : 0.0;
+            T* ob = out + t;
+#pragma unroll 4
+            for (int q = tc; q < qn; q += cols) {
+                const int qq = q0 + q;
+                double v = cov_fast_entry<NU, PREF, true>(pc0, pc1, pc2, ga, ca, ssa, ba_h, sx[q], sy[q], sz[q], sg[q],
+                                                    PREF == 1 ? s4[q] : 0.0, PREF == 1 ? 0.0 : s4[q],
+                                                    PREF == 1 ? 0.0 : s5[q]);
+                if (self && t == qq) v = diag;  // sigma^2 + tau^2 (evaluate_covariance.cpp:103,307)
+                ob[(long)qq * ld] = (T)v;
+            }
+        }
+    }
+    __syncthreads();
+}
+
+// Block out[t + q ld] = C(A_{a0+t}, B_{b0+q}), t < nr, q < nc (with the
+// sigma^2 + tau^2 diagonal when `self`), by the whole CTA.  KIND (cov_kind on the
+// host): 1..4 the straight-line nonstationary FP64 forms (Matern 3/2 or 1/2 x
+// prefactor exponent 1 or 3/2), 0 every other model.
+// CH: column points staged per chunk by the other models (7 CH doubles of stage).
+template <typename T, int KIND, int CH = kCovChunk>
+__device__ __forceinline__ void cov_block(const Geom& g, const PointSet& P, long a0, int nr, long b0, int nc, bool self,
+                                          T* out, long ld, double* stage) {
+    if constexpr (KIND == 0) {
+        fill_cov_staged<T, CH>(g, P, &a0, 1, nr, b0, nc, self, out, ld, 0, stage);
+    } else {
+        const double hs = g.dist_scale * (KIND <= 2 ? 1.7320508075688772 : 1.0);
+        const double ihs2 = 1.0 / (hs * hs), ih2 = 0.5 * ihs2;
+        constexpr int NU = KIND <= 2 ? 3 : 1, PREF = (KIND & 1) ? 1 : 0;
+        cov_block_fast<T, NU, PREF>(P, a0, nr, b0, nc, self, out, ld, ih2, ihs2, stage);
+    }
+}
+
+inline int cov_kind(const Geom& g, bool fp64) {
+    if (!(fp64 && g.nonstat && g.distance != 1 && g.pref_kind != 2)) return 0;
+    return g.nu_x2 == 3 ? (g.pref_kind == 1 ? 1 : 2) : (g.pref_kind == 1 ? 3 : 4);
+}
+
+
 // ---- FP64: warp tile (8 NW) rows x 16 columns --------------------------------
 template <int NW>
 struct AccD {
@@ -456,6 +536,13 @@ __device__ __forceinline__ void cp_async8(double* dst, const double* src, bool p
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
     const int n = pred ? 8 : 0;
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+// 16-byte asynchronous global -> shared copy through L2 only; pred == false
+// writes zeros (src must then still be a valid 16-byte aligned address).
+__device__ __forceinline__ void cp_async16z(double* dst, const double* src, bool pred) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    const int n = pred ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(n) : "memory");
 }
 // Bulk prefetch into L2 of the 16-byte aligned part of [p, p + bytes) (the
 // instruction takes a 16-byte aligned address and a multiple of 16 bytes).

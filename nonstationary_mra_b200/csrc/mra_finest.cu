@@ -1,0 +1,652 @@
+// Finest level of the MRA hot path (...-loop-regions-at-finest-level-in-prior.cpp:
+// 90-269, class_approximation.cpp:52-82): conditioning of the observations on
+// their ancestors, the finest regions' conditional covariances with their
+// Cholesky factors, and the log-likelihood terms.
+//
+// The level runs as separate launches, each split by what is independent in it,
+// so that neither a few heavily clustered regions nor a tree with few regions
+// leaves the chip to a handful of CTAs (one CTA per level M-3 region with all of
+// these steps inside took 2.43 of the 2.61 ms of an 8,192-point evaluation,
+// 16 CTAs in flight, and 79 of 93 ms of a 262,144-point clustered prediction,
+// one CTA finishing the largest regions):
+//   k_cov_finest            C(Q_{a_j}, S) of every ancestor level, into B^
+//   k_finest_condition*     V_j and U_j of a chunk of at most 64 observations:
+//                           every observation conditions on its own, so the
+//                           chunks are as many as the chip needs
+//   k_finest_children       Sigma, L_Sigma, y~, B^ of one finest region of at most
+//                           64 observations, or of a sibling group of small ones
+//   k_heavy_*               the same of larger finest regions in 64 x 64 tiles,
+//                           one CTA per tile, the block columns in turn
+//   k_finest_terms          log-lik terms summed per sibling group
+#include "mra_kernels.cuh"
+
+namespace mra {
+
+// ---------------------------------------------------------------------------
+// covariance of the observations with their ancestors' knots
+// ---------------------------------------------------------------------------
+// Task (chunk, j): block C(Q_{a_j}, S_chunk), r x n, into row block j of B^.  The
+// deepest ancestor (level M-2) differs between the sibling groups of a chunk.
+// Issue-bound like k_cov_level: its own launch keeps 4 CTAs per SM busy.
+template <typename T, int KIND>
+__global__ void __launch_bounds__(kCovThreads, 4) k_cov_finest(Geom g, DevTree<T> t) {
+    constexpr int CH = sizeof(T) == 8 ? kCovChunk : 96;  // FP32: the chunk of fill_cov, and so its compiled code
+    __shared__ double stage[7 * CH];
+    const int r = t.r, L = t.L, m = t.M - 2;
+    const long Lr = (long)L * r;
+    const long ntask = t.n_chunks * L;
+    for (long b = blockIdx.x; b < ntask; b += gridDim.x) {
+        const long q = b / L;
+        const int j = (int)(b - q * L);
+        const FinChunk ch = t.chunks[q];
+        const long unit = ch.unit;  // local index at level M-3 (0 when M == 2)
+        if (skipped(t, chunk_region(t, unit))) continue;
+        if (j < m) {
+            long a = chunk_region(t, unit);  // level m-1, up to level j
+            for (int l = m - 1; l > j; --l) a = (a - 1) / t.J;
+            cov_block<T, KIND, CH>(g, t.pts, a * r, r, t.obs0 + ch.lo, ch.n, false, t.Bhat + ch.lo * Lr + (long)j * r, Lr,
+                               stage);
+        } else {
+            const long g0 = m > 0 ? unit * t.J : 0, g1 = m > 0 ? g0 + t.J : 1;
+            const long s2 = level_start(t.J, m);
+            for (long gl = g0; gl < g1; ++gl) {
+                const long glo = t.sub_lo[s2 + gl], ghi = t.sub_hi[s2 + gl];
+                const long lo = glo > ch.lo ? glo : ch.lo, hi = ghi < ch.lo + ch.n ? ghi : ch.lo + ch.n;
+                if (lo >= hi) continue;
+                cov_block<T, KIND, CH>(g, t.pts, (s2 + gl) * r, r, t.obs0 + lo, (int)(hi - lo), false,
+                                   t.Bhat + lo * Lr + (long)m * r, Lr, stage);
+            }
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// conditioning: V_j = C_j - U_{a_j}^T U_{S,0..j-1},  U_{S,j} = L_{a_j}^{-1} V_j
+// ---------------------------------------------------------------------------
+// FP64, r <= RC <= 64.  One CTA per chunk walks the ancestors; per ancestor one
+// product over K = j r (slabs of 32, three in flight: U_a of the deepest
+// ancestor is read once and comes from HBM) and one with the stored inverse,
+// whose operand V_j stays in shared memory.  RC is the tile height (16, 32 or
+// 64): 8 warps as RC / 8 row groups x 64 / RC column groups, each warp 8 rows x
+// up to RC columns, so that small r and narrow chunks leave no warp multiplying
+// padding.  EVEN: r even, operand rows 16-byte aligned, copied in pairs.
+template <int RC>
+struct CondSmem {
+    static constexpr int AS = RC * KS64 > TK64 * (RC + 4) ? RC * KS64 : TK64 * (RC + 4);
+    double A[3][AS];
+    double B[3][64 * KS64];  // also V, [column][row], row stride RC + 4
+};
+
+template <int RC, bool EVEN>
+__device__ __forceinline__ void cond_step(CondSmem<RC>& sm, int r, const double* Ua, int K, const double* Us, long Lr,
+                                          int N, const double* P, double* V, double* U) {
+    constexpr int RW = RC / 8, CW = 8 / RW, NF = RC / 8;  // row groups, column groups, fragments per warp
+    constexpr int RS = RC + 4, VS = RC + 4;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int g = lane >> 2, t = lane & 3;
+    const int wr = w % RW, wc = w / RW;
+    const int N8 = (N + 7) & ~7;
+    const int row = 8 * wr + g;
+    double acc[NF][2];
+    // accumulators start at -C, so that acc ends at -(C - U_a^T U_S)
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+        const int c = (f * CW + wc) * 8 + 2 * t;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) acc[f][h] = (row < r && c + h < N) ? -V[row + (long)(c + h) * Lr] : 0.0;
+    }
+    auto issue = [&](int k0, int s) {
+        double* sA = sm.A[s];
+        double* sB = sm.B[s];
+        if (EVEN) {
+            for (int e = tid; e < RC * (TK64 / 2); e += kThreads) {
+                const int i = e / (TK64 / 2), k = 2 * (e % (TK64 / 2));
+                const bool ok = i < r && k0 + k < K;
+                cp_async16z(sA + i * KS64 + k, ok ? Ua + (k0 + k) + (long)i * K : Ua, ok);
+            }
+            for (int e = tid; e < N8 * (TK64 / 2); e += kThreads) {
+                const int j = e / (TK64 / 2), k = 2 * (e % (TK64 / 2));
+                const bool ok = j < N && k0 + k < K;
+                cp_async16z(sB + j * KS64 + k, ok ? Us + (k0 + k) + (long)j * Lr : Us, ok);
+            }
+        } else {
+            for (int e = tid; e < RC * TK64; e += kThreads) {
+                const int i = e / TK64, k = e % TK64;
+                const bool ok = i < r && k0 + k < K;
+                cp_async8(sA + i * KS64 + k, ok ? Ua + (k0 + k) + (long)i * K : Ua, ok);
+            }
+            for (int e = tid; e < N8 * TK64; e += kThreads) {
+                const int j = e / TK64, k = e % TK64;
+                const bool ok = j < N && k0 + k < K;
+                cp_async8(sB + j * KS64 + k, ok ? Us + (k0 + k) + (long)j * Lr : Us, ok);
+            }
+        }
+    };
+    const int ns = (K + TK64 - 1) / TK64;
+    if (ns > 0) issue(0, 0);
+    cp_async_commit();
+    if (ns > 1) issue(TK64, 1);
+    cp_async_commit();
+    int s = 0;
+    for (int i = 0; i < ns; ++i) {
+        cp_async_wait<1>();  // slab i has landed (for this thread; the barrier makes it so for all)
+        __syncthreads();     // and every warp is done with slab i - 1, whose stage slab i + 2 takes
+        const int s2 = s == 0 ? 2 : s - 1;
+        if (i + 2 < ns) issue((i + 2) * TK64, s2);
+        cp_async_commit();
+        const double* sA = sm.A[s] + row * KS64 + t;
+        const double* sB = sm.B[s] + g * KS64 + t;
+#pragma unroll
+        for (int k4 = 0; k4 < TK64; k4 += 4) {
+            const double a = sA[k4];
+#pragma unroll
+            for (int f = 0; f < NF; ++f) {
+                const int c0 = (f * CW + wc) * 8;
+                if (c0 < N8) mma_f64(acc[f], a, sB[c0 * KS64 + k4]);
+            }
+        }
+        s = s == 2 ? 0 : s + 1;
+    }
+    __syncthreads();
+    // L_a^{-1} (lower triangular, zeros above) as two slabs [k][row]; V_j to memory and as the next operand
+    for (int e = tid; e < RC * (EVEN ? RC / 2 : RC); e += kThreads) {
+        const int i = EVEN ? 2 * (e % (RC / 2)) : e % RC, k = EVEN ? e / (RC / 2) : e / RC;
+        double* dst = sm.A[k / TK64] + (k % TK64) * RS + i;
+        const bool ok = i < r && k < r;
+        if (EVEN) cp_async16z(dst, ok ? P + i + (long)k * r : P, ok);
+        else cp_async8(dst, ok ? P + i + (long)k * r : P, ok);
+    }
+    cp_async_commit();
+    double* sV = &sm.B[0][0];
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+        const int c = (f * CW + wc) * 8 + 2 * t;
+        if ((f * CW + wc) * 8 >= N8) continue;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const double v = -acc[f][h];
+            sV[(c + h) * VS + row] = v;
+            if (row < r && c + h < N) V[row + (long)(c + h) * Lr] = v;
+            acc[f][h] = 0.0;
+        }
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    const int kend = 8 * (wr + 1);  // rows 8 wr .. 8 wr + 7 of a lower-triangular factor
+#pragma unroll 4
+    for (int k4 = 0; k4 < kend; k4 += 4) {
+        const double a = sm.A[k4 / TK64][(k4 % TK64 + t) * RS + row];
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+            const int c0 = (f * CW + wc) * 8;
+            if (c0 < N8) mma_f64(acc[f], a, sV[(c0 + g) * VS + k4 + t]);
+        }
+    }
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+        const int c = (f * CW + wc) * 8 + 2 * t;
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            if (row < r && c + h < N) U[row + (long)(c + h) * Lr] = acc[f][h];
+    }
+    __syncthreads();
+}
+
+template <int RC, bool EVEN>
+__global__ void __launch_bounds__(kThreads, 2) k_finest_condition(DevTree<double> t) {
+    extern __shared__ __align__(16) unsigned char la_dyn_smem[];
+    CondSmem<RC>& sm = *reinterpret_cast<CondSmem<RC>*>(la_dyn_smem);
+    const int r = t.r, L = t.L, m = t.M - 2;
+    const long rr = (long)r * r, Lr = (long)L * r;
+    const FinChunk ch = t.chunks[blockIdx.x];
+    const long unit = ch.unit;
+    if (skipped(t, chunk_region(t, unit))) return;
+    double* V = t.Bhat + ch.lo * Lr;
+    double* U = t.Ufin + ch.lo * Lr;
+    for (int j = 0; j < m; ++j) {
+        long a = chunk_region(t, unit);
+        for (int l = m - 1; l > j; --l) a = (a - 1) / t.J;
+        const double* Ua = t.U + t.u_off[j] + (a - level_start(t.J, j)) * (long)j * rr;
+        cond_step<RC, EVEN>(sm, r, Ua, j * r, U, Lr, ch.n, t.Pinv + a * rr, V + (long)j * r, U + (long)j * r);
+    }
+    const long g0 = m > 0 ? unit * t.J : 0, g1 = m > 0 ? g0 + t.J : 1;
+    const long s2 = level_start(t.J, m);
+    for (long gl = g0; gl < g1; ++gl) {
+        const long glo = t.sub_lo[s2 + gl], ghi = t.sub_hi[s2 + gl];
+        const long lo = glo > ch.lo ? glo : ch.lo, hi = ghi < ch.lo + ch.n ? ghi : ch.lo + ch.n;
+        if (lo >= hi) continue;
+        const long d = (lo - ch.lo) * Lr;
+        cond_step<RC, EVEN>(sm, r, t.U + t.u_off[m] + gl * (long)m * rr, m * r, U + d, Lr, (int)(hi - lo),
+                            t.Pinv + (s2 + gl) * rr, V + d + (long)m * r, U + d + (long)m * r);
+    }
+}
+
+// The same through the general products: FP32 storage, or r > 64.
+template <typename T>
+__global__ void __launch_bounds__(kThreads, 2) k_finest_condition_any(DevTree<T> t) {
+    LaSmem<T>& sm = la_smem<T>();
+    const int r = t.r, L = t.L, m = t.M - 2;
+    const long rr = (long)r * r, Lr = (long)L * r;
+    const FinChunk ch = t.chunks[blockIdx.x];
+    const long unit = ch.unit;
+    if (skipped(t, chunk_region(t, unit))) return;
+    auto step = [&](long a, int j, const T* Ua, long d, int n) {
+        T* V = t.Bhat + (ch.lo + d) * Lr + (long)j * r;
+        T* U = t.Ufin + (ch.lo + d) * Lr;
+        if (j > 0) gemm<T, true, false>(r, n, j * r, (T)-1, Ua, (long)j * r, U, Lr, (T)1, V, Lr, sm);
+        gemm<T, false, false>(r, n, r, (T)1, t.Pinv + a * rr, r, V, Lr, (T)0, U + (long)j * r, Lr, sm);
+    };
+    const long g0 = m > 0 ? unit * t.J : 0, g1 = m > 0 ? g0 + t.J : 1;
+    const long s2 = level_start(t.J, m);
+    long gl = g0 - 1;
+    for (int j = 0; j < m || gl + 1 < g1;) {
+        long a, lo = ch.lo, hi = ch.lo + ch.n;
+        const T* Ua;
+        int jj;
+        if (j < m) {
+            jj = j++;
+            a = chunk_region(t, unit);
+            for (int l = m - 1; l > jj; --l) a = (a - 1) / t.J;
+            Ua = t.U + t.u_off[jj] + (a - level_start(t.J, jj)) * (long)jj * rr;
+        } else {
+            ++gl;
+            jj = m;
+            a = s2 + gl;
+            if (t.sub_lo[a] > lo) lo = t.sub_lo[a];
+            if (t.sub_hi[a] < hi) hi = t.sub_hi[a];
+            if (lo >= hi) continue;
+            Ua = t.U + t.u_off[m] + gl * (long)m * rr;
+        }
+        step(a, jj, Ua, lo - ch.lo, (int)(hi - lo));
+    }
+}
+
+// ---------------------------------------------------------------------------
+// the finest children of one level M-2 region, all at once
+// ---------------------------------------------------------------------------
+// Used when every child has at most 32 observations and the group at most 64
+// (T = double): one covariance block and one product form the whole group's
+// conditional covariance, one warp per child factors its diagonal block,
+// solves y~ and inverts its factor into a block-diagonal matrix, and one
+// product forms the whole group's B^ (in place: each 64-row tile of the
+// product reads exactly the rows it then writes, and the group fits one
+// column tile).  Returns the group's log-likelihood terms (thread 0).
+
+template <typename T>
+__device__ __noinline__ double finest_children_grouped(const Geom& g, const DevTree<T>& t, long clo, long chi,
+                                                       long lo, int np, T* ws, LaSmem<T>& sm) {
+    if constexpr (sizeof(T) != 8) {
+        return 0.0;
+    } else {
+        const long Lr = (long)t.L * t.r;
+        const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+        T* Sg = ws;                      // np x np conditional covariance of the group
+        T* Binv = ws + (long)np * np;    // np x np block-diagonal L_Sigma^{-1}
+        fill_cov<T>(g, t.pts, t.obs0 + lo, np, t.obs0 + lo, np, true, Sg, np, sm);
+        for (int e = tid; e < np * np; e += kThreads) Binv[e] = 0.0;
+        __syncthreads();
+        gemm<T, true, false>(np, np, (int)Lr, (T)-1, t.Ufin + lo * Lr, Lr, t.Ufin + lo * Lr, Lr, (T)1, Sg, np, sm);
+        constexpr int LD = kChildMax + 1;
+        double* Sw = &sm.A[0][0] + w * (kChildMax * LD);  // per-warp 32 x 33 (A and B tiles are contiguous)
+        double part = 0.0;
+        const long c = clo + w;
+        if (c < chi) {
+            const long o0 = t.obs_off[c];
+            const int n = (int)(t.obs_off[c + 1] - o0), q0 = (int)(o0 - lo);
+            if (n > 0) {
+                for (int e = lane; e < n * n; e += 32) {
+                    const int i = e % n, j = e / n;
+                    Sw[i + j * LD] = Sg[(q0 + i) + (long)(q0 + j) * np];
+                }
+                __syncwarp();
+                int bad = 0;
+                for (int k = 0; k < n; ++k) {  // lane i owns row i
+                    const double d = Sw[k + k * LD];
+                    __syncwarp();
+                    if (!(d > 0.0)) bad = 1;
+                    const double sq = sqrt(d);
+                    if (lane == k) Sw[k + k * LD] = sq;
+                    if (lane > k && lane < n) Sw[lane + k * LD] *= 1.0 / sq;
+                    __syncwarp();
+                    const double lik = lane < n ? Sw[lane + k * LD] : 0.0;
+                    for (int j = k + 1; j < n; ++j)  // uniform trip count across the warp
+                        if (lane >= j && lane < n) Sw[lane + j * LD] -= lik * Sw[j + k * LD];
+                    __syncwarp();
+                }
+                T* Lc = t.Lsig + t.lsig_off[c];
+                for (int e = lane; e < n * n; e += 32) {
+                    const int i = e % n, j = e / n;
+                    Lc[i + (long)j * n] = i >= j ? Sw[i + j * LD] : 0.0;
+                }
+                double ldp = lane < n ? log(Sw[lane + lane * LD]) : 0.0;
+                for (int o = 16; o > 0; o >>= 1) ldp += __shfl_xor_sync(0xffffffffu, ldp, o);
+                // y~ = L_Sigma^{-1} y: lane i ends holding x_i
+                double xl = 0.0;
+                for (int i = 0; i < n; ++i) {
+                    double sp = lane < i ? Sw[i + lane * LD] * xl : 0.0;
+                    for (int o = 16; o > 0; o >>= 1) sp += __shfl_xor_sync(0xffffffffu, sp, o);
+                    if (lane == i) xl = (t.y[o0 + i] - sp) / Sw[i + i * LD];
+                }
+                if (lane < n) t.yt[o0 + lane] = xl;
+                double yy = lane < n ? xl * xl : 0.0;
+                for (int o = 16; o > 0; o >>= 1) yy += __shfl_xor_sync(0xffffffffu, yy, o);
+                // column j of L_Sigma^{-1} by lane j, into the child's diagonal block
+                {
+                    // lanes walk the same rows and terms (X[k] = 0 above the
+                    // diagonal): no divergence, broadcast reads of L
+                    const int j = lane;
+                    double xs[kChildMax];  // column j of the inverse, in registers
+#pragma unroll
+                    for (int i = 0; i < kChildMax; ++i) xs[i] = 0.0;
+                    double* col = Binv + q0 + (long)(q0 + (j < n ? j : 0)) * np;
+                    for (int i = 0; i < n; ++i) {
+                        double v = 0.0;
+#pragma unroll
+                        for (int k = 0; k < kChildMax; ++k)
+                            if (k < i) v += Sw[i + k * LD] * xs[k];
+                        const double xi = i == j ? 1.0 / Sw[i + i * LD] : (i > j ? -v / Sw[i + i * LD] : 0.0);
+#pragma unroll
+                        for (int k = 0; k < kChildMax; ++k)
+                            if (k == i) xs[k] = xi;
+                        if (j < n && i >= j) col[i] = xi;
+                    }
+                }
+                part = yy + 2.0 * ldp;
+                if (bad && lane == 0) report_error(t.err, t.n_int + c);
+            }
+        }
+        __syncthreads();
+        if (lane == 0) sm.red[w] = part;
+        __syncthreads();
+        double tot = 0.0;
+        if (tid == 0)
+            for (int k = 0; k < kThreads / 32; ++k) tot += sm.red[k];
+        __syncthreads();
+        gemm<T, false, true, true>((int)Lr, np, np, (T)1, t.Bhat + lo * Lr, Lr, Binv, np, (T)0, t.Bhat + lo * Lr, Lr,
+                                   sm);
+        return tot;
+    }
+}
+
+// Work items: a value v < J^(M-2) is that sibling group, else the finest region
+// v - J^(M-2); most expensive first, from a queue.
+template <typename T>
+__global__ void __launch_bounds__(kThreads, 2) k_finest_children(Geom g, DevTree<T> t) {
+    LaSmem<T>& sm = la_smem<T>();
+    __shared__ long s_u;
+    const int L = t.L, m = t.M - 2;
+    const long Lr = (long)L * t.r;
+    const long s2 = level_start(t.J, m), cnt2 = level_count(t.J, m);
+    T* ws = t.ws + blockIdx.x * t.ws_stride;
+    for (;;) {
+        if (threadIdx.x == 0) {
+            int q = atomicAdd(&t.queue[0], 1);
+            s_u = q < t.n_fin_items ? t.fin_items[q] : -1;
+        }
+        __syncthreads();
+        const long item = s_u;
+        __syncthreads();
+        if (item < 0) break;
+        if (item < cnt2) {
+            if (skipped(t, s2 + item)) continue;
+            const long clo = t.child_lo[item], chi = t.child_hi[item];
+            const long lo = t.obs_off[clo];
+            const double d = finest_children_grouped<T>(g, t, clo, chi, lo, (int)(t.obs_off[chi] - lo), ws, sm);
+            if (threadIdx.x == 0) t.dchild[clo] = d;
+            __syncthreads();
+            continue;
+        }
+        const long c = item - cnt2;
+        if (skipped(t, (long)t.fin_anc[c * L + L - 1])) continue;
+        const long o0 = t.obs_off[c];
+        const int n = (int)(t.obs_off[c + 1] - o0);
+        T* S = t.Lsig + t.lsig_off[c];
+        fill_cov<T>(g, t.pts, t.obs0 + o0, n, t.obs0 + o0, n, true, S, n, sm);
+        __syncthreads();
+        gemm<T, true, false>(n, n, (int)Lr, (T)-1, t.Ufin + o0 * Lr, Lr, t.Ufin + o0 * Lr, Lr, (T)1, S, n, sm);
+        double ld = 0.0;
+        constexpr bool small = sizeof(T) == 8;  // FP64 items hold at most 64 observations
+        T* Sinv = ws;  // n x n
+        int info = potrf_lower<T>(n, S, n, sm, &ld, small ? Sinv : nullptr, n);
+        double* ytc = t.yt + o0;
+        for (int e = threadIdx.x; e < n; e += kThreads) ytc[e] = t.y[o0 + e];
+        __syncthreads();
+        if constexpr (small) {
+            trmv_lower_inv<T>(n, Sinv, n, ytc, ytc);  // y~ = L_Sigma^{-1} y
+            // B^ = V L_Sigma^{-T}, in place: each 64-row tile of the product
+            // reads exactly the rows it then writes
+            gemm<T, false, true, true>((int)Lr, n, n, (T)1, t.Bhat + o0 * Lr, Lr, Sinv, n, (T)0, t.Bhat + o0 * Lr, Lr,
+                                       sm);
+        } else {
+            trsv_lower_f64<T>(n, S, n, ytc);
+            trsm_right_lower_trans<T>((int)Lr, n, S, n, t.Bhat + o0 * Lr, Lr, sm);
+        }
+        double part = 0.0;
+        for (int e = threadIdx.x; e < n; e += kThreads) part += ytc[e] * ytc[e];
+        double yy = cta_sum(part, sm);
+        if (threadIdx.x == 0) {
+            t.dchild[c] = yy + ld;
+            if (info) report_error(t.err, t.n_int + c);
+        }
+        __syncthreads();
+    }
+}
+
+// ---------------------------------------------------------------------------
+// finest regions of more than 64 observations (FP64), in 64 x 64 tiles
+// ---------------------------------------------------------------------------
+// Sigma's lower tiles: one CTA per tile (region h, row tile bi, column tile bj).
+__global__ void __launch_bounds__(kThreads, 2) k_heavy_sigma(Geom g, DevTree<double> t) {
+    LaSmem<double>& sm = la_smem<double>();
+    const long Lr = (long)t.L * t.r;
+    const HeavyTile ht = t.heavy_tiles[blockIdx.x];
+    const long c = t.heavy[ht.h];
+    if (skipped(t, (long)t.fin_anc[c * t.L + t.L - 1])) return;
+    const long o0 = t.obs_off[c];
+    const int n = (int)(t.obs_off[c + 1] - o0);
+    const int i0 = 64 * ht.bi, j0 = 64 * ht.bj;
+    const int ni = min(64, n - i0), nj = min(64, n - j0);
+    double* S = t.Lsig + t.lsig_off[c] + i0 + (long)j0 * n;
+    fill_cov<double>(g, t.pts, t.obs0 + o0 + i0, ni, t.obs0 + o0 + j0, nj, ht.bi == ht.bj, S, n, sm);
+    __syncthreads();
+    gemm<double, true, false>(ni, nj, (int)Lr, -1.0, t.Ufin + (o0 + i0) * Lr, Lr, t.Ufin + (o0 + j0) * Lr, Lr, 1.0, S, n,
+                              sm);
+}
+
+// Left-looking block column k of the factorization of [Sigma; V]: the tiles of
+// the block column (rows k.. of Sigma, then the row tiles of V) subtract the
+// product of what is already factored; the diagonal tile is then factored and
+// inverted, and y~_k solved.  blockIdx.x = region * tiles + tile.
+__global__ void __launch_bounds__(kThreads, 2) k_heavy_column(DevTree<double> t, int k, int tiles) {
+    LaSmem<double>& sm = la_smem<double>();
+    const long Lr = (long)t.L * t.r;
+    const int h = blockIdx.x / tiles, tile = blockIdx.x % tiles;
+    const long c = t.heavy[h];
+    if (skipped(t, (long)t.fin_anc[c * t.L + t.L - 1])) return;
+    const long o0 = t.obs_off[c];
+    const int n = (int)(t.obs_off[c + 1] - o0);
+    const int rows = (n + 63) / 64 - k;  // row tiles of Sigma in this block column
+    const int j0 = 64 * k, nj = min(64, n - j0);
+    double* S = t.Lsig + t.lsig_off[c];
+    if (tile >= rows) {
+        const long x0 = 64L * (tile - rows);
+        if (x0 >= Lr) return;
+        double* W = t.Bhat + o0 * Lr + x0;
+        gemm<double, false, true>((int)min(64L, Lr - x0), nj, j0, -1.0, W, Lr, S + j0, n, 1.0, W + (long)j0 * Lr, Lr,
+                                  sm);
+        return;
+    }
+    const int i0 = j0 + 64 * tile, ni = min(64, n - i0);
+    double* W = S + i0 + (long)j0 * n;
+    if (k > 0) gemm<double, false, true>(ni, nj, j0, -1.0, S + i0, n, S + j0, n, 1.0, W, n, sm);
+    if (tile > 0) return;
+    double* X = t.heavy_inv + (long)h * 64 * 64;
+    double ld = 0.0;
+    const int info = potrf_small(nj, W, n, sm, &ld, X, 64);
+    // y~_k = X (y_k - L_(k,0..k-1) y~_(0..k-1)): 4 threads per row over the columns
+    double* yt = t.yt + o0;
+    double* part = &sm.A[0][0];
+    {
+        const int q = threadIdx.x & 63, cg = threadIdx.x >> 6;
+        double s = 0.0;
+        if (q < nj)
+            for (int x = cg; x < j0; x += 4) s += S[j0 + q + (long)x * n] * yt[x];
+        part[threadIdx.x] = s;
+        __syncthreads();
+        if (threadIdx.x < nj) {
+            const int e = threadIdx.x;
+            yt[j0 + e] = t.y[o0 + j0 + e] - ((part[e] + part[64 + e]) + (part[128 + e] + part[192 + e]));
+        }
+        __syncthreads();
+    }
+    trmv_lower_inv<double>(nj, X, 64, yt + j0, yt + j0);
+    double p2 = 0.0;
+    for (int e = threadIdx.x; e < nj; e += kThreads) p2 += yt[j0 + e] * yt[j0 + e];
+    const double yy = cta_sum(p2, sm);
+    if (threadIdx.x == 0) {
+        t.dchild[c] = (k == 0 ? 0.0 : t.dchild[c]) + yy + ld;
+        if (info) report_error(t.err, t.n_int + c);
+    }
+}
+
+// The tiles below the diagonal of block column k (and V's) times L_kk^{-T}, in place.
+__global__ void __launch_bounds__(kThreads, 2) k_heavy_panel(DevTree<double> t, int k, int tiles) {
+    LaSmem<double>& sm = la_smem<double>();
+    const long Lr = (long)t.L * t.r;
+    const int h = blockIdx.x / tiles, tile = blockIdx.x % tiles;
+    const long c = t.heavy[h];
+    if (skipped(t, (long)t.fin_anc[c * t.L + t.L - 1])) return;
+    const long o0 = t.obs_off[c];
+    const int n = (int)(t.obs_off[c + 1] - o0);
+    const int rows = (n + 63) / 64 - k - 1;  // row tiles of Sigma below the diagonal
+    const int j0 = 64 * k, nj = min(64, n - j0);
+    const double* X = t.heavy_inv + (long)h * 64 * 64;
+    double* W;
+    long ldw;
+    int ni;
+    if (tile < rows) {
+        const int i0 = j0 + 64 * (tile + 1);
+        W = t.Lsig + t.lsig_off[c] + i0 + (long)j0 * n;
+        ldw = n;
+        ni = min(64, n - i0);
+    } else {
+        const long x0 = 64L * (tile - rows);
+        if (x0 >= Lr) return;
+        W = t.Bhat + (o0 + j0) * Lr + x0;
+        ldw = Lr;
+        ni = (int)min(64L, Lr - x0);
+    }
+    gemm<double, false, true, true>(ni, nj, nj, 1.0, W, ldw, X, 64, 0.0, W, ldw, sm);
+}
+
+// dfin of each sibling group: the sum of its children's terms, in order (the
+// slots of regions without observations, and of all but the first of a group
+// processed together, stay zero).
+template <typename T>
+__global__ void k_finest_terms(DevTree<T> t) {
+    const long s2 = level_start(t.J, t.M - 2), cnt2 = level_count(t.J, t.M - 2);
+    const long q = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= cnt2 || skipped(t, s2 + q)) return;
+    double s = 0.0;
+    for (long c = t.child_lo[q]; c < t.child_hi[q]; ++c) s += t.dchild[c];
+    t.dfin[q] = s;
+}
+
+// ---------------------------------------------------------------------------
+// launchers
+// ---------------------------------------------------------------------------
+template <typename T>
+static void launch_cov_finest(const Geom& g, const DevTree<T>& t, cudaStream_t st) {
+    const long tasks = t.n_chunks * t.L;
+    const unsigned grid = (unsigned)(tasks < 148L * 32 ? tasks : 148L * 32);
+    switch (cov_kind(g, sizeof(T) == 8)) {
+        case 1: k_cov_finest<T, 1><<<grid, kCovThreads, 0, st>>>(g, t); break;
+        case 2: k_cov_finest<T, 2><<<grid, kCovThreads, 0, st>>>(g, t); break;
+        case 3: k_cov_finest<T, 3><<<grid, kCovThreads, 0, st>>>(g, t); break;
+        case 4: k_cov_finest<T, 4><<<grid, kCovThreads, 0, st>>>(g, t); break;
+        default: k_cov_finest<T, 0><<<grid, kCovThreads, 0, st>>>(g, t); break;
+    }
+}
+
+template <int RC>
+static void launch_condition(const DevTree<double>& t, cudaStream_t st) {
+    const unsigned grid = (unsigned)t.n_chunks;
+    if (t.r % 2 == 0) k_finest_condition<RC, true><<<grid, kThreads, sizeof(CondSmem<RC>), st>>>(t);
+    else k_finest_condition<RC, false><<<grid, kThreads, sizeof(CondSmem<RC>), st>>>(t);
+}
+
+template <typename T>
+int launch_finest(const Geom& g, const DevTree<T>& t, int grid, cudaStream_t st, const FinestFork& fk) {
+    int launches = 0;
+    if (t.n_chunks > 0) {
+        launch_cov_finest<T>(g, t, st);
+        if constexpr (sizeof(T) == 8) {
+            if (t.r <= 16) launch_condition<16>(t, st);
+            else if (t.r <= 32) launch_condition<32>(t, st);
+            else if (t.r <= 64) launch_condition<64>(t, st);
+            else k_finest_condition_any<T><<<(unsigned)t.n_chunks, kThreads, sizeof(LaSmem<T>), st>>>(t);
+        } else {
+            k_finest_condition_any<T><<<(unsigned)t.n_chunks, kThreads, sizeof(LaSmem<T>), st>>>(t);
+        }
+        launches += 2;
+    }
+    if constexpr (sizeof(T) == 8) {
+        if (t.n_heavy > 0) {
+            // the heavy regions' chain of block columns beside the small regions
+            cudaEventRecord(fk.fork, st);
+            cudaStreamWaitEvent(fk.side, fk.fork, 0);
+            const int LT = (int)(((long)t.L * t.r + 63) / 64);
+            k_heavy_sigma<<<(unsigned)t.n_heavy_tiles, kThreads, sizeof(LaSmem<T>), fk.side>>>(g, t);
+            ++launches;
+            const int nb = fk.heavy_blocks[0];
+            long act = t.n_heavy;
+            for (int k = 0; k < nb; ++k) {
+                while (act > 0 && fk.heavy_blocks[act - 1] <= k) --act;
+                const int tiles = k == 0 ? 1 : nb - k + LT;
+                k_heavy_column<<<(unsigned)(act * tiles), kThreads, sizeof(LaSmem<T>), fk.side>>>(t, k, tiles);
+                const int below = nb - k - 1 + LT;
+                k_heavy_panel<<<(unsigned)(act * below), kThreads, sizeof(LaSmem<T>), fk.side>>>(t, k, below);
+                launches += 2;
+            }
+            cudaEventRecord(fk.join, fk.side);
+        }
+    }
+    if (t.n_fin_items > 0) {
+        k_finest_children<T><<<(unsigned)(t.n_fin_items < grid ? t.n_fin_items : grid), kThreads, sizeof(LaSmem<T>),
+                               st>>>(g, t);
+        ++launches;
+    }
+    if constexpr (sizeof(T) == 8)
+        if (t.n_heavy > 0) cudaStreamWaitEvent(st, fk.join, 0);
+    const long cnt2 = level_count(t.J, t.M - 2);
+    k_finest_terms<T><<<(unsigned)((cnt2 + 255) / 256), 256, 0, st>>>(t);
+    return launches + 1;
+}
+
+cudaError_t prepare_finest() {
+    cudaError_t e = cudaSuccess;
+    auto set = [&](const void* fn, size_t bytes) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    };
+    set((const void*)k_finest_condition<16, true>, sizeof(CondSmem<16>));
+    set((const void*)k_finest_condition<16, false>, sizeof(CondSmem<16>));
+    set((const void*)k_finest_condition<32, true>, sizeof(CondSmem<32>));
+    set((const void*)k_finest_condition<32, false>, sizeof(CondSmem<32>));
+    set((const void*)k_finest_condition<64, true>, sizeof(CondSmem<64>));
+    set((const void*)k_finest_condition<64, false>, sizeof(CondSmem<64>));
+    set((const void*)k_finest_condition_any<double>, sizeof(LaSmem<double>));
+    set((const void*)k_finest_condition_any<float>, sizeof(LaSmem<float>));
+    set((const void*)k_finest_children<double>, sizeof(LaSmem<double>));
+    set((const void*)k_finest_children<float>, sizeof(LaSmem<float>));
+    set((const void*)k_heavy_sigma, sizeof(LaSmem<double>));
+    set((const void*)k_heavy_column, sizeof(LaSmem<double>));
+    set((const void*)k_heavy_panel, sizeof(LaSmem<double>));
+    return e;
+}
+
+cudaError_t set_gemm_tiles_finest(const int nw[3]) { return cudaMemcpyToSymbol(c_gemm_nw, nw, 3 * sizeof(int)); }
+
+template int launch_finest<double>(const Geom&, const DevTree<double>&, int, cudaStream_t, const FinestFork&);
+template int launch_finest<float>(const Geom&, const DevTree<float>&, int, cudaStream_t, const FinestFork&);
+
+}  // namespace mra

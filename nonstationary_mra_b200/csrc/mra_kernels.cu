@@ -7,15 +7,10 @@
 //                       prediction point (class_nonstationary_covariance.cpp:479-573)
 //   k_prior_level(m)    levels 0..M-2, one CTA per region: U_{i,j} = L_{a_j}^{-1} V_j,
 //                       L_i = chol(K_i)   (class_approximation.cpp:46-50,84-169)
-//   k_finest_group      one CTA per level M-3 region: conditioning of all its
-//                       observations on the shared ancestors (levels 0..M-3),
-//                       then per level M-2 child (a sibling group of finest
-//                       regions) the level M-2 step and per finest region
-//                       Sigma, L_Sigma, y~,
-//                       B^ and the log-lik terms
-//                       (...-loop-regions-at-finest-level-in-prior.cpp:90-269),
-//                       then the level M-2 posterior of the parent
-//   k_posterior_level(m) levels M-3..0 (...-posterior-inference.cpp:14-265,
+//   (mra_finest.cu)     finest level: conditioning, Sigma, L_Sigma, y~, B^ and
+//                       the log-lik terms
+//                       (...-loop-regions-at-finest-level-in-prior.cpp:90-269)
+//   k_posterior_level(m) levels M-2..0 (...-posterior-inference.cpp:14-265,
 //                       class_approximation.cpp:186-306)
 //   k_reduce            deterministic sum of the per-region terms
 //   k_predict           prediction, one CTA per level M-2 region (its finest
@@ -39,13 +34,6 @@
 #include "mra_kernels.cuh"
 
 namespace mra {
-
-__device__ inline void report_error(int* err, long region) {
-    if (atomicCAS(&err[0], 0, 4 /* MRA_ERR_NOT_SPD */) == 0) {
-        err[1] = (int)(region & 0x7fffffff);
-        err[2] = (int)(region >> 31);
-    }
-}
 
 // ---------------------------------------------------------------------------
 // a1: fields
@@ -100,84 +88,6 @@ __global__ void k_fields(Geom g, FieldParams fp, const double* __restrict__ c0, 
 // products beside it the launch keeps every SM full of independent entry
 // chains, which the per-region kernel, two CTAs per SM between its products,
 // cannot.
-constexpr int kCovThreads = 256;
-constexpr int kCovChunk = 64;  // column points staged per chunk (7 x 64 doubles of shared memory)
-
-// The straight-line nonstationary FP64 block: one row point per thread with its
-// parameters in registers, the column points staged in chunks, entries of
-// cov_fast_entry (the same arithmetic as fill_row_fast).
-template <typename T, int NU, int PREF>
-__device__ __forceinline__ void cov_block_fast(const PointSet& P, long a0, int nr, long b0, int nc, bool self,
-                                               T* __restrict__ out, long ld, double ih2, double ihs2,
-                                               double* stage) {
-    double* sx = stage;
-    double* sy = sx + kCovChunk;
-    double* sz = sy + kCovChunk;
-    double* sg = sz + kCovChunk;
-    double* s4 = sg + kCovChunk;  // sqrt(s2) b (PREF 1) or sqrt(s2) (PREF 0)
-    double* s5 = s4 + kCovChunk;  // b (PREF 0)
-    const int tid = threadIdx.x, nt = blockDim.x;
-    const int rows = nr < nt ? nr : nt;
-    const int cols = nt / rows;
-    const bool worker = tid < rows * cols;
-    const int tr = tid % rows, tc = tid / rows;
-    for (int q0 = 0; q0 < nc; q0 += kCovChunk) {
-        const int qn = nc - q0 < kCovChunk ? nc - q0 : kCovChunk;
-        __syncthreads();
-        for (int e = tid; e < qn; e += nt) {
-            const long ib = b0 + q0 + e;
-            const double bb = P.beta[ib], ssq = sqrt(P.s2[ib]);
-            sx[e] = P.c0[ib];
-            sy[e] = P.c1[ib];
-            sz[e] = P.c2[ib];
-            sg[e] = bb * bb * ih2;
-            s4[e] = PREF == 1 ? ssq * bb : ssq;
-            s5[e] = bb;
-        }
-        __syncthreads();
-        if (!worker) continue;
-        for (int t = tr; t < nr; t += rows) {
-            const long ia = a0 + t;
-            const double pc0 = P.c0[ia], pc1 = P.c1[ia], pc2 = P.c2[ia], sa = P.s2[ia], ba = P.beta[ia];
-            const double ssa = sqrt(sa), ga = ba * ba * ih2, ca = ssa * ba * ihs2, ba_h = ba * ihs2;
-            const double diag = self ? sa + P.t2[ia] : 0.0;
-            T* ob = out + t;
-#pragma unroll 4
-            for (int q = tc; q < qn; q += cols) {
-                const int qq = q0 + q;
-                double v = cov_fast_entry<NU, PREF, true>(pc0, pc1, pc2, ga, ca, ssa, ba_h, sx[q], sy[q], sz[q], sg[q],
-                                                    PREF == 1 ? s4[q] : 0.0, PREF == 1 ? 0.0 : s4[q],
-                                                    PREF == 1 ? 0.0 : s5[q]);
-                if (self && t == qq) v = diag;  // sigma^2 + tau^2 (evaluate_covariance.cpp:103,307)
-                ob[(long)qq * ld] = (T)v;
-            }
-        }
-    }
-    __syncthreads();
-}
-
-// Block out[t + q ld] = C(A_{a0+t}, B_{b0+q}), t < nr, q < nc (with the
-// sigma^2 + tau^2 diagonal when `self`), by the whole CTA.  KIND (cov_kind on the
-// host): 1..4 the straight-line nonstationary FP64 forms (Matern 3/2 or 1/2 x
-// prefactor exponent 1 or 3/2), 0 every other model.
-template <typename T, int KIND>
-__device__ __forceinline__ void cov_block(const Geom& g, const PointSet& P, long a0, int nr, long b0, int nc, bool self,
-                                          T* out, long ld, double* stage) {
-    if constexpr (KIND == 0) {
-        fill_cov_staged<T, kCovChunk>(g, P, &a0, 1, nr, b0, nc, self, out, ld, 0, stage);
-    } else {
-        const double hs = g.dist_scale * (KIND <= 2 ? 1.7320508075688772 : 1.0);
-        const double ihs2 = 1.0 / (hs * hs), ih2 = 0.5 * ihs2;
-        constexpr int NU = KIND <= 2 ? 3 : 1, PREF = (KIND & 1) ? 1 : 0;
-        cov_block_fast<T, NU, PREF>(P, a0, nr, b0, nc, self, out, ld, ih2, ihs2, stage);
-    }
-}
-
-inline int cov_kind(const Geom& g, bool fp64) {
-    if (!(fp64 && g.nonstat && g.distance != 1 && g.pref_kind != 2)) return 0;
-    return g.nu_x2 == 3 ? (g.pref_kind == 1 ? 1 : 2) : (g.pref_kind == 1 ? 3 : 4);
-}
-
 template <typename T, int KIND>
 __global__ void __launch_bounds__(kCovThreads, 4) k_cov_level(Geom g, DevTree<T> t, int m, long loc0, long nloc,
                                                                T* __restrict__ out) {
@@ -274,8 +184,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_prior_level(Geom g, DevTree<T> 
 // ---------------------------------------------------------------------------
 // The products of the posterior steps go through a separate function: the
 // steps keep many values live across their products, and inlined there the
-// product loops would share (and spill) their registers.  (The finest-level
-// kernel measured faster with its products inlined.)
+// product loops would share (and spill) their registers.
 template <typename T, bool TA, bool TB, bool ONE_TILE = false>
 __device__ __noinline__ void gemm_call(int M, int N, int K, T alpha, const T* A, long lda, const T* B, long ldb,
                                        T beta, T* C, long ldc, LaSmem<T>& sm, const T* Cin = nullptr,
@@ -453,257 +362,6 @@ __device__ __noinline__ void accumulate_factored(const DevTree<T>& t, int m, int
         wagg[x] = init ? s : wagg[x] + s;
     }
     __syncthreads();
-}
-
-// ---------------------------------------------------------------------------
-// a7/a8: the finest children of one level M-2 region, all at once
-// ---------------------------------------------------------------------------
-// Used when every child has at most 32 observations and the group at most 64
-// (T = double): one covariance block and one product form the whole group's
-// conditional covariance, one warp per child factors its diagonal block,
-// solves y~ and inverts its factor into a block-diagonal matrix, and one
-// product forms the whole group's B^ (in place: each 64-row tile of the
-// product reads exactly the rows it then writes, and the group fits one
-// column tile).  Returns the group's log-likelihood terms (thread 0).
-constexpr int kGroupMax = 64;
-constexpr int kChildMax = 32;
-
-template <typename T>
-__device__ __noinline__ double finest_children_grouped(const Geom& g, const DevTree<T>& t, long clo, long chi,
-                                                       long lo, int np, T* ws, LaSmem<T>& sm) {
-    if constexpr (sizeof(T) != 8) {
-        return 0.0;
-    } else {
-        const long Lr = (long)t.L * t.r;
-        const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-        T* Sg = ws;                      // np x np conditional covariance of the group
-        T* Binv = ws + (long)np * np;    // np x np block-diagonal L_Sigma^{-1}
-        fill_cov<T>(g, t.pts, t.obs0 + lo, np, t.obs0 + lo, np, true, Sg, np, sm);
-        for (int e = tid; e < np * np; e += kThreads) Binv[e] = 0.0;
-        __syncthreads();
-        gemm<T, true, false>(np, np, (int)Lr, (T)-1, t.Ufin + lo * Lr, Lr, t.Ufin + lo * Lr, Lr, (T)1, Sg, np, sm);
-        constexpr int LD = kChildMax + 1;
-        double* Sw = &sm.A[0][0] + w * (kChildMax * LD);  // per-warp 32 x 33 (A and B tiles are contiguous)
-        double part = 0.0;
-        const long c = clo + w;
-        if (c < chi) {
-            const long o0 = t.obs_off[c];
-            const int n = (int)(t.obs_off[c + 1] - o0), q0 = (int)(o0 - lo);
-            if (n > 0) {
-                for (int e = lane; e < n * n; e += 32) {
-                    const int i = e % n, j = e / n;
-                    Sw[i + j * LD] = Sg[(q0 + i) + (long)(q0 + j) * np];
-                }
-                __syncwarp();
-                int bad = 0;
-                for (int k = 0; k < n; ++k) {  // lane i owns row i
-                    const double d = Sw[k + k * LD];
-                    __syncwarp();
-                    if (!(d > 0.0)) bad = 1;
-                    const double sq = sqrt(d);
-                    if (lane == k) Sw[k + k * LD] = sq;
-                    if (lane > k && lane < n) Sw[lane + k * LD] *= 1.0 / sq;
-                    __syncwarp();
-                    const double lik = lane < n ? Sw[lane + k * LD] : 0.0;
-                    for (int j = k + 1; j < n; ++j)  // uniform trip count across the warp
-                        if (lane >= j && lane < n) Sw[lane + j * LD] -= lik * Sw[j + k * LD];
-                    __syncwarp();
-                }
-                T* Lc = t.Lsig + t.lsig_off[c];
-                for (int e = lane; e < n * n; e += 32) {
-                    const int i = e % n, j = e / n;
-                    Lc[i + (long)j * n] = i >= j ? Sw[i + j * LD] : 0.0;
-                }
-                double ldp = lane < n ? log(Sw[lane + lane * LD]) : 0.0;
-                for (int o = 16; o > 0; o >>= 1) ldp += __shfl_xor_sync(0xffffffffu, ldp, o);
-                // y~ = L_Sigma^{-1} y: lane i ends holding x_i
-                double xl = 0.0;
-                for (int i = 0; i < n; ++i) {
-                    double sp = lane < i ? Sw[i + lane * LD] * xl : 0.0;
-                    for (int o = 16; o > 0; o >>= 1) sp += __shfl_xor_sync(0xffffffffu, sp, o);
-                    if (lane == i) xl = (t.y[o0 + i] - sp) / Sw[i + i * LD];
-                }
-                if (lane < n) t.yt[o0 + lane] = xl;
-                double yy = lane < n ? xl * xl : 0.0;
-                for (int o = 16; o > 0; o >>= 1) yy += __shfl_xor_sync(0xffffffffu, yy, o);
-                // column j of L_Sigma^{-1} by lane j, into the child's diagonal block
-                {
-                    // lanes walk the same rows and terms (X[k] = 0 above the
-                    // diagonal): no divergence, broadcast reads of L
-                    const int j = lane;
-                    double xs[kChildMax];  // column j of the inverse, in registers
-#pragma unroll
-                    for (int i = 0; i < kChildMax; ++i) xs[i] = 0.0;
-                    double* col = Binv + q0 + (long)(q0 + (j < n ? j : 0)) * np;
-                    for (int i = 0; i < n; ++i) {
-                        double v = 0.0;
-#pragma unroll
-                        for (int k = 0; k < kChildMax; ++k)
-                            if (k < i) v += Sw[i + k * LD] * xs[k];
-                        const double xi = i == j ? 1.0 / Sw[i + i * LD] : (i > j ? -v / Sw[i + i * LD] : 0.0);
-#pragma unroll
-                        for (int k = 0; k < kChildMax; ++k)
-                            if (k == i) xs[k] = xi;
-                        if (j < n && i >= j) col[i] = xi;
-                    }
-                }
-                part = yy + 2.0 * ldp;
-                if (bad && lane == 0) report_error(t.err, t.n_int + c);
-            }
-        }
-        __syncthreads();
-        if (lane == 0) sm.red[w] = part;
-        __syncthreads();
-        double tot = 0.0;
-        if (tid == 0)
-            for (int k = 0; k < kThreads / 32; ++k) tot += sm.red[k];
-        __syncthreads();
-        gemm<T, false, true, true>((int)Lr, np, np, (T)1, t.Bhat + lo * Lr, Lr, Binv, np, (T)0, t.Bhat + lo * Lr, Lr,
-                                   sm);
-        return tot;
-    }
-}
-
-// ---------------------------------------------------------------------------
-// a7/a8 (+ a9 at level M-2): finest level, one CTA per level M-3 region
-// ---------------------------------------------------------------------------
-// A work item is either a unit -- a level M-3 region with its J level M-2
-// children (sibling groups), taken together when it holds few observations --
-// or a single level M-2 group (large units are split for load balance; for
-// M = 2 the single level-0 group).  The observations of an item are
-// contiguous and all of them share the ancestors at levels 0..M-3: their
-// conditioning on those levels runs once per item (for a unit: products J
-// times wider, the ancestors' U read once).  The level M-2 step, the finest
-// children and the level M-2 posterior then run per group.
-template <typename T>
-__global__ void __launch_bounds__(kThreads, 2) k_finest_group(Geom g, DevTree<T> t, int keep) {
-    LaSmem<T>& sm = la_smem<T>();
-    __shared__ long s_u;
-    const int r = t.r, L = t.L, m = t.M - 2;
-    const long rr = (long)r * r, Lr = (long)L * r;
-    const long s2 = level_start(t.J, m);
-    const long n_units = t.M >= 3 ? level_count(t.J, m - 1) : 0;
-    T* ws = t.ws + blockIdx.x * t.ws_stride;
-    double* wsd = t.wsd + blockIdx.x * t.wsd_stride;
-    for (;;) {
-        if (threadIdx.x == 0) {
-            int q = atomicAdd(&t.queue[0], 1);
-            s_u = q < t.n_fin_items ? t.par_order[q] : -1;
-        }
-        __syncthreads();
-        const long item = s_u;
-        __syncthreads();
-        if (item < 0) break;
-        // item < n_units: unit (level M-3 local index); else group item - n_units (level M-2 local index)
-        const bool unit = item < n_units;
-        const long g_lo = unit ? item * t.J : item - n_units, g_hi = unit ? g_lo + t.J : g_lo + 1;
-        const long ui = unit ? level_start(t.J, m - 1) + item : s2 + g_lo;  // region whose subtree is the item
-        if (skipped(t, ui)) continue;  // uniform: the item is the same for the whole CTA
-        long anc[kMaxLevels];
-        if (m > 0) {
-            long c = unit ? ui : (ui - 1) / t.J;
-            anc[m - 1] = c;
-            for (int a = m - 2; a >= 0; --a) {
-                c = (c - 1) / t.J;
-                anc[a] = c;
-            }
-        }
-        const long ulo = t.sub_lo[ui];
-        const int nu = (int)(t.sub_hi[ui] - ulo);
-        if (m > 0 && nu > 0) {
-            // C(Q_{a_j}, S) of levels 0..M-3 for all observations of the unit, into B^
-            T* Uf = t.Ufin + ulo * Lr;  // (L r) x nu, ld = L r
-            T* Bh = t.Bhat + ulo * Lr;
-            long aoff[kMaxLevels];
-            for (int j = 0; j < m; ++j) aoff[j] = anc[j] * r;
-            fill_cov_blocks<T>(g, t.pts, aoff, m, r, t.obs0 + ulo, nu, false, Bh, Lr, r, sm);
-            for (int j = 0; j < m; ++j) {
-                const long a = anc[j];
-                T* V = Bh + (long)j * r;  // V_j (kept: B^ is L_Sigma^{-1} V^T)
-                if (j > 0) {
-                    const T* Ua = t.U + t.u_off[j] + (a - level_start(t.J, j)) * (long)j * rr;
-                    gemm<T, true, false>(r, nu, j * r, (T)-1, Ua, (long)j * r, Uf, Lr, (T)1, V, Lr, sm);
-                }
-                gemm<T, false, false>(r, nu, r, (T)1, t.Pinv + a * rr, r, V, Lr, (T)0, Uf + (long)j * r, Lr, sm);
-            }
-        }
-        for (long ploc = g_lo; ploc < g_hi; ++ploc) {
-            const long p = s2 + ploc;
-            const long clo = t.child_lo[ploc], chi = t.child_hi[ploc];
-            const long lo = t.obs_off[clo];
-            const int np = (int)(t.obs_off[chi] - lo);
-            double dterm = 0.0;
-            if (np > 0) {
-                // level M-2: the group's own parent p
-                T* Uf = t.Ufin + lo * Lr;
-                T* V = t.Bhat + lo * Lr + (long)m * r;
-                const long ap = p * r;
-                fill_cov_blocks<T>(g, t.pts, &ap, 1, r, t.obs0 + lo, np, false, V, Lr, 0, sm);
-                if (m > 0) {
-                    const T* Ua = t.U + t.u_off[m] + ploc * (long)m * rr;
-                    gemm<T, true, false>(r, np, m * r, (T)-1, Ua, (long)m * r, Uf, Lr, (T)1, V, Lr, sm);
-                }
-                gemm<T, false, false>(r, np, r, (T)1, t.Pinv + p * rr, r, V, Lr, (T)0, Uf + (long)m * r, Lr, sm);
-                int nmax = 0;
-                for (long c = clo; c < chi; ++c) nmax = max(nmax, (int)(t.obs_off[c + 1] - t.obs_off[c]));
-                const bool grouped = sizeof(T) == 8 && nmax <= kChildMax && np <= kGroupMax &&
-                                     chi - clo <= kThreads / 32;
-                if (grouped) dterm += finest_children_grouped<T>(g, t, clo, chi, lo, np, ws, sm);
-                for (long c = clo; c < chi && !grouped; ++c) {
-                    const long o0 = t.obs_off[c];
-                    const int n = (int)(t.obs_off[c + 1] - o0);
-                    if (n == 0) continue;
-                    T* S = t.Lsig + t.lsig_off[c];
-                    fill_cov<T>(g, t.pts, t.obs0 + o0, n, t.obs0 + o0, n, true, S, n, sm);
-                    __syncthreads();
-                    gemm<T, true, false>(n, n, (int)Lr, (T)-1, t.Ufin + o0 * Lr, Lr, t.Ufin + o0 * Lr, Lr, (T)1, S,
-                                         n, sm);
-                    double ld = 0.0;
-                    const bool small = sizeof(T) == 8 && n <= 64;
-                    T* Sinv = ws;  // n x n
-                    int info = potrf_lower<T>(n, S, n, sm, &ld, small ? Sinv : nullptr, n);
-                    double* ytc = t.yt + o0;
-                    for (int e = threadIdx.x; e < n; e += kThreads) ytc[e] = t.y[o0 + e];
-                    __syncthreads();
-                    if (small) trmv_lower_inv<T>(n, Sinv, n, ytc, ytc);  // y~ = L_Sigma^{-1} y
-                    else trsv_lower_f64<T>(n, S, n, ytc);
-                    if (small) {
-                        // B^ = V L_Sigma^{-T}, in place: each 64-row tile of the product
-                        // reads exactly the rows it then writes
-                        gemm<T, false, true, true>((int)Lr, n, n, (T)1, t.Bhat + o0 * Lr, Lr, Sinv, n, (T)0,
-                                                   t.Bhat + o0 * Lr, Lr, sm);
-                    } else {
-                        trsm_right_lower_trans<T>((int)Lr, n, S, n, t.Bhat + o0 * Lr, Lr, sm);
-                    }
-                    double part = 0.0;
-                    for (int e = threadIdx.x; e < n; e += kThreads) part += ytc[e] * ytc[e];
-                    double yy = cta_sum(part, sm);
-                    if (threadIdx.x == 0) {
-                        dterm += yy + ld;
-                        if (info) report_error(t.err, t.n_int + c);
-                    }
-                }
-            }
-            if (threadIdx.x == 0) t.dfin[ploc] = dterm;
-            if (!t.fuse_post) continue;
-            dterm = 0.0;
-            // posterior of the parent at level m = M-2 from F = B^ rows, f = y~
-            const T* F = t.Bhat + lo * Lr;
-            const double* f = t.yt + lo;
-            if (t.factored[p]) {
-                T* Fo = m > 0 ? t.Fbuf[m & 1] + lo * (long)m * r : nullptr;
-                double* fo = m > 0 ? t.fbuf[m & 1] + lo : nullptr;
-                factored_step<T>(t, m, p, np, F, Lr, f, Fo, fo, keep != 0, ws, wsd, sm, dterm);
-            } else {
-                T* Aagg = ws;
-                double* wagg = wsd;
-                accumulate_factored<T>(t, m, np, F, Lr, f, Aagg, wagg, true, sm);
-                dense_step<T>(t, m, p, Aagg, wagg, keep != 0, Aagg + n_slices(m + 1) * rr, sm, dterm);
-            }
-            if (threadIdx.x == 0) t.dpost[p] = dterm;
-            __syncthreads();
-        }
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1003,12 +661,6 @@ int launch_prior_level(const Geom& g, const DevTree<T>& t, int m, int grid, cuda
     return launches;
 }
 template <typename T>
-int launch_finest_group(const Geom& g, const DevTree<T>& t, int grid, bool keep, cudaStream_t st) {
-    long cnt = t.n_fin_items;
-    k_finest_group<T><<<(unsigned)(cnt < grid ? cnt : grid), kThreads, sizeof(LaSmem<T>), st>>>(g, t, keep ? 1 : 0);
-    return 1;
-}
-template <typename T>
 void launch_posterior_level(const Geom& g, const DevTree<T>& t, int m, int grid, bool keep, cudaStream_t st) {
     long cnt = level_count(t.J, m);
     k_posterior_level<T><<<(unsigned)(cnt < grid ? cnt : grid), kThreads, sizeof(LaSmem<T>), st>>>(g, t, m, keep ? 1 : 0);
@@ -1051,7 +703,6 @@ static cudaError_t prepare_type() {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     };
     set((const void*)k_prior_level<T>);
-    set((const void*)k_finest_group<T>);
     set((const void*)k_posterior_level<T>);
     set((const void*)k_predict<T>);
     set((const void*)k_reduce<T>);
@@ -1063,12 +714,12 @@ cudaError_t set_gemm_tiles(const int nw[3]) { return cudaMemcpyToSymbol(c_gemm_n
 
 cudaError_t prepare_kernels() {
     cudaError_t e = prepare_type<double>();
-    return e == cudaSuccess ? prepare_type<float>() : e;
+    if (e == cudaSuccess) e = prepare_type<float>();
+    return e == cudaSuccess ? prepare_finest() : e;
 }
 
 #define MRA_INSTANTIATE(T)                                                                                   \
     template int launch_prior_level<T>(const Geom&, const DevTree<T>&, int, int, cudaStream_t, CovTiming*); \
-    template int launch_finest_group<T>(const Geom&, const DevTree<T>&, int, bool, cudaStream_t);           \
     template void launch_posterior_level<T>(const Geom&, const DevTree<T>&, int, int, bool, cudaStream_t);  \
     template void launch_predict<T>(const Geom&, const DevTree<T>&, int, cudaStream_t);                     \
     template void launch_reduce<T>(const DevTree<T>&, double*, cudaStream_t);                               \

@@ -11,6 +11,22 @@
 
 namespace mra {
 
+// A run of observations that share their ancestors of levels 0..M-3 (unit: the
+// local index of the level M-3 region, 0 when M = 2), conditioned by one CTA.
+struct FinChunk {
+    int64_t lo;
+    int32_t n;
+    int32_t unit;
+};
+// A finest region of at most kFinTile observations is one work item; a sibling
+// group is one item when its children hold at most kChildMax and together at
+// most kGroupMax observations (FP64).
+constexpr int kFinTile = 64, kGroupMax = 64, kChildMax = 32;
+struct HeavyTile {
+    int32_t h;       // index into DevTree::heavy
+    uint16_t bi, bj; // 64 x 64 tile of Sigma, bi >= bj
+};
+
 // Everything a kernel needs to address the resident structure and buffers.
 template <typename T>
 struct DevTree {
@@ -27,9 +43,15 @@ struct DevTree {
     const int64_t* sub_hi;     // [n_int] one past the last
     const int64_t* child_lo;   // [J^(M-2)] first finest child of each level M-2 region
     const int64_t* child_hi;   // one past the last
-    const int64_t* par_order;  // [n_fin_items] finest-kernel work items, most expensive first: a value
-                               // v < J^(M-3) is the level M-3 unit v, else the level M-2 group v - J^(M-3)
+    const FinChunk* chunks;    // [n_chunks] runs of observations conditioned together
+    long n_chunks;
+    const int64_t* fin_items;  // [n_fin_items] small finest regions, most expensive first: a value v < J^(M-2)
+                               // is the sibling group v, else the finest region v - J^(M-2)
     long n_fin_items;
+    const int64_t* heavy;      // [n_heavy] finest regions of more than 64 observations (FP64), largest first
+    long n_heavy;
+    const HeavyTile* heavy_tiles;  // [n_heavy_tiles] lower tiles of their Sigma
+    long n_heavy_tiles;
     const int64_t* pred_order; // [J^(M-2)] level M-2 regions (local index), most expensive prediction work first
     const int64_t* post_order; // [n_int] per level m, at level_start(m): the level's regions (local index),
                                // most expensive posterior step first
@@ -55,8 +77,10 @@ struct DevTree {
     T* G;                      // like U: [J^m][r x (m r)], ld = r (prediction mode)
     T* Lpinv;                  // [n_int][r*r] inverse of each posterior factor (FP64 prediction mode, r <= 64), else null
     double* dpost;             // [n_int] posterior log-lik terms
+    double* dchild;            // [n_fin] log-lik terms of each finest region (or of the group it leads)
     double* dfin;              // [J^(M-2)] finest-level log-lik terms of each sibling group
-    int fuse_post;             // 1: the finest-group kernel also runs the level M-2 posterior
+    int fuse_post;             // 1: the finest stage ends with the level M-2 posterior
+    double* heavy_inv;         // [n_heavy][64 x 64] inverse of the current diagonal tile
     T* aout[2];                // dense A~ slices of one level's dense regions (by dslot), ping-pong by level parity
     double* wout[2];           // dense w~ of one level's dense regions (by dslot)
     T* Fbuf[2];                // factored F of one level: [n_obs][m r]
@@ -75,7 +99,7 @@ struct DevTree {
     double* var;               // [n_pred]
     // bookkeeping
     int* queue;                // work-queue counters (kQueueCounters, zeroed before every evaluation):
-                               // [0] finest items, [1] prediction items, [kQueuePost + m] posterior level m
+                               // [0] small finest regions, [1] prediction items, [kQueuePost + m] posterior level m
     int* err;                  // [0]: status, [1]: region (low), [2]: region (high)
 };
 
@@ -97,9 +121,21 @@ template <typename T>
 __device__ __forceinline__ bool skipped(const DevTree<T>& t, long region) {
     return t.active && !t.active[region];
 }
+// the region whose sub-tree holds a chunk: the level M-3 region (the root when M = 2)
+template <typename T>
+__device__ __forceinline__ long chunk_region(const DevTree<T>& t, long unit) {
+    return t.M >= 3 ? level_start(t.J, t.M - 3) + unit : 0;
+}
 // slice index of block (j,k), j <= k < m, row-major over the upper triangle
 // (the order of class_approximation.cpp:62-73)
 __host__ __device__ inline long slice_index(int m, int j, int k) { return (long)j * m - (long)j * (j - 1) / 2 + (k - j); }
+
+__device__ inline void report_error(int* err, long region) {
+    if (atomicCAS(&err[0], 0, 4 /* MRA_ERR_NOT_SPD */) == 0) {
+        err[1] = (int)(region & 0x7fffffff);
+        err[2] = (int)(region >> 31);
+    }
+}
 
 // θ-dependent field evaluation parameters (device pointers)
 struct FieldParams {
@@ -142,9 +178,19 @@ struct CovTiming {
 // of regions whose blocks fit t.cbuf; returns the number of kernels launched.
 template <typename T>
 int launch_prior_level(const Geom& g, const DevTree<T>& t, int m, int grid, cudaStream_t st, CovTiming* tm = nullptr);
-// The finest groups; returns the number of kernels launched (1).
+// Stream and events (timing disabled) on which the heavy finest regions run
+// beside the small ones, and the number of 64-wide block columns of each heavy
+// region (host memory, largest first).
+struct FinestFork {
+    cudaStream_t side;
+    cudaEvent_t fork, join;
+    const int* heavy_blocks;
+};
+// The finest level (without the level M-2 posterior); returns the number of kernels launched.
 template <typename T>
-int launch_finest_group(const Geom& g, const DevTree<T>& t, int grid, bool keep, cudaStream_t st);
+int launch_finest(const Geom& g, const DevTree<T>& t, int grid, cudaStream_t st, const FinestFork& fk);
+cudaError_t prepare_finest();
+cudaError_t set_gemm_tiles_finest(const int nw[3]);
 template <typename T>
 void launch_posterior_level(const Geom& g, const DevTree<T>& t, int m, int grid, bool keep, cudaStream_t st);
 template <typename T>
