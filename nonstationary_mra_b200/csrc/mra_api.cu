@@ -297,6 +297,7 @@ mra_status run_eval(mra_ctx* c, bool predict) {
     const long np_all = c->n_int * c->r + c->n_obs + c->n_pred;
     const long rr = (long)c->r * c->r;
     int i = 0, launched = 0;
+    const Fork fk{c->side, c->fork, c->join, c->heavy_blocks.data()};
     c->timed_plan.clear();
     CovTiming cov{c->cev, mra_ctx::kMaxCovTimed, 0, capturing, false};
     for (size_t pi = 0; pi < c->plan.size(); ++pi) {
@@ -338,14 +339,12 @@ mra_status run_eval(mra_ctx* c, bool predict) {
                     launched += 3;
                 }
                 {
-                    const FinestFork fk{c->side, c->fork, c->join, c->heavy_blocks.data()};
                     if (mixed && c->mixed_finest32) {
                         launched += launch_finest<float>(c->geom, tf, c->grid, st, fk);
                     } else {
                         launched += launch_finest<double>(c->geom, td, c->grid, st, fk);
                         if (td.fuse_post) {
-                            launch_posterior_level<double>(c->geom, td, c->M - 2, c->grid, predict, st);
-                            launched += 1;
+                            launched += launch_posterior_level(td, c->M - 2, c->grid, predict, st, fk);
                         }
                     }
                 }
@@ -362,8 +361,7 @@ mra_status run_eval(mra_ctx* c, bool predict) {
                 }
                 break;
             case MRA_KERNEL_POSTERIOR_LEVEL:
-                launch_posterior_level<double>(c->geom, td, l.level, c->grid, predict, st);
-                launched += 1;
+                launched += launch_posterior_level(td, l.level, c->grid, predict, st, fk);
                 break;
             case MRA_KERNEL_REDUCE:
                 launch_reduce<double>(td, c->d_result, st);
@@ -488,6 +486,8 @@ mra_status setup_tree(mra_ctx* c, DevTree<T>& t, const HostTree& h, const PointS
     t.n_heavy_tiles = (long)h.heavy_tiles.size();
     t.heavy_inv = sh.heavy_inv;
     // sizes of the level-parity buffers
+    for (int m = 0; m < kMaxLevels; ++m) t.n_dense[m] = 0;
+    t.n_dense[0] = h.factored[0] ? 0 : 1;
     size_t aout_sz[2] = {1, 1}, wout_sz[2] = {1, 1}, F_sz[2] = {1, 1}, f_sz[2] = {1, 1};
     for (int m = 1; m <= M - 2; ++m) {
         const long s0 = level_start(J, m), cnt = level_count(J, m);
@@ -497,6 +497,7 @@ mra_status setup_tree(mra_ctx* c, DevTree<T>& t, const HostTree& h, const PointS
             if (h.factored[s0 + q]) any_fact = true;
             else ++n_dense;
         }
+        t.n_dense[m] = n_dense;
         if (n_dense > 0) {
             aout_sz[m & 1] = std::max(aout_sz[m & 1], (size_t)(n_dense * n_slices(m) * rr));
             wout_sz[m & 1] = std::max(wout_sz[m & 1], (size_t)(n_dense * m * r));
@@ -506,13 +507,12 @@ mra_status setup_tree(mra_ctx* c, DevTree<T>& t, const HostTree& h, const PointS
             f_sz[m & 1] = std::max(f_sz[m & 1], (size_t)c->n_obs);
         }
     }
-    t.ws_stride = post_part ? std::max((long)r * c->tf + 2L * c->tf * c->tf, n_slices(M - 1) * rr + (long)(M - 2) * rr + rr) + 64
-                            : 64;
+    t.ws_stride = post_part ? (long)r * c->tf + 2L * c->tf * c->tf + 64 : 64;
     // prior: V of one conditioning step (r x r); finest: the inverse of a small
     // region's L_Sigma (n x n, n <= 64), or a whole sibling group's conditional
     // covariance and block-diagonal inverse (2 x 64 x 64)
     if (prior_part) t.ws_stride = std::max(t.ws_stride, std::max(rr, 2L * 64 * 64) + 64);
-    t.wsd_stride = post_part ? (long)(M - 1) * r + c->tf + 64 : 64;
+    t.wsd_stride = post_part ? (long)c->tf + 64 : 64;
     if (!post_part) {
         for (int p = 0; p < 2; ++p) aout_sz[p] = wout_sz[p] = F_sz[p] = f_sz[p] = 1;
     }
@@ -557,7 +557,10 @@ mra_status setup_tree(mra_ctx* c, DevTree<T>& t, const HostTree& h, const PointS
             cap_mb = 8192;
         if (const char* e = std::getenv("MRA_COV_BUF_MB")) cap_mb = std::max(1L, std::atol(e));
         long elems = std::min(need, cap_mb * (1L << 20) / (long)sizeof(T));
-        const long floor_elems = std::min(need, (long)(M - 1) * rr * c->grid);  // one region per CTA slot
+        long floor_elems = std::min(need, (long)(M - 1) * rr * c->grid);  // one region per CTA slot
+        if (post_part)  // and the scratch of one dense region of each posterior level
+            for (int m = 0; m <= M - 2; ++m)
+                if (t.n_dense[m]) floor_elems = std::max(floor_elems, dense_scratch(m, r));
         elems = std::max(elems, floor_elems);
         for (;;) {
             cudaError_t e2 = cudaSuccess;
@@ -568,6 +571,15 @@ mra_status setup_tree(mra_ctx* c, DevTree<T>& t, const HostTree& h, const PointS
             elems = std::max(floor_elems, elems / 4);
         }
         t.cbuf_elems = elems;
+    } else if (post_part) {
+        // the mixed path's posterior: the FP32 tree's buffer, read as doubles
+        t.cbuf = reinterpret_cast<T*>(c->tf32.cbuf);
+        t.cbuf_elems = c->tf32.cbuf_elems / 2;
+        for (int m = 0; m <= M - 2; ++m)
+            if (t.n_dense[m] && t.cbuf_elems < dense_scratch(m, r)) {
+                t.cbuf_elems = dense_scratch(m, r);
+                TALLOC(t.cbuf, T, t.cbuf_elems);
+            }
     }
     TALLOC(t.wsd, double, (long)c->grid * t.wsd_stride);
     TALLOC(t.P, T, pred_part ? c->n_pred * (long)L * r : 1);
@@ -779,7 +791,7 @@ mra_status mra_create(const mra_structure* s, const mra_model* m, int32_t precis
             if (!h.factored[s0 + q]) h.dslot[s0 + q] = k++;
     }
     c->h_dslot = h.dslot;
-    // posterior work items of each level, most expensive first: a factored
+    // posterior work items of each level, dense regions first, most expensive first: a factored
     // region costs about n^2 (m r) for its n observations, a dense one the
     // accumulation of its factored children ((m+1) r)^2 per row plus its
     // r^3-sized step
@@ -805,8 +817,10 @@ mra_status mra_create(const mra_structure* s, const mra_model* m, int32_t precis
             }
         }
         for (long q = 0; q < cnt; ++q) h.post_order[s0 + q] = q;
-        std::stable_sort(h.post_order.begin() + s0, h.post_order.begin() + s0 + cnt,
-                         [&](int64_t a, int64_t b) { return cost[a] > cost[b]; });
+        std::stable_sort(h.post_order.begin() + s0, h.post_order.begin() + s0 + cnt, [&](int64_t a, int64_t b) {
+            const int8_t fa = h.factored[s0 + a], fb = h.factored[s0 + b];
+            return fa != fb ? fa < fb : cost[a] > cost[b];
+        });
     }
     // finest level, conditioning: runs of at most 64 observations below one
     // level M-3 region (the root when M = 2).  Every run walks the same chain of
@@ -1304,6 +1318,7 @@ mra_status mra_autotune(mra_ctx* c, int32_t evals, int32_t* choice_out, double* 
     for (int k = 0; k < nc; ++k) {
         CU(set_gemm_tiles(cand[k]));
         CU(set_gemm_tiles_finest(cand[k]));
+        CU(set_gemm_tiles_posterior(cand[k]));
         double d, ll, ms = 0.0;
         mra_status st = mra_loglik(c, &d, &ll);  // warm-up with this choice
         if (st != MRA_OK) return st;
@@ -1319,6 +1334,7 @@ mra_status mra_autotune(mra_ctx* c, int32_t evals, int32_t* choice_out, double* 
     }
     CU(set_gemm_tiles(cand[ib]));
     CU(set_gemm_tiles_finest(cand[ib]));
+    CU(set_gemm_tiles_posterior(cand[ib]));
     if (choice_out)
         for (int b = 0; b < 3; ++b) choice_out[b] = cand[ib][b];
     if (ms_out) *ms_out = best / evals;

@@ -576,7 +576,7 @@ static void launch_condition(const DevTree<double>& t, cudaStream_t st) {
 }
 
 template <typename T>
-int launch_finest(const Geom& g, const DevTree<T>& t, int grid, cudaStream_t st, const FinestFork& fk) {
+int launch_finest(const Geom& g, const DevTree<T>& t, int grid, cudaStream_t st, const Fork& fk) {
     int launches = 0;
     if (t.n_chunks > 0) {
         launch_cov_finest<T>(g, t, st);
@@ -646,7 +646,7 @@ cudaError_t prepare_finest() {
 
 cudaError_t set_gemm_tiles_finest(const int nw[3]) { return cudaMemcpyToSymbol(c_gemm_nw, nw, 3 * sizeof(int)); }
 
-template int launch_finest<double>(const Geom&, const DevTree<double>&, int, cudaStream_t, const FinestFork&);
-template int launch_finest<float>(const Geom&, const DevTree<float>&, int, cudaStream_t, const FinestFork&);
+template int launch_finest<double>(const Geom&, const DevTree<double>&, int, cudaStream_t, const Fork&);
+template int launch_finest<float>(const Geom&, const DevTree<float>&, int, cudaStream_t, const Fork&);
 
 }  // namespace mra

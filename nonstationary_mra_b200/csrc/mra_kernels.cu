@@ -10,27 +10,12 @@
 //   (mra_finest.cu)     finest level: conditioning, Sigma, L_Sigma, y~, B^ and
 //                       the log-lik terms
 //                       (...-loop-regions-at-finest-level-in-prior.cpp:90-269)
-//   k_posterior_level(m) levels M-2..0 (...-posterior-inference.cpp:14-265,
+//   (mra_posterior.cu)  posterior, levels M-2..0 (...-posterior-inference.cpp:14-265,
 //                       class_approximation.cpp:186-306)
 //   k_reduce            deterministic sum of the per-region terms
 //   k_predict           prediction, one CTA per level M-2 region (its finest
 //                       children's predictions together)
 //                       (...-prior.cpp:271-392, class_approximation-predict.cpp:105-189)
-//
-// Posterior representation.  A region's contribution to its parent is the pair
-// (A~, w~) of the reference (class_approximation.cpp:266-306).  Below a size
-// threshold it is carried in factored observation-space form instead: a matrix
-// F (n x m r, one row per observation of the subtree) and a vector f with
-// A~_(j,k) = F_j^T F_k and w~_j = F_j^T f.  The finest level starts in this
-// form (F = B^, f = y~).  For a region i at level m with factored input (F, f):
-//   Y = L_i^{-1} F_m^T,  R R^T = I + Y^T Y,
-//   output F' = R^{-1} F_{0..m-1},  f' = R^{-1} f,
-//   log-lik term 2 log|R| - (f^T f - f'^T f'),
-// which equals the reference's -2 log|L_i| + 2 log|L~_i| - v^T v with
-// L~ L~^T = L L^T + F_m^T F_m (Sylvester's determinant identity and Woodbury),
-// and F'^T F' / F'^T f' equal the reference's A~ / w~ of the region.  Larger
-// regions use the reference's dense r x r slices.  Prediction mode also forms
-// L~, v and G of factored regions from (F, f).
 #include "mra_kernels.cuh"
 
 namespace mra {
@@ -176,277 +161,6 @@ __global__ void __launch_bounds__(kThreads, 2) k_prior_level(Geom g, DevTree<T> 
             t.ldprior[i] = ld;
             if (info) report_error(t.err, i);
         }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// posterior steps of one region (level m): factored and dense forms
-// ---------------------------------------------------------------------------
-// The products of the posterior steps go through a separate function: the
-// steps keep many values live across their products, and inlined there the
-// product loops would share (and spill) their registers.
-template <typename T, bool TA, bool TB, bool ONE_TILE = false>
-__device__ __noinline__ void gemm_call(int M, int N, int K, T alpha, const T* A, long lda, const T* B, long ldb,
-                                       T beta, T* C, long ldc, LaSmem<T>& sm, const T* Cin = nullptr,
-                                       long ldcin = 0) {
-    gemm<T, TA, TB, ONE_TILE>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, sm, Cin, ldcin);
-}
-
-// Factored input (F: n rows of width (m+1) r, row stride ldF; f: n doubles).
-// Writes F' (n rows of width m r) to Fo and f' to fo when m > 0.
-template <typename T>
-__device__ __noinline__ void factored_step(const DevTree<T>& t, int m, long i, int n, const T* F, long ldF, const double* f, T* Fo,
-                              double* fo, bool keep, T* ws, double* wsd, LaSmem<T>& sm, double& dterm) {
-    const int r = t.r;
-    const long rr = (long)r * r, mr = (long)m * r;
-    const T* Li = t.Lprior + i * rr;
-    T* Y = ws;                  // r x n
-    T* S = ws + (long)r * n;    // n x n
-    T* Rinv = S + (long)n * n;  // n x n (n <= 128)
-    // Y = L_i^{-1} F_m^T as a product with the stored inverse of the prior factor
-    gemm_call<T, false, false>(r, n, r, (T)1, t.Pinv + i * rr, r, F + mr, ldF, (T)0, Y, r, sm);
-    gemm_call<T, true, false>(n, n, r, (T)1, Y, r, Y, r, (T)0, S, n, sm);
-    for (int q = threadIdx.x; q < n; q += kThreads) S[q + (long)q * n] += (T)1;
-    __syncthreads();
-    double ld = 0.0;
-    const bool small = sizeof(T) == 8 && n <= 128;
-    int info = potrf_lower<T>(n, S, n, sm, &ld, small ? Rinv : nullptr, n);
-    double* fp = m > 0 ? fo : wsd;
-    double part = 0.0;
-    for (int q = threadIdx.x; q < n; q += kThreads) {
-        fp[q] = f[q];
-        part += f[q] * f[q];
-    }
-    double ff = cta_sum(part, sm);
-    if (small) trmv_lower_inv<T>(n, Rinv, n, fp, fp);  // f' = R^{-1} f with the inverse formed above
-    else trsv_lower_f64<T>(n, S, n, fp);
-    part = 0.0;
-    for (int q = threadIdx.x; q < n; q += kThreads) part += fp[q] * fp[q];
-    double pp = cta_sum(part, sm);
-    if (threadIdx.x == 0) {
-        dterm += ld - (ff - pp);
-        if (info) report_error(t.err, i);
-    }
-    if (m > 0) {
-        if (small) {
-            // F' = F_{0..m-1} R^{-T}
-            gemm_call<T, false, true>((int)mr, n, n, (T)1, F, ldF, Rinv, n, (T)0, Fo, mr, sm);
-        } else {
-            for (long e = threadIdx.x; e < mr * n; e += kThreads) {
-                long x = e % mr, q = e / mr;
-                Fo[q * mr + x] = F[q * ldF + x];
-            }
-            __syncthreads();
-            trsm_right_lower_trans<T>((int)mr, n, S, n, Fo, mr, sm);
-        }
-    }
-    if (keep) {
-        // predictive factors of the region: L~ L~^T = L L^T + F_m^T F_m, v = L~^{-1} F_m^T f,
-        // G = L~^{-1} F_m^T F_{0..m-1}
-        T* Lt = t.Lpost + i * rr;
-        gemm_call<T, false, true>(r, r, r, (T)1, Li, r, Li, r, (T)0, Lt, r, sm);
-        gemm_call<T, false, true>(r, r, n, (T)1, F + mr, ldF, F + mr, ldF, (T)1, Lt, r, sm);
-        T* Lti = t.Lpinv ? t.Lpinv + i * rr : nullptr;  // L~^{-1}, kept for prediction
-        int info2 = potrf_lower<T>(r, Lt, r, sm, nullptr, Lti, r);
-        double* v = t.vpost + i * r;
-        for (int tt = threadIdx.x; tt < r; tt += kThreads) {
-            double s = 0.0;
-            for (int q = 0; q < n; ++q) s += (double)F[(long)q * ldF + mr + tt] * f[q];
-            v[tt] = s;
-        }
-        __syncthreads();
-        if (Lti) trmv_lower_inv<T>(r, Lti, r, v, v);
-        else trsv_lower_f64<T>(r, Lt, r, v);
-        if (m > 0) {
-            T* Gi = t.G + t.u_off[m] + (i - level_start(t.J, m)) * mr * r;
-            gemm_call<T, false, true>(r, (int)mr, n, (T)1, F + mr, ldF, F, ldF, (T)0, Gi, r, sm);
-            // G = L~^{-1} G in place: one row tile (r <= 64) reads all of its
-            // column block before writing it
-            if (Lti) gemm_call<T, false, false>(r, (int)mr, r, (T)1, Lti, r, Gi, r, (T)0, Gi, r, sm);
-            else trsm_left_lower<T>(r, (int)mr, Lt, r, Gi, r, sm);
-        }
-        if (info2 && threadIdx.x == 0) report_error(t.err, i);
-    }
-}
-
-// Dense input: Aagg holds the slices (j,k), j <= k <= m, of the summed children
-// contributions, wagg the (m+1) x r summed w.
-template <typename T>
-__device__ __noinline__ void dense_step(const DevTree<T>& t, int m, long i, const T* Aagg, const double* wagg, bool keep, T* Gw,
-                           LaSmem<T>& sm, double& dterm) {
-    const int r = t.r;
-    const long rr = (long)r * r, mr = (long)m * r;
-    const long loc = i - level_start(t.J, m);
-    const T* Lp = t.Lprior + i * rr;
-    T* Lt = t.Lpost + i * rr;
-    gemm_call<T, false, true>(r, r, r, (T)1, Lp, r, Lp, r, (T)0, Lt, r, sm);
-    const T* Amm = Aagg + slice_index(m + 1, m, m) * rr;
-    for (long e = threadIdx.x; e < rr; e += kThreads) Lt[e] += Amm[e];
-    __syncthreads();
-    double ld = 0.0;
-    // L~^{-1}: kept for prediction when that is on, else an r x r scratch after the G scratch
-    const bool kept = keep && t.Lpinv;
-    T* Ltinv = kept ? t.Lpinv + i * rr : Gw + mr * r;
-    const bool small = sizeof(T) == 8 && r <= 64 && (m > 0 || kept);
-    int info = potrf_lower<T>(r, Lt, r, sm, &ld, small ? Ltinv : nullptr, r);
-    double* v = t.vpost + i * r;
-    for (int e = threadIdx.x; e < r; e += kThreads) v[e] = wagg[mr + e];
-    __syncthreads();
-    if (small) trmv_lower_inv<T>(r, Ltinv, r, v, v);  // v = L~^{-1} w_m with the inverse formed above
-    else trsv_lower_f64<T>(r, Lt, r, v);
-    double part = 0.0;
-    for (int e = threadIdx.x; e < r; e += kThreads) part += v[e] * v[e];
-    double vv = cta_sum(part, sm);
-    if (threadIdx.x == 0) {
-        dterm += ld - t.ldprior[i] - vv;
-        if (info) report_error(t.err, i);
-    }
-    if (m == 0) return;
-    T* Gi = keep ? t.G + t.u_off[m] + loc * mr * r : Gw;  // r x (m r), ld = r
-    if (small) {
-        // G_j = L~^{-1} A_(j,m)^T
-        for (int j = 0; j < m; ++j)
-            gemm_call<T, false, true>(r, r, r, (T)1, Ltinv, r, Aagg + slice_index(m + 1, j, m) * rr, r, (T)0,
-                                 Gi + (long)j * rr, r, sm);
-    } else {
-        for (long e = threadIdx.x; e < mr * r; e += kThreads) {
-            int j = (int)(e / rr);
-            long w = e % rr;
-            int p = (int)(w % r), q = (int)(w / r);
-            Gi[e] = Aagg[slice_index(m + 1, j, m) * rr + q + (long)p * r];  // G_j = A_(j,m)^T
-        }
-        __syncthreads();
-        trsm_left_lower<T>(r, (int)mr, Lt, r, Gi, r, sm);
-    }
-    const long slot = t.dslot[i];  // compact index among the level's dense regions
-    double* wo = t.wout[m & 1] + slot * mr;
-    for (long x = threadIdx.x; x < mr; x += kThreads) {
-        double s = 0.0;
-        for (int tt = 0; tt < r; ++tt) s += (double)Gi[tt + x * r] * v[tt];
-        wo[x] = wagg[x] - s;
-    }
-    // A_out(j, j..m-1) = A(j, j..m-1) - G_j^T G_{j..m-1}: both slice rows are
-    // contiguous r x r blocks, one product per j reading A from Aagg
-    T* ao = t.aout[m & 1] + slot * n_slices(m) * rr;
-    for (int j = 0; j < m; ++j) {
-        T* dst = ao + slice_index(m, j, j) * rr;
-        const T* src = Aagg + slice_index(m + 1, j, j) * rr;
-        gemm_call<T, true, false>(r, (m - j) * r, r, (T)-1, Gi + (long)j * rr, r, Gi + (long)j * rr, r, (T)1, dst, r,
-                                  sm, src, r);
-    }
-}
-
-// Aagg/wagg += the (A~, w~) of factored rows F (n x (m+1) r, row stride ldF), f;
-// with `init` they are set instead (the first contribution: no zeroing pass).
-// The slices (j, j..m) of A~ are contiguous r x r blocks, so block row j is
-// one product F_j^T F_{j..m} (r x (m+1-j) r).
-template <typename T>
-__device__ __noinline__ void accumulate_factored(const DevTree<T>& t, int m, int n, const T* F, long ldF, const double* f, T* Aagg,
-                                    double* wagg, bool init, LaSmem<T>& sm) {
-    const int r = t.r;
-    const long rr = (long)r * r, mr1 = (long)(m + 1) * r;
-    if (n == 0) {
-        if (init) {
-            for (long e = threadIdx.x; e < n_slices(m + 1) * rr; e += kThreads) Aagg[e] = (T)0;
-            for (long e = threadIdx.x; e < mr1; e += kThreads) wagg[e] = 0.0;
-            __syncthreads();
-        }
-        return;
-    }
-    for (int j = 0; j <= m; ++j)
-        gemm_call<T, false, true>(r, (m + 1 - j) * r, n, (T)1, F + (long)j * r, ldF, F + (long)j * r, ldF,
-                                  init ? (T)0 : (T)1, Aagg + slice_index(m + 1, j, j) * rr, r, sm);
-    for (long x = threadIdx.x; x < mr1; x += kThreads) {
-        double s = 0.0;
-        for (int q = 0; q < n; ++q) s += (double)F[(long)q * ldF + x] * f[q];
-        wagg[x] = init ? s : wagg[x] + s;
-    }
-    __syncthreads();
-}
-
-// ---------------------------------------------------------------------------
-// a9/a10/a11: posterior, one level (m = M-3 .. 0)
-// ---------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(kThreads, 2) k_posterior_level(Geom g, DevTree<T> t, int m, int keep) {
-    LaSmem<T>& sm = la_smem<T>();
-    const int r = t.r;
-    const long rr = (long)r * r, mr1 = (long)(m + 1) * r;
-    const long s0 = level_start(t.J, m), cnt = level_count(t.J, m);
-    const long ns_in = n_slices(m + 1);
-    T* ws = t.ws + blockIdx.x * t.ws_stride;
-    double* wsd = t.wsd + blockIdx.x * t.wsd_stride;
-    const T* Fin = t.Fbuf[(m + 1) & 1];
-    const double* fin = t.fbuf[(m + 1) & 1];
-    const T* ain = t.aout[(m + 1) & 1];
-    const double* win = t.wout[(m + 1) & 1];
-    const bool from_finest = m == t.M - 2;  // children are finest regions: rows of B^, y~
-    // regions taken from a shared counter, most expensive first (the clustered
-    // regions' dense steps cost tens of factored ones)
-    __shared__ long s_loc;
-    for (;;) {
-        __syncthreads();  // every thread has read the previous s_loc
-        if (threadIdx.x == 0) {
-            const int q = atomicAdd(&t.queue[kQueuePost + m], 1);
-            s_loc = q < cnt ? t.post_order[s0 + q] : -1;
-        }
-        __syncthreads();
-        const long loc = s_loc;
-        if (loc < 0) break;
-        const long i = s0 + loc;
-        if (skipped(t, i)) continue;
-        double dterm = 0.0;
-        if (from_finest) {
-            const long lo = t.sub_lo[i];
-            const int n = (int)(t.sub_hi[i] - lo);
-            const T* F = t.Bhat + lo * mr1;
-            const double* f = t.yt + lo;
-            if (t.factored[i]) {
-                T* Fo = m > 0 ? t.Fbuf[m & 1] + lo * (long)m * r : nullptr;
-                double* fo = m > 0 ? t.fbuf[m & 1] + lo : nullptr;
-                factored_step<T>(t, m, i, n, F, mr1, f, Fo, fo, keep != 0, ws, wsd, sm, dterm);
-            } else {
-                T* Aagg = ws;
-                double* wagg = wsd;
-                accumulate_factored<T>(t, m, n, F, mr1, f, Aagg, wagg, true, sm);
-                dense_step<T>(t, m, i, Aagg, wagg, keep != 0, Aagg + ns_in * rr, sm, dterm);
-            }
-        } else if (t.factored[i]) {
-            const long lo = t.sub_lo[i];
-            const int n = (int)(t.sub_hi[i] - lo);
-            T* Fo = m > 0 ? t.Fbuf[m & 1] + lo * (long)m * r : nullptr;
-            double* fo = m > 0 ? t.fbuf[m & 1] + lo : nullptr;
-            factored_step<T>(t, m, i, n, Fin + lo * mr1, mr1, fin + lo, Fo, fo, keep != 0, ws, wsd, sm, dterm);
-        } else {
-            T* Aagg = ws;
-            double* wagg = wsd;
-            bool first = true;  // the first contribution sets Aagg / wagg
-            for (int cc = 1; cc <= t.J; ++cc) {
-                const long c = i * t.J + cc;
-                if (t.factored[c]) {
-                    // factored children with adjacent rows are accumulated together
-                    const long lo = t.sub_lo[c];
-                    long hi = t.sub_hi[c], cl = c;
-                    while (cc < t.J && t.factored[cl + 1] && t.sub_lo[cl + 1] == hi) {
-                        ++cc;
-                        ++cl;
-                        hi = t.sub_hi[cl];
-                    }
-                    accumulate_factored<T>(t, m, (int)(hi - lo), Fin + lo * mr1, mr1, fin + lo, Aagg, wagg, first, sm);
-                } else {
-                    const long cl = t.dslot[c];
-                    const T* as = ain + cl * ns_in * rr;
-                    const double* wsrc = win + cl * mr1;
-                    for (long e = threadIdx.x; e < ns_in * rr; e += kThreads) Aagg[e] = first ? as[e] : Aagg[e] + as[e];
-                    for (long e = threadIdx.x; e < mr1; e += kThreads) wagg[e] = first ? wsrc[e] : wagg[e] + wsrc[e];
-                    __syncthreads();
-                }
-                first = false;
-            }
-            dense_step<T>(t, m, i, Aagg, wagg, keep != 0, Aagg + ns_in * rr, sm, dterm);
-        }
-        if (threadIdx.x == 0) t.dpost[i] = dterm;
-        __syncthreads();
     }
 }
 
@@ -661,11 +375,6 @@ int launch_prior_level(const Geom& g, const DevTree<T>& t, int m, int grid, cuda
     return launches;
 }
 template <typename T>
-void launch_posterior_level(const Geom& g, const DevTree<T>& t, int m, int grid, bool keep, cudaStream_t st) {
-    long cnt = level_count(t.J, m);
-    k_posterior_level<T><<<(unsigned)(cnt < grid ? cnt : grid), kThreads, sizeof(LaSmem<T>), st>>>(g, t, m, keep ? 1 : 0);
-}
-template <typename T>
 void launch_predict(const Geom& g, const DevTree<T>& t, int grid, cudaStream_t st) {
     const long cnt2 = level_count(t.J, t.M - 2);
     k_predict<T><<<(unsigned)(cnt2 < grid ? cnt2 : grid), kThreads, sizeof(LaSmem<T>), st>>>(g, t);
@@ -703,7 +412,6 @@ static cudaError_t prepare_type() {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     };
     set((const void*)k_prior_level<T>);
-    set((const void*)k_posterior_level<T>);
     set((const void*)k_predict<T>);
     set((const void*)k_reduce<T>);
     set((const void*)k_sample<T>);
@@ -715,12 +423,12 @@ cudaError_t set_gemm_tiles(const int nw[3]) { return cudaMemcpyToSymbol(c_gemm_n
 cudaError_t prepare_kernels() {
     cudaError_t e = prepare_type<double>();
     if (e == cudaSuccess) e = prepare_type<float>();
+    if (e == cudaSuccess) e = prepare_posterior();
     return e == cudaSuccess ? prepare_finest() : e;
 }
 
 #define MRA_INSTANTIATE(T)                                                                                   \
     template int launch_prior_level<T>(const Geom&, const DevTree<T>&, int, int, cudaStream_t, CovTiming*); \
-    template void launch_posterior_level<T>(const Geom&, const DevTree<T>&, int, int, bool, cudaStream_t);  \
     template void launch_predict<T>(const Geom&, const DevTree<T>&, int, cudaStream_t);                     \
     template void launch_reduce<T>(const DevTree<T>&, double*, cudaStream_t);                               \
     template void launch_sample<T>(const DevTree<T>&, const double*, const double*, double*, int, cudaStream_t);

@@ -53,8 +53,9 @@ struct DevTree {
     const HeavyTile* heavy_tiles;  // [n_heavy_tiles] lower tiles of their Sigma
     long n_heavy_tiles;
     const int64_t* pred_order; // [J^(M-2)] level M-2 regions (local index), most expensive prediction work first
-    const int64_t* post_order; // [n_int] per level m, at level_start(m): the level's regions (local index),
-                               // most expensive posterior step first
+    const int64_t* post_order; // [n_int] per level m, at level_start(m): the level's regions (local index), its
+                               // n_dense[m] dense ones first, each kind most expensive step first
+    long n_dense[kMaxLevels];
     const int8_t* factored;    // [n_int] 1: the region's posterior output is kept as F, f
     const int8_t* active;      // [n_int] sub-tree sharding: 0 = the region belongs to another rank's
                                // sub-tree and is skipped; nullptr: every region is computed
@@ -85,8 +86,9 @@ struct DevTree {
     double* wout[2];           // dense w~ of one level's dense regions (by dslot)
     T* Fbuf[2];                // factored F of one level: [n_obs][m r]
     double* fbuf[2];           // factored f of one level: [n_obs]
-    T* cbuf;                   // covariance blocks of a chunk of one prior level's regions
-    long cbuf_elems;           // its size in elements (a multiple of nothing in particular)
+    T* cbuf;                   // covariance blocks of a chunk of one prior level's regions; later the scratch of
+                               // a chunk of one posterior level's dense regions
+    long cbuf_elems;           // its size in elements
     T* ws;                     // per-CTA workspace (T)
     long ws_stride;
     double* wsd;               // per-CTA workspace (FP64)
@@ -178,21 +180,27 @@ struct CovTiming {
 // of regions whose blocks fit t.cbuf; returns the number of kernels launched.
 template <typename T>
 int launch_prior_level(const Geom& g, const DevTree<T>& t, int m, int grid, cudaStream_t st, CovTiming* tm = nullptr);
-// Stream and events (timing disabled) on which the heavy finest regions run
-// beside the small ones, and the number of 64-wide block columns of each heavy
+// Stream and events (timing disabled) for work beside the main stream's (heavy
+// finest regions beside small ones, factored regions beside dense ones), and the
+// number of 64-wide block columns of each heavy
 // region (host memory, largest first).
-struct FinestFork {
+struct Fork {
     cudaStream_t side;
     cudaEvent_t fork, join;
     const int* heavy_blocks;
 };
 // The finest level (without the level M-2 posterior); returns the number of kernels launched.
 template <typename T>
-int launch_finest(const Geom& g, const DevTree<T>& t, int grid, cudaStream_t st, const FinestFork& fk);
+int launch_finest(const Geom& g, const DevTree<T>& t, int grid, cudaStream_t st, const Fork& fk);
 cudaError_t prepare_finest();
 cudaError_t set_gemm_tiles_finest(const int nw[3]);
-template <typename T>
-void launch_posterior_level(const Geom& g, const DevTree<T>& t, int m, int grid, bool keep, cudaStream_t st);
+// One posterior level (FP64): its dense regions in chunks whose scratch fits
+// t.cbuf, its factored ones beside them; returns the number of kernels launched.
+int launch_posterior_level(const DevTree<double>& t, int m, int grid, bool keep, cudaStream_t st, const Fork& fk);
+cudaError_t prepare_posterior();
+cudaError_t set_gemm_tiles_posterior(const int nw[3]);
+// doubles of scratch of one dense region of level m: the slices (j, m), G and the inverse of L~
+inline long dense_scratch(int m, int r) { return (2L * m + 1) * r * r; }
 template <typename T>
 void launch_predict(const Geom& g, const DevTree<T>& t, int grid, cudaStream_t st);
 template <typename T>
