@@ -549,7 +549,9 @@ mra_status setup_tree(mra_ctx* c, DevTree<T>& t, const HostTree& h, const PointS
     t.cbuf_elems = 0;
     if (prior_part) {
         long need = 0;
-        for (int m = 0; m <= M - 2; ++m) need = std::max(need, level_count(J, m) * (long)(m + 1) * rr);
+        const int SB = prior_batch(sizeof(T) == 8, r, J);
+        for (int m = 0; m <= M - 2; ++m)
+            need = std::max(need, (level_count(J, m) + SB - 1) / SB * SB * (long)(m + 1) * rr);
         long cap_mb = 2048;
         size_t free_b = 0, total_b = 0;
         if (sizeof(T) == 8 && c->precision == MRA_PRECISION_FP64 && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
@@ -1317,6 +1319,7 @@ mra_status mra_autotune(mra_ctx* c, int32_t evals, int32_t* choice_out, double* 
     int ib = 0;
     for (int k = 0; k < nc; ++k) {
         CU(set_gemm_tiles(cand[k]));
+        CU(set_gemm_tiles_prior(cand[k]));
         CU(set_gemm_tiles_finest(cand[k]));
         CU(set_gemm_tiles_posterior(cand[k]));
         double d, ll, ms = 0.0;
@@ -1333,6 +1336,7 @@ mra_status mra_autotune(mra_ctx* c, int32_t evals, int32_t* choice_out, double* 
         if (ms < best) best = ms, ib = k;
     }
     CU(set_gemm_tiles(cand[ib]));
+    CU(set_gemm_tiles_prior(cand[ib]));
     CU(set_gemm_tiles_finest(cand[ib]));
     CU(set_gemm_tiles_posterior(cand[ib]));
     if (choice_out)

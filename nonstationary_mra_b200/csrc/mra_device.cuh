@@ -1136,70 +1136,138 @@ __device__ inline int potrf_blocked(int n, T* A, long lda, LaSmem<T>& sm, double
 
 
 // FP64 Cholesky (and optionally the inverse of the factor) of an n x n
-// matrix, n <= 64, staged whole in shared memory (column-major, ld 65),
-// right-looking in 16-wide block columns:
-//  * each 16 x 16 diagonal block is factored by one warp with lane l holding
-//    row l in registers (pivots broadcast by shuffles, 1/sqrt(pivot) by
-//    rsqrt), and the same warp inverts the block (lane l: column l);
-//  * the panel below it is the product of the panel with the block's inverse
-//    (transposed), and the trailing update a rank-16 product, each thread
-//    owning rows tx + 16a / columns ty + 16c of the 16 x 16 thread grid;
-//  * X = L^{-1} is completed block by block away from the diagonal:
-//    X_ij = -X_ii sum_{k=j}^{i-1} L_ik X_kj.
-// n that is not a multiple of 16 is padded with an identity block.  A
+// matrix, n <= 64, staged whole in shared memory (column-major, ld 68: 4 mod 16
+// doubles, conflict-free m8n8k4 fragments), right-looking in 8-wide blocks.
+// What bounds it is the chain of the 64 pivots (1/sqrt, scale, update), so each
+// block's 8 x 8 diagonal is factored redundantly in the registers of every
+// thread that needs it -- no shuffles or barriers inside the chain -- and the
+// inverse rides along: with X = I to start with, block row k of X = L^{-1} is the
+// same 8-step substitution as a panel row, and its update another tile of the
+// trailing product.
+//  * threads 0..63: row of the panel (the diagonal block's rows among them);
+//    threads 64..127: column of X's block row;
+//  * all warps: 8 x 8 tiles of the trailing matrix and of X by m8n8k4.
+// n that is not a multiple of 8 is padded with an identity block.  A
 // non-positive or NaN pivot sets sm.flag (1-based index, first wins) and the
 // factorization goes on with NaNs.  logdet (thread 0) = 2 sum log L_ii.
-constexpr int SLD = 65;
-constexpr unsigned kFullMask = 0xffffffffu;
+// n = 64 with the inverse, one CTA of 256: 21,100 cycles, n = 16: 5,900 (16-wide
+// blocks with the diagonal block's rows in lanes and shuffled pivots: 55,800 and
+// 11,800); two CTAs per SM: 27,000 each (62,100).
+constexpr int SLD = 68;
 
-// One warp: factors the 16 x 16 block of S at (b0, b0) in place and writes its
-// inverse to the same block of X (both with zeros above the diagonal).
-static __device__ __noinline__ void potrf_diag16(double* S, double* X, int b0, LaSmem<double>& sm) {
-    const int l = threadIdx.x & 31;
-    double x[16];
-#pragma unroll
-    for (int c = 0; c < 16; ++c) x[c] = (l < 16 && c <= l) ? S[(b0 + l) + (b0 + c) * SLD] : 0.0;
+// S (N x N valid lower part, N = n rounded up to 8) -> L; X -> L^{-1} if kInv.
+// Starts after a barrier on S, ends with one.
+// NT (128 or 256): threads of the CTA.
+template <bool kInv, typename Sm, int NT = kThreads>
+__device__ __forceinline__ void potrf_core(int n, double* S, double* X, Sm& sm) {
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int g = lane >> 2, t = lane & 3;
+    const int nbk = (n + 7) >> 3, N = nbk << 3;
+    if (kInv) {
+        for (int e = tid; e < N * 64; e += NT) X[(e & 63) + (e >> 6) * SLD] = (e & 63) == (e >> 6) ? 1.0 : 0.0;
+        __syncthreads();
+    }
     int bad = 0;
+    for (int k = 0; k < nbk; ++k) {
+        const int k0 = k << 3;
+        const int row = k0 + tid, c = tid - 64;
+        const bool prow = tid < 64 && row < N, pcol = kInv && tid >= 64 && c < k0 + 8;
+        double* base = tid < 64 ? S + row + k0 * SLD : X + k0 + c * SLD;
+        const int step = tid < 64 ? SLD : 1;
+        double l[36], x[8];  // the diagonal block, row by row; this thread's panel row or column of X
+        if (tid < 128) {
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-        const double d = __shfl_sync(kFullMask, x[k], k);
-        if (!(d > 0.0) && bad == 0) bad = b0 + k + 1;
-        const double r = rsqrt(d);
-        if (l == 0) sm.inv[k] = r;
-        x[k] = l == k ? d * r : (l > k ? x[k] * r : x[k]);
+            for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = k + 1; j < 16; ++j) {
-            const double ljk = __shfl_sync(kFullMask, x[k], j);
-            if (l >= j) x[j] = fma(-x[k], ljk, x[j]);
+                for (int j = 0; j <= i; ++j) l[i * (i + 1) / 2 + j] = S[(k0 + i) + (k0 + j) * SLD];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) x[j] = prow || pcol ? base[j * step] : 0.0;
+        }
+        __syncthreads();  // the block is read before its rows are rewritten
+        if (tid < 128) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const double d = l[j * (j + 1) / 2 + j];
+                if (!(d > 0.0) && bad == 0 && k0 + j < n) bad = k0 + j + 1;
+                const double r = rsqrt(d);
+#pragma unroll
+                for (int i = j + 1; i < 8; ++i) l[i * (i + 1) / 2 + j] *= r;
+                x[j] *= r;
+#pragma unroll
+                for (int i = j + 1; i < 8; ++i) {
+#pragma unroll
+                    for (int q = j + 1; q <= i; ++q)
+                        l[i * (i + 1) / 2 + q] = fma(-l[i * (i + 1) / 2 + j], l[q * (q + 1) / 2 + j], l[i * (i + 1) / 2 + q]);
+                    x[i] = fma(-l[i * (i + 1) / 2 + j], x[j], x[i]);
+                }
+            }
+            if (prow || pcol) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) base[j * step] = tid < 64 && j > tid ? 0.0 : x[j];  // zeros above the diagonal
+            }
+        }
+        __syncthreads();
+        // trailing tiles by block columns: column q <= k of X (rows below k), column q > k of S (rows from q)
+        for (int q = w; q < nbk; q += NT / 32) {
+            if (!kInv && q <= k) continue;
+            const bool inX = q <= k;
+            const double* B = inX ? X + k0 + 8 * q * SLD : S + 8 * q + k0 * SLD;
+            const int bs = inX ? SLD : 1, bt = inX ? 1 : SLD;
+            const double b0 = B[g * bs + t * bt], b1 = B[g * bs + (4 + t) * bt];
+            double* C = (inX ? X : S) + g + (8 * q + 2 * t) * SLD;
+            const double* A = S + g + (k0 + t) * SLD;
+            int bi = inX ? k + 1 : q;
+#pragma unroll 4
+            for (; bi < nbk; ++bi) {
+                double acc[2] = {-C[8 * bi], -C[8 * bi + SLD]};
+                mma_f64(acc, A[8 * bi], b0);
+                mma_f64(acc, A[8 * bi + 4 * SLD], b1);
+                C[8 * bi] = -acc[0];
+                C[8 * bi + SLD] = -acc[1];
+            }
+        }
+        __syncthreads();
+    }
+    if (tid == 0) sm.flag = bad;
+}
+
+// Factors S = sm.A (after a barrier) and writes L to A and, if kInv, its inverse
+// (formed in sm.B) to inv, zeros above the diagonals; returns the first bad pivot.
+// A function of its own, with its registers to itself; sm is the kernel's dynamic
+// shared memory, taken here so that its accesses are known to be shared ones.
+template <bool kInv, typename Sm, int NT = kThreads>
+__device__ __noinline__ int potrf_finish(int n, double* A, long lda, double* logdet, double* inv, long ldinv) {
+    extern __shared__ __align__(16) unsigned char la_dyn_smem[];
+    Sm& sm = *reinterpret_cast<Sm*>(la_dyn_smem);
+    double* S = &sm.A[0][0];
+    double* X = &sm.B[0][0];
+    const int tid = threadIdx.x;
+    potrf_core<kInv, Sm, NT>(n, S, X, sm);
+    if (tid < 64) {
+        double part = tid < n ? log(S[tid + tid * SLD]) : 0.0;
+        for (int o = 16; o > 0; o >>= 1) part += __shfl_down_sync(0xffffffffu, part, o);
+        if ((tid & 31) == 0) sm.red[tid >> 5] = part;
+    }
+    const int i = tid & 63;
+    if (i < n) {
+#pragma unroll 4
+        for (int j = tid >> 6; j < n; j += NT / 64) {
+            A[i + (long)j * lda] = i >= j ? S[i + j * SLD] : 0.0;
+            if (kInv) inv[i + (long)j * ldinv] = i >= j ? X[i + j * SLD] : 0.0;
         }
     }
-    if (l < 16) {
-#pragma unroll
-        for (int c = 0; c < 16; ++c) S[(b0 + l) + (b0 + c) * SLD] = c <= l ? x[c] : 0.0;
-    }
-    if (l == 0 && bad && sm.flag == 0) sm.flag = bad;
-    __syncwarp();
-    double y[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) y[i] = i == l ? 1.0 : 0.0;
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-        y[k] *= sm.inv[k];
-#pragma unroll
-        for (int i = k + 1; i < 16; ++i) y[i] = fma(-S[(b0 + i) + (b0 + k) * SLD], y[k], y[i]);
-    }
-    if (l < 16) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) X[(b0 + i) + (b0 + l) * SLD] = y[i];
-    }
+    __syncthreads();
+    if (tid == 0 && logdet) *logdet = 2.0 * (sm.red[0] + sm.red[1]);
+    const int flag = sm.flag;
+    __syncthreads();  // the shared memory is free again
+    return flag;
 }
 
 __device__ inline int potrf_small(int n, double* A, long lda, LaSmem<double>& sm, double* logdet, double* inv,
                                   long ldinv) {
     const int tid = threadIdx.x;
-    double* S = &sm.A[0][0];  // 64 x 65 (fits in the operand tile buffers)
-    double* X = &sm.B[0][0];
-    const int nbk = (n + 15) >> 4, N = nbk << 4;
+    double* S = &sm.A[0][0];  // 64 x 68 (fits in the operand tile buffers)
+    const int N = (n + 7) & ~7;
     {
         // every load issued before the first store (16 columns per thread)
         const int i = tid & 63, j0 = tid >> 6;
@@ -1215,115 +1283,9 @@ __device__ inline int potrf_small(int n, double* A, long lda, LaSmem<double>& sm
             if (i < N && j < N) S[i + j * SLD] = v[q];
         }
     }
-    if (tid == 0) sm.flag = 0;
     __syncthreads();
-    const int tx = tid & 15, ty = tid >> 4;
-    for (int b = 0; b < nbk; ++b) {
-        const int b0 = b << 4;
-        if (tid < 32) potrf_diag16(S, X, b0, sm);
-        __syncthreads();
-        const int rest = N - b0 - 16;
-        if (rest > 0) {
-            const int r0 = b0 + 16, na = rest >> 4;
-            // panel: L[i][b0+k] = sum_{c<=k} A[i][b0+c] Y[k][c], Y the block's inverse
-            double v[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-            for (int c = 0; c < 16; ++c) {
-                if (c <= ty) {
-                    const double yk = X[(b0 + ty) + (b0 + c) * SLD];
-#pragma unroll
-                    for (int a = 0; a < 3; ++a)
-                        if (a < na) v[a] = fma(S[(r0 + tx + 16 * a) + (b0 + c) * SLD], yk, v[a]);
-                }
-            }
-            __syncthreads();
-#pragma unroll
-            for (int a = 0; a < 3; ++a)
-                if (a < na) S[(r0 + tx + 16 * a) + (b0 + ty) * SLD] = v[a];
-            __syncthreads();
-            // trailing update of the lower triangle
-            double acc[3][3];
-#pragma unroll
-            for (int a = 0; a < 3; ++a)
-#pragma unroll
-                for (int e = 0; e < 3; ++e) acc[a][e] = 0.0;
-#pragma unroll
-            for (int k = 0; k < 16; ++k) {
-                double li[3], lj[3];
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    li[a] = a < na ? S[(r0 + tx + 16 * a) + (b0 + k) * SLD] : 0.0;
-                    lj[a] = a < na ? S[(r0 + ty + 16 * a) + (b0 + k) * SLD] : 0.0;
-                }
-#pragma unroll
-                for (int a = 0; a < 3; ++a)
-#pragma unroll
-                    for (int e = 0; e <= a; ++e) acc[a][e] = fma(li[a], lj[e], acc[a][e]);
-            }
-#pragma unroll
-            for (int a = 0; a < 3; ++a)
-#pragma unroll
-                for (int e = 0; e <= a; ++e)
-                    if (a < na && (a > e || tx >= ty)) S[(r0 + tx + 16 * a) + (r0 + ty + 16 * e) * SLD] -= acc[a][e];
-            __syncthreads();
-        }
-    }
-    double part = 0.0;
-    for (int i = tid; i < n; i += kThreads) part += log(S[i + i * SLD]);
-    const double sum = cta_sum(part, sm);
-    if (tid == 0 && logdet) *logdet = 2.0 * sum;
-    {
-        const int i = tid & 63;
-        for (int j = tid >> 6; j < n; j += kThreads / 64)
-            if (i < n) A[i + (long)j * lda] = i >= j ? S[i + j * SLD] : 0.0;
-    }
-    if (inv) {
-        // off-diagonal blocks of X by distance dd from the diagonal; thread
-        // (tx, ty) forms element (tx, ty) of each block
-        for (int dd = 1; dd < nbk; ++dd) {
-            const int np = nbk - dd;
-            double v[3];
-#pragma unroll
-            for (int u = 0; u < 3; ++u) {
-                v[u] = 0.0;
-                if (u < np) {
-                    const int row = 16 * (u + dd) + tx, col = 16 * u + ty;
-                    double s[4] = {0.0, 0.0, 0.0, 0.0};
-                    for (int kb = u; kb < u + dd; ++kb) {
-#pragma unroll
-                        for (int c = 0; c < 16; ++c)
-                            s[c & 3] = fma(S[row + (16 * kb + c) * SLD], X[(16 * kb + c) + col * SLD], s[c & 3]);
-                    }
-                    v[u] = (s[0] + s[1]) + (s[2] + s[3]);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < 3; ++u)
-                if (u < np) X[(16 * (u + dd) + tx) + (16 * u + ty) * SLD] = v[u];
-            __syncthreads();
-#pragma unroll
-            for (int u = 0; u < 3; ++u) {
-                if (u < np) {
-                    const int ib = u + dd, row = 16 * ib + tx, col = 16 * u + ty;
-                    double s[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-                    for (int c = 0; c < 16; ++c)
-                        if (c <= tx) s[c & 3] = fma(X[row + (16 * ib + c) * SLD], X[(16 * ib + c) + col * SLD], s[c & 3]);
-                    v[u] = -((s[0] + s[1]) + (s[2] + s[3]));
-                }
-            }
-            __syncthreads();
-#pragma unroll
-            for (int u = 0; u < 3; ++u)
-                if (u < np) X[(16 * (u + dd) + tx) + (16 * u + ty) * SLD] = v[u];
-            __syncthreads();
-        }
-        const int i = tid & 63;
-        for (int j = tid >> 6; j < n; j += kThreads / 64)
-            if (i < n) inv[i + (long)j * ldinv] = i >= j ? X[i + j * SLD] : 0.0;
-    }
-    __syncthreads();
-    return sm.flag;
+    return inv ? potrf_finish<true, LaSmem<double>>(n, A, lda, logdet, inv, ldinv)
+               : potrf_finish<false, LaSmem<double>>(n, A, lda, logdet, inv, ldinv);
 }
 
 // FP64 Cholesky with the inverse of the factor for 64 < n <= 128, as a 2 x 2

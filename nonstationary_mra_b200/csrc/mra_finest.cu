@@ -18,7 +18,7 @@
 //   k_heavy_*               the same of larger finest regions in 64 x 64 tiles,
 //                           one CTA per tile, the block columns in turn
 //   k_finest_terms          log-lik terms summed per sibling group
-#include "mra_kernels.cuh"
+#include "mra_cond.cuh"
 
 namespace mra {
 
@@ -63,161 +63,38 @@ __global__ void __launch_bounds__(kCovThreads, 4) k_cov_finest(Geom g, DevTree<T
 // ---------------------------------------------------------------------------
 // conditioning: V_j = C_j - U_{a_j}^T U_{S,0..j-1},  U_{S,j} = L_{a_j}^{-1} V_j
 // ---------------------------------------------------------------------------
-// FP64, r <= RC <= 64.  One CTA per chunk walks the ancestors; per ancestor one
-// product over K = j r (slabs of 32, three in flight: U_a of the deepest
-// ancestor is read once and comes from HBM) and one with the stored inverse,
-// whose operand V_j stays in shared memory.  RC is the tile height (16, 32 or
-// 64): 8 warps as RC / 8 row groups x 64 / RC column groups, each warp 8 rows x
-// up to RC columns, so that small r and narrow chunks leave no warp multiplying
-// padding.  EVEN: r even, operand rows 16-byte aligned, copied in pairs.
-template <int RC>
-struct CondSmem {
-    static constexpr int AS = RC * KS64 > TK64 * (RC + 4) ? RC * KS64 : TK64 * (RC + 4);
-    double A[3][AS];
-    double B[3][64 * KS64];  // also V, [column][row], row stride RC + 4
-};
-
+// FP64, r <= RC <= 64 (mra_cond.cuh): one CTA per chunk.
 template <int RC, bool EVEN>
-__device__ __forceinline__ void cond_step(CondSmem<RC>& sm, int r, const double* Ua, int K, const double* Us, long Lr,
-                                          int N, const double* P, double* V, double* U) {
-    constexpr int RW = RC / 8, CW = 8 / RW, NF = RC / 8;  // row groups, column groups, fragments per warp
-    constexpr int RS = RC + 4, VS = RC + 4;
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const int g = lane >> 2, t = lane & 3;
-    const int wr = w % RW, wc = w / RW;
-    const int N8 = (N + 7) & ~7;
-    const int row = 8 * wr + g;
-    double acc[NF][2];
-    // accumulators start at -C, so that acc ends at -(C - U_a^T U_S)
-#pragma unroll
-    for (int f = 0; f < NF; ++f) {
-        const int c = (f * CW + wc) * 8 + 2 * t;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) acc[f][h] = (row < r && c + h < N) ? -V[row + (long)(c + h) * Lr] : 0.0;
-    }
-    auto issue = [&](int k0, int s) {
-        double* sA = sm.A[s];
-        double* sB = sm.B[s];
-        if (EVEN) {
-            for (int e = tid; e < RC * (TK64 / 2); e += kThreads) {
-                const int i = e / (TK64 / 2), k = 2 * (e % (TK64 / 2));
-                const bool ok = i < r && k0 + k < K;
-                cp_async16z(sA + i * KS64 + k, ok ? Ua + (k0 + k) + (long)i * K : Ua, ok);
-            }
-            for (int e = tid; e < N8 * (TK64 / 2); e += kThreads) {
-                const int j = e / (TK64 / 2), k = 2 * (e % (TK64 / 2));
-                const bool ok = j < N && k0 + k < K;
-                cp_async16z(sB + j * KS64 + k, ok ? Us + (k0 + k) + (long)j * Lr : Us, ok);
-            }
-        } else {
-            for (int e = tid; e < RC * TK64; e += kThreads) {
-                const int i = e / TK64, k = e % TK64;
-                const bool ok = i < r && k0 + k < K;
-                cp_async8(sA + i * KS64 + k, ok ? Ua + (k0 + k) + (long)i * K : Ua, ok);
-            }
-            for (int e = tid; e < N8 * TK64; e += kThreads) {
-                const int j = e / TK64, k = e % TK64;
-                const bool ok = j < N && k0 + k < K;
-                cp_async8(sB + j * KS64 + k, ok ? Us + (k0 + k) + (long)j * Lr : Us, ok);
-            }
-        }
-    };
-    const int ns = (K + TK64 - 1) / TK64;
-    if (ns > 0) issue(0, 0);
-    cp_async_commit();
-    if (ns > 1) issue(TK64, 1);
-    cp_async_commit();
-    int s = 0;
-    for (int i = 0; i < ns; ++i) {
-        cp_async_wait<1>();  // slab i has landed (for this thread; the barrier makes it so for all)
-        __syncthreads();     // and every warp is done with slab i - 1, whose stage slab i + 2 takes
-        const int s2 = s == 0 ? 2 : s - 1;
-        if (i + 2 < ns) issue((i + 2) * TK64, s2);
-        cp_async_commit();
-        const double* sA = sm.A[s] + row * KS64 + t;
-        const double* sB = sm.B[s] + g * KS64 + t;
-#pragma unroll
-        for (int k4 = 0; k4 < TK64; k4 += 4) {
-            const double a = sA[k4];
-#pragma unroll
-            for (int f = 0; f < NF; ++f) {
-                const int c0 = (f * CW + wc) * 8;
-                if (c0 < N8) mma_f64(acc[f], a, sB[c0 * KS64 + k4]);
-            }
-        }
-        s = s == 2 ? 0 : s + 1;
-    }
-    __syncthreads();
-    // L_a^{-1} (lower triangular, zeros above) as two slabs [k][row]; V_j to memory and as the next operand
-    for (int e = tid; e < RC * (EVEN ? RC / 2 : RC); e += kThreads) {
-        const int i = EVEN ? 2 * (e % (RC / 2)) : e % RC, k = EVEN ? e / (RC / 2) : e / RC;
-        double* dst = sm.A[k / TK64] + (k % TK64) * RS + i;
-        const bool ok = i < r && k < r;
-        if (EVEN) cp_async16z(dst, ok ? P + i + (long)k * r : P, ok);
-        else cp_async8(dst, ok ? P + i + (long)k * r : P, ok);
-    }
-    cp_async_commit();
-    double* sV = &sm.B[0][0];
-#pragma unroll
-    for (int f = 0; f < NF; ++f) {
-        const int c = (f * CW + wc) * 8 + 2 * t;
-        if ((f * CW + wc) * 8 >= N8) continue;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const double v = -acc[f][h];
-            sV[(c + h) * VS + row] = v;
-            if (row < r && c + h < N) V[row + (long)(c + h) * Lr] = v;
-            acc[f][h] = 0.0;
-        }
-    }
-    cp_async_wait<0>();
-    __syncthreads();
-    const int kend = 8 * (wr + 1);  // rows 8 wr .. 8 wr + 7 of a lower-triangular factor
-#pragma unroll 4
-    for (int k4 = 0; k4 < kend; k4 += 4) {
-        const double a = sm.A[k4 / TK64][(k4 % TK64 + t) * RS + row];
-#pragma unroll
-        for (int f = 0; f < NF; ++f) {
-            const int c0 = (f * CW + wc) * 8;
-            if (c0 < N8) mma_f64(acc[f], a, sV[(c0 + g) * VS + k4 + t]);
-        }
-    }
-#pragma unroll
-    for (int f = 0; f < NF; ++f) {
-        const int c = (f * CW + wc) * 8 + 2 * t;
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-            if (row < r && c + h < N) U[row + (long)(c + h) * Lr] = acc[f][h];
-    }
-    __syncthreads();
-}
-
-template <int RC, bool EVEN>
-__global__ void __launch_bounds__(kThreads, 2) k_finest_condition(DevTree<double> t) {
+__global__ void __launch_bounds__(kCondThreads, CondSmem<RC>::CTAS) k_finest_condition(DevTree<double> t) {
     extern __shared__ __align__(16) unsigned char la_dyn_smem[];
-    CondSmem<RC>& sm = *reinterpret_cast<CondSmem<RC>*>(la_dyn_smem);
     const int r = t.r, L = t.L, m = t.M - 2;
     const long rr = (long)r * r, Lr = (long)L * r;
     const FinChunk ch = t.chunks[blockIdx.x];
     const long unit = ch.unit;
     if (skipped(t, chunk_region(t, unit))) return;
+    Cond<RC, EVEN> cond(*reinterpret_cast<CondSmem<RC>*>(la_dyn_smem), r);
     double* V = t.Bhat + ch.lo * Lr;
     double* U = t.Ufin + ch.lo * Lr;
-    for (int j = 0; j < m; ++j) {
-        long a = chunk_region(t, unit);
-        for (int l = m - 1; l > j; --l) a = (a - 1) / t.J;
-        const double* Ua = t.U + t.u_off[j] + (a - level_start(t.J, j)) * (long)j * rr;
-        cond_step<RC, EVEN>(sm, r, Ua, j * r, U, Lr, ch.n, t.Pinv + a * rr, V + (long)j * r, U + (long)j * r);
-    }
-    const long g0 = m > 0 ? unit * t.J : 0, g1 = m > 0 ? g0 + t.J : 1;
-    const long s2 = level_start(t.J, m);
-    for (long gl = g0; gl < g1; ++gl) {
-        const long glo = t.sub_lo[s2 + gl], ghi = t.sub_hi[s2 + gl];
-        const long lo = glo > ch.lo ? glo : ch.lo, hi = ghi < ch.lo + ch.n ? ghi : ch.lo + ch.n;
-        if (lo >= hi) continue;
+    // levels 0..M-3, then level M-2 per sibling group of the chunk; one call of
+    // step, whose code then stays in the instruction cache
+    const int ng = m > 0 ? t.J : 1;
+    const long g0 = m > 0 ? unit * t.J : 0, s2 = level_start(t.J, m);
+    for (int s = 0; s < m + ng; ++s) {
+        long a, lo = ch.lo, hi = ch.lo + ch.n;
+        const int j = s < m ? s : m;
+        if (s < m) {
+            a = chunk_region(t, unit);  // level m-1, up to level j
+            for (int l = m - 1; l > j; --l) a = (a - 1) / t.J;
+        } else {
+            a = s2 + g0 + (s - m);
+            if (t.sub_lo[a] > lo) lo = t.sub_lo[a];
+            if (t.sub_hi[a] < hi) hi = t.sub_hi[a];
+            if (lo >= hi) continue;
+        }
         const long d = (lo - ch.lo) * Lr;
-        cond_step<RC, EVEN>(sm, r, t.U + t.u_off[m] + gl * (long)m * rr, m * r, U + d, Lr, (int)(hi - lo),
-                            t.Pinv + (s2 + gl) * rr, V + d + (long)m * r, U + d + (long)m * r);
+        const CondOp o{t.U + t.u_off[j] + (a - level_start(t.J, j)) * (long)j * rr, j * r, U + d, Lr, (int)(hi - lo)};
+        double* Vj = V + d + (long)j * r;
+        cond.step(o, t.Pinv + a * rr, Vj, Lr, Vj, U + d + (long)j * r);
     }
 }
 
@@ -571,8 +448,8 @@ static void launch_cov_finest(const Geom& g, const DevTree<T>& t, cudaStream_t s
 template <int RC>
 static void launch_condition(const DevTree<double>& t, cudaStream_t st) {
     const unsigned grid = (unsigned)t.n_chunks;
-    if (t.r % 2 == 0) k_finest_condition<RC, true><<<grid, kThreads, sizeof(CondSmem<RC>), st>>>(t);
-    else k_finest_condition<RC, false><<<grid, kThreads, sizeof(CondSmem<RC>), st>>>(t);
+    if (t.r % 2 == 0) k_finest_condition<RC, true><<<grid, kCondThreads, sizeof(CondSmem<RC>), st>>>(t);
+    else k_finest_condition<RC, false><<<grid, kCondThreads, sizeof(CondSmem<RC>), st>>>(t);
 }
 
 template <typename T>

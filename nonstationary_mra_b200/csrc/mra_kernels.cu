@@ -5,7 +5,7 @@
 // Schedule of one log-likelihood (one launch per stage and tree level):
 //   k_fields            sigma^2/beta/tau^2 at every knot, observation and
 //                       prediction point (class_nonstationary_covariance.cpp:479-573)
-//   k_prior_level(m)    levels 0..M-2, one CTA per region: U_{i,j} = L_{a_j}^{-1} V_j,
+//   (mra_prior.cu)      prior, levels 0..M-2: U_{i,j} = L_{a_j}^{-1} V_j,
 //                       L_i = chol(K_i)   (class_approximation.cpp:46-50,84-169)
 //   (mra_finest.cu)     finest level: conditioning, Sigma, L_Sigma, y~, B^ and
 //                       the log-lik terms
@@ -59,109 +59,6 @@ __global__ void k_fields(Geom g, FieldParams fp, const double* __restrict__ c0, 
     s2[i] = out[0];
     beta[i] = out[1];
     t2[i] = out[2];
-}
-
-// ---------------------------------------------------------------------------
-// a2/a3 for the prior: the covariance blocks of one level, in their own launch
-// ---------------------------------------------------------------------------
-// Regions loc0 .. loc0+nloc-1 (local indices) of level m: block j < m of region
-// i is C(Q_{a_j}, Q_i) (rows: the knots of ancestor a_j, columns: the region's
-// own knots; evaluate_nonstationary_cross_covariance, evaluate_covariance.cpp:
-// 155-234), block m is C(Q_i, Q_i) with sigma^2 + tau^2 on its diagonal
-// (:248-313).  Block j of the q-th region goes to out + (q (m+1) + j) r^2,
-// column-major with ld r.  One CTA per block at a time; with no barrier-bound
-// products beside it the launch keeps every SM full of independent entry
-// chains, which the per-region kernel, two CTAs per SM between its products,
-// cannot.
-template <typename T, int KIND>
-__global__ void __launch_bounds__(kCovThreads, 4) k_cov_level(Geom g, DevTree<T> t, int m, long loc0, long nloc,
-                                                               T* __restrict__ out) {
-    __shared__ double stage[7 * kCovChunk];
-    const int r = t.r;
-    const long rr = (long)r * r;
-    const long s0 = level_start(t.J, m);
-    const long nblocks = nloc * (m + 1);
-    for (long b = blockIdx.x; b < nblocks; b += gridDim.x) {
-        const long q = b / (m + 1);
-        const int j = (int)(b - q * (m + 1));
-        const long i = s0 + loc0 + q;
-        if (skipped(t, i)) continue;
-        long a = i;  // the ancestor of level j (the region itself for j == m)
-        for (int l = m; l > j; --l) a = (a - 1) / t.J;
-        cov_block<T, KIND>(g, t.pts, a * r, r, i * r, r, j == m, out + b * rr, r, stage);
-    }
-}
-
-// Host-side dispatch of the covariance-block launches on the model's form.
-template <typename T>
-void launch_cov_level(const Geom& g, const DevTree<T>& t, int m, long loc0, long n, unsigned grid, cudaStream_t st) {
-    switch (cov_kind(g, sizeof(T) == 8)) {
-        case 1: k_cov_level<T, 1><<<grid, kCovThreads, 0, st>>>(g, t, m, loc0, n, t.cbuf); break;
-        case 2: k_cov_level<T, 2><<<grid, kCovThreads, 0, st>>>(g, t, m, loc0, n, t.cbuf); break;
-        case 3: k_cov_level<T, 3><<<grid, kCovThreads, 0, st>>>(g, t, m, loc0, n, t.cbuf); break;
-        case 4: k_cov_level<T, 4><<<grid, kCovThreads, 0, st>>>(g, t, m, loc0, n, t.cbuf); break;
-        default: k_cov_level<T, 0><<<grid, kCovThreads, 0, st>>>(g, t, m, loc0, n, t.cbuf); break;
-    }
-}
-
-// ---------------------------------------------------------------------------
-// a5/a6: prior, one level of interior regions
-// ---------------------------------------------------------------------------
-// One CTA per region.  The inverse L_a^{-1} of every prior factor is formed
-// once, right after its Cholesky, so that the m triangular solves of each
-// descendant become tensor-pipe products.  The covariance blocks come from
-// k_cov_level (C: the q-th region's m+1 blocks at C + q (m+1) r^2); each
-// conditioning product takes its block as the added term, so nothing is
-// copied: V_j = C_j - U_{a_j}^T U_{i,0..j-1}, U_{i,j} = L_{a_j}^{-1} V_j and
-// K_i = C_i - U_i^T U_i straight into the factor's storage.
-template <typename T>
-__global__ void __launch_bounds__(kThreads, 2) k_prior_level(Geom g, DevTree<T> t, int m, long loc0, long nloc,
-                                                            const T* __restrict__ C) {
-    LaSmem<T>& sm = la_smem<T>();
-    const int r = t.r;
-    const long rr = (long)r * r;
-    const long s0 = level_start(t.J, m);
-    const long mr = (long)m * r;
-    for (long q = blockIdx.x; q < nloc; q += gridDim.x) {
-        const long loc = loc0 + q;
-        const long i = s0 + loc;
-        if (skipped(t, i)) continue;
-        long anc[kMaxLevels];
-        {
-            long c = i;
-            for (int a = m - 1; a >= 0; --a) {
-                c = (c - 1) / t.J;
-                anc[a] = c;
-            }
-        }
-        const T* Cq = C + q * (long)(m + 1) * rr;
-        T* Ui = t.U + t.u_off[m] + loc * mr * r;  // (m r) x r, ld = m r
-        // one r x r scratch per CTA (stays in L2)
-        T* V = t.ws + blockIdx.x * t.ws_stride;
-        for (int j = 0; j < m; ++j) {
-            const long a = anc[j];
-            const T* Cj = Cq + j * rr;
-            const T* Vj = Cj;  // level 0 has nothing to condition on
-            // the next covariance block (or the self block) into L2 while this step's products run
-            if (threadIdx.x == 0) prefetch_l2(Cj + rr, rr * sizeof(T));
-            if (j > 0) {
-                const T* Ua = t.U + t.u_off[j] + (a - level_start(t.J, j)) * (long)j * rr;
-                gemm_wide<T, true, false>(r, r, j * r, (T)-1, Ua, (long)j * r, Ui, mr, (T)1, V, r, sm, Cj, r);
-                Vj = V;
-            }
-            // U_{i,j} = L_a^{-1} V as a product with the stored inverse
-            gemm<T, false, false>(r, r, r, (T)1, t.Pinv + a * rr, r, Vj, r, (T)0, Ui + (long)j * r, mr, sm);
-        }
-        T* Li = t.Lprior + i * rr;
-        // K_i = C_i - U_i^T U_i (for m == 0 a product with K = 0: the copy of C_i)
-        gemm<T, true, false>(r, r, (int)mr, (T)-1, Ui, mr, Ui, mr, (T)1, Li, r, sm, Cq + (long)m * rr, r);
-        double ld = 0.0;
-        int info = potrf_lower<T>(r, Li, r, sm, &ld, t.Pinv + i * rr, r);
-        if (threadIdx.x == 0) {
-            t.ldprior[i] = ld;
-            if (info) report_error(t.err, i);
-        }
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -349,32 +246,6 @@ void launch_fields(const Geom& g, const FieldParams& fp, const double* c0, const
     k_fields<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(g, fp, c0, c1, c2, n, s2, beta, t2);
 }
 template <typename T>
-int launch_prior_level(const Geom& g, const DevTree<T>& t, int m, int grid, cudaStream_t st, CovTiming* tm) {
-    auto mark = [&](cudaEvent_t e) {
-        if (tm->capturing) cudaEventRecordWithFlags(e, st, cudaEventRecordExternal);
-        else cudaEventRecord(e, st);
-    };
-    const long cnt = level_count(t.J, m);
-    const long per_region = (long)(m + 1) * t.r * t.r;
-    long per = t.cbuf_elems / per_region;  // regions whose blocks fit the buffer at once
-    if (per < 1) per = 1;
-    int launches = 0;
-    for (long loc0 = 0; loc0 < cnt; loc0 += per) {
-        const long n = cnt - loc0 < per ? cnt - loc0 : per;
-        const long nb = n * (m + 1);
-        const long cov_grid = (long)grid * 16;  // 16 per region-kernel slot: 32 CTAs per SM
-        const bool timed = tm && tm->used < tm->cap;
-        if (tm && !timed) tm->overflow = true;
-        if (timed) mark(tm->ev[2 * tm->used]);
-        launch_cov_level<T>(g, t, m, loc0, n, (unsigned)(nb < cov_grid ? nb : cov_grid), st);
-        if (timed) mark(tm->ev[2 * tm->used++ + 1]);
-        k_prior_level<T><<<(unsigned)(n < grid ? n : grid), kThreads, sizeof(LaSmem<T>), st>>>(g, t, m, loc0, n,
-                                                                                                t.cbuf);
-        launches += 2;
-    }
-    return launches;
-}
-template <typename T>
 void launch_predict(const Geom& g, const DevTree<T>& t, int grid, cudaStream_t st) {
     const long cnt2 = level_count(t.J, t.M - 2);
     k_predict<T><<<(unsigned)(cnt2 < grid ? cnt2 : grid), kThreads, sizeof(LaSmem<T>), st>>>(g, t);
@@ -411,7 +282,6 @@ static cudaError_t prepare_type() {
     auto set = [&](const void* fn) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     };
-    set((const void*)k_prior_level<T>);
     set((const void*)k_predict<T>);
     set((const void*)k_reduce<T>);
     set((const void*)k_sample<T>);
@@ -423,12 +293,12 @@ cudaError_t set_gemm_tiles(const int nw[3]) { return cudaMemcpyToSymbol(c_gemm_n
 cudaError_t prepare_kernels() {
     cudaError_t e = prepare_type<double>();
     if (e == cudaSuccess) e = prepare_type<float>();
+    if (e == cudaSuccess) e = prepare_prior();
     if (e == cudaSuccess) e = prepare_posterior();
     return e == cudaSuccess ? prepare_finest() : e;
 }
 
 #define MRA_INSTANTIATE(T)                                                                                   \
-    template int launch_prior_level<T>(const Geom&, const DevTree<T>&, int, int, cudaStream_t, CovTiming*); \
     template void launch_predict<T>(const Geom&, const DevTree<T>&, int, cudaStream_t);                     \
     template void launch_reduce<T>(const DevTree<T>&, double*, cudaStream_t);                               \
     template void launch_sample<T>(const DevTree<T>&, const double*, const double*, double*, int, cudaStream_t);

@@ -197,6 +197,14 @@ cudaError_t set_gemm_tiles_finest(const int nw[3]);
 // One posterior level (FP64): its dense regions in chunks whose scratch fits
 // t.cbuf, its factored ones beside them; returns the number of kernels launched.
 int launch_posterior_level(const DevTree<double>& t, int m, int grid, bool keep, cudaStream_t st, const Fork& fk);
+cudaError_t prepare_prior();
+cudaError_t set_gemm_tiles_prior(const int nw[3]);
+// sibling regions that one CTA of the prior takes together (their covariance
+// blocks lie side by side): up to 64 columns, FP64 and r <= 64
+inline int prior_batch(bool fp64, int r, int J) {
+    const int sb = !fp64 || r > 64 ? 1 : (r <= 16 ? 4 : (r <= 32 ? 2 : 1));
+    return sb < J ? sb : J;
+}
 cudaError_t prepare_posterior();
 cudaError_t set_gemm_tiles_posterior(const int nw[3]);
 // doubles of scratch of one dense region of level m: the slices (j, m), G and the inverse of L~
