@@ -184,6 +184,7 @@ struct HostTree {
     std::vector<int64_t> nfin, npred, obs_off, pred_off, fin_anc, pred_order, lsig_off, pc_off;
     std::vector<int64_t> child_lo, child_hi, fin_items, heavy, sub_lo, sub_hi, dslot, post_order;
     std::vector<int8_t> factored;
+    long fin_class[3] = {0, 0, 0}, n_fused = 0;
     std::vector<FinChunk> chunks;
     std::vector<HeavyTile> heavy_tiles;
 };
@@ -340,9 +341,9 @@ mra_status run_eval(mra_ctx* c, bool predict) {
                 }
                 {
                     if (mixed && c->mixed_finest32) {
-                        launched += launch_finest<float>(c->geom, tf, c->grid, st, fk);
+                        launched += launch_finest<float>(c->geom, tf, c->grid, predict, st, fk);
                     } else {
-                        launched += launch_finest<double>(c->geom, td, c->grid, st, fk);
+                        launched += launch_finest<double>(c->geom, td, c->grid, predict || !td.fuse_post, st, fk);
                         if (td.fuse_post) {
                             launched += launch_posterior_level(td, c->M - 2, c->grid, predict, st, fk);
                         }
@@ -478,6 +479,8 @@ mra_status setup_tree(mra_ctx* c, DevTree<T>& t, const HostTree& h, const PointS
     t.dslot = idx[11];
     t.post_order = idx[12];
     t.n_fin_items = (long)h.fin_items.size();
+    for (int q = 0; q < 3; ++q) t.n_fin_class[q] = h.fin_class[q];
+    t.n_fused = h.n_fused;
     t.heavy = idx[13];
     t.n_heavy = (long)h.heavy.size();
     t.chunks = sh.chunks;
@@ -508,10 +511,8 @@ mra_status setup_tree(mra_ctx* c, DevTree<T>& t, const HostTree& h, const PointS
         }
     }
     t.ws_stride = post_part ? (long)r * c->tf + 2L * c->tf * c->tf + 64 : 64;
-    // prior: V of one conditioning step (r x r); finest: the inverse of a small
-    // region's L_Sigma (n x n, n <= 64), or a whole sibling group's conditional
-    // covariance and block-diagonal inverse (2 x 64 x 64)
-    if (prior_part) t.ws_stride = std::max(t.ws_stride, std::max(rr, 2L * 64 * 64) + 64);
+    // prior: V of one conditioning step (r x r)
+    if (prior_part) t.ws_stride = std::max(t.ws_stride, rr + 64);
     t.wsd_stride = post_part ? (long)c->tf + 64 : 64;
     if (!post_part) {
         for (int p = 0; p < 2; ++p) aout_sz[p] = wout_sz[p] = F_sz[p] = f_sz[p] = 1;
@@ -847,41 +848,56 @@ mra_status mra_create(const mra_structure* s, const mra_model* m, int32_t precis
     }
     // finest level, small regions: a sibling group whose children hold at most
     // kChildMax observations each and kGroupMax together is one item (FP64), any
-    // other region of at most kFinTile is its own; most expensive first.  FP64
-    // regions beyond that are factored tile by tile.
+    // other region of at most kFinTile is its own; by tile class, most expensive
+    // first.  FP64 regions beyond that are factored tile by tile.  The posterior of
+    // a factored group taken whole comes with it (FP64 path).
+    std::vector<int8_t> fused(cnt2, 0);
     {
         const bool fp64 = !(precision == MRA_PRECISION_MIXED && c->mixed_finest32);
-        std::vector<std::pair<double, int64_t>> items, heavy;
+        struct Item {
+            int cls;
+            double cost;
+            int64_t v;
+        };
+        std::vector<Item> items, heavy;
+        auto tile_class = [&](long n) { return !fp64 || n > 32 ? 0 : (n > 16 ? 1 : 2); };
         for (long q = 0; q < cnt2; ++q) {
             const long clo = h.child_lo[q], chi = h.child_hi[q];
             const long np = h.obs_off[chi] - h.obs_off[clo];
+            fused[q] = precision == MRA_PRECISION_FP64 && h.factored[lvl2 + q] && np == 0;
             if (np == 0) continue;
             long nmax = 0;
             for (long k = clo; k < chi; ++k) nmax = std::max<long>(nmax, h.nfin[k]);
-            if (fp64 && nmax <= kChildMax && np <= kGroupMax && chi - clo <= kThreads / 32) {
-                items.push_back({(double)np * (np + L * r), (int64_t)q});
+            if (fp64 && nmax <= kChildMax && np <= kGroupMax) {
+                items.push_back({tile_class(np), (double)np * (np + L * r), (int64_t)q});
+                fused[q] = precision == MRA_PRECISION_FP64 && h.factored[lvl2 + q];
                 continue;
             }
             for (long k = clo; k < chi; ++k) {
                 const double n = (double)h.nfin[k];
                 if (n == 0) continue;
-                if (fp64 && n > kFinTile) heavy.push_back({n, (int64_t)k});
-                else items.push_back({n * n * (n + 2.0 * L * r) + 64.0 * n * L * r, (int64_t)(cnt2 + k)});
+                if (fp64 && n > kFinTile) heavy.push_back({0, n, (int64_t)k});
+                else items.push_back({tile_class((long)n), n * n * (n + 2.0 * L * r) + 64.0 * n * L * r, (int64_t)(cnt2 + k)});
             }
         }
-        auto more = [](const std::pair<double, int64_t>& x, const std::pair<double, int64_t>& y) {
-            return x.first > y.first;
-        };
+        auto more = [](const Item& x, const Item& y) { return x.cls != y.cls ? x.cls < y.cls : x.cost > y.cost; };
         std::stable_sort(items.begin(), items.end(), more);
         std::stable_sort(heavy.begin(), heavy.end(), more);
-        for (const auto& it : items) h.fin_items.push_back(it.second);
+        for (const auto& it : items) {
+            h.fin_items.push_back(it.v);
+            ++h.fin_class[it.cls];
+        }
         for (size_t q = 0; q < heavy.size(); ++q) {
-            h.heavy.push_back(heavy[q].second);
-            const int nb = (int)((h.nfin[heavy[q].second] + kFinTile - 1) / kFinTile);
+            h.heavy.push_back(heavy[q].v);
+            const int nb = (int)((h.nfin[heavy[q].v] + kFinTile - 1) / kFinTile);
             c->heavy_blocks.push_back(nb);
             for (int bi = 0; bi < nb; ++bi)
                 for (int bj = 0; bj <= bi; ++bj) h.heavy_tiles.push_back({(int32_t)q, (uint16_t)bi, (uint16_t)bj});
         }
+        // level M-2: the fused regions behind its other factored ones
+        std::stable_partition(h.post_order.begin() + lvl2, h.post_order.begin() + lvl2 + cnt2,
+                              [&](int64_t q) { return !fused[q]; });
+        for (long q = 0; q < cnt2; ++q) h.n_fused += fused[q];
     }
     int64_t u_total = 0;
     for (int mm = 0; mm <= M - 2; ++mm) u_total += level_count(J, mm) * (int64_t)mm * r * r;

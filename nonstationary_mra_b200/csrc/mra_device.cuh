@@ -1157,14 +1157,15 @@ constexpr int SLD = 68;
 
 // S (N x N valid lower part, N = n rounded up to 8) -> L; X -> L^{-1} if kInv.
 // Starts after a barrier on S, ends with one.
-// NT (128 or 256): threads of the CTA.
-template <bool kInv, typename Sm, int NT = kThreads>
+// NT (128 or 256): threads of the CTA; LD: row stride of S and X (4 mod 16 doubles).
+template <bool kInv, typename Sm, int NT = kThreads, int LD = SLD>
 __device__ __forceinline__ void potrf_core(int n, double* S, double* X, Sm& sm) {
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int nbk = (n + 7) >> 3, N = nbk << 3;
     if (kInv) {
-        for (int e = tid; e < N * 64; e += NT) X[(e & 63) + (e >> 6) * SLD] = (e & 63) == (e >> 6) ? 1.0 : 0.0;
+        for (int c = w; c < N; c += NT / 32)
+            for (int i = lane; i < N; i += 32) X[i + c * LD] = i == c ? 1.0 : 0.0;
         __syncthreads();
     }
     int bad = 0;
@@ -1172,14 +1173,14 @@ __device__ __forceinline__ void potrf_core(int n, double* S, double* X, Sm& sm) 
         const int k0 = k << 3;
         const int row = k0 + tid, c = tid - 64;
         const bool prow = tid < 64 && row < N, pcol = kInv && tid >= 64 && c < k0 + 8;
-        double* base = tid < 64 ? S + row + k0 * SLD : X + k0 + c * SLD;
-        const int step = tid < 64 ? SLD : 1;
+        double* base = tid < 64 ? S + row + k0 * LD : X + k0 + c * LD;
+        const int step = tid < 64 ? LD : 1;
         double l[36], x[8];  // the diagonal block, row by row; this thread's panel row or column of X
         if (tid < 128) {
 #pragma unroll
             for (int i = 0; i < 8; ++i)
 #pragma unroll
-                for (int j = 0; j <= i; ++j) l[i * (i + 1) / 2 + j] = S[(k0 + i) + (k0 + j) * SLD];
+                for (int j = 0; j <= i; ++j) l[i * (i + 1) / 2 + j] = S[(k0 + i) + (k0 + j) * LD];
 #pragma unroll
             for (int j = 0; j < 8; ++j) x[j] = prow || pcol ? base[j * step] : 0.0;
         }
@@ -1211,19 +1212,19 @@ __device__ __forceinline__ void potrf_core(int n, double* S, double* X, Sm& sm) 
         for (int q = w; q < nbk; q += NT / 32) {
             if (!kInv && q <= k) continue;
             const bool inX = q <= k;
-            const double* B = inX ? X + k0 + 8 * q * SLD : S + 8 * q + k0 * SLD;
-            const int bs = inX ? SLD : 1, bt = inX ? 1 : SLD;
+            const double* B = inX ? X + k0 + 8 * q * LD : S + 8 * q + k0 * LD;
+            const int bs = inX ? LD : 1, bt = inX ? 1 : LD;
             const double b0 = B[g * bs + t * bt], b1 = B[g * bs + (4 + t) * bt];
-            double* C = (inX ? X : S) + g + (8 * q + 2 * t) * SLD;
-            const double* A = S + g + (k0 + t) * SLD;
+            double* C = (inX ? X : S) + g + (8 * q + 2 * t) * LD;
+            const double* A = S + g + (k0 + t) * LD;
             int bi = inX ? k + 1 : q;
 #pragma unroll 4
             for (; bi < nbk; ++bi) {
-                double acc[2] = {-C[8 * bi], -C[8 * bi + SLD]};
+                double acc[2] = {-C[8 * bi], -C[8 * bi + LD]};
                 mma_f64(acc, A[8 * bi], b0);
-                mma_f64(acc, A[8 * bi + 4 * SLD], b1);
+                mma_f64(acc, A[8 * bi + 4 * LD], b1);
                 C[8 * bi] = -acc[0];
-                C[8 * bi + SLD] = -acc[1];
+                C[8 * bi + LD] = -acc[1];
             }
         }
         __syncthreads();

@@ -13,8 +13,9 @@
 //   k_finest_condition*     V_j and U_j of a chunk of at most 64 observations:
 //                           every observation conditions on its own, so the
 //                           chunks are as many as the chip needs
-//   k_finest_children       Sigma, L_Sigma, y~, B^ of one finest region of at most
-//                           64 observations, or of a sibling group of small ones
+//   (mra_small.cu)          Sigma, L_Sigma, y~, B^ of finest regions of at most 64
+//                           observations, sibling groups of small ones together
+//                           with their parent's posterior
 //   k_heavy_*               the same of larger finest regions in 64 x 64 tiles,
 //                           one CTA per tile, the block columns in turn
 //   k_finest_terms          log-lik terms summed per sibling group
@@ -139,122 +140,15 @@ __global__ void __launch_bounds__(kThreads, 2) k_finest_condition_any(DevTree<T>
 }
 
 // ---------------------------------------------------------------------------
-// the finest children of one level M-2 region, all at once
+// finest regions in FP32 storage (mixed path): one CTA per region, from a queue,
+// most expensive first
 // ---------------------------------------------------------------------------
-// Used when every child has at most 32 observations and the group at most 64
-// (T = double): one covariance block and one product form the whole group's
-// conditional covariance, one warp per child factors its diagonal block,
-// solves y~ and inverts its factor into a block-diagonal matrix, and one
-// product forms the whole group's B^ (in place: each 64-row tile of the
-// product reads exactly the rows it then writes, and the group fits one
-// column tile).  Returns the group's log-likelihood terms (thread 0).
-
-template <typename T>
-__device__ __noinline__ double finest_children_grouped(const Geom& g, const DevTree<T>& t, long clo, long chi,
-                                                       long lo, int np, T* ws, LaSmem<T>& sm) {
-    if constexpr (sizeof(T) != 8) {
-        return 0.0;
-    } else {
-        const long Lr = (long)t.L * t.r;
-        const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-        T* Sg = ws;                      // np x np conditional covariance of the group
-        T* Binv = ws + (long)np * np;    // np x np block-diagonal L_Sigma^{-1}
-        fill_cov<T>(g, t.pts, t.obs0 + lo, np, t.obs0 + lo, np, true, Sg, np, sm);
-        for (int e = tid; e < np * np; e += kThreads) Binv[e] = 0.0;
-        __syncthreads();
-        gemm<T, true, false>(np, np, (int)Lr, (T)-1, t.Ufin + lo * Lr, Lr, t.Ufin + lo * Lr, Lr, (T)1, Sg, np, sm);
-        constexpr int LD = kChildMax + 1;
-        double* Sw = &sm.A[0][0] + w * (kChildMax * LD);  // per-warp 32 x 33 (A and B tiles are contiguous)
-        double part = 0.0;
-        const long c = clo + w;
-        if (c < chi) {
-            const long o0 = t.obs_off[c];
-            const int n = (int)(t.obs_off[c + 1] - o0), q0 = (int)(o0 - lo);
-            if (n > 0) {
-                for (int e = lane; e < n * n; e += 32) {
-                    const int i = e % n, j = e / n;
-                    Sw[i + j * LD] = Sg[(q0 + i) + (long)(q0 + j) * np];
-                }
-                __syncwarp();
-                int bad = 0;
-                for (int k = 0; k < n; ++k) {  // lane i owns row i
-                    const double d = Sw[k + k * LD];
-                    __syncwarp();
-                    if (!(d > 0.0)) bad = 1;
-                    const double sq = sqrt(d);
-                    if (lane == k) Sw[k + k * LD] = sq;
-                    if (lane > k && lane < n) Sw[lane + k * LD] *= 1.0 / sq;
-                    __syncwarp();
-                    const double lik = lane < n ? Sw[lane + k * LD] : 0.0;
-                    for (int j = k + 1; j < n; ++j)  // uniform trip count across the warp
-                        if (lane >= j && lane < n) Sw[lane + j * LD] -= lik * Sw[j + k * LD];
-                    __syncwarp();
-                }
-                T* Lc = t.Lsig + t.lsig_off[c];
-                for (int e = lane; e < n * n; e += 32) {
-                    const int i = e % n, j = e / n;
-                    Lc[i + (long)j * n] = i >= j ? Sw[i + j * LD] : 0.0;
-                }
-                double ldp = lane < n ? log(Sw[lane + lane * LD]) : 0.0;
-                for (int o = 16; o > 0; o >>= 1) ldp += __shfl_xor_sync(0xffffffffu, ldp, o);
-                // y~ = L_Sigma^{-1} y: lane i ends holding x_i
-                double xl = 0.0;
-                for (int i = 0; i < n; ++i) {
-                    double sp = lane < i ? Sw[i + lane * LD] * xl : 0.0;
-                    for (int o = 16; o > 0; o >>= 1) sp += __shfl_xor_sync(0xffffffffu, sp, o);
-                    if (lane == i) xl = (t.y[o0 + i] - sp) / Sw[i + i * LD];
-                }
-                if (lane < n) t.yt[o0 + lane] = xl;
-                double yy = lane < n ? xl * xl : 0.0;
-                for (int o = 16; o > 0; o >>= 1) yy += __shfl_xor_sync(0xffffffffu, yy, o);
-                // column j of L_Sigma^{-1} by lane j, into the child's diagonal block
-                {
-                    // lanes walk the same rows and terms (X[k] = 0 above the
-                    // diagonal): no divergence, broadcast reads of L
-                    const int j = lane;
-                    double xs[kChildMax];  // column j of the inverse, in registers
-#pragma unroll
-                    for (int i = 0; i < kChildMax; ++i) xs[i] = 0.0;
-                    double* col = Binv + q0 + (long)(q0 + (j < n ? j : 0)) * np;
-                    for (int i = 0; i < n; ++i) {
-                        double v = 0.0;
-#pragma unroll
-                        for (int k = 0; k < kChildMax; ++k)
-                            if (k < i) v += Sw[i + k * LD] * xs[k];
-                        const double xi = i == j ? 1.0 / Sw[i + i * LD] : (i > j ? -v / Sw[i + i * LD] : 0.0);
-#pragma unroll
-                        for (int k = 0; k < kChildMax; ++k)
-                            if (k == i) xs[k] = xi;
-                        if (j < n && i >= j) col[i] = xi;
-                    }
-                }
-                part = yy + 2.0 * ldp;
-                if (bad && lane == 0) report_error(t.err, t.n_int + c);
-            }
-        }
-        __syncthreads();
-        if (lane == 0) sm.red[w] = part;
-        __syncthreads();
-        double tot = 0.0;
-        if (tid == 0)
-            for (int k = 0; k < kThreads / 32; ++k) tot += sm.red[k];
-        __syncthreads();
-        gemm<T, false, true, true>((int)Lr, np, np, (T)1, t.Bhat + lo * Lr, Lr, Binv, np, (T)0, t.Bhat + lo * Lr, Lr,
-                                   sm);
-        return tot;
-    }
-}
-
-// Work items: a value v < J^(M-2) is that sibling group, else the finest region
-// v - J^(M-2); most expensive first, from a queue.
-template <typename T>
-__global__ void __launch_bounds__(kThreads, 2) k_finest_children(Geom g, DevTree<T> t) {
-    LaSmem<T>& sm = la_smem<T>();
+__global__ void __launch_bounds__(kThreads, 2) k_finest_regions_f32(Geom g, DevTree<float> t) {
+    LaSmem<float>& sm = la_smem<float>();
     __shared__ long s_u;
-    const int L = t.L, m = t.M - 2;
+    const int L = t.L;
     const long Lr = (long)L * t.r;
-    const long s2 = level_start(t.J, m), cnt2 = level_count(t.J, m);
-    T* ws = t.ws + blockIdx.x * t.ws_stride;
+    const long cnt2 = level_count(t.J, t.M - 2);
     for (;;) {
         if (threadIdx.x == 0) {
             int q = atomicAdd(&t.queue[0], 1);
@@ -264,40 +158,21 @@ __global__ void __launch_bounds__(kThreads, 2) k_finest_children(Geom g, DevTree
         const long item = s_u;
         __syncthreads();
         if (item < 0) break;
-        if (item < cnt2) {
-            if (skipped(t, s2 + item)) continue;
-            const long clo = t.child_lo[item], chi = t.child_hi[item];
-            const long lo = t.obs_off[clo];
-            const double d = finest_children_grouped<T>(g, t, clo, chi, lo, (int)(t.obs_off[chi] - lo), ws, sm);
-            if (threadIdx.x == 0) t.dchild[clo] = d;
-            __syncthreads();
-            continue;
-        }
         const long c = item - cnt2;
         if (skipped(t, (long)t.fin_anc[c * L + L - 1])) continue;
         const long o0 = t.obs_off[c];
         const int n = (int)(t.obs_off[c + 1] - o0);
-        T* S = t.Lsig + t.lsig_off[c];
-        fill_cov<T>(g, t.pts, t.obs0 + o0, n, t.obs0 + o0, n, true, S, n, sm);
+        float* S = t.Lsig + t.lsig_off[c];
+        fill_cov<float>(g, t.pts, t.obs0 + o0, n, t.obs0 + o0, n, true, S, n, sm);
         __syncthreads();
-        gemm<T, true, false>(n, n, (int)Lr, (T)-1, t.Ufin + o0 * Lr, Lr, t.Ufin + o0 * Lr, Lr, (T)1, S, n, sm);
+        gemm<float, true, false>(n, n, (int)Lr, -1.f, t.Ufin + o0 * Lr, Lr, t.Ufin + o0 * Lr, Lr, 1.f, S, n, sm);
         double ld = 0.0;
-        constexpr bool small = sizeof(T) == 8;  // FP64 items hold at most 64 observations
-        T* Sinv = ws;  // n x n
-        int info = potrf_lower<T>(n, S, n, sm, &ld, small ? Sinv : nullptr, n);
+        int info = potrf_lower<float>(n, S, n, sm, &ld);
         double* ytc = t.yt + o0;
         for (int e = threadIdx.x; e < n; e += kThreads) ytc[e] = t.y[o0 + e];
         __syncthreads();
-        if constexpr (small) {
-            trmv_lower_inv<T>(n, Sinv, n, ytc, ytc);  // y~ = L_Sigma^{-1} y
-            // B^ = V L_Sigma^{-T}, in place: each 64-row tile of the product
-            // reads exactly the rows it then writes
-            gemm<T, false, true, true>((int)Lr, n, n, (T)1, t.Bhat + o0 * Lr, Lr, Sinv, n, (T)0, t.Bhat + o0 * Lr, Lr,
-                                       sm);
-        } else {
-            trsv_lower_f64<T>(n, S, n, ytc);
-            trsm_right_lower_trans<T>((int)Lr, n, S, n, t.Bhat + o0 * Lr, Lr, sm);
-        }
+        trsv_lower_f64<float>(n, S, n, ytc);
+        trsm_right_lower_trans<float>((int)Lr, n, S, n, t.Bhat + o0 * Lr, Lr, sm);
         double part = 0.0;
         for (int e = threadIdx.x; e < n; e += kThreads) part += ytc[e] * ytc[e];
         double yy = cta_sum(part, sm);
@@ -453,7 +328,7 @@ static void launch_condition(const DevTree<double>& t, cudaStream_t st) {
 }
 
 template <typename T>
-int launch_finest(const Geom& g, const DevTree<T>& t, int grid, cudaStream_t st, const Fork& fk) {
+int launch_finest(const Geom& g, const DevTree<T>& t, int grid, bool keep, cudaStream_t st, const Fork& fk) {
     int launches = 0;
     if (t.n_chunks > 0) {
         launch_cov_finest<T>(g, t, st);
@@ -488,8 +363,10 @@ int launch_finest(const Geom& g, const DevTree<T>& t, int grid, cudaStream_t st,
             cudaEventRecord(fk.join, fk.side);
         }
     }
-    if (t.n_fin_items > 0) {
-        k_finest_children<T><<<(unsigned)(t.n_fin_items < grid ? t.n_fin_items : grid), kThreads, sizeof(LaSmem<T>),
+    if constexpr (sizeof(T) == 8) {
+        launches += launch_finest_small(g, t, keep, st);
+    } else if (t.n_fin_items > 0) {
+        k_finest_regions_f32<<<(unsigned)(t.n_fin_items < grid ? t.n_fin_items : grid), kThreads, sizeof(LaSmem<T>),
                                st>>>(g, t);
         ++launches;
     }
@@ -513,17 +390,17 @@ cudaError_t prepare_finest() {
     set((const void*)k_finest_condition<64, false>, sizeof(CondSmem<64>));
     set((const void*)k_finest_condition_any<double>, sizeof(LaSmem<double>));
     set((const void*)k_finest_condition_any<float>, sizeof(LaSmem<float>));
-    set((const void*)k_finest_children<double>, sizeof(LaSmem<double>));
-    set((const void*)k_finest_children<float>, sizeof(LaSmem<float>));
+    set((const void*)k_finest_regions_f32, sizeof(LaSmem<float>));
     set((const void*)k_heavy_sigma, sizeof(LaSmem<double>));
     set((const void*)k_heavy_column, sizeof(LaSmem<double>));
     set((const void*)k_heavy_panel, sizeof(LaSmem<double>));
+    if (e == cudaSuccess) e = prepare_finest_small();
     return e;
 }
 
 cudaError_t set_gemm_tiles_finest(const int nw[3]) { return cudaMemcpyToSymbol(c_gemm_nw, nw, 3 * sizeof(int)); }
 
-template int launch_finest<double>(const Geom&, const DevTree<double>&, int, cudaStream_t, const Fork&);
-template int launch_finest<float>(const Geom&, const DevTree<float>&, int, cudaStream_t, const Fork&);
+template int launch_finest<double>(const Geom&, const DevTree<double>&, int, bool, cudaStream_t, const Fork&);
+template int launch_finest<float>(const Geom&, const DevTree<float>&, int, bool, cudaStream_t, const Fork&);
 
 }  // namespace mra

@@ -45,9 +45,10 @@ struct DevTree {
     const int64_t* child_hi;   // one past the last
     const FinChunk* chunks;    // [n_chunks] runs of observations conditioned together
     long n_chunks;
-    const int64_t* fin_items;  // [n_fin_items] small finest regions, most expensive first: a value v < J^(M-2)
-                               // is the sibling group v, else the finest region v - J^(M-2)
-    long n_fin_items;
+    const int64_t* fin_items;  // [n_fin_items] small finest regions: a value v < J^(M-2) is the sibling group v,
+                               // else the finest region v - J^(M-2); FP64: by tile class (64, 32, 16), each most
+                               // expensive first
+    long n_fin_items, n_fin_class[3];
     const int64_t* heavy;      // [n_heavy] finest regions of more than 64 observations (FP64), largest first
     long n_heavy;
     const HeavyTile* heavy_tiles;  // [n_heavy_tiles] lower tiles of their Sigma
@@ -56,6 +57,8 @@ struct DevTree {
     const int64_t* post_order; // [n_int] per level m, at level_start(m): the level's regions (local index), its
                                // n_dense[m] dense ones first, each kind most expensive step first
     long n_dense[kMaxLevels];
+    long n_fused;              // last factored regions of level M-2 in post_order whose posterior (outside
+                               // prediction) comes with their finest group
     const int8_t* factored;    // [n_int] 1: the region's posterior output is kept as F, f
     const int8_t* active;      // [n_int] sub-tree sharding: 0 = the region belongs to another rank's
                                // sub-tree and is skipped; nullptr: every region is computed
@@ -191,7 +194,10 @@ struct Fork {
 };
 // The finest level (without the level M-2 posterior); returns the number of kernels launched.
 template <typename T>
-int launch_finest(const Geom& g, const DevTree<T>& t, int grid, cudaStream_t st, const Fork& fk);
+int launch_finest(const Geom& g, const DevTree<T>& t, int grid, bool keep, cudaStream_t st, const Fork& fk);
+// its small regions (FP64), with the posterior of groups taken whole unless `keep`
+int launch_finest_small(const Geom& g, const DevTree<double>& t, bool keep, cudaStream_t st);
+cudaError_t prepare_finest_small();
 cudaError_t prepare_finest();
 cudaError_t set_gemm_tiles_finest(const int nw[3]);
 // One posterior level (FP64): its dense regions in chunks whose scratch fits

@@ -126,7 +126,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_posterior_factored(DevTree<doub
     LaSmem<double>& sm = la_smem<double>();
     const int r = t.r;
     const long mr1 = (long)(m + 1) * r;
-    const long s0 = level_start(t.J, m), nd = t.n_dense[m], cnt = level_count(t.J, m);
+    const long s0 = level_start(t.J, m), nd = t.n_dense[m];
+    const long cnt = level_count(t.J, m) - (m == t.M - 2 && !keep ? t.n_fused : 0);
     double* ws = t.ws + blockIdx.x * t.ws_stride;
     double* wsd = t.wsd + blockIdx.x * t.wsd_stride;
     // the children's rows: B^, y~ of the finest level, else F, f of the level below
@@ -403,7 +404,7 @@ static int launch_dense(const DevTree<double>& t, int m, bool keep, cudaStream_t
 }
 
 int launch_posterior_level(const DevTree<double>& t, int m, int grid, bool keep, cudaStream_t st, const Fork& fk) {
-    const long nf = level_count(t.J, m) - t.n_dense[m];
+    const long nf = level_count(t.J, m) - t.n_dense[m] - (m == t.M - 2 && !keep ? t.n_fused : 0);
     int launches = 0;
     // factored regions beside the dense ones (both need only the level below)
     const bool both = nf > 0 && t.n_dense[m] > 0;
