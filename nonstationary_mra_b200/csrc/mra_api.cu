@@ -314,7 +314,8 @@ mra_status run_eval(mra_ctx* c, bool predict) {
         switch (l.kind) {
             case MRA_KERNEL_FIELDS:
                 launch_fields(c->geom, c->fp, td.pts.c0, td.pts.c1, td.pts.c2, np_all, const_cast<double*>(td.pts.s2),
-                              const_cast<double*>(td.pts.beta), const_cast<double*>(td.pts.t2), st);
+                              const_cast<double*>(td.pts.beta), const_cast<double*>(td.pts.t2),
+                              const_cast<double*>(td.pts.ss), st);
                 launched += 1;
                 break;
             case MRA_KERNEL_PRIOR_LEVEL: {
@@ -468,6 +469,8 @@ mra_status setup_tree(mra_ctx* c, DevTree<T>& t, const HostTree& h, const PointS
     const long rr = (long)r * r;
     cudaError_t ce = cudaSuccess;
     t.J = J; t.M = M; t.r = r; t.L = L; t.tf = c->tf;
+    t.lj = J == 4 ? 2 : 1;
+    for (int m = 0; m < kMaxLevels; ++m) t.lstart[m] = m <= M - 2 ? (int)level_start(J, m) : 0;
     t.n_int = c->n_int; t.n_fin = c->n_fin; t.n_obs = c->n_obs; t.n_pred = c->n_pred;
     t.obs0 = c->n_int * r;
     t.pred0 = c->n_int * r + c->n_obs;
@@ -906,13 +909,15 @@ mra_status mra_create(const mra_structure* s, const mra_model* m, int32_t precis
     cudaError_t ce = cudaSuccess;
     const long np_all = n_int * r + n_obs + n_pred;
     double* pc[3];
-    double* fields[3];
+    double* fields[4];
     for (int d = 0; d < 3; ++d) {
         pc[d] = c->alloc<double>(np_all, &ce);
         if (ce) return bail(fail(MRA_ERR_OOM, "device allocation failed: coordinates"));
         fields[d] = c->alloc<double>(np_all, &ce);
         if (ce) return bail(fail(MRA_ERR_OOM, "device allocation failed: fields"));
     }
+    fields[3] = c->alloc<double>(np_all, &ce);
+    if (ce) return bail(fail(MRA_ERR_OOM, "device allocation failed: fields"));
     double* y = c->alloc<double>(n_obs, &ce);
     if (ce) return bail(fail(MRA_ERR_OOM, "device allocation failed: y"));
     const std::vector<int64_t>* tabs[14] = {&h.obs_off, &h.pred_off, &h.fin_anc, &h.pred_order, &h.lsig_off,
@@ -948,7 +953,7 @@ mra_status mra_create(const mra_structure* s, const mra_model* m, int32_t precis
     c->fp.basis = m->basis;
     c->fp.basis_len = m->basis_len;
     c->fp.theta = c->d_theta;
-    PointSet pts{pc[0], pc[1], pc[2], fields[0], fields[1], fields[2]};
+    PointSet pts{pc[0], pc[1], pc[2], fields[0], fields[1], fields[2], fields[3]};
     Shared sh{};
     sh.yt = c->alloc<double>(n_obs, &ce);
     if (!ce) sh.ldprior = c->alloc<double>(n_int, &ce);
@@ -1397,7 +1402,9 @@ mra_status mra_sample_prior(mra_ctx* c, const double* z_int, const double* z_obs
 static mra_status eval_points(const mra_model* m, const mra_theta* th, const double* p, uint64_t n,
                               std::vector<void*>& frees, PointSet* ps, cudaStream_t st) {
     Geom g = make_geom(m);
-    double *c[3], *f[3];
+    double *c[3], *f[4];
+    CU(cudaMalloc(&f[3], std::max<uint64_t>(n, 1) * sizeof(double)));
+    frees.push_back(f[3]);
     for (int d = 0; d < 3; ++d) {
         CU(cudaMalloc(&c[d], std::max<uint64_t>(n, 1) * sizeof(double)));
         frees.push_back(c[d]);
@@ -1433,8 +1440,8 @@ static mra_status eval_points(const mra_model* m, const mra_theta* th, const dou
     }
     CU(cudaMemcpyAsync(dth, v, sizeof(v), cudaMemcpyHostToDevice, st));
     fp.theta = dth;
-    launch_fields(g, fp, c[0], c[1], c[2], (long)n, f[0], f[1], f[2], st);
-    *ps = PointSet{c[0], c[1], c[2], f[0], f[1], f[2]};
+    launch_fields(g, fp, c[0], c[1], c[2], (long)n, f[0], f[1], f[2], f[3], st);
+    *ps = PointSet{c[0], c[1], c[2], f[0], f[1], f[2], f[3]};
     return MRA_OK;
 }
 
@@ -1477,20 +1484,20 @@ mra_status mra_eval_covariance(const mra_model* m, const mra_theta* th, const do
                 launch_cov_block(make_geom(m), a, 0, (int)n1, 0, (int)n1, true, d, 0);
             } else {
                 // one point set with both: set 2 rows, set 1 columns (out[i1*n2 + i2])
-                double* cc[6];
-                for (int q = 0; q < 6 && e == cudaSuccess; ++q) {
+                double* cc[7];
+                for (int q = 0; q < 7 && e == cudaSuccess; ++q) {
                     e = cudaMalloc(&cc[q], std::max<uint64_t>(n1 + n2, 1) * sizeof(double));
                     if (e == cudaSuccess) frees.push_back(cc[q]);
                 }
-                const double* srcA[6] = {a.c0, a.c1, a.c2, a.s2, a.beta, a.t2};
-                const double* srcB[6] = {b.c0, b.c1, b.c2, b.s2, b.beta, b.t2};
-                for (int q = 0; q < 6 && e == cudaSuccess; ++q) {
+                const double* srcA[7] = {a.c0, a.c1, a.c2, a.s2, a.beta, a.t2, a.ss};
+                const double* srcB[7] = {b.c0, b.c1, b.c2, b.s2, b.beta, b.t2, b.ss};
+                for (int q = 0; q < 7 && e == cudaSuccess; ++q) {
                     if (n2) e = cudaMemcpy(cc[q], srcB[q], n2 * sizeof(double), cudaMemcpyDeviceToDevice);
                     if (e == cudaSuccess && n1)
                         e = cudaMemcpy(cc[q] + n2, srcA[q], n1 * sizeof(double), cudaMemcpyDeviceToDevice);
                 }
                 if (e == cudaSuccess) {
-                    PointSet both{cc[0], cc[1], cc[2], cc[3], cc[4], cc[5]};
+                    PointSet both{cc[0], cc[1], cc[2], cc[3], cc[4], cc[5], cc[6]};
                     launch_cov_block(make_geom(m), both, 0, (int)n2, (long)n2, (int)n1, false, d, 0);
                 }
             }

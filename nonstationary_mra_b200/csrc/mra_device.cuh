@@ -18,6 +18,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 namespace mra {
 
 constexpr int kThreads = 256;   // every region kernel runs 256-thread CTAs
@@ -112,7 +114,7 @@ __device__ __forceinline__ float cov_entry_f(const Geom& g, const Pt& p1, float 
 }
 
 // A point set laid out SoA: coordinates c0/c1/c2 and fields s2 (sigma^2),
-// beta, t2 (tau^2), all indexed by the same global point index.
+// beta, t2 (tau^2), ss (sigma), all indexed by the same global point index.
 struct PointSet {
     const double* c0;
     const double* c1;
@@ -120,6 +122,7 @@ struct PointSet {
     const double* s2;
     const double* beta;
     const double* t2;
+    const double* ss;
     __device__ __forceinline__ Pt pt(long i) const { return Pt{c0[i], c1[i], c2[i]}; }
 };
 
@@ -203,114 +206,105 @@ __device__ __forceinline__ LaSmem<T>& la_smem() {
     return *reinterpret_cast<LaSmem<T>*>(la_dyn_smem);
 }
 
-// ---- branch-free FP64 elementary functions for the covariance entries ----
-// e^{-s} for s >= 0 (s clamped at 700, where the result is below 1e-304):
-// Cody-Waite reduction s = n ln2 + r, |r| <= ln2/2, with ln2 split in a
-// 32-bit head (n * head exact) and a tail; e^{-r} from its Taylor polynomial
-// of degree 13 in Horner form (truncation below 5e-18 relative); 2^{-n} built
-// in the exponent field.  Within 1 ulp of exp(-s) on this range (checked on
-// 4M arguments against the CUDA library).
+// ---- FP64 elementary functions of the covariance entries ----
+// The fills are bound by instruction issue and the FP64 pipe, so the entry is
+// written for few instructions of both kinds: coefficients come from constant
+// memory (a DFMA reads them there; as immediates they cost two moves each), range
+// checks and exponents are integer operations on the high word, and one inverse
+// square root serves the distance and the prefactor.  Per entry of a 32-lane warp 155 -> 98
+// instructions issued; blocks of 1,024 regions of 64 knots with 5 ancestors: 144 ->
+// 109 us (230 G entries/s).
+static __constant__ double c_exp[15] = {
+    1.4426950408889634,      // 1 / ln 2
+    6755399441055744.0,      // 1.5 * 2^52: rounds to an integer in the low word
+    0.6931471803691238,      // ln 2, 32-bit head (n * head exact)
+    1.9082149292705877e-10,  // and tail
+    1.6059043836821613e-10, 2.08767569878681e-09, 2.505210838544172e-08, 2.755731922398589e-07,
+    2.7557319223985893e-06, 2.48015873015873e-05, 0.0001984126984126984, 0.001388888888888889,
+    0.008333333333333333, 0.041666666666666664, 0.16666666666666666};  // 1/13! .. 1/3!
+
+__device__ __forceinline__ unsigned hi_word(double x) { return (unsigned)__double2hiint(x); }
+
+// e^{-s} for s >= 0: Cody-Waite reduction s = n ln2 + r, |r| <= ln2/2; e^{-r} from
+// its Taylor polynomial of degree 13 in Horner form (truncation below 5e-18
+// relative); 2^{-n} added to the exponent field.  s is taken as at most 700.25 (the
+// result is then below 1e-303).  Within 1 ulp of exp(-s) on this range.
 __device__ __forceinline__ double exp_neg(double s) {
-    s = fmin(s, 700.0);
-    const double kShift = 6755399441055744.0;  // 1.5 * 2^52: rounds s/ln2 to an integer in the low word
-    const double t = fma(s, 1.4426950408889634, kShift);
-    const double n = t - kShift;
-    double r = fma(-n, 0.6931471803691238, s);
-    r = fma(-n, 1.9082149292705877e-10, r);
-    const double u = -r;
-    double p = 1.6059043836821613e-10;  // 1/13!
-    p = fma(p, u, 2.08767569878681e-09);
-    p = fma(p, u, 2.505210838544172e-08);
-    p = fma(p, u, 2.755731922398589e-07);
-    p = fma(p, u, 2.7557319223985893e-06);
-    p = fma(p, u, 2.48015873015873e-05);
-    p = fma(p, u, 0.0001984126984126984);
-    p = fma(p, u, 0.001388888888888889);
-    p = fma(p, u, 0.008333333333333333);
-    p = fma(p, u, 0.041666666666666664);
-    p = fma(p, u, 0.16666666666666666);
+    s = __hiloint2double((int)min(hi_word(s), 0x4085E000u), __double2loint(s));
+    const double t = fma(s, c_exp[0], c_exp[1]);
+    const double n = t - c_exp[1];
+    double u = fma(n, c_exp[2], -s);
+    u = fma(n, c_exp[3], u);  // -r
+    double p = c_exp[4];
+#pragma unroll
+    for (int k = 5; k < 15; ++k) p = fma(p, u, c_exp[k]);
     p = fma(p, u, 0.5);
     p = fma(p, u, 1.0);
     p = fma(p, u, 1.0);
-    return p * __hiloint2double((1023 - __double2loint(t)) << 20, 0);
+    return __hiloint2double(__double2hiint(p) - (__double2loint(t) << 20), __double2loint(p));
 }
 
-// 1/s from the PTX approximation refined by one third-order Newton step
-// (y <- y (1 + e + e^2), e = 1 - s y); s positive and normal.
-__device__ __forceinline__ double rcp_nr(double s) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(s));
-    const double e = fma(-s, y, 1.0);
-    return fma(y, fma(e, e, e), y);
-}
-
-// 1/sqrt(x) from the PTX approximation refined by one third-order Newton step
-// (y <- y (1 + e/2 + 3e^2/8), e = 1 - x y^2); x positive and normal.
-__device__ __forceinline__ double rsqrt_nr(double x) {
-    double y;
-    asm("rsqrt.approx.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x * y, y, 1.0);
-    return fma(y * e, fma(0.375, e, 0.5), y);
-}
-
-// The same two quantities seeded by the single-precision approximations
-// (rcp.approx.ftz.f32 / rsqrt.approx.ftz.f32 of the argument rounded to FP32,
-// relative error near 2^-23) and refined by the same third-order Newton step,
-// whose cubic convergence takes the seed error below 2^-66: the result is within
-// an ulp or two of the FP64-seeded form.  The FP32 units issue these far faster
-// than the FP64 approximations; arguments outside [1e-30, 1e30], where the FP32
-// seed would underflow or overflow, take the FP64-seeded path.
-__device__ __forceinline__ double rcp_fast(double s) {
-    if (!(s > 1e-30 && s < 1e30)) return rcp_nr(s);
-    float yf;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(__double2float_rn(s)));
-    const double y = (double)yf;
-    const double e = fma(-s, y, 1.0);
-    return fma(y, fma(e, e, e), y);
-}
-
-__device__ __forceinline__ double rsqrt_fast(double x) {
-    if (!(x > 1e-30 && x < 1e30)) return rsqrt_nr(x);
+// 1/sqrt(x): the single-precision approximation (relative error near 2^-23) refined
+// by one third-order Householder step y (1 + e/2 + 3 e^2/8), e = 1 - x y^2, which
+// takes the error below 2^-66: within an ulp of the exact value.  x must be in
+// [2^-100, 2^100) (rsqrt_ok), where the single-precision seed is normal.
+__device__ __forceinline__ bool rsqrt_ok(double x) { return hi_word(x) - 0x39B00000u < 0x0C800000u; }
+__device__ __forceinline__ double rsqrt_seeded(double x) {
     float yf;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(__double2float_rn(x)));
     const double y = (double)yf;
-    const double e = fma(-x * y, y, 1.0);
+    const double s = x * y;  // e = 1 - x y^2 with the rounding of x y taken back: the distance enters an exponential
+    const double e = fma(-fma(x, y, -s), y, fma(-s, y, 1.0));
     return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
-// One nonstationary straight-line entry from per-point quantities (see
-// fill_row_fast): row point (pc, ga, ca = sqrt(s1) b1 / scale^2 for PREF 1;
-// ssa, ba_h = b1 / scale^2 for PREF 0), column point (q, gq, ssbq = sqrt(s2) b2;
-// ssq, bq).  F32SEED: reciprocal and inverse square root seeded in FP32
-// (rcp_fast / rsqrt_fast; more independent work per issue slot, for launches
-// that are issue-bound) or in FP64 (rcp_nr / rsqrt_nr; shorter dependent
-// chains, for fills that are latency-bound inside the region kernels).
-template <int NU, int PREF, bool F32SEED = false>
+// One nonstationary straight-line entry from per-point quantities (sqrt(s1 s2)
+// pre(x) matern(h), x = 2 b1 b2 / (b1^2 + b2^2), h = scale sqrt(2 d^2 / (b1^2 + b2^2))):
+// with g = b^2 / (2 scale^2) per point and b = g1 + g2, h = sqrt(d^2 / b) and x =
+// b1 b2 / (scale^2 b).  q = 1/sqrt(d^2 b) gives h = d^2 q and 1/b = h q, refined by
+// one Newton step.  Row point (pc, ga, ca = sqrt(s1) b1 / scale^2 for PREF 1; ssa,
+// ba_h = b1 / scale^2 for PREF 0), column point (q*, gq, ssbq = sqrt(s2) b2; ssq,
+// bq).  NU: 1 exponential, 3 Matern 3/2; PREF: 0 prefactor x^1.5, 1 prefactor x;
+// PLANAR: no third coordinate.  SAFE = false sets `bad` where an argument is out of
+// rsqrt_seeded's range (coincident points, extreme scales, NaN) and the caller takes
+// the SAFE form: tested once per batch of entries, so that the entries' dependent
+// chains interleave (a branch in each entry serialised them, 125 us where this form
+// takes 109).
+template <int NU, int PREF, bool PLANAR, bool SAFE>
 __device__ __forceinline__ double cov_fast_entry(double pc0, double pc1, double pc2, double ga, double ca,
                                                  double ssa, double ba_h, double qx, double qy, double qz, double gq,
-                                                 double ssbq, double ssq, double bq) {
-    const double dx = qx - pc0, dy = qy - pc1, dz = qz - pc2;
-    const double d2 = fma(dx, dx, fma(dy, dy, dz * dz));
-    const double w = F32SEED ? rcp_fast(ga + gq) : rcp_nr(ga + gq);  // 2 scale^2 / (b1^2 + b2^2)
-    const double u = d2 * w;                                            // h^2
-    const double h = u > 1e-300 ? u * (F32SEED ? rsqrt_fast(u) : rsqrt_nr(u)) : 0.0;
+                                                 double ssbq, double ssq, double bq, bool& bad) {
+    const double dx = qx - pc0, dy = qy - pc1;
+    double d2 = dy * dy;
+    if (!PLANAR) {
+        const double dz = qz - pc2;
+        d2 = fma(dz, dz, d2);
+    }
+    d2 = fma(dx, dx, d2);
+    const double b = ga + gq;
+    double h, w;
+    if (SAFE) {
+        w = 1.0 / b;
+        h = sqrt(d2 * w);
+    } else {
+        const double z = d2 * b;
+        bad = bad || !rsqrt_ok(z);
+        const double q = rsqrt_seeded(z);
+        h = d2 * q;
+        w = h * q;
+        w = fma(w, fma(-b, w, 1.0), w);
+    }
     const double em = exp_neg(h);
-    const double m = NU == 3 ? (1.0 + h) * em : em;
+    const double m = NU == 3 ? fma(h, em, em) : em;
     if (PREF == 1) return (ca * ssbq) * w * m;
     const double x = ba_h * bq * w;
-    return (ssa * ssq) * (x * sqrt(x)) * m;
+    if (!SAFE) bad = bad || !rsqrt_ok(x);
+    const double sx = SAFE ? sqrt(x) : x * rsqrt_seeded(x);
+    return (ssa * ssq) * (x * sx) * m;
 }
 
 // One row point against the staged column points q_begin, q_begin + q_step,
 // ... < q_end (straight-line distance, nonstationary): writes ob[(qoff + q) ld].
-// NU: 1 exponential, 3 Matern 3/2; PREF: 0 prefactor x^1.5, 1 prefactor x.
-// Entry: sqrt(s1 s2) pre(x) matern(h), x = 2 b1 b2 / (b1^2 + b2^2),
-// h = scale sqrt(2 d^2 / (b1^2 + b2^2)).  With g = b^2 / (2 scale^2) staged per
-// point, w = 1 / (g1 + g2) gives h = sqrt(d^2 w) and x = b1 b2 w / scale^2,
-// so the entry is (sqrt(s1) b1 / scale^2) (sqrt(s2) b2) w matern(h) for
-// PREF 1.  Every parameter is in registers so the loop carries no reloads;
-// one reciprocal, one inverse square root and one exponential per entry,
-// none with a branch.
 template <typename T, int NU, int PREF>
 __device__ __noinline__ void fill_row_fast(const double* __restrict__ sx, const double* __restrict__ sy,
                                            const double* __restrict__ sz, const double* __restrict__ ss,
@@ -319,12 +313,24 @@ __device__ __noinline__ void fill_row_fast(const double* __restrict__ sx, const 
                                            double ssa, double ba, double ga, double ihs2, int q_begin, int q_end,
                                            int q_step, int qoff, T* __restrict__ ob, long ld) {
     const double ca = ssa * ba * ihs2, ba_h = ba * ihs2;
-#pragma unroll 4
-    for (int q = q_begin; q < q_end; q += q_step) {
-        const double v = cov_fast_entry<NU, PREF>(pc0, pc1, pc2, ga, ca, ssa, ba_h, sx[q], sy[q], sz[q], sg[q],
-                                                  PREF == 1 ? ssb[q] : 0.0, PREF == 1 ? 0.0 : ss[q],
-                                                  PREF == 1 ? 0.0 : sb[q]);
-        ob[(long)(qoff + q) * ld] = (T)v;
+    for (int q = q_begin; q < q_end; q += 4 * q_step) {
+        double v[4];
+        bool bad = false;
+        auto entry = [&](int k, auto safe) {
+            const int e = q + k * q_step < q_end ? q + k * q_step : q;
+            v[k] = cov_fast_entry<NU, PREF, false, decltype(safe)::value>(
+                pc0, pc1, pc2, ga, ca, ssa, ba_h, sx[e], sy[e], sz[e], sg[e], PREF == 1 ? ssb[e] : 0.0,
+                PREF == 1 ? 0.0 : ss[e], PREF == 1 ? 0.0 : sb[e], bad);
+        };
+#pragma unroll
+        for (int k = 0; k < 4; ++k) entry(k, std::false_type());
+        if (bad) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) entry(k, std::true_type());
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (q + k * q_step < q_end) ob[(long)(qoff + q + k * q_step) * ld] = (T)v[k];
     }
 }
 
@@ -372,7 +378,7 @@ __device__ __noinline__ void fill_cov_staged(const Geom& g, const PointSet& P, c
             sx[e] = P.c0[ib];
             sy[e] = P.c1[ib];
             sz[e] = P.c2[ib];
-            ss[e] = fast ? sqrt(P.s2[ib]) : P.s2[ib];
+            ss[e] = fast ? P.ss[ib] : P.s2[ib];
             const double bb = P.beta[ib];
             sb[e] = bb;
             if (fast) {
@@ -389,7 +395,7 @@ __device__ __noinline__ void fill_cov_staged(const Geom& g, const PointSet& P, c
                 T* ob = out + kb * blk + t;
                 const double pc0 = P.c0[ia], pc1 = P.c1[ia], pc2 = P.c2[ia];
                 const double sa = P.s2[ia], ba = P.beta[ia];
-                const double ssa = sqrt(sa), ga = ba * ba * ih2;
+                const double ssa = P.ss[ia], ga = ba * ba * ih2;
                 if (nu == 3 && pk == 1)
                     fill_row_fast<T, 3, 1>(sx, sy, sz, ss, sb, sg, ssb, pc0, pc1, pc2, ssa, ba, ga, ihs2, tq, qn, cols,
                                            q0, ob, ld);
@@ -446,23 +452,22 @@ __device__ inline void fill_cov(const Geom& g, const PointSet& P, long a0, int n
 }
 
 constexpr int kCovThreads = 256;
-constexpr int kCovChunk = 64;  // column points staged per chunk (7 x 64 doubles of shared memory)
+constexpr int kCovChunk = 64;  // column points staged per chunk (7 x 64 doubles of shared memory, 16-byte aligned)
 
-// The straight-line nonstationary FP64 block: one row point per thread with its
-// parameters in registers, the column points staged in chunks, entries of
-// cov_fast_entry (the same arithmetic as fill_row_fast).
-template <typename T, int NU, int PREF>
-__device__ __forceinline__ void cov_block_fast(const PointSet& P, long a0, int nr, long b0, int nc, bool self,
+// The straight-line nonstationary FP64 block: two row points per thread with their
+// parameters in registers, the column points staged in chunks as pairs (x, y), (z,
+// g), (sqrt(s2) b or sqrt(s2), b), which both rows read.
+// self: row t is the point of column t + doff.
+template <typename T, int NU, int PREF, bool PLANAR>
+__device__ __forceinline__ void cov_block_fast(const PointSet& P, long a0, int nr, long b0, int nc, bool self, int doff,
                                                T* __restrict__ out, long ld, double ih2, double ihs2,
                                                double* stage) {
-    double* sx = stage;
-    double* sy = sx + kCovChunk;
-    double* sz = sy + kCovChunk;
-    double* sg = sz + kCovChunk;
-    double* s4 = sg + kCovChunk;  // sqrt(s2) b (PREF 1) or sqrt(s2) (PREF 0)
-    double* s5 = s4 + kCovChunk;  // b (PREF 0)
+    double2* sxy = reinterpret_cast<double2*>(stage);
+    double2* szg = sxy + kCovChunk;
+    double2* s45 = szg + kCovChunk;
     const int tid = threadIdx.x, nt = blockDim.x;
-    const int rows = nr < nt ? nr : nt;
+    const int half = (nr + 1) / 2;
+    const int rows = half < nt ? half : nt;
     const int cols = nt / rows;
     const bool worker = tid < rows * cols;
     const int tr = tid % rows, tc = tid / rows;
@@ -471,40 +476,73 @@ __device__ __forceinline__ void cov_block_fast(const PointSet& P, long a0, int n
         __syncthreads();
         for (int e = tid; e < qn; e += nt) {
             const long ib = b0 + q0 + e;
-            const double bb = P.beta[ib], ssq = sqrt(P.s2[ib]);
-            sx[e] = P.c0[ib];
-            sy[e] = P.c1[ib];
-            sz[e] = P.c2[ib];
-            sg[e] = bb * bb * ih2;
-            s4[e] = PREF == 1 ? ssq * bb : ssq;
-            s5[e] = bb;
+            const double bb = P.beta[ib], ssq = P.ss[ib];
+            sxy[e] = make_double2(P.c0[ib], P.c1[ib]);
+            szg[e] = make_double2(PLANAR ? 0.0 : P.c2[ib], bb * bb * ih2);
+            s45[e] = make_double2(PREF == 1 ? ssq * bb : ssq, bb);
         }
         __syncthreads();
         if (!worker) continue;
-        for (int t = tr; t < nr; t += rows) {
-            const long ia = a0 + t;
-            const double pc0 = P.c0[ia], pc1 = P.c1[ia], pc2 = P.c2[ia], sa = P.s2[ia], ba = P.beta[ia];
-            const double ssa = sqrt(sa), ga = ba * ba * ih2, ca = ssa * ba * ihs2, ba_h = ba * ihs2;
-            const double diag = self ? sa + P.t2[ia] : 0.0;
-            T* ob = out + t;
-#pragma unroll 4
-            for (int q = tc; q < qn; q += cols) {
-                const int qq = q0 + q;
-                double v = cov_fast_entry<NU, PREF, true>(pc0, pc1, pc2, ga, ca, ssa, ba_h, sx[q], sy[q], sz[q], sg[q],
-                                                    PREF == 1 ? s4[q] : 0.0, PREF == 1 ? 0.0 : s4[q],
-                                                    PREF == 1 ? 0.0 : s5[q]);
-                if (self && t == qq) v = diag;  // sigma^2 + tau^2 (evaluate_covariance.cpp:103,307)
-                ob[(long)qq * ld] = (T)v;
+        for (int t = tr; t < half; t += rows) {
+            const bool two = t + half < nr;
+            double pc0[2], pc1[2], pc2[2], ga[2], ca[2], ssa[2], bh[2], diag[2];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const long ia = a0 + t + (k && two ? half : 0);
+                const double ba = P.beta[ia];
+                pc0[k] = P.c0[ia];
+                pc1[k] = P.c1[ia];
+                pc2[k] = PLANAR ? 0.0 : P.c2[ia];
+                ssa[k] = P.ss[ia];
+                ga[k] = ba * ba * ih2;
+                bh[k] = ba * ihs2;
+                ca[k] = ssa[k] * bh[k];
+                diag[k] = self ? P.s2[ia] + P.t2[ia] : 0.0;
+            }
+            T* ob = out + t + (long)(q0 + tc) * ld;
+            const long step = (long)cols * ld;
+            for (int q = tc; q < qn; q += 2 * cols, ob += 2 * step) {
+                const int qb = q + cols < qn ? q + cols : q;  // two columns at a time: four entries
+                double v[4];
+                bool bad = false;
+                auto entry = [&](int e, auto safe) {
+                    const int k = e & 1, c = e < 2 ? q : qb;
+                    const double2 xy = sxy[c], zg = szg[c], r45 = s45[c];
+                    bool b1 = false;
+                    v[e] = cov_fast_entry<NU, PREF, PLANAR, decltype(safe)::value>(
+                        pc0[k], pc1[k], pc2[k], ga[k], ca[k], ssa[k], bh[k], xy.x, xy.y, zg.x, zg.y, r45.x, r45.x, r45.y,
+                        b1);
+                    bad = bad || (b1 && !(self && t + k * half + doff == q0 + c));  // the diagonal is replaced below
+                };
+#pragma unroll
+                for (int e = 0; e < 4; ++e) entry(e, std::false_type());
+                if (bad) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) entry(e, std::true_type());
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int k = e & 1, c = e < 2 ? q : qb;
+                    if (self && t + k * half + doff == q0 + c) v[e] = diag[k];  // sigma^2 + tau^2 (evaluate_covariance.cpp:103,307)
+                    if ((k == 0 || two) && (e < 2 || q + cols < qn)) ob[k * half + (e < 2 ? 0 : step)] = (T)v[e];
+                }
             }
         }
     }
     __syncthreads();
 }
 
+template <int KIND>
+struct CovForm {
+    static constexpr int NU = ((KIND - 1) & 3) < 2 ? 3 : 1, PREF = KIND & 1;
+    static constexpr bool PLANAR = KIND > 4;
+};
+
 // Block out[t + q ld] = C(A_{a0+t}, B_{b0+q}), t < nr, q < nc (with the
 // sigma^2 + tau^2 diagonal when `self`), by the whole CTA.  KIND (cov_kind on the
 // host): 1..4 the straight-line nonstationary FP64 forms (Matern 3/2 or 1/2 x
-// prefactor exponent 1 or 3/2), 0 every other model.
+// prefactor exponent 1 or 3/2) in space, 5..8 the same in the plane, 0 every other
+// model.
 // CH: column points staged per chunk by the other models (7 CH doubles of stage).
 template <typename T, int KIND, int CH = kCovChunk>
 __device__ __forceinline__ void cov_block(const Geom& g, const PointSet& P, long a0, int nr, long b0, int nc, bool self,
@@ -512,16 +550,32 @@ __device__ __forceinline__ void cov_block(const Geom& g, const PointSet& P, long
     if constexpr (KIND == 0) {
         fill_cov_staged<T, CH>(g, P, &a0, 1, nr, b0, nc, self, out, ld, 0, stage);
     } else {
-        const double hs = g.dist_scale * (KIND <= 2 ? 1.7320508075688772 : 1.0);
+        using F = CovForm<KIND>;
+        const double hs = g.dist_scale * (F::NU == 3 ? 1.7320508075688772 : 1.0);
         const double ihs2 = 1.0 / (hs * hs), ih2 = 0.5 * ihs2;
-        constexpr int NU = KIND <= 2 ? 3 : 1, PREF = (KIND & 1) ? 1 : 0;
-        cov_block_fast<T, NU, PREF>(P, a0, nr, b0, nc, self, out, ld, ih2, ihs2, stage);
+        cov_block_fast<T, F::NU, F::PREF, F::PLANAR>(P, a0, nr, b0, nc, self, 0, out, ld, ih2, ihs2, stage);
     }
 }
 
 inline int cov_kind(const Geom& g, bool fp64) {
     if (!(fp64 && g.nonstat && g.distance != 1 && g.pref_kind != 2)) return 0;
-    return g.nu_x2 == 3 ? (g.pref_kind == 1 ? 1 : 2) : (g.pref_kind == 1 ? 3 : 4);
+    return (g.nu_x2 == 3 ? (g.pref_kind == 1 ? 1 : 2) : (g.pref_kind == 1 ? 3 : 4)) + (g.distance == 2 ? 4 : 0);
+}
+
+// Calls f(std::integral_constant<int, KIND>) for the model's form.
+template <typename Fn>
+inline void with_cov_kind(int kind, Fn&& f) {
+    switch (kind) {
+        case 1: f(std::integral_constant<int, 1>()); break;
+        case 2: f(std::integral_constant<int, 2>()); break;
+        case 3: f(std::integral_constant<int, 3>()); break;
+        case 4: f(std::integral_constant<int, 4>()); break;
+        case 5: f(std::integral_constant<int, 5>()); break;
+        case 6: f(std::integral_constant<int, 6>()); break;
+        case 7: f(std::integral_constant<int, 7>()); break;
+        case 8: f(std::integral_constant<int, 8>()); break;
+        default: f(std::integral_constant<int, 0>()); break;
+    }
 }
 
 

@@ -32,24 +32,23 @@ namespace mra {
 template <typename T, int KIND>
 __global__ void __launch_bounds__(kCovThreads, 4) k_cov_finest(Geom g, DevTree<T> t) {
     constexpr int CH = sizeof(T) == 8 ? kCovChunk : 96;  // FP32: the chunk of fill_cov, and so its compiled code
-    __shared__ double stage[7 * CH];
+    __shared__ __align__(16) double stage[7 * CH];
     const int r = t.r, L = t.L, m = t.M - 2;
     const long Lr = (long)L * r;
     const long ntask = t.n_chunks * L;
     for (long b = blockIdx.x; b < ntask; b += gridDim.x) {
-        const long q = b / L;
+        const long q = (unsigned)b / (unsigned)L;  // at most 2^31 tasks
         const int j = (int)(b - q * L);
         const FinChunk ch = t.chunks[q];
         const long unit = ch.unit;  // local index at level M-3 (0 when M == 2)
         if (skipped(t, chunk_region(t, unit))) continue;
         if (j < m) {
-            long a = chunk_region(t, unit);  // level m-1, up to level j
-            for (int l = m - 1; l > j; --l) a = (a - 1) / t.J;
+            const long a = ancestor(t, m - 1, unit, j);
             cov_block<T, KIND, CH>(g, t.pts, a * r, r, t.obs0 + ch.lo, ch.n, false, t.Bhat + ch.lo * Lr + (long)j * r, Lr,
                                stage);
         } else {
             const long g0 = m > 0 ? unit * t.J : 0, g1 = m > 0 ? g0 + t.J : 1;
-            const long s2 = level_start(t.J, m);
+            const long s2 = t.lstart[m];
             for (long gl = g0; gl < g1; ++gl) {
                 const long glo = t.sub_lo[s2 + gl], ghi = t.sub_hi[s2 + gl];
                 const long lo = glo > ch.lo ? glo : ch.lo, hi = ghi < ch.lo + ch.n ? ghi : ch.lo + ch.n;
@@ -79,13 +78,12 @@ __global__ void __launch_bounds__(kCondThreads, CondSmem<RC>::CTAS) k_finest_con
     // levels 0..M-3, then level M-2 per sibling group of the chunk; one call of
     // step, whose code then stays in the instruction cache
     const int ng = m > 0 ? t.J : 1;
-    const long g0 = m > 0 ? unit * t.J : 0, s2 = level_start(t.J, m);
+    const long g0 = m > 0 ? unit * t.J : 0, s2 = t.lstart[m];
     for (int s = 0; s < m + ng; ++s) {
         long a, lo = ch.lo, hi = ch.lo + ch.n;
         const int j = s < m ? s : m;
         if (s < m) {
-            a = chunk_region(t, unit);  // level m-1, up to level j
-            for (int l = m - 1; l > j; --l) a = (a - 1) / t.J;
+            a = ancestor(t, m - 1, unit, j);
         } else {
             a = s2 + g0 + (s - m);
             if (t.sub_lo[a] > lo) lo = t.sub_lo[a];
@@ -93,7 +91,7 @@ __global__ void __launch_bounds__(kCondThreads, CondSmem<RC>::CTAS) k_finest_con
             if (lo >= hi) continue;
         }
         const long d = (lo - ch.lo) * Lr;
-        const CondOp o{t.U + t.u_off[j] + (a - level_start(t.J, j)) * (long)j * rr, j * r, U + d, Lr, (int)(hi - lo)};
+        const CondOp o{t.U + t.u_off[j] + (a - t.lstart[j]) * (long)j * rr, j * r, U + d, Lr, (int)(hi - lo)};
         double* Vj = V + d + (long)j * r;
         cond.step(o, t.Pinv + a * rr, Vj, Lr, Vj, U + d + (long)j * r);
     }
@@ -115,7 +113,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_finest_condition_any(DevTree<T>
         gemm<T, false, false>(r, n, r, (T)1, t.Pinv + a * rr, r, V, Lr, (T)0, U + (long)j * r, Lr, sm);
     };
     const long g0 = m > 0 ? unit * t.J : 0, g1 = m > 0 ? g0 + t.J : 1;
-    const long s2 = level_start(t.J, m);
+    const long s2 = t.lstart[m];
     long gl = g0 - 1;
     for (int j = 0; j < m || gl + 1 < g1;) {
         long a, lo = ch.lo, hi = ch.lo + ch.n;
@@ -123,9 +121,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_finest_condition_any(DevTree<T>
         int jj;
         if (j < m) {
             jj = j++;
-            a = chunk_region(t, unit);
-            for (int l = m - 1; l > jj; --l) a = (a - 1) / t.J;
-            Ua = t.U + t.u_off[jj] + (a - level_start(t.J, jj)) * (long)jj * rr;
+            a = ancestor(t, m - 1, unit, jj);
+            Ua = t.U + t.u_off[jj] + (a - t.lstart[jj]) * (long)jj * rr;
         } else {
             ++gl;
             jj = m;
@@ -296,7 +293,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_heavy_panel(DevTree<double> t, 
 // processed together, stay zero).
 template <typename T>
 __global__ void k_finest_terms(DevTree<T> t) {
-    const long s2 = level_start(t.J, t.M - 2), cnt2 = level_count(t.J, t.M - 2);
+    const long s2 = t.lstart[t.M - 2], cnt2 = level_count(t.J, t.M - 2);
     const long q = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= cnt2 || skipped(t, s2 + q)) return;
     double s = 0.0;
@@ -311,13 +308,11 @@ template <typename T>
 static void launch_cov_finest(const Geom& g, const DevTree<T>& t, cudaStream_t st) {
     const long tasks = t.n_chunks * t.L;
     const unsigned grid = (unsigned)(tasks < 148L * 32 ? tasks : 148L * 32);
-    switch (cov_kind(g, sizeof(T) == 8)) {
-        case 1: k_cov_finest<T, 1><<<grid, kCovThreads, 0, st>>>(g, t); break;
-        case 2: k_cov_finest<T, 2><<<grid, kCovThreads, 0, st>>>(g, t); break;
-        case 3: k_cov_finest<T, 3><<<grid, kCovThreads, 0, st>>>(g, t); break;
-        case 4: k_cov_finest<T, 4><<<grid, kCovThreads, 0, st>>>(g, t); break;
-        default: k_cov_finest<T, 0><<<grid, kCovThreads, 0, st>>>(g, t); break;
-    }
+    if constexpr (sizeof(T) == 8)
+        with_cov_kind(cov_kind(g, true),
+                      [&](auto k) { k_cov_finest<T, decltype(k)::value><<<grid, kCovThreads, 0, st>>>(g, t); });
+    else
+        k_cov_finest<T, 0><<<grid, kCovThreads, 0, st>>>(g, t);
 }
 
 template <int RC>

@@ -23,42 +23,77 @@ namespace mra {
 // ---------------------------------------------------------------------------
 // a1: fields
 // ---------------------------------------------------------------------------
-__global__ void k_fields(Geom g, FieldParams fp, const double* __restrict__ c0, const double* __restrict__ c1,
-                         const double* __restrict__ c2, long n, double* __restrict__ s2, double* __restrict__ beta,
-                         double* __restrict__ t2) {
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+// One thread per point and field (blockIdx.y): a point's basis sums are chains of
+// an exponential or a polynomial per basis function, so the three fields run side
+// by side, in small blocks that spread over the chip (8,192 points with two fields
+// of 9 functions: 11.2 us with one thread per point in blocks of 256, 8.5 us now).
+constexpr int kFieldThreads = 64;
+
+__device__ __forceinline__ double field_value(const Geom& g, const FieldParams& fp, int f, const Pt& p) {
     const double* th = fp.theta;
-    if (!g.nonstat) {
-        s2[i] = th[6];
-        beta[i] = th[7];
-        t2[i] = th[8];
-        return;
-    }
-    Pt p{c0[i], c1[i], c2[i]};
-    double out[3];
-#pragma unroll
-    for (int f = 0; f < 3; ++f) {
-        double v = th[3 + f];
-        const long nb = fp.nb[f];
-        const double* c = fp.centers[f];
-        const double* w = fp.weights[f];
-        for (long b = 0; b < nb; ++b) {
-            Pt q{c[b], c[nb + b], c[2 * nb + b]};
-            double d = point_distance(g, p, q) / fp.basis_len;
-            if (fp.basis == 0) {
-                if (d >= 1) continue;
-                double u = 1 - d, u2 = u * u;
-                v += u2 * u2 * u2 * (35 * d * d + 18 * d + 3) * w[b] / 3;
-            } else {
-                v += exp(-0.5 * d * d) * w[b];
-            }
+    if (!g.nonstat) return th[6 + f];
+    double v = th[3 + f];
+    const long nb = fp.nb[f];
+    const double* c = fp.centers[f];
+    const double* w = fp.weights[f];
+#pragma unroll 3
+    for (long b = 0; b < nb; ++b) {
+        const Pt q{c[b], c[nb + b], c[2 * nb + b]};
+        const double d = point_distance(g, p, q) / fp.basis_len;
+        if (fp.basis == 0) {
+            const double u = 1 - d, u2 = u * u;
+            const double phi = u2 * u2 * u2 * (35 * d * d + 18 * d + 3) * w[b] / 3;
+            v += d >= 1 ? 0.0 : phi;
+        } else {
+            v += exp(-0.5 * d * d) * w[b];
         }
-        out[f] = th[f] * exp(v);
     }
-    s2[i] = out[0];
-    beta[i] = out[1];
-    t2[i] = out[2];
+    return th[f] * exp(v);
+}
+
+__device__ __forceinline__ void store_field(int f, long i, double v, double* s2, double* beta, double* t2, double* ss) {
+    if (f == 0) {
+        s2[i] = v;
+        ss[i] = sqrt(v);
+    } else {
+        (f == 1 ? beta : t2)[i] = v;
+    }
+}
+
+__global__ void __launch_bounds__(kFieldThreads)
+    k_fields(Geom g, FieldParams fp, const double* __restrict__ c0, const double* __restrict__ c1,
+             const double* __restrict__ c2, long n, double* __restrict__ s2, double* __restrict__ beta,
+             double* __restrict__ t2, double* __restrict__ ss) {
+    const long i = (long)blockIdx.x * kFieldThreads + threadIdx.x;
+    if (i >= n) return;
+    const int f = blockIdx.y;
+    store_field(f, i, field_value(g, fp, f, Pt{c0[i], c1[i], c2[i]}), s2, beta, t2, ss);
+}
+
+// The same for the points p2 [3][n2] then p1 [3][n1] with the parameters passed by
+// value (small models: nothing to copy first); also gathers the coordinates.
+__global__ void __launch_bounds__(kFieldThreads)
+    k_fields_inline(Geom g, FieldParams fp, const __grid_constant__ InlineTables tab, const double* __restrict__ p2,
+                    long n2, const double* __restrict__ p1, long n1, PointBuffers o) {
+    const long i = (long)blockIdx.x * kFieldThreads + threadIdx.x;
+    if (i >= n1 + n2) return;
+    const int f = blockIdx.y;
+    const double* src = i < n2 ? p2 + i : p1 + (i - n2);
+    const long n = i < n2 ? n2 : n1;
+    const Pt p{src[0], src[n], src[2 * n]};
+    long off = 0;
+    fp.theta = tab.theta;
+    for (int q = 0; q < 3; ++q) {
+        fp.centers[q] = tab.v + off;
+        fp.weights[q] = tab.v + off + 3 * fp.nb[q];
+        off += 4 * fp.nb[q];
+    }
+    if (f == 0) {
+        o.c[0][i] = p.c0;
+        o.c[1][i] = p.c1;
+        o.c[2][i] = p.c2;
+    }
+    store_field(f, i, field_value(g, fp, f, p), o.f[0], o.f[1], o.f[2], o.f[3]);
 }
 
 // ---------------------------------------------------------------------------
@@ -218,6 +253,22 @@ __global__ void __launch_bounds__(kThreads, 2) k_sample(DevTree<T> t, const doub
 // ---------------------------------------------------------------------------
 // evaluate_*covariance blocks (layout out[i1*n2 + i2])
 // ---------------------------------------------------------------------------
+// Straight-line nonstationary forms: tiles of RT rows x CT columns by the blocks of
+// mra_device.cuh (4001 x 3003 entries: 54 us, 1.8 TB/s of results; by the
+// entry-per-thread kernel below about 130).
+template <int KIND>
+__global__ void __launch_bounds__(kCovThreads, 4) k_cov_tiles(Geom g, PointSet P, long a0, int na, long b0, int nb,
+                                                              int self, int RT, int CT, double* out) {
+    __shared__ __align__(16) double stage[7 * kCovChunk];
+    const int t0 = blockIdx.x * RT, q0 = blockIdx.y * CT;
+    const int nr = min(RT, na - t0), nc = min(CT, nb - q0);
+    using F = CovForm<KIND>;
+    const double hs = g.dist_scale * (F::NU == 3 ? 1.7320508075688772 : 1.0);
+    const double ihs2 = 1.0 / (hs * hs), ih2 = 0.5 * ihs2;
+    cov_block_fast<double, F::NU, F::PREF, F::PLANAR>(P, a0 + t0, nr, b0 + q0, nc, self != 0, t0 - q0,
+                                                      out + t0 + (long)q0 * na, na, ih2, ihs2, stage);
+}
+
 __global__ void k_cov_block(Geom g, PointSet P, long a0, int na, long b0, int nb, int self, double* out) {
     long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= (long)na * nb) return;
@@ -241,9 +292,17 @@ __global__ void k_convert(const Ti* __restrict__ in, To* __restrict__ out, long 
 // launchers
 // ---------------------------------------------------------------------------
 void launch_fields(const Geom& g, const FieldParams& fp, const double* c0, const double* c1, const double* c2,
-                   long n, double* s2, double* beta, double* t2, cudaStream_t st) {
+                   long n, double* s2, double* beta, double* t2, double* ss, cudaStream_t st) {
     if (n <= 0) return;
-    k_fields<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(g, fp, c0, c1, c2, n, s2, beta, t2);
+    const dim3 grid((unsigned)((n + kFieldThreads - 1) / kFieldThreads), 3);
+    k_fields<<<grid, kFieldThreads, 0, st>>>(g, fp, c0, c1, c2, n, s2, beta, t2, ss);
+}
+void launch_fields_inline(const Geom& g, const FieldParams& fp, const InlineTables& tab, const double* p2, long n2,
+                          const double* p1, long n1, const PointBuffers& o, cudaStream_t st) {
+    const long n = n1 + n2;
+    if (n <= 0) return;
+    const dim3 grid((unsigned)((n + kFieldThreads - 1) / kFieldThreads), 3);
+    k_fields_inline<<<grid, kFieldThreads, 0, st>>>(g, fp, tab, p2, n2, p1, n1, o);
 }
 template <typename T>
 void launch_predict(const Geom& g, const DevTree<T>& t, int grid, cudaStream_t st) {
@@ -263,6 +322,22 @@ void launch_cov_block(const Geom& g, const PointSet& P, long a0, int na, long b0
                       cudaStream_t st) {
     long n = (long)na * nb;
     if (n <= 0) return;
+    const int kind = cov_kind(g, true);
+    if (kind > 0) {
+        // long column runs, unless that leaves the chip short of blocks
+        int RT = 256, CT = kCovChunk;
+        while ((long)((na + RT - 1) / RT) * ((nb + CT - 1) / CT) < 4 * 148 && CT > 8) RT > 64 ? RT /= 2 : CT /= 2;
+        const long gy = (nb + CT - 1) / CT;
+        if (gy <= 65535) {
+            const dim3 grid((unsigned)((na + RT - 1) / RT), (unsigned)gy);
+            with_cov_kind(kind, [&](auto k) {
+                if constexpr (decltype(k)::value > 0)
+                    k_cov_tiles<decltype(k)::value><<<grid, kCovThreads, 0, st>>>(g, P, a0, na, b0, nb, self ? 1 : 0, RT,
+                                                                                  CT, out);
+            });
+            return;
+        }
+    }
     k_cov_block<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(g, P, a0, na, b0, nb, self ? 1 : 0, out);
 }
 

@@ -31,6 +31,8 @@ struct HeavyTile {
 template <typename T>
 struct DevTree {
     int J, M, r, L;            // L = M-1 ancestor levels of a finest region
+    int lj;                    // log2 J
+    int lstart[kMaxLevels];    // first region of each interior level
     long n_int, n_fin, n_obs, n_pred;
     long obs0, pred0;          // first obs / pred index in the joint point arrays
     int tf;                    // largest subtree (in observations) kept in factored form
@@ -129,7 +131,12 @@ __device__ __forceinline__ bool skipped(const DevTree<T>& t, long region) {
 // the region whose sub-tree holds a chunk: the level M-3 region (the root when M = 2)
 template <typename T>
 __device__ __forceinline__ long chunk_region(const DevTree<T>& t, long unit) {
-    return t.M >= 3 ? level_start(t.J, t.M - 3) + unit : 0;
+    return t.M >= 3 ? t.lstart[t.M - 3] + unit : 0;
+}
+// the level-j ancestor of region `loc` (local index) of level m
+template <typename T>
+__device__ __forceinline__ long ancestor(const DevTree<T>& t, int m, long loc, int j) {
+    return t.lstart[j] + (loc >> (t.lj * (m - j)));
 }
 // slice index of block (j,k), j <= k < m, row-major over the upper triangle
 // (the order of class_approximation.cpp:62-73)
@@ -168,7 +175,19 @@ cudaError_t prepare_kernels();
 cudaError_t set_gemm_tiles(const int nw[3]);
 
 void launch_fields(const Geom& g, const FieldParams& fp, const double* c0, const double* c1, const double* c2,
-                   long n, double* s2, double* beta, double* t2, cudaStream_t st);
+                   long n, double* s2, double* beta, double* t2, double* ss, cudaStream_t st);
+// theta and the basis tables of a small model by value: per field the centers
+// [3][nb] and the weights [nb], one after the other.
+struct InlineTables {
+    double theta[16];
+    double v[432];
+};
+struct PointBuffers {
+    double* c[3];
+    double* f[4];  // sigma^2, beta, tau^2, sigma
+};
+void launch_fields_inline(const Geom& g, const FieldParams& fp, const InlineTables& tab, const double* p2, long n2,
+                          const double* p1, long n1, const PointBuffers& o, cudaStream_t st);
 // Events recorded around each covariance-block launch of a prior level, so
 // that the caller can split the level's device time between the covariance
 // launches and the region launches.

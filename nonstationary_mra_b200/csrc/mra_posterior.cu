@@ -110,7 +110,7 @@ __device__ __noinline__ void factored_step(const DevTree<double>& t, int m, long
         if (Lti) trmv_lower_inv<double>(r, Lti, r, v, v);
         else trsv_lower_f64<double>(r, Lt, r, v);
         if (m > 0) {
-            double* Gi = t.G + t.u_off[m] + (i - level_start(t.J, m)) * mr * r;
+            double* Gi = t.G + t.u_off[m] + (i - t.lstart[m]) * mr * r;
             gemm_call<false, true>(r, (int)mr, n, 1.0, F + mr, ldF, F, ldF, 0.0, Gi, r, sm);
             // G = L~^{-1} G in place: one row tile (r <= 64) reads all of its
             // column block before writing it
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_posterior_factored(DevTree<doub
     LaSmem<double>& sm = la_smem<double>();
     const int r = t.r;
     const long mr1 = (long)(m + 1) * r;
-    const long s0 = level_start(t.J, m), nd = t.n_dense[m];
+    const long s0 = t.lstart[m], nd = t.n_dense[m];
     const long cnt = level_count(t.J, m) - (m == t.M - 2 && !keep ? t.n_fused : 0);
     double* ws = t.ws + blockIdx.x * t.ws_stride;
     double* wsd = t.wsd + blockIdx.x * t.wsd_stride;
@@ -172,7 +172,7 @@ struct DenseArgs {
 
 __device__ __forceinline__ double* dense_G(const DevTree<double>& t, const DenseArgs& a, long q, long i) {
     const long rr = (long)t.r * t.r;
-    return a.keep ? t.G + t.u_off[a.m] + (i - level_start(t.J, a.m)) * (long)a.m * rr
+    return a.keep ? t.G + t.u_off[a.m] + (i - t.lstart[a.m]) * (long)a.m * rr
                   : a.scr + q * a.per + (long)a.m * rr;
 }
 __device__ __forceinline__ double* dense_inv(const DevTree<double>& t, const DenseArgs& a, long q, long i) {
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(Tile<TS>::NT, Tile<TS>::CTAS) k_dense_gather(D
     int j = 0;  // slice s = (j, k), j <= k <= m, row by row
     while (s >= m + 1 - j) s -= m + 1 - j, ++j;
     const int k = j + s;
-    const long i = level_start(t.J, m) + t.post_order[level_start(t.J, m) + a.q0 + q];
+    const long i = t.lstart[m] + t.post_order[t.lstart[m] + a.q0 + q];
     if (skipped(t, i)) return;
     const int r0 = ti * TS, c0 = tj * TS;
     const int M = min(TS, r - r0), N = min(TS, r - c0);
@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_dense_factor(DevTree<double> t,
     LaSmem<double>& sm = la_smem<double>();
     const int r = t.r;
     const long q = blockIdx.x;
-    const long i = level_start(t.J, a.m) + t.post_order[level_start(t.J, a.m) + a.q0 + q];
+    const long i = t.lstart[a.m] + t.post_order[t.lstart[a.m] + a.q0 + q];
     if (skipped(t, i)) return;
     double* Lt = t.Lpost + i * (long)r * r;
     double* X = r <= 128 ? dense_inv(t, a, q, i) : nullptr;
@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(Tile<TS>::NT, Tile<TS>::CTAS) k_dense_solve(De
     const long q = blockIdx.x / (m * nt2);
     const int s = (int)(blockIdx.x - q * (m * nt2));
     const int j = s / nt2, ti = s % nt2 / nt, tj = s % nt;
-    const long i = level_start(t.J, m) + t.post_order[level_start(t.J, m) + a.q0 + q];
+    const long i = t.lstart[m] + t.post_order[t.lstart[m] + a.q0 + q];
     if (skipped(t, i)) return;
     const int r0 = ti * TS, c0 = tj * TS;
     const int M = min(TS, r - r0), N = min(TS, r - c0);
@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_dense_solve_any(DevTree<double>
     const int r = t.r, m = a.m;
     const long rr = (long)r * r, mr = (long)m * r;
     const long q = blockIdx.x;
-    const long i = level_start(t.J, m) + t.post_order[level_start(t.J, m) + a.q0 + q];
+    const long i = t.lstart[m] + t.post_order[t.lstart[m] + a.q0 + q];
     if (skipped(t, i)) return;
     const double* A = a.scr + q * a.per;
     double* G = dense_G(t, a, q, i);
@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(Tile<TS>::NT, Tile<TS>::CTAS) k_dense_out(DevT
     int j = 0;
     while (s >= m - j) s -= m - j, ++j;
     const int k = j + s;
-    const long i = level_start(t.J, m) + t.post_order[level_start(t.J, m) + a.q0 + q];
+    const long i = t.lstart[m] + t.post_order[t.lstart[m] + a.q0 + q];
     if (skipped(t, i)) return;
     const int r0 = ti * TS, c0 = tj * TS;
     const int M = min(TS, r - r0), N = min(TS, r - c0);

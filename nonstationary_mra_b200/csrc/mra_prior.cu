@@ -25,18 +25,17 @@ __host__ __device__ inline long cov_slot(long q, int j, int m, int SB) {
 template <typename T, int KIND>
 __global__ void __launch_bounds__(kCovThreads, 4) k_cov_level(Geom g, DevTree<T> t, int m, long loc0, long nloc, int SB,
                                                                T* __restrict__ out) {
-    __shared__ double stage[7 * kCovChunk];
+    __shared__ __align__(16) double stage[7 * kCovChunk];
     const int r = t.r;
     const long rr = (long)r * r;
-    const long s0 = level_start(t.J, m);
+    const long s0 = t.lstart[m];
     const long nblocks = nloc * (m + 1);
     for (long b = blockIdx.x; b < nblocks; b += gridDim.x) {
-        const long q = b / (m + 1);
+        const long q = (unsigned)b / (unsigned)(m + 1);  // at most 2^31 blocks
         const int j = (int)(b - q * (m + 1));
         const long i = s0 + loc0 + q;
         if (skipped(t, i)) continue;
-        long a = i;  // the ancestor of level j (the region itself for j == m)
-        for (int l = m; l > j; --l) a = (a - 1) / t.J;
+        const long a = ancestor(t, m, loc0 + q, j);  // the region itself for j == m
         cov_block<T, KIND>(g, t.pts, a * r, r, i * r, r, j == m, out + cov_slot(q, j, m, SB) * rr, r, stage);
     }
 }
@@ -45,13 +44,12 @@ __global__ void __launch_bounds__(kCovThreads, 4) k_cov_level(Geom g, DevTree<T>
 template <typename T>
 void launch_cov_level(const Geom& g, const DevTree<T>& t, int m, long loc0, long n, int SB, unsigned grid,
                       cudaStream_t st) {
-    switch (cov_kind(g, sizeof(T) == 8)) {
-        case 1: k_cov_level<T, 1><<<grid, kCovThreads, 0, st>>>(g, t, m, loc0, n, SB, t.cbuf); break;
-        case 2: k_cov_level<T, 2><<<grid, kCovThreads, 0, st>>>(g, t, m, loc0, n, SB, t.cbuf); break;
-        case 3: k_cov_level<T, 3><<<grid, kCovThreads, 0, st>>>(g, t, m, loc0, n, SB, t.cbuf); break;
-        case 4: k_cov_level<T, 4><<<grid, kCovThreads, 0, st>>>(g, t, m, loc0, n, SB, t.cbuf); break;
-        default: k_cov_level<T, 0><<<grid, kCovThreads, 0, st>>>(g, t, m, loc0, n, SB, t.cbuf); break;
-    }
+    if constexpr (sizeof(T) == 8)
+        with_cov_kind(cov_kind(g, true), [&](auto k) {
+            k_cov_level<T, decltype(k)::value><<<grid, kCovThreads, 0, st>>>(g, t, m, loc0, n, SB, t.cbuf);
+        });
+    else
+        k_cov_level<T, 0><<<grid, kCovThreads, 0, st>>>(g, t, m, loc0, n, SB, t.cbuf);
 }
 
 // ---------------------------------------------------------------------------
@@ -83,7 +81,7 @@ __global__ void __launch_bounds__(kCondThreads, CondSmem<RC>::CTAS)
     const long mr = (long)m * r;
     const long q = (long)blockIdx.x * SB;
     const int nsib = (int)(nloc - q < SB ? nloc - q : SB);
-    const long i0 = level_start(t.J, m) + loc0 + q;
+    const long i0 = t.lstart[m] + loc0 + q;
     // at the split level of a sharded evaluation siblings belong to different ranks: the columns of a sibling that
     // is not computed here are carried along (columns are independent) and left out below
     bool any = false;
@@ -93,9 +91,8 @@ __global__ void __launch_bounds__(kCondThreads, CondSmem<RC>::CTAS)
     const double* Cq = C + cov_slot(q, 0, m, SB) * rr;
     double* Ui = t.U + t.u_off[m] + (loc0 + q) * mr * r;  // (m r) x (nsib r), ld = m r
     for (int j = 0; j < m; ++j) {
-        long a = i0;
-        for (int l = m; l > j; --l) a = (a - 1) / t.J;
-        const CondOp o{t.U + t.u_off[j] + (a - level_start(t.J, j)) * (long)j * rr, j * r, Ui, mr, nsib * r};
+        const long a = ancestor(t, m, loc0 + q, j);
+        const CondOp o{t.U + t.u_off[j] + (a - t.lstart[j]) * (long)j * rr, j * r, Ui, mr, nsib * r};
         const double* Cj = Cq + (long)j * SB * rr;
         // the next covariance block (or the self blocks) into L2 while this step's products run
         if (threadIdx.x == 0) prefetch_l2(Cj + (long)SB * rr, (unsigned long)nsib * rr * sizeof(double));

@@ -61,9 +61,9 @@ template <int KIND>
 __global__ void __launch_bounds__(256) k_cov_group(Geom g, DevTree<double> t) {
     const int lane = threadIdx.x & 31;
     const long nw = (long)gridDim.x * (blockDim.x / 32);
-    const double hs = g.dist_scale * (KIND <= 2 ? 1.7320508075688772 : 1.0);
+    using F = CovForm<KIND>;
+    const double hs = g.dist_scale * (F::NU == 3 ? 1.7320508075688772 : 1.0);
     const double ihs2 = 1.0 / (hs * hs), ih2 = 0.5 * ihs2;
-    constexpr int NU = KIND <= 2 ? 3 : 1, PREF = (KIND & 1) ? 1 : 0;
     const PointSet& P = t.pts;
     for (long c = (long)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); c < t.n_fin; c += nw) {
         const long o0 = t.obs_off[c];
@@ -73,17 +73,22 @@ __global__ void __launch_bounds__(256) k_cov_group(Geom g, DevTree<double> t) {
         for (int e = lane; e < n * n; e += 32) {
             const int i = e % n, j = e / n;
             const long ia = t.obs0 + o0 + i, ib = t.obs0 + o0 + j;
-            const double sa = P.s2[ia], ba = P.beta[ia], sb = P.s2[ib], bb = P.beta[ib];
+            const double sa = P.s2[ia], ba = P.beta[ia], bb = P.beta[ib];
             double v;
             if (i == j) {
                 v = sa + P.t2[ia];
             } else if constexpr (KIND == 0) {
-                v = cov_entry(g, P.pt(ia), sa, ba, P.pt(ib), sb, bb);
+                v = cov_entry(g, P.pt(ia), sa, ba, P.pt(ib), P.s2[ib], bb);
             } else {
-                const double ssa = sqrt(sa), ssb = sqrt(sb);
-                v = cov_fast_entry<NU, PREF, true>(P.c0[ia], P.c1[ia], P.c2[ia], ba * ba * ih2, ssa * ba * ihs2, ssa,
-                                                   ba * ihs2, P.c0[ib], P.c1[ib], P.c2[ib], bb * bb * ih2, ssb * bb,
-                                                   ssb, bb);
+                const double ssa = P.ss[ia], ssb = P.ss[ib];
+                auto entry = [&](auto safe) {
+                    bool bad = false;
+                    v = cov_fast_entry<F::NU, F::PREF, F::PLANAR, decltype(safe)::value>(
+                        P.c0[ia], P.c1[ia], P.c2[ia], ba * ba * ih2, ssa * ba * ihs2, ssa, ba * ihs2, P.c0[ib],
+                        P.c1[ib], P.c2[ib], bb * bb * ih2, ssb * bb, ssb, bb, bad);
+                    return bad;
+                };
+                if (entry(std::false_type())) entry(std::true_type());
             }
             S[e] = v;
         }
@@ -103,7 +108,7 @@ __global__ void __launch_bounds__(SmallSmem<RC>::NT, SmallSmem<RC>::CTAS)
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, tt = lane & 3;
     const int r = t.r, L = t.L, m = t.M - 2;
     const long Lr = (long)L * r, mr = (long)m * r;
-    const long s2 = level_start(t.J, m), cnt2 = level_count(t.J, m);
+    const long s2 = t.lstart[m], cnt2 = level_count(t.J, m);
     const long item = items[blockIdx.x];
     const bool group = item < cnt2;
     const long clo = group ? t.child_lo[item] : item - cnt2, chi = group ? t.child_hi[item] : clo + 1;
@@ -408,13 +413,7 @@ int launch_finest_small(const Geom& g, const DevTree<double>& t, bool keep, cuda
     if (t.n_fin_items == 0) return 0;
     const long blocks = (t.n_fin + 7) / 8;
     const unsigned grid = (unsigned)(blocks < 148L * 32 ? blocks : 148L * 32);
-    switch (cov_kind(g, true)) {
-        case 1: k_cov_group<1><<<grid, 256, 0, st>>>(g, t); break;
-        case 2: k_cov_group<2><<<grid, 256, 0, st>>>(g, t); break;
-        case 3: k_cov_group<3><<<grid, 256, 0, st>>>(g, t); break;
-        case 4: k_cov_group<4><<<grid, 256, 0, st>>>(g, t); break;
-        default: k_cov_group<0><<<grid, 256, 0, st>>>(g, t); break;
-    }
+    with_cov_kind(cov_kind(g, true), [&](auto k) { k_cov_group<decltype(k)::value><<<grid, 256, 0, st>>>(g, t); });
     // largest class first
     const long n64 = t.n_fin_class[0], n32 = t.n_fin_class[1], n16 = t.n_fin_class[2];
     launch_class<64>(t, t.fin_items, n64, keep, st);

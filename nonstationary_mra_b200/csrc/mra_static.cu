@@ -14,6 +14,7 @@
 // exits.
 #include <cuda_runtime.h>
 
+#include <cstring>
 #include <mutex>
 
 #include "../../include/mra_b200.h"
@@ -24,13 +25,13 @@ using namespace mra;
 namespace {
 
 // scratch layout (doubles): theta [16] | centers [3 fields][3][MAX_BASIS] |
-// weights [3][MAX_BASIS] | coordinates [3][MAX_POINTS] | fields [3][MAX_POINTS]
+// weights [3][MAX_BASIS] | coordinates [3][MAX_POINTS] | fields [4][MAX_POINTS]
 constexpr long kTheta = 0;
 constexpr long kCenters = 16;
 constexpr long kWeights = kCenters + 3L * 3 * MRA_STATIC_MAX_BASIS;
 constexpr long kCoords = kWeights + 3L * MRA_STATIC_MAX_BASIS;
 constexpr long kFields = kCoords + 3L * MRA_STATIC_MAX_POINTS;
-constexpr long kScratchDoubles = kFields + 3L * MRA_STATIC_MAX_POINTS;
+constexpr long kScratchDoubles = kFields + 4L * MRA_STATIC_MAX_POINTS;
 
 }  // namespace
 
@@ -101,33 +102,15 @@ extern "C" mra_status mra_eval_covariance_static(const mra_model* m, const mra_t
     FieldParams fp{};
     fp.basis = m->basis;
     fp.basis_len = m->basis_len;
+    PointBuffers pb{};
+    for (int c = 0; c < 3; ++c) pb.c[c] = scr + kCoords + (long)c * MRA_STATIC_MAX_POINTS;
+    for (int f = 0; f < 4; ++f) pb.f[f] = scr + kFields + (long)f * MRA_STATIC_MAX_POINTS;
+    long n_tab = 0;
     for (int f = 0; f < 3; ++f) {
-        long nb = m->nonstationary ? (long)m->field[f].n_basis : 0;
+        fp.nb[f] = m->nonstationary ? (long)m->field[f].n_basis : 0;
         v[3 + f] = th->intercepts ? th->intercepts[f] : (m->nonstationary ? m->field[f].intercept : 0.0);
-        double* cen = scr + kCenters + (long)f * 3 * MRA_STATIC_MAX_BASIS;
-        double* w = scr + kWeights + (long)f * MRA_STATIC_MAX_BASIS;
-        if (nb) {
-            for (int c = 0; c < 3; ++c)
-                SCU(cudaMemcpyAsync(cen + (long)c * nb, m->field[f].centers + (long)c * nb, nb * sizeof(double),
-                                    cudaMemcpyHostToDevice, st));
-            const double* wsrc = th->weights[f] ? th->weights[f] : m->field[f].weights;
-            SCU(cudaMemcpyAsync(w, wsrc, nb * sizeof(double), cudaMemcpyHostToDevice, st));
-        }
-        fp.nb[f] = nb;
-        fp.centers[f] = cen;
-        fp.weights[f] = w;
+        n_tab += 4 * fp.nb[f];
     }
-    SCU(cudaMemcpyAsync(scr + kTheta, v, sizeof(v), cudaMemcpyHostToDevice, st));
-    fp.theta = scr + kTheta;
-    // coordinates: set 2 first, then set 1 (rows of the output are set-2 points)
-    double* cc[3];
-    for (int c = 0; c < 3; ++c) {
-        cc[c] = scr + kCoords + (long)c * MRA_STATIC_MAX_POINTS;
-        if (n2) SCU(cudaMemcpyAsync(cc[c], p2_dev + (long)c * n2, n2 * sizeof(double), cudaMemcpyDeviceToDevice, st));
-        SCU(cudaMemcpyAsync(cc[c] + n2, p1_dev + (long)c * n1, n1 * sizeof(double), cudaMemcpyDeviceToDevice, st));
-    }
-    double* fl[3];
-    for (int f = 0; f < 3; ++f) fl[f] = scr + kFields + (long)f * MRA_STATIC_MAX_POINTS;
     Geom g{};
     g.nonstat = m->nonstationary ? 1 : 0;
     g.distance = m->distance;
@@ -135,8 +118,45 @@ extern "C" mra_status mra_eval_covariance_static(const mra_model* m, const mra_t
     g.pref_exp = m->prefactor_exp;
     g.pref_kind = m->prefactor_exp == 1.5 ? 0 : (m->prefactor_exp == 1.0 ? 1 : 2);
     g.dist_scale = m->dist_scale;
-    launch_fields(g, fp, cc[0], cc[1], cc[2], np, fl[0], fl[1], fl[2], st);
-    PointSet P{cc[0], cc[1], cc[2], fl[0], fl[1], fl[2]};
+    // set 2 first, then set 1 (rows of the output are set-2 points)
+    const long nt2 = self ? 0 : (long)n2;
+    InlineTables tab;
+    if (n_tab <= (long)(sizeof(tab.v) / sizeof(double))) {
+        // small models travel with the launch: no copies (15 of them, and their issue on the host, took
+        // longer than a small block's kernels)
+        std::memcpy(tab.theta, v, sizeof(v));
+        long off = 0;
+        for (int f = 0; f < 3; ++f) {
+            const long nb = fp.nb[f];
+            if (!nb) continue;
+            std::memcpy(tab.v + off, m->field[f].centers, 3 * nb * sizeof(double));
+            std::memcpy(tab.v + off + 3 * nb, th->weights[f] ? th->weights[f] : m->field[f].weights, nb * sizeof(double));
+            off += 4 * nb;
+        }
+        launch_fields_inline(g, fp, tab, p2_dev, nt2, p1_dev, (long)n1, pb, st);
+    } else {
+        for (int f = 0; f < 3; ++f) {
+            const long nb = fp.nb[f];
+            double* cen = scr + kCenters + (long)f * 3 * MRA_STATIC_MAX_BASIS;
+            double* w = scr + kWeights + (long)f * MRA_STATIC_MAX_BASIS;
+            if (nb) {
+                SCU(cudaMemcpyAsync(cen, m->field[f].centers, 3 * nb * sizeof(double), cudaMemcpyHostToDevice, st));
+                SCU(cudaMemcpyAsync(w, th->weights[f] ? th->weights[f] : m->field[f].weights, nb * sizeof(double),
+                                    cudaMemcpyHostToDevice, st));
+            }
+            fp.centers[f] = cen;
+            fp.weights[f] = w;
+        }
+        SCU(cudaMemcpyAsync(scr + kTheta, v, sizeof(v), cudaMemcpyHostToDevice, st));
+        fp.theta = scr + kTheta;
+        for (int c = 0; c < 3; ++c) {
+            if (nt2)
+                SCU(cudaMemcpyAsync(pb.c[c], p2_dev + (long)c * nt2, nt2 * sizeof(double), cudaMemcpyDeviceToDevice, st));
+            SCU(cudaMemcpyAsync(pb.c[c] + nt2, p1_dev + (long)c * n1, n1 * sizeof(double), cudaMemcpyDeviceToDevice, st));
+        }
+        launch_fields(g, fp, pb.c[0], pb.c[1], pb.c[2], np, pb.f[0], pb.f[1], pb.f[2], pb.f[3], st);
+    }
+    PointSet P{pb.c[0], pb.c[1], pb.c[2], pb.f[0], pb.f[1], pb.f[2], pb.f[3]};
     if (self)
         launch_cov_block(g, P, 0, (int)n1, 0, (int)n1, true, out_dev, st);
     else
