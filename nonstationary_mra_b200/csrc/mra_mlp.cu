@@ -8,10 +8,14 @@
 // Predictions without input gradients (the screening of candidate parameter
 // vectors) run k_mlp_forward_tc instead, whose 128 x 128 layer is a
 // tcgen05.mma product in tensor memory.
-// Thread h of a CTA owns hidden unit h: row h of W2 sits in its registers for
-// the forward product, and the backward product through W2 reads the BF16
-// copy of W2 in shared memory column-wise (consecutive threads, consecutive
-// addresses).
+// Four threads of a CTA share hidden unit h, each a quarter of the tile's
+// samples; W2 sits in shared memory in BF16 with padded rows, read along row h in the
+// forward product and column-wise in the backward one, both free of bank conflicts.  The passes are
+// chains of dependent sums of fixed order, a few tiles at most in flight, so what
+// counts is how many of them run side by side: with one thread per hidden unit
+// and 16 samples each the training pass of 160 samples took 42 us, now 19, and the
+// gradients of 64 samples 55 us, now 9 (4-sample tiles); every sum keeps its order,
+// so the results are bitwise the same.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -27,11 +31,13 @@
 namespace {
 
 constexpr int H = 128;     // hidden width
-constexpr int S = 16;      // samples per tile
+constexpr int S = 16;      // samples per training tile
+constexpr int SQ = 4;      // samples per tile of a small prediction
+constexpr int NT = 4 * H;  // threads of a pass
 constexpr int MAXD = 64;   // largest input width
 constexpr long MAXN = 65536;
 
-enum Mode { TRAIN = 0, PREDICT = 1, PREDICT_GRAD = 2 };
+enum Mode { TRAIN = 0, PREDICT_GRAD = 1 };
 
 struct Layout {
     long W1, b1, W2, b2, w3, b3, P;
@@ -63,177 +69,249 @@ struct MlpArgs {
 
 __device__ __forceinline__ float sigm(float z) { return 1.0f / (1.0f + expf(-z)); }
 
-size_t smem_bytes(int mode, int D) {
-    size_t b = (size_t)H * H * sizeof(__nv_bfloat16)   // W2 (row-major)
-               + (size_t)D * H * sizeof(__nv_bfloat16) // W1 transposed [d][h]
-               + (size_t)S * MAXD * sizeof(float)      // x tile
-               + 2 * (size_t)S * H * sizeof(float)     // a1, g_z2 tiles
-               + (size_t)S * 4 * sizeof(float);        // y partial sums per warp
-    if (mode == TRAIN) b += (size_t)H * H * sizeof(float) + (size_t)D * H * sizeof(float);
-    return b;
+// 4-byte asynchronous global -> shared copies: every load of a prologue in flight at once
+__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
+constexpr int WS = H + 2;  // row stride of W2 and of W1 transposed: consecutive rows fall on different banks
+
+size_t smem_bytes(int mode, int D, int ns) {
+    return (size_t)H * WS * sizeof(__nv_bfloat16)        // W2 (row-major)
+           + (((size_t)D * WS * sizeof(__nv_bfloat16) + 15) & ~(size_t)15)  // W1 transposed [d][h]
+           + (size_t)ns * MAXD * sizeof(float)           // x tile
+           + (mode == TRAIN ? 4 : 3) * (size_t)ns * H * sizeof(float)  // a1, g_z2, g_z1 tiles; a2
+           + (size_t)ns * 6 * sizeof(float);             // y partial sums per warp, g_y, errors
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(H) k_mlp_pass(MlpArgs a) {
+// ST: samples per tile; thread (h, sg) handles hidden unit h of samples sg ST/4 ...
+template <int MODE, int ST>
+__global__ void __launch_bounds__(NT, 1) k_mlp_pass(MlpArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
+    constexpr int PT = ST / 4;
     const int D = a.D;
-    const int h = threadIdx.x, warp = h >> 5, lane = h & 31;
+    const int tid = threadIdx.x, h = tid & (H - 1), sg = tid >> 7, warp = (tid >> 5) & 3, lane = tid & 31;
     __nv_bfloat16* W2s = reinterpret_cast<__nv_bfloat16*>(smem);
-    __nv_bfloat16* W1t = W2s + H * H;
-    float* xs = reinterpret_cast<float*>(W1t + D * H);
-    float* a1s = xs + S * MAXD;
-    float* gzs = a1s + S * H;
-    float* red = gzs + S * H;
-    float* dW2 = red + S * 4;   // TRAIN only: [o][i], thread i owns column i
-    float* dW1 = dW2 + H * H;   // TRAIN only: [d][h]
+    __nv_bfloat16* W1t = W2s + H * WS;
+    float* xs = reinterpret_cast<float*>(smem + (size_t)H * WS * 2 + (((size_t)D * WS * 2 + 15) & ~(size_t)15));
+    float* a1s = xs + ST * MAXD;
+    float* gzs = a1s + ST * H;
+    float* g1s = gzs + ST * H;
+    float* red = g1s + ST * H;
+    float* gys = red + ST * 4;
+    float* es = gys + ST;
+    float* a2s = es + ST;  // TRAIN only
 
-    // row h of W2 in registers (bf16 pairs)
-    __nv_bfloat162 w2r[H / 2];
-    const __nv_bfloat162* w2row = reinterpret_cast<const __nv_bfloat162*>(a.W2b + (long)h * H);
 #pragma unroll
-    for (int q = 0; q < H / 2; ++q) w2r[q] = w2row[q];
-    for (int e = h; e < H * H; e += H) W2s[e] = a.W2b[e];
-    for (int e = h; e < H * D; e += H) {
-        int hh = e / D, d = e % D;
-        W1t[d * H + hh] = a.W1b[e];
+    for (int q = 0; q < H * H / 2 / NT; ++q) {
+        const int e = tid + q * NT;
+        cp_async4(reinterpret_cast<unsigned*>(W2s) + (e >> 6) * (WS / 2) + (e & 63),
+                  reinterpret_cast<const unsigned*>(a.W2b) + e);
+    }
+    // the first tile's inputs with the weights; the next tiles' at the end of the loop
+    auto load_x = [&](long tile) {
+        for (int d = lane; d < D; d += 32)
+            for (int s = tid >> 5; s < ST; s += NT / 32) {
+                const long i = tile * ST + s;
+                if (i < a.N) cp_async4(xs + s * MAXD + d, a.X + i * D + d);
+                else xs[s * MAXD + d] = 0.f;
+            }
+    };
+    load_x(blockIdx.x);
+    {
+        __nv_bfloat16 v[MAXD / 4];
+#pragma unroll
+        for (int q = 0; q < MAXD / 4; ++q)
+            if (sg + 4 * q < D) v[q] = a.W1b[h * D + sg + 4 * q];
+#pragma unroll
+        for (int q = 0; q < MAXD / 4; ++q)
+            if (sg + 4 * q < D) W1t[(sg + 4 * q) * WS + h] = v[q];
     }
     const float b1h = a.master[a.b1 + h], b2h = a.master[a.b2 + h], b3 = a.master[a.b3];
     const float w3h = __bfloat162float(a.w3b[h]);
     float db1 = 0.f, db2 = 0.f, dw3 = 0.f, db3 = 0.f, lsum = 0.f;
+    // TRAIN: dW2[32 sg + q][h] and dW1[sg + 4 q][h]
+    float dW2[MODE == TRAIN ? H / 4 : 1], dW1[MODE == TRAIN ? MAXD / 4 : 1];
     if (MODE == TRAIN) {
-        for (int o = 0; o < H; ++o) dW2[o * H + h] = 0.f;
-        for (int d = 0; d < D; ++d) dW1[d * H + h] = 0.f;
+#pragma unroll
+        for (int q = 0; q < H / 4; ++q) dW2[q] = 0.f;
+#pragma unroll
+        for (int q = 0; q < MAXD / 4; ++q) dW1[q] = 0.f;
     }
-    __syncthreads();
 
-    const long ntiles = (a.N + S - 1) / S;
+    const long ntiles = (a.N + ST - 1) / ST;
     for (long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const long s0 = tile * S;
-        const int ns = (int)min((long)S, a.N - s0);
-        for (int e = h; e < S * D; e += H) {
-            int s = e / D, d = e % D;
-            xs[s * MAXD + d] = s < ns ? a.X[(s0 + s) * D + d] : 0.f;
+        const long s0 = tile * ST;
+        const int ns = (int)min((long)ST, a.N - s0);
+        float tgt[MODE == TRAIN ? PT : 1];
+        if (MODE == TRAIN) {
+#pragma unroll
+            for (int j = 0; j < PT; ++j) tgt[j] = sg * PT + j < ns ? a.T[s0 + sg * PT + j] : 0.f;
         }
+        cp_async_all();
         __syncthreads();
         // layer 1
-        float z1[S], z2[S];
+        float z1[PT], z2[PT];
 #pragma unroll
-        for (int s = 0; s < S; ++s) {
-            float acc = b1h;
-            for (int d = 0; d < D; ++d) acc = fmaf(__bfloat162float(W1t[d * H + h]), xs[s * MAXD + d], acc);
-            z1[s] = acc;
-            a1s[s * H + h] = acc * sigm(acc);
+        for (int j = 0; j < PT; ++j) z1[j] = b1h;
+#pragma unroll 4
+        for (int d = 0; d < D; ++d) {
+            const float w = __bfloat162float(W1t[d * WS + h]);
+#pragma unroll
+            for (int j = 0; j < PT; ++j) z1[j] = fmaf(w, xs[(sg * PT + j) * MAXD + d], z1[j]);
         }
+#pragma unroll
+        for (int j = 0; j < PT; ++j) a1s[(sg * PT + j) * H + h] = z1[j] * sigm(z1[j]);
         __syncthreads();
         // layer 2 and the output
 #pragma unroll
-        for (int s = 0; s < S; ++s) {
-            float acc = b2h;
-            const float2* ar = reinterpret_cast<const float2*>(a1s + s * H);
+        for (int j = 0; j < PT; ++j) z2[j] = b2h;
+        const float4* ar = reinterpret_cast<const float4*>(a1s + sg * PT * H);
+        const __nv_bfloat162* w2r = reinterpret_cast<const __nv_bfloat162*>(W2s + h * WS);
+#pragma unroll 8
+        for (int q = 0; q < H / 4; ++q) {
+            const float2 w0 = __bfloat1622float2(w2r[2 * q]), w1 = __bfloat1622float2(w2r[2 * q + 1]);
 #pragma unroll
-            for (int q = 0; q < H / 2; ++q) {
-                float2 w = __bfloat1622float2(w2r[q]);
-                float2 x = ar[q];
-                acc = fmaf(w.x, x.x, acc);
-                acc = fmaf(w.y, x.y, acc);
+            for (int j = 0; j < PT; ++j) {
+                const float4 x = ar[j * (H / 4) + q];
+                z2[j] = fmaf(w0.x, x.x, z2[j]);
+                z2[j] = fmaf(w0.y, x.y, z2[j]);
+                z2[j] = fmaf(w1.x, x.z, z2[j]);
+                z2[j] = fmaf(w1.y, x.w, z2[j]);
             }
-            z2[s] = acc;
-            float p = w3h * (acc * sigm(acc));
+        }
+#pragma unroll
+        for (int j = 0; j < PT; ++j) {
+            float p = w3h * (z2[j] * sigm(z2[j]));
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
-            if (lane == 0) red[s * 4 + warp] = p;
+            if (lane == 0) red[(sg * PT + j) * 4 + warp] = p;
         }
         __syncthreads();
-        float gy[S];
+        // output errors and the backward step through the output layer
 #pragma unroll
-        for (int s = 0; s < S; ++s) {
-            float y = b3 + ((red[s * 4 + 0] + red[s * 4 + 1]) + (red[s * 4 + 2] + red[s * 4 + 3]));
+        for (int j = 0; j < PT; ++j) {
+            const int s = sg * PT + j;
+            const float y = b3 + ((red[s * 4 + 0] + red[s * 4 + 1]) + (red[s * 4 + 2] + red[s * 4 + 3]));
+            float gy;
             if (MODE == TRAIN) {
-                float e = s < ns ? y - a.T[s0 + s] : 0.f;
-                gy[s] = 2.f * e / (float)a.N;
-                if (h == 0) lsum += e * e;
+                const float e = s < ns ? y - tgt[j] : 0.f;
+                gy = 2.f * e / (float)a.N;
+                if (h == 0) es[s] = e;
             } else {
-                gy[s] = s < ns ? 1.f : 0.f;
+                gy = s < ns ? 1.f : 0.f;
                 if (h == 0 && s < ns) a.Y[s0 + s] = y;
             }
+            const float sg2 = sigm(z2[j]);
+            gzs[s * H + h] = gy * w3h * (sg2 * (1.f + z2[j] * (1.f - sg2)));
+            if (MODE == TRAIN) {
+                a2s[s * H + h] = z2[j] * sg2;
+                if (h == 0) gys[s] = gy;
+            }
         }
-        if constexpr (MODE == PREDICT) {
-            __syncthreads();
+        __syncthreads();
+        if constexpr (MODE == TRAIN) {
+            float a1h[ST];
+#pragma unroll
+            for (int s = 0; s < ST; ++s) a1h[s] = a1s[s * H + h];
+#pragma unroll
+            for (int q = 0; q < H / 4; q += 4) {
+                float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int s = 0; s < ST; ++s) {
+                    const float4 gz = *reinterpret_cast<const float4*>(gzs + s * H + 32 * sg + q);
+                    acc[0] = fmaf(gz.x, a1h[s], acc[0]);
+                    acc[1] = fmaf(gz.y, a1h[s], acc[1]);
+                    acc[2] = fmaf(gz.z, a1h[s], acc[2]);
+                    acc[3] = fmaf(gz.w, a1h[s], acc[3]);
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) dW2[q + u] += acc[u];
+            }
+            if (sg == 0) {
+#pragma unroll
+                for (int s = 0; s < ST; ++s) dw3 = fmaf(gys[s], a2s[s * H + h], dw3);
+            } else if (sg == 1) {
+#pragma unroll
+                for (int s = 0; s < ST; ++s) db2 += gzs[s * H + h];
+            } else if (sg == 3 && h == 0) {
+                for (int s = 0; s < ST; ++s) {
+                    lsum += es[s] * es[s];
+                    db3 += gys[s];
+                }
+            }
+        }
+        // through W2 and the first activation
+        float gz1[PT];
+#pragma unroll
+        for (int j = 0; j < PT; ++j) gz1[j] = 0.f;
+#pragma unroll 4
+        for (int o = 0; o < H; o += 4) {
+            float w[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) w[u] = __bfloat162float(W2s[(o + u) * WS + h]);
+#pragma unroll
+            for (int j = 0; j < PT; ++j) {
+                const float4 gz = *reinterpret_cast<const float4*>(gzs + (sg * PT + j) * H + o);
+                gz1[j] = fmaf(w[0], gz.x, gz1[j]);
+                gz1[j] = fmaf(w[1], gz.y, gz1[j]);
+                gz1[j] = fmaf(w[2], gz.z, gz1[j]);
+                gz1[j] = fmaf(w[3], gz.w, gz1[j]);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < PT; ++j) {
+            const float sg1 = sigm(z1[j]);
+            gz1[j] *= sg1 * (1.f + z1[j] * (1.f - sg1));
+            g1s[(sg * PT + j) * H + h] = gz1[j];
+        }
+        __syncthreads();
+        if constexpr (MODE == TRAIN) {
+            float g1h[ST];
+#pragma unroll
+            for (int s = 0; s < ST; ++s) g1h[s] = g1s[s * H + h];
+            if (sg == 2) {
+#pragma unroll
+                for (int s = 0; s < ST; ++s) db1 += g1h[s];
+            }
+#pragma unroll
+            for (int q = 0; q < MAXD / 4; ++q) {
+                const int d = sg + 4 * q;
+                if (d >= D) break;
+                float acc = 0.f;
+#pragma unroll
+                for (int s = 0; s < ST; ++s) acc = fmaf(g1h[s], xs[s * MAXD + d], acc);
+                dW1[q] += acc;
+            }
         } else {
-            // backward through the output layer
-#pragma unroll
-            for (int s = 0; s < S; ++s) {
-                float sg = sigm(z2[s]);
-                float a2 = z2[s] * sg;
-                float g = gy[s] * w3h * (sg * (1.f + z2[s] * (1.f - sg)));
-                gzs[s * H + h] = g;
-                if (MODE == TRAIN) {
-                    dw3 = fmaf(gy[s], a2, dw3);
-                    db2 += g;
-                    if (h == 0) db3 += gy[s];
-                }
+            // d y / d x: sum over hidden units of W1[h][d] g_z1[h]
+            for (int e = tid; e < ST * D; e += NT) {
+                int s = e / D, d = e % D;
+                float acc = 0.f;
+#pragma unroll 8
+                for (int k = 0; k < H; ++k) acc = fmaf(__bfloat162float(W1t[d * WS + k]), g1s[s * H + k], acc);
+                if (s < ns) a.G[(s0 + s) * D + d] = acc;
             }
-            __syncthreads();
-            float a1h[S];
-#pragma unroll
-            for (int s = 0; s < S; ++s) a1h[s] = a1s[s * H + h];
-            if (MODE == TRAIN) {
-                for (int o = 0; o < H; ++o) {
-                    float acc = 0.f;
-#pragma unroll
-                    for (int s = 0; s < S; ++s) acc = fmaf(gzs[s * H + o], a1h[s], acc);
-                    dW2[o * H + h] += acc;
-                }
-            }
-            // through W2 and the first activation
-            float gz1[S];
-#pragma unroll
-            for (int s = 0; s < S; ++s) gz1[s] = 0.f;
-            for (int o = 0; o < H; ++o) {
-                float w = __bfloat162float(W2s[o * H + h]);
-#pragma unroll
-                for (int s = 0; s < S; ++s) gz1[s] = fmaf(w, gzs[s * H + o], gz1[s]);
-            }
-#pragma unroll
-            for (int s = 0; s < S; ++s) {
-                float sg = sigm(z1[s]);
-                gz1[s] *= sg * (1.f + z1[s] * (1.f - sg));
-            }
-            if (MODE == TRAIN) {
-#pragma unroll
-                for (int s = 0; s < S; ++s) db1 += gz1[s];
-                for (int d = 0; d < D; ++d) {
-                    float acc = 0.f;
-#pragma unroll
-                    for (int s = 0; s < S; ++s) acc = fmaf(gz1[s], xs[s * MAXD + d], acc);
-                    dW1[d * H + h] += acc;
-                }
-            } else {
-                // d y / d x: sum over hidden units of W1[h][d] g_z1[h]
-                __syncthreads();
-#pragma unroll
-                for (int s = 0; s < S; ++s) gzs[s * H + h] = gz1[s];
-                __syncthreads();
-                for (int e = h; e < S * D; e += H) {
-                    int s = e / D, d = e % D;
-                    float acc = 0.f;
-                    for (int k = 0; k < H; ++k) acc = fmaf(__bfloat162float(W1t[d * H + k]), gzs[s * H + k], acc);
-                    if (s < ns) a.G[(s0 + s) * D + d] = acc;
-                }
-            }
-            __syncthreads();
         }
+        __syncthreads();
+        if (tile + gridDim.x < ntiles) load_x(tile + gridDim.x);
     }
-    if (MODE != TRAIN) return;
-    float* out = a.partial + (long)blockIdx.x * (a.P + 1);
-    for (int d = 0; d < D; ++d) out[a.W1 + (long)h * D + d] = dW1[d * H + h];
-    out[a.b1 + h] = db1;
-    for (int o = 0; o < H; ++o) out[a.W2 + (long)o * H + h] = dW2[o * H + h];
-    out[a.b2 + h] = db2;
-    out[a.w3 + h] = dw3;
-    if (h == 0) {
-        out[a.b3] = db3;
-        out[a.P] = lsum;
+    if constexpr (MODE == TRAIN) {
+        float* out = a.partial + (long)blockIdx.x * (a.P + 1);
+#pragma unroll
+        for (int q = 0; q < MAXD / 4; ++q)
+            if (sg + 4 * q < D) out[a.W1 + (long)h * D + sg + 4 * q] = dW1[q];
+#pragma unroll
+        for (int q = 0; q < H / 4; ++q) out[a.W2 + (long)(32 * sg + q) * H + h] = dW2[q];
+        if (sg == 0) out[a.w3 + h] = dw3;
+        if (sg == 1) out[a.b2 + h] = db2;
+        if (sg == 2) out[a.b1 + h] = db1;
+        if (sg == 3 && h == 0) {
+            out[a.b3] = db3;
+            out[a.P] = lsum;
+        }
     }
 }
 
@@ -247,6 +325,7 @@ __global__ void k_mlp_reduce_adam(long P, int nblk, const float* __restrict__ pa
     long p = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p > P) return;
     float g = 0.f;
+#pragma unroll 8
     for (int c = 0; c < nblk; ++c) g += partial[(long)c * (P + 1) + p];
     if (p == P) {
         if (loss_out) *loss_out = g;
@@ -280,8 +359,8 @@ __global__ void k_mlp_sync_bf16(long P, const float* master, __nv_bfloat16* W1b,
 
 // ---------------------------------------------------------------------------
 // Forward pass on the 5th-generation tensor cores (prediction without input
-// gradients).  One CTA of 128 threads takes tiles of 128 samples, thread t =
-// sample t of the tile = TMEM lane t:
+// gradients).  One CTA of 512 threads takes tiles of 128 samples (sample s = TMEM
+// lane s), four threads per sample, each a quarter of the hidden units:
 //   layer 1 (n_in x 128, small) on the FP32 cores, exactly as k_mlp_pass;
 //   layer 2 (128 x 128 x 128) as tcgen05.mma kind::tf32 with the product in
 //     tensor memory: a1 is split into a TF32 high part and the FP32 remainder
@@ -289,6 +368,8 @@ __global__ void k_mlp_sync_bf16(long P, const float* master, __nv_bfloat16* W1b,
 //     hi W2^T + lo W2^T is FP32-accurate (the remainder's own truncation to TF32
 //     costs at most 2^-21 |a1|);
 //   the output layer on the FP32 cores from the product read back by tcgen05.ld.
+// The FP32 parts (layer 1 and 256 SiLUs per sample) set the time: 65,536 samples
+// took 140 us with one thread per sample, 50 us now.
 // Operands sit in shared memory in the canonical K-major layout without
 // swizzle: 8-row x 16-byte core matrices, the two core matrices of one MMA's K
 // slice 128 bytes apart (leading byte offset), consecutive 8-row groups 4096
@@ -296,13 +377,15 @@ __global__ void k_mlp_sync_bf16(long P, const float* master, __nv_bfloat16* W1b,
 // them to an mbarrier; the others wait on it with a bounded spin.
 constexpr int TC_M = 128;                    // samples per tile = MMA M = TMEM lanes
 constexpr unsigned TC_LBO = 128, TC_SBO = 4096;
+constexpr int TC_T = 4 * TC_M;               // threads of the CTA
 constexpr long kTcSpin = 1L << 24;           // bounded waits (about a second)
 
 struct TcSmem {
-    float Ahi[TC_M * H];                     // 64 KB each, canonical K-major layout
-    float Alo[TC_M * H];
+    float Ahi[TC_M * H];                     // 64 KB each, canonical K-major layout; after the product the output sums
+                                             // of each quarter of the hidden units [4][sample]
+    float Alo[TC_M * H];                     // first the tile's inputs [sample][n_in | 1]
     float W2f[H * H];                        // rows = output units
-    __nv_bfloat16 W1t[MAXD * H];             // layer 1 weights [d][h]
+    float W1t[MAXD * H];                     // layer 1 weights [d][h]
     float b1[H], b2[H], w3[H];
     unsigned long long bar;                  // MMA completion
     unsigned tmem_base;
@@ -359,14 +442,60 @@ __device__ __forceinline__ void tc_ld32(unsigned taddr, float (&v)[32]) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
 
+// z[0..1] += a * b, two FP32 multiply-adds in one instruction
+__device__ __forceinline__ void fma2(float* z, float2 a, float2 b) {
+    float2 c = make_float2(z[0], z[1]);
+    unsigned long long& cc = *reinterpret_cast<unsigned long long*>(&c);
+    asm("fma.rn.f32x2 %0, %1, %2, %0;"
+        : "+l"(cc)
+        : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));
+    z[0] = c.x;
+    z[1] = c.y;
+}
+
 // y = MLP(x) for a.N samples (a.Y); *err = 1 if a bounded wait gave up.
-__global__ void __launch_bounds__(TC_M, 1) k_mlp_forward_tc(MlpArgs a, int* err) {
+__global__ void __launch_bounds__(TC_T, 1) k_mlp_forward_tc(MlpArgs a, int* err) {
     extern __shared__ __align__(1024) unsigned char tc_raw[];
     TcSmem& sm = *reinterpret_cast<TcSmem*>(tc_raw);
     const int tid = threadIdx.x, warp = tid >> 5, D = a.D;
-    for (int e = tid; e < H * H; e += TC_M) sm.W2f[tc_idx(e / H, e % H)] = __bfloat162float(a.W2b[e]);
-    for (int e = tid; e < H * D; e += TC_M) sm.W1t[(e % D) * H + e / D] = a.W1b[e];
-    for (int h = tid; h < H; h += TC_M) {
+    const int smp = tid & (TC_M - 1), hq = tid / TC_M;  // sample of the tile, quarter of the hidden units
+    const int XD = D | 1;
+    auto load_x = [&](long tile) {
+        const long left = a.N - tile * TC_M;
+        const int n = (int)(left < TC_M ? left : TC_M) * D;
+        const float* X = a.X + tile * TC_M * D;
+        for (int e = tid; e < TC_M * D; e += TC_T) {
+            const int q = e / D;
+            float* dst = sm.Alo + e + q * (XD - D);
+            if (e < n) cp_async4(dst, X + e);
+            else *dst = 0.f;
+        }
+    };
+    load_x(blockIdx.x);
+    {
+        uint4 v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = reinterpret_cast<const uint4*>(a.W2b)[tid + q * TC_T];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int e = 8 * (tid + q * TC_T);
+            const unsigned u[4] = {v[q].x, v[q].y, v[q].z, v[q].w};
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u[2 * x]));
+                const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u[2 * x + 1]));
+                *reinterpret_cast<float4*>(sm.W2f + tc_idx(e / H, e % H + 4 * x)) = make_float4(lo.x, lo.y, hi.x, hi.y);
+            }
+        }
+        __nv_bfloat16 w[MAXD / 4];
+#pragma unroll
+        for (int q = 0; q < MAXD / 4; ++q)
+            if (hq + 4 * q < D) w[q] = a.W1b[smp * D + hq + 4 * q];
+#pragma unroll
+        for (int q = 0; q < MAXD / 4; ++q)
+            if (hq + 4 * q < D) sm.W1t[(hq + 4 * q) * H + smp] = __bfloat162float(w[q]);
+    }
+    for (int h = tid; h < H; h += TC_T) {
         sm.b1[h] = a.master[a.b1 + h];
         sm.b2[h] = a.master[a.b2 + h];
         sm.w3[h] = __bfloat162float(a.w3b[h]);
@@ -387,28 +516,46 @@ __global__ void __launch_bounds__(TC_M, 1) k_mlp_forward_tc(MlpArgs a, int* err)
     __syncthreads();
     tc_fence_after();
     const unsigned tmem = sm.tmem_base;
-    const unsigned lane_addr = tmem + ((unsigned)(warp * 32) << 16);
+    const unsigned lane_addr = tmem + ((unsigned)((warp & 3) * 32) << 16) + (unsigned)(32 * hq);
     const float b3 = a.master[a.b3];
     const long ntiles = (a.N + TC_M - 1) / TC_M;
     unsigned parity = 0;
     for (long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const long s = tile * TC_M + tid;
-        const bool valid = s < a.N;
+        const long s0 = tile * TC_M;
+        const bool valid = s0 + smp < a.N;
+        const float* xs = sm.Alo;
+        cp_async_all();
+        __syncthreads();
         // layer 1 on the FP32 cores, in k_mlp_pass's order: z1 = b1 + sum_d W1[h][d] x[d]
-        float z[H];
+        float z[H / 4];
 #pragma unroll
-        for (int h = 0; h < H; ++h) z[h] = sm.b1[h];
+        for (int h = 0; h < H / 4; ++h) z[h] = sm.b1[32 * hq + h];
         for (int d = 0; d < D; ++d) {
-            const float xd = valid ? a.X[s * D + d] : 0.f;
+            const float xd = xs[smp * XD + d];
+            const float2 x2 = make_float2(xd, xd);
+            const float4* wr = reinterpret_cast<const float4*>(sm.W1t + d * H + 32 * hq);
 #pragma unroll
-            for (int h = 0; h < H; ++h) z[h] = fmaf(__bfloat162float(sm.W1t[d * H + h]), xd, z[h]);
+            for (int q = 0; q < H / 16; ++q) {
+                const float4 w = wr[q];
+                fma2(z + 4 * q, make_float2(w.x, w.y), x2);
+                fma2(z + 4 * q + 2, make_float2(w.z, w.w), x2);
+            }
         }
+        __syncthreads();  // the inputs have been read
 #pragma unroll
-        for (int h = 0; h < H; ++h) {
-            const float a1 = z[h] * sigm(z[h]);
-            const float hi = __uint_as_float(__float_as_uint(a1) & 0xffffe000u);  // exact in TF32
-            sm.Ahi[tc_idx(tid, h)] = hi;
-            sm.Alo[tc_idx(tid, h)] = a1 - hi;
+        for (int h = 0; h < H / 4; h += 4) {
+            float4 hi, lo;
+            float* ph = &hi.x;
+            float* pl = &lo.x;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float a1 = z[h + e] * sigm(z[h + e]);
+                ph[e] = __uint_as_float(__float_as_uint(a1) & 0xffffe000u);  // exact in TF32
+                pl[e] = a1 - ph[e];
+            }
+            const int at = tc_idx(smp, 32 * hq + h);  // four consecutive k of one core-matrix row
+            *reinterpret_cast<float4*>(sm.Ahi + at) = hi;
+            *reinterpret_cast<float4*>(sm.Alo + at) = lo;
         }
         // the tile's operands, written by every thread, become visible to the tensor core
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -434,22 +581,24 @@ __global__ void __launch_bounds__(TC_M, 1) k_mlp_forward_tc(MlpArgs a, int* err)
             break;
         }
         tc_fence_after();
-        float y = b3;
-#pragma unroll
-        for (int c = 0; c < H / 32; ++c) {
-            float v[32];
-            tc_ld32(lane_addr + (unsigned)(32 * c), v);
+        // the operands are free: the next tile's inputs arrive during the output layer
+        if (tile + gridDim.x < ntiles) load_x(tile + gridDim.x);
+        {
+            float v[32], y = 0.f;
+            tc_ld32(lane_addr, v);
             asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
             for (int q = 0; q < 32; ++q) {
-                const float z2 = v[q] + sm.b2[32 * c + q];
-                y = fmaf(sm.w3[32 * c + q], z2 * sigm(z2), y);
+                const float z2 = v[q] + sm.b2[32 * hq + q];
+                y = fmaf(sm.w3[32 * hq + q], z2 * sigm(z2), y);
             }
+            sm.Ahi[hq * TC_M + smp] = y;  // the product is complete: its operands are free
         }
-        if (valid) a.Y[s] = y;
         // every thread's reads of the product precede the next tile's MMAs into it
         tc_fence_before();
         __syncthreads();
+        if (hq == 0 && valid)
+            a.Y[s0 + smp] = b3 + ((sm.Ahi[smp] + sm.Ahi[TC_M + smp]) + (sm.Ahi[2 * TC_M + smp] + sm.Ahi[3 * TC_M + smp]));
     }
     __syncthreads();
     if (warp == 0) {
@@ -509,7 +658,7 @@ mra_status launch_train_pass(mra_mlp* n) {
     MlpArgs a = args_of(n, n->N, n->X);
     long ntiles = (n->N + S - 1) / S;
     n->grid_train = (int)std::min<long>(ntiles, n->sms);
-    k_mlp_pass<TRAIN><<<n->grid_train, H, smem_bytes(TRAIN, n->D), n->stream>>>(a);
+    k_mlp_pass<TRAIN, S><<<n->grid_train, NT, smem_bytes(TRAIN, n->D, S), n->stream>>>(a);
     MCU(cudaGetLastError());
     return MRA_OK;
 }
@@ -579,11 +728,15 @@ mra_status mra_mlp_create(int32_t n_in, int32_t hidden, uint64_t seed, mra_mlp**
     MALLOC(n->grad, (size_t)(P + 1) * sizeof(float));
     MALLOC(n->loss, sizeof(float));
 #undef MALLOC
-    for (int mode = 0; mode < 3; ++mode) {
-        size_t sb = smem_bytes(mode, n_in);
-        cudaError_t e = mode == TRAIN ? cudaFuncSetAttribute(k_mlp_pass<TRAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb)
-                        : mode == PREDICT ? cudaFuncSetAttribute(k_mlp_pass<PREDICT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb)
-                                          : cudaFuncSetAttribute(k_mlp_pass<PREDICT_GRAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb);
+    {
+        cudaError_t e = cudaFuncSetAttribute(k_mlp_pass<TRAIN, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)smem_bytes(TRAIN, n_in, S));
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k_mlp_pass<PREDICT_GRAD, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)smem_bytes(PREDICT_GRAD, n_in, S));
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k_mlp_pass<PREDICT_GRAD, SQ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)smem_bytes(PREDICT_GRAD, n_in, SQ));
         if (e != cudaSuccess) return fail_free(mfail(MRA_ERR_CUDA, std::string("mra_mlp: smem attribute: ") + cudaGetErrorString(e)));
     }
     {
@@ -712,15 +865,20 @@ mra_status mra_mlp_predict(mra_mlp* n, const float* x, int64_t N, float* y, floa
     a.Y = n->Yq;
     a.G = n->Gq;
     if (dydx) {
-        const long ntiles = (N + S - 1) / S;
-        const int grid = (int)std::min<long>(ntiles, 4L * n->sms);
-        k_mlp_pass<PREDICT_GRAD><<<grid, H, smem_bytes(PREDICT_GRAD, n->D), n->stream>>>(a);
+        // few samples: small tiles over many CTAs (the pass is latency); many: more work per weight load
+        if (N <= (long)SQ * 2 * n->sms) {
+            const int grid = (int)((N + SQ - 1) / SQ);
+            k_mlp_pass<PREDICT_GRAD, SQ><<<grid, NT, smem_bytes(PREDICT_GRAD, n->D, SQ), n->stream>>>(a);
+        } else {
+            const int grid = (int)std::min<long>((N + S - 1) / S, (long)n->sms);
+            k_mlp_pass<PREDICT_GRAD, S><<<grid, NT, smem_bytes(PREDICT_GRAD, n->D, S), n->stream>>>(a);
+        }
     } else {
         // values only: the 128 x 128 layer on the tensor cores (tcgen05), 128 samples per tile
         MCU(cudaMemsetAsync(n->tc_err, 0, sizeof(int), n->stream));
         const long ntiles = (N + TC_M - 1) / TC_M;
         const int grid = (int)std::min<long>(ntiles, n->sms);
-        k_mlp_forward_tc<<<grid, TC_M, sizeof(TcSmem), n->stream>>>(a, n->tc_err);
+        k_mlp_forward_tc<<<grid, TC_T, sizeof(TcSmem), n->stream>>>(a, n->tc_err);
     }
     MCU(cudaGetLastError());
     MCU(cudaMemcpyAsync(y, n->Yq, (size_t)N * sizeof(float), cudaMemcpyDeviceToHost, n->stream));
