@@ -95,12 +95,23 @@ struct mra_ctx {
     int graph_timed[2] = {0, 0};     // timed stages of the log-likelihood / prediction graph
     int graph_launches[2] = {0, 0};  // kernels launched by each
     int graph_cov[2] = {0, 0};       // timed covariance-block launches of each
-    double* d_theta = nullptr;  // 16 doubles
+    double* d_theta = nullptr;  // 16 doubles, then the three fields' weights
+    std::vector<double> h_theta;
     double* d_weights[3]{};
     long nb[3]{};
     std::vector<double> model_weights[3];
     double model_intercept[3]{};
-    double* d_result = nullptr;  // [0] d
+    // one evaluation's outcome: work-queue counters and error words (cleared by one
+    // memset), then d; copied to host memory by the evaluation itself
+    static constexpr int kStatusInts = kQueueCounters + 4;
+    int* d_status = nullptr;     // kStatusInts ints, then d
+    double* d_result = nullptr;  // d
+    struct Outcome {
+        int err[4];
+        double d;
+    };
+    Outcome* h_outcome = nullptr;  // pinned
+    bool stats_pending = false;    // the last evaluation's event times are still to be read
     double flop_loglik = 0, flop_reference = 0;
     int64_t u_total = 0;
     mra_stats stats{};
@@ -134,6 +145,7 @@ struct mra_ctx {
             if (e) cudaEventDestroy(e);
         for (auto& e : cev)
             if (e) cudaEventDestroy(e);
+        if (h_outcome) cudaFreeHost(h_outcome);
         if (fork) cudaEventDestroy(fork);
         if (join) cudaEventDestroy(join);
         if (side) cudaStreamDestroy(side);
@@ -293,8 +305,7 @@ mra_status run_eval(mra_ctx* c, bool predict) {
     const bool mixed = c->precision == MRA_PRECISION_MIXED;
     DevTree<double>& td = c->td;
     DevTree<float>& tf = c->tf32;
-    CU(cudaMemsetAsync(td.queue, 0, kQueueCounters * sizeof(int), st));
-    CU(cudaMemsetAsync(td.err, 0, 4 * sizeof(int), st));
+    CU(cudaMemsetAsync(c->d_status, 0, mra_ctx::kStatusInts * sizeof(int), st));
     const long np_all = c->n_int * c->r + c->n_obs + c->n_pred;
     const long rr = (long)c->r * c->r;
     int i = 0, launched = 0;
@@ -388,6 +399,7 @@ mra_status run_eval(mra_ctx* c, bool predict) {
         CU(record(c->tev[2 * i + 1], st, capturing));
         ++i;
     }
+    CU(cudaMemcpyAsync(c->h_outcome, td.err, sizeof(mra_ctx::Outcome), cudaMemcpyDeviceToHost, st));
     CU(cudaGetLastError());
     c->n_timed = i;
     c->n_cov = cov.used;
@@ -396,14 +408,12 @@ mra_status run_eval(mra_ctx* c, bool predict) {
     return MRA_OK;
 }
 
-int* err_ptr(mra_ctx* c) { return c->td.err; }
-
-mra_status finish_eval(mra_ctx* c) {
-    CU(cudaStreamSynchronize(c->stream));
-    int err[4];
-    double d;
-    CU(cudaMemcpy(err, err_ptr(c), sizeof(err), cudaMemcpyDeviceToHost));
-    CU(cudaMemcpy(&d, c->d_result, sizeof(double), cudaMemcpyDeviceToHost));
+// The event times of the last evaluation, read when the statistics are asked for:
+// an optimizer's thousands of evaluations read none, and reading some 40 pairs
+// took longer than the synchronisation itself.
+mra_status read_times(mra_ctx* c) {
+    if (!c->stats_pending) return MRA_OK;
+    c->stats_pending = false;
     mra_stats& s = c->stats;
     s.ms_fields = s.ms_prior = s.ms_finest = s.ms_posterior = s.ms_predict = s.ms_total = 0;
     s.n_timed = c->n_timed;
@@ -433,8 +443,16 @@ mra_status finish_eval(mra_ctx* c) {
     if (c->cov_overflow)  // some covariance launches went untimed: the split is unknown
         for (int i = 0; i < c->n_timed; ++i)
             if (s.timed_kind[i] == MRA_KERNEL_PRIOR_LEVEL) s.timed_ms_cov[i] = -1;
-    s.d = d;
-    s.loglik = -0.5 * (d + (double)c->n_obs * std::log(2 * 3.14159265359));
+    return MRA_OK;
+}
+
+mra_status finish_eval(mra_ctx* c) {
+    CU(cudaStreamSynchronize(c->stream));
+    const int* err = c->h_outcome->err;
+    mra_stats& s = c->stats;
+    c->stats_pending = true;
+    s.d = c->h_outcome->d;
+    s.loglik = -0.5 * (s.d + (double)c->n_obs * std::log(2 * 3.14159265359));
     s.flop_last = c->flop_loglik;
     s.flop_reference = c->flop_reference;
     s.bytes_device = c->bytes;
@@ -930,13 +948,18 @@ mra_status mra_create(const mra_structure* s, const mra_model* m, int32_t precis
         mra_status u = upload(idx[q], tabs[q]->data(), tabs[q]->size() * sizeof(int64_t), c->stream);
         if (u) return bail(u);
     }
-    c->d_theta = c->alloc<double>(16, &ce);
-    if (!ce) c->d_result = c->alloc<double>(4, &ce);
+    for (int f = 0; f < 3; ++f) c->nb[f] = m->nonstationary ? (long)m->field[f].n_basis : 0;
+    c->h_theta.resize(16 + c->nb[0] + c->nb[1] + c->nb[2]);
+    c->d_theta = c->alloc<double>(c->h_theta.size(), &ce);
+    static_assert(mra_ctx::kStatusInts % 2 == 0, "d follows the error words on an 8-byte boundary");
+    if (!ce) c->d_status = static_cast<int*>(c->alloc_bytes(mra_ctx::kStatusInts * sizeof(int) + sizeof(double), &ce));
     if (ce) return bail(fail(MRA_ERR_OOM, "device allocation failed"));
+    c->d_result = reinterpret_cast<double*>(c->d_status + mra_ctx::kStatusInts);
+    if (cudaMallocHost((void**)&c->h_outcome, sizeof(mra_ctx::Outcome)) != cudaSuccess)
+        return bail(fail(MRA_ERR_OOM, "host allocation failed"));
     for (int f = 0; f < 3; ++f) {
-        c->nb[f] = m->nonstationary ? (long)m->field[f].n_basis : 0;
         double* centers = c->alloc<double>(3 * c->nb[f], &ce);
-        if (!ce) c->d_weights[f] = c->alloc<double>(c->nb[f], &ce);
+        c->d_weights[f] = f == 0 ? c->d_theta + 16 : c->d_weights[f - 1] + c->nb[f - 1];
         if (ce) return bail(fail(MRA_ERR_OOM, "device allocation failed: basis"));
         c->model_weights[f].assign(m->nonstationary && c->nb[f] ? m->field[f].weights : nullptr,
                                    m->nonstationary && c->nb[f] ? m->field[f].weights + c->nb[f] : nullptr);
@@ -968,8 +991,8 @@ mra_status mra_create(const mra_structure* s, const mra_model* m, int32_t precis
     if (!ce) sh.heavy_tiles = heavy_tiles = c->alloc<HeavyTile>(h.heavy_tiles.size(), &ce);
     if (!ce) sh.mean = c->alloc<double>(n_pred, &ce);
     if (!ce) sh.var = c->alloc<double>(n_pred, &ce);
-    if (!ce) sh.queue = c->alloc<int>(kQueueCounters, &ce);
-    if (!ce) sh.err = c->alloc<int>(4, &ce);
+    sh.queue = c->d_status;
+    sh.err = c->d_status + kQueueCounters;
     if (!ce) sh.factored = c->alloc<int8_t>(n_int, &ce);
     if (ce) return bail(fail(MRA_ERR_OOM, "device allocation failed: shared vectors"));
     {
@@ -1041,12 +1064,16 @@ mra_status mra_set_theta(mra_ctx* c, const mra_theta* th) {
         return fail(MRA_ERR_ARG, "sill and range must be positive, nugget non-negative");
     for (int f = 3; f < 6; ++f)
         if (!std::isfinite(v[f])) return fail(MRA_ERR_ARG, "intercepts must be finite");
-    CU(cudaMemcpyAsync(c->d_theta, v, sizeof(v), cudaMemcpyHostToDevice, c->stream));
+    // theta and the weights in one copy
+    std::memcpy(c->h_theta.data(), v, sizeof(v));
+    double* at = c->h_theta.data() + 16;
     for (int f = 0; f < 3; ++f) {
         if (!c->nb[f]) continue;
-        const double* w = th->weights[f] ? th->weights[f] : c->model_weights[f].data();
-        CU(cudaMemcpyAsync(c->d_weights[f], w, c->nb[f] * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+        std::memcpy(at, th->weights[f] ? th->weights[f] : c->model_weights[f].data(), c->nb[f] * sizeof(double));
+        at += c->nb[f];
     }
+    CU(cudaMemcpyAsync(c->d_theta, c->h_theta.data(), c->h_theta.size() * sizeof(double), cudaMemcpyHostToDevice,
+                       c->stream));
     return MRA_OK;
 }
 
@@ -1133,6 +1160,7 @@ mra_status capture_one(mra_ctx* c, bool predict, cudaGraph_t* graph, cudaGraphEx
 mra_status mra_capture_graph(mra_ctx* c) {
     if (!c) return fail(MRA_ERR_ARG, "NULL context");
     if (c->shard_split) return fail(MRA_ERR_STATE, "sharded evaluations are not captured");
+    if (mra_status s = read_times(c)) return s;  // capturing replaces the list of timed launches
     if (!c->graph_exec) {
         mra_status s = capture_one(c, false, &c->graph, &c->graph_exec);
         if (s) return s;
@@ -1308,6 +1336,7 @@ mra_status mra_get_terms(mra_ctx* c, double* out, int32_t n_out) {
 
 mra_status mra_get_stats(const mra_ctx* c, mra_stats* out) {
     if (!c || !out) return fail(MRA_ERR_ARG, "NULL argument");
+    if (mra_status s = read_times(const_cast<mra_ctx*>(c))) return s;
     *out = c->stats;
     out->bytes_device = c->bytes;
     out->flop_last = c->flop_loglik;

@@ -40,3 +40,17 @@ def test_finest_level_vs_oracle(case):
     ctx.capture_graph()
     assert ctx.loglik()[0] == d       # the forked launches replay in order
     ctx.close()
+
+
+def test_stats_survive_graph_capture():
+    """The event times of an evaluation are read when the statistics are asked for,
+    also after a capture (which lists the launches of another evaluation) in between."""
+    st, md = random_case(*CASES[0])
+    ctx, (d, _) = run_loglik(st, md)
+    ctx.capture_graph()
+    s = ctx.stats()
+    assert s["d"] == d and s["ms_predict"] == 0 and s["ms_prior"] > 0
+    assert [l["kernel"] for l in s["launches"]].count("prior_level") == st.M - 1
+    ctx.predict()
+    assert ctx.stats()["ms_predict"] > 0
+    ctx.close()
