@@ -121,8 +121,30 @@ struct mra_ctx {
     // the prior levels and the finest level; the posterior is always FP64
     bool mixed_prior32 = true, mixed_finest32 = true;
 
+    // Buffers of at most kSmall bytes share slabs: a cudaMalloc costs some 60 us, and a
+    // small context holds about 60 buffers.
+    static constexpr size_t kSmall = 256 << 10, kSlab = 2 << 20;
+    char* slab = nullptr;
+    size_t slab_left = 0;
     void* alloc_bytes(size_t bytes_, cudaError_t* err) {
         DevBuf b;
+        const size_t need = (std::max<size_t>(bytes_, 16) + 255) & ~size_t(255);
+        if (need <= kSmall) {
+            if (need > slab_left) {
+                b.bytes = kSlab;
+                *err = cudaMalloc(&b.p, b.bytes);
+                if (*err != cudaSuccess) return nullptr;
+                bufs.push_back(b);
+                bytes += b.bytes;
+                slab = static_cast<char*>(b.p);
+                slab_left = kSlab;
+            }
+            void* p = slab;
+            slab += need;
+            slab_left -= need;
+            *err = cudaSuccess;
+            return p;
+        }
         b.bytes = std::max<size_t>(bytes_, 16);
         *err = cudaMalloc(&b.p, b.bytes);
         if (*err != cudaSuccess) return nullptr;
@@ -704,9 +726,10 @@ mra_status mra_create(const mra_structure* s, const mra_model* m, int32_t precis
     int dev = 0, count = 0;
     if (cudaGetDeviceCount(&count) != cudaSuccess || count == 0) return fail(MRA_ERR_NO_DEVICE, "no CUDA device");
     CU(cudaGetDevice(&dev));
-    cudaDeviceProp prop;
-    CU(cudaGetDeviceProperties(&prop, dev));
-    if (prop.major < 10) return fail(MRA_ERR_NO_DEVICE, "an sm_100 (B200) device is required");
+    int major = 0, sms = 0;  // (cudaGetDeviceProperties takes milliseconds)
+    CU(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev));
+    CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if (major < 10) return fail(MRA_ERR_NO_DEVICE, "an sm_100 (B200) device is required");
 
     mra_ctx* c = new mra_ctx();
     auto bail = [&](mra_status st) {
@@ -715,7 +738,7 @@ mra_status mra_create(const mra_structure* s, const mra_model* m, int32_t precis
     };
     c->device = dev;
     c->precision = precision;
-    c->sms = prop.multiProcessorCount;
+    c->sms = sms;
     c->grid = 2 * c->sms;
     c->J = J; c->M = M; c->r = r; c->L = L;
     c->n_int = n_int; c->n_fin = n_fin; c->n_obs = n_obs; c->n_pred = n_pred;

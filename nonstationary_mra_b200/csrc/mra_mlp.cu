@@ -699,13 +699,14 @@ mra_status mra_mlp_create(int32_t n_in, int32_t hidden, uint64_t seed, mra_mlp**
     int dev = 0, count = 0;
     if (cudaGetDeviceCount(&count) != cudaSuccess || count == 0) return mfail(MRA_ERR_NO_DEVICE, "no CUDA device");
     MCU(cudaGetDevice(&dev));
-    cudaDeviceProp prop;
-    MCU(cudaGetDeviceProperties(&prop, dev));
-    if (prop.major != 10) return mfail(MRA_ERR_NO_DEVICE, "mra_mlp: needs an sm_100 device");
+    int major = 0, sms = 0;
+    MCU(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev));
+    MCU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if (major != 10) return mfail(MRA_ERR_NO_DEVICE, "mra_mlp: needs an sm_100 device");
     mra_mlp* n = new mra_mlp();
     n->D = n_in;
     n->lay = Layout(n_in);
-    n->sms = prop.multiProcessorCount;
+    n->sms = sms;
     const long P = n->lay.P;
     auto fail_free = [&](mra_status s) {
         mra_mlp_destroy(n);
