@@ -20,6 +20,7 @@
 //                           one CTA per tile, the block columns in turn
 //   k_finest_terms          log-lik terms summed per sibling group
 #include "mra_cond.cuh"
+#include "mra_tile.cuh"
 
 namespace mra {
 
@@ -184,9 +185,31 @@ __global__ void __launch_bounds__(kThreads, 2) k_finest_regions_f32(Geom g, DevT
 // ---------------------------------------------------------------------------
 // finest regions of more than 64 observations (FP64), in 64 x 64 tiles
 // ---------------------------------------------------------------------------
-// Sigma's lower tiles: one CTA per tile (region h, row tile bi, column tile bj).
-__global__ void __launch_bounds__(kThreads, 2) k_heavy_sigma(Geom g, DevTree<double> t) {
-    LaSmem<double>& sm = la_smem<double>();
+// One CTA per tile throughout, on the tile products of mra_tile.cuh (8-byte copies
+// where a region's odd size leaves its columns unaligned).
+__device__ __forceinline__ bool aligned16(const double* p, long ld) {
+    return ((unsigned long)p & 15ul) == 0 && ld % 2 == 0;
+}
+
+// C(S, S) into Sigma's lower tiles.
+template <int KIND>
+__global__ void __launch_bounds__(kCovThreads, 4) k_cov_heavy(Geom g, DevTree<double> t) {
+    __shared__ __align__(16) double stage[7 * kCovChunk];
+    const HeavyTile ht = t.heavy_tiles[blockIdx.x];
+    const long c = t.heavy[ht.h];
+    if (skipped(t, (long)t.fin_anc[c * t.L + t.L - 1])) return;
+    const long o0 = t.obs_off[c];
+    const int n = (int)(t.obs_off[c + 1] - o0);
+    const int i0 = 64 * ht.bi, j0 = 64 * ht.bj;
+    cov_block<double, KIND>(g, t.pts, t.obs0 + o0 + i0, min(64, n - i0), t.obs0 + o0 + j0, min(64, n - j0),
+                            ht.bi == ht.bj, t.Lsig + t.lsig_off[c] + i0 + (long)j0 * n, n, stage);
+}
+
+// Sigma = C - U_S^T U_S, lower tiles.
+__global__ void __launch_bounds__(kThreads, 2) k_heavy_sigma(DevTree<double> t) {
+    extern __shared__ __align__(16) unsigned char la_dyn_smem[];
+    using TT = Tile<64>;
+    TT::Smem& sm = *reinterpret_cast<TT::Smem*>(la_dyn_smem);
     const long Lr = (long)t.L * t.r;
     const HeavyTile ht = t.heavy_tiles[blockIdx.x];
     const long c = t.heavy[ht.h];
@@ -196,10 +219,12 @@ __global__ void __launch_bounds__(kThreads, 2) k_heavy_sigma(Geom g, DevTree<dou
     const int i0 = 64 * ht.bi, j0 = 64 * ht.bj;
     const int ni = min(64, n - i0), nj = min(64, n - j0);
     double* S = t.Lsig + t.lsig_off[c] + i0 + (long)j0 * n;
-    fill_cov<double>(g, t.pts, t.obs0 + o0 + i0, ni, t.obs0 + o0 + j0, nj, ht.bi == ht.bj, S, n, sm);
-    __syncthreads();
-    gemm<double, true, false>(ni, nj, (int)Lr, -1.0, t.Ufin + (o0 + i0) * Lr, Lr, t.Ufin + (o0 + j0) * Lr, Lr, 1.0, S, n,
-                              sm);
+    const bool vec = Lr % 2 == 0;
+    TT::Acc acc;
+    TT::zero(acc);
+    TT::add(acc, -1.0, S, n, ni, nj);
+    TT::product<true, true>(acc, sm, t.Ufin + (o0 + i0) * Lr, Lr, ni, t.Ufin + (o0 + j0) * Lr, Lr, nj, (int)Lr, vec, vec);
+    TT::store(acc, -1.0, S, n, ni, nj);
 }
 
 // Left-looking block column k of the factorization of [Sigma; V]: the tiles of
@@ -207,7 +232,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_heavy_sigma(Geom g, DevTree<dou
 // product of what is already factored; the diagonal tile is then factored and
 // inverted, and y~_k solved.  blockIdx.x = region * tiles + tile.
 __global__ void __launch_bounds__(kThreads, 2) k_heavy_column(DevTree<double> t, int k, int tiles) {
-    LaSmem<double>& sm = la_smem<double>();
+    extern __shared__ __align__(16) unsigned char la_dyn_smem[];
+    using TT = Tile<64>;
+    TT::Smem& tm = *reinterpret_cast<TT::Smem*>(la_dyn_smem);
     const long Lr = (long)t.L * t.r;
     const int h = blockIdx.x / tiles, tile = blockIdx.x % tiles;
     const long c = t.heavy[h];
@@ -217,18 +244,27 @@ __global__ void __launch_bounds__(kThreads, 2) k_heavy_column(DevTree<double> t,
     const int rows = (n + 63) / 64 - k;  // row tiles of Sigma in this block column
     const int j0 = 64 * k, nj = min(64, n - j0);
     double* S = t.Lsig + t.lsig_off[c];
-    if (tile >= rows) {
-        const long x0 = 64L * (tile - rows);
-        if (x0 >= Lr) return;
-        double* W = t.Bhat + o0 * Lr + x0;
-        gemm<double, false, true>((int)min(64L, Lr - x0), nj, j0, -1.0, W, Lr, S + j0, n, 1.0, W + (long)j0 * Lr, Lr,
-                                  sm);
-        return;
+    const bool vs = aligned16(S, n);
+    const bool inV = tile >= rows;
+    const long x0 = 64L * (tile - rows);
+    if (inV && x0 >= Lr) return;
+    const int i0 = j0 + 64 * tile;
+    double* A = inV ? t.Bhat + o0 * Lr + x0 : S + i0;  // factored columns 0..j0-1 of the row tile
+    const long lda = inV ? Lr : n;
+    const int ni = inV ? (int)min(64L, Lr - x0) : min(64, n - i0);
+    double* W = A + (long)j0 * lda;
+    if (k > 0) {
+        TT::Acc acc;
+        TT::zero(acc);
+        TT::add(acc, -1.0, W, lda, ni, nj);
+        // a pair copy starts at an even row: the valid rows must be even, or rows beyond the tile be readable
+        TT::product<false, false>(acc, tm, A, lda, ni, S + j0, n, nj, j0, (inV ? Lr % 2 == 0 : vs) && ni % 2 == 0,
+                                  vs && nj % 2 == 0);
+        TT::store(acc, -1.0, W, lda, ni, nj);
+        __syncthreads();
     }
-    const int i0 = j0 + 64 * tile, ni = min(64, n - i0);
-    double* W = S + i0 + (long)j0 * n;
-    if (k > 0) gemm<double, false, true>(ni, nj, j0, -1.0, S + i0, n, S + j0, n, 1.0, W, n, sm);
-    if (tile > 0) return;
+    if (inV || tile > 0) return;
+    LaSmem<double>& sm = la_smem<double>();
     double* X = t.heavy_inv + (long)h * 64 * 64;
     double ld = 0.0;
     const int info = potrf_small(nj, W, n, sm, &ld, X, 64);
@@ -238,8 +274,10 @@ __global__ void __launch_bounds__(kThreads, 2) k_heavy_column(DevTree<double> t,
     {
         const int q = threadIdx.x & 63, cg = threadIdx.x >> 6;
         double s = 0.0;
-        if (q < nj)
+        if (q < nj) {
+#pragma unroll 4
             for (int x = cg; x < j0; x += 4) s += S[j0 + q + (long)x * n] * yt[x];
+        }
         part[threadIdx.x] = s;
         __syncthreads();
         if (threadIdx.x < nj) {
@@ -260,7 +298,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_heavy_column(DevTree<double> t,
 
 // The tiles below the diagonal of block column k (and V's) times L_kk^{-T}, in place.
 __global__ void __launch_bounds__(kThreads, 2) k_heavy_panel(DevTree<double> t, int k, int tiles) {
-    LaSmem<double>& sm = la_smem<double>();
+    extern __shared__ __align__(16) unsigned char la_dyn_smem[];
+    using TT = Tile<64>;
+    TT::Smem& sm = *reinterpret_cast<TT::Smem*>(la_dyn_smem);
     const long Lr = (long)t.L * t.r;
     const int h = blockIdx.x / tiles, tile = blockIdx.x % tiles;
     const long c = t.heavy[h];
@@ -285,7 +325,10 @@ __global__ void __launch_bounds__(kThreads, 2) k_heavy_panel(DevTree<double> t, 
         ldw = Lr;
         ni = (int)min(64L, Lr - x0);
     }
-    gemm<double, false, true, true>(ni, nj, nj, 1.0, W, ldw, X, 64, 0.0, W, ldw, sm);
+    TT::Acc acc;
+    TT::zero(acc);
+    TT::product<false, false>(acc, sm, W, ldw, ni, X, 64, nj, nj, aligned16(W, ldw) && ni % 2 == 0, nj % 2 == 0);
+    TT::store(acc, 1.0, W, ldw, ni, nj);
 }
 
 // dfin of each sibling group: the sum of its children's terms, in order (the
@@ -343,16 +386,20 @@ int launch_finest(const Geom& g, const DevTree<T>& t, int grid, bool keep, cudaS
             cudaEventRecord(fk.fork, st);
             cudaStreamWaitEvent(fk.side, fk.fork, 0);
             const int LT = (int)(((long)t.L * t.r + 63) / 64);
-            k_heavy_sigma<<<(unsigned)t.n_heavy_tiles, kThreads, sizeof(LaSmem<T>), fk.side>>>(g, t);
-            ++launches;
+            const size_t sb = sizeof(Tile<64>::Smem);
+            with_cov_kind(cov_kind(g, true), [&](auto k) {
+                k_cov_heavy<decltype(k)::value><<<(unsigned)t.n_heavy_tiles, kCovThreads, 0, fk.side>>>(g, t);
+            });
+            k_heavy_sigma<<<(unsigned)t.n_heavy_tiles, kThreads, sb, fk.side>>>(t);
+            launches += 2;
             const int nb = fk.heavy_blocks[0];
             long act = t.n_heavy;
             for (int k = 0; k < nb; ++k) {
                 while (act > 0 && fk.heavy_blocks[act - 1] <= k) --act;
                 const int tiles = k == 0 ? 1 : nb - k + LT;
-                k_heavy_column<<<(unsigned)(act * tiles), kThreads, sizeof(LaSmem<T>), fk.side>>>(t, k, tiles);
+                k_heavy_column<<<(unsigned)(act * tiles), kThreads, sb, fk.side>>>(t, k, tiles);
                 const int below = nb - k - 1 + LT;
-                k_heavy_panel<<<(unsigned)(act * below), kThreads, sizeof(LaSmem<T>), fk.side>>>(t, k, below);
+                k_heavy_panel<<<(unsigned)(act * below), kThreads, sb, fk.side>>>(t, k, below);
                 launches += 2;
             }
             cudaEventRecord(fk.join, fk.side);
@@ -386,9 +433,9 @@ cudaError_t prepare_finest() {
     set((const void*)k_finest_condition_any<double>, sizeof(LaSmem<double>));
     set((const void*)k_finest_condition_any<float>, sizeof(LaSmem<float>));
     set((const void*)k_finest_regions_f32, sizeof(LaSmem<float>));
-    set((const void*)k_heavy_sigma, sizeof(LaSmem<double>));
-    set((const void*)k_heavy_column, sizeof(LaSmem<double>));
-    set((const void*)k_heavy_panel, sizeof(LaSmem<double>));
+    set((const void*)k_heavy_sigma, sizeof(Tile<64>::Smem));
+    set((const void*)k_heavy_column, sizeof(Tile<64>::Smem));
+    set((const void*)k_heavy_panel, sizeof(Tile<64>::Smem));
     if (e == cudaSuccess) e = prepare_finest_small();
     return e;
 }
