@@ -556,6 +556,7 @@ mra_status setup_tree(mra_ctx* c, DevTree<T>& t, const HostTree& h, const PointS
     t.ws_stride = post_part ? (long)r * c->tf + 2L * c->tf * c->tf + 64 : 64;
     // prior: V of one conditioning step (r x r)
     if (prior_part) t.ws_stride = std::max(t.ws_stride, rr + 64);
+    if (post_part && c->tf <= 128) t.ws_stride = 64;  // the factored steps use the scratch of the covariance buffer
     t.wsd_stride = post_part ? (long)c->tf + 64 : 64;
     if (!post_part) {
         for (int p = 0; p < 2; ++p) aout_sz[p] = wout_sz[p] = F_sz[p] = f_sz[p] = 1;
@@ -591,6 +592,10 @@ mra_status setup_tree(mra_ctx* c, DevTree<T>& t, const HostTree& h, const PointS
     // allocation fails)
     t.cbuf = nullptr;
     t.cbuf_elems = 0;
+    // posterior levels: the scratch of one dense and one factored region at a time, at least
+    long post_need = 0;
+    for (int m = 0; m <= M - 2; ++m)
+        post_need = std::max(post_need, dense_scratch(m, r) + fact_scratch(m, r, std::min(c->tf, 128), c->have_pred) + 4);
     if (prior_part) {
         long need = 0;
         const int SB = prior_batch(sizeof(T) == 8, r, J);
@@ -604,9 +609,7 @@ mra_status setup_tree(mra_ctx* c, DevTree<T>& t, const HostTree& h, const PointS
         if (const char* e = std::getenv("MRA_COV_BUF_MB")) cap_mb = std::max(1L, std::atol(e));
         long elems = std::min(need, cap_mb * (1L << 20) / (long)sizeof(T));
         long floor_elems = std::min(need, (long)(M - 1) * rr * c->grid);  // one region per CTA slot
-        if (post_part)  // and the scratch of one dense region of each posterior level
-            for (int m = 0; m <= M - 2; ++m)
-                if (t.n_dense[m]) floor_elems = std::max(floor_elems, dense_scratch(m, r));
+        if (post_part) floor_elems = std::max(floor_elems, post_need);
         elems = std::max(elems, floor_elems);
         for (;;) {
             cudaError_t e2 = cudaSuccess;
@@ -621,11 +624,10 @@ mra_status setup_tree(mra_ctx* c, DevTree<T>& t, const HostTree& h, const PointS
         // the mixed path's posterior: the FP32 tree's buffer, read as doubles
         t.cbuf = reinterpret_cast<T*>(c->tf32.cbuf);
         t.cbuf_elems = c->tf32.cbuf_elems / 2;
-        for (int m = 0; m <= M - 2; ++m)
-            if (t.n_dense[m] && t.cbuf_elems < dense_scratch(m, r)) {
-                t.cbuf_elems = dense_scratch(m, r);
-                TALLOC(t.cbuf, T, t.cbuf_elems);
-            }
+        if (t.cbuf_elems < post_need) {
+            t.cbuf_elems = post_need;
+            TALLOC(t.cbuf, T, t.cbuf_elems);
+        }
     }
     TALLOC(t.wsd, double, (long)c->grid * t.wsd_stride);
     TALLOC(t.P, T, pred_part ? c->n_pred * (long)L * r : 1);

@@ -233,7 +233,12 @@ inline int prior_batch(bool fp64, int r, int J) {
 cudaError_t prepare_posterior();
 cudaError_t set_gemm_tiles_posterior(const int nw[3]);
 // doubles of scratch of one dense region of level m: the slices (j, m), G and the inverse of L~
-inline long dense_scratch(int m, int r) { return (2L * m + 1) * r * r; }
+inline long dense_scratch(int m, int r) { return ((2L * m + 1) * r * r + 1) & ~1L; }
+// of one factored region (tf rows at most): Y, S and R^{-1}; with `keep` also a dense region's
+inline long fact_scratch(int m, int r, int tf, bool keep) {
+    const long n = (long)r * tf + 2L * tf * tf, d = keep ? dense_scratch(m, r) : 0;
+    return ((n > d ? n : d) + 1) & ~1L;
+}
 template <typename T>
 void launch_predict(const Geom& g, const DevTree<T>& t, int grid, cudaStream_t st);
 template <typename T>

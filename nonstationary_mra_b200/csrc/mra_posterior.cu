@@ -16,8 +16,9 @@
 // regions use the reference's dense r x r slices.  Prediction mode also forms
 // L~, v and G of factored regions from (F, f).
 //
-// A level's factored regions run one CTA each from a queue (k_posterior_factored).
-// Its dense regions run tile by tile, in launches split by what is independent:
+// A level's factored regions (k_fact_*; beyond 128 rows one CTA each from a queue,
+// k_posterior_factored) and its dense ones run tile by tile, in launches split by
+// what is independent.  Dense:
 //   k_dense_gather   slices (j, k) of the summed children contributions, and
 //                    L L^T + A_(m,m): one CTA per tile of a slice
 //   k_dense_factor   L~ with its inverse, v, the log-lik term: one CTA per region
@@ -27,13 +28,15 @@
 // few regions left the chip to as many CTAs (100 to 900 us per level), and a
 // clustered region's thousands of rows were summed by one (1.6 of 3.7 ms of the
 // posterior of a clustered 65,536-point evaluation in one launch).
+#include <algorithm>
+
 #include "mra_kernels.cuh"
 #include "mra_tile.cuh"
 
 namespace mra {
 
 // ---------------------------------------------------------------------------
-// factored regions
+// factored regions of more than 128 rows (MRA_FACTORED_MAX above 128)
 // ---------------------------------------------------------------------------
 // The products of the posterior steps go through a separate function: the
 // steps keep many values live across their products, and inlined there the
@@ -165,7 +168,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_posterior_factored(DevTree<doub
 // prior's covariance buffer, idle by now).
 struct DenseArgs {
     int m, keep;
-    long q0;      // first region of the launch in the level's dense list
+    int col;      // predictive factors of factored regions: only the slices (j, m), from the region's own rows
+    long q0;      // first region of the launch in the level's list (post_order)
     double* scr;  // scratch of region q0
     long per;     // doubles of scratch per region: m slices (j, m), m blocks G, the inverse
 };
@@ -188,14 +192,16 @@ __global__ void __launch_bounds__(Tile<TS>::NT, Tile<TS>::CTAS) k_dense_gather(D
     const int r = t.r, m = a.m;
     const long rr = (long)r * r, mr1 = (long)(m + 1) * r;
     const bool vec = r % 2 == 0;
-    const int ns = (int)n_slices(m + 1), nt2 = nt * nt;
-    const long q = blockIdx.x / (ns * nt2);
-    int s = (int)(blockIdx.x - q * (ns * nt2));
+    const int ns = (int)n_slices(m + 1), tasks = a.col ? m + 1 : ns, nt2 = nt * nt;
+    const long q = blockIdx.x / (tasks * nt2);
+    int s = (int)(blockIdx.x - q * (tasks * nt2));
     const int ti = s % nt2 / nt, tj = s % nt;
     s /= nt2;
-    int j = 0;  // slice s = (j, k), j <= k <= m, row by row
-    while (s >= m + 1 - j) s -= m + 1 - j, ++j;
-    const int k = j + s;
+    int j = a.col ? s : 0, k = m;  // slice s = (j, k), j <= k <= m, row by row; a.col: (s, m)
+    if (!a.col) {
+        while (s >= m + 1 - j) s -= m + 1 - j, ++j;
+        k = j + s;
+    }
     const long i = t.lstart[m] + t.post_order[t.lstart[m] + a.q0 + q];
     if (skipped(t, i)) return;
     const int r0 = ti * TS, c0 = tj * TS;
@@ -215,9 +221,10 @@ __global__ void __launch_bounds__(Tile<TS>::NT, Tile<TS>::CTAS) k_dense_gather(D
             for (int x = wg; x < n; x += WG) w += F[(long)x * mr1 + j * r + r0 + wx] * f[x];
         }
     };
-    if (m == t.M - 2) {
+    if (m == t.M - 2 || a.col) {
         const long lo = t.sub_lo[i];
-        rows(t.Bhat + lo * mr1, t.yt + lo, (int)(t.sub_hi[i] - lo));
+        rows((m == t.M - 2 ? t.Bhat : t.Fbuf[(m + 1) & 1]) + lo * mr1, (m == t.M - 2 ? t.yt : t.fbuf[(m + 1) & 1]) + lo,
+             (int)(t.sub_hi[i] - lo));
     } else {
         const double* Fin = t.Fbuf[(m + 1) & 1];
         const double* fin = t.fbuf[(m + 1) & 1];
@@ -283,7 +290,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_dense_factor(DevTree<double> t,
     for (int e = threadIdx.x; e < r; e += kThreads) part += v[e] * v[e];
     const double vv = cta_sum(part, sm);
     if (threadIdx.x == 0) {
-        t.dpost[i] = ld - t.ldprior[i] - vv;
+        if (!a.col) t.dpost[i] = ld - t.ldprior[i] - vv;
         if (info) report_error(t.err, i);
     }
 }
@@ -380,14 +387,112 @@ __global__ void __launch_bounds__(Tile<TS>::NT, Tile<TS>::CTAS) k_dense_out(DevT
 }
 
 // ---------------------------------------------------------------------------
+// factored regions of at most 128 rows, in tiles
+// ---------------------------------------------------------------------------
+// k_fact_y       Y = L^{-1} F_m^T                      one CTA per tile
+// k_fact_factor  R R^T = I + Y^T Y with R^{-1}, f'     one CTA per region
+// k_fact_out     F' = F_{0..m-1} R^{-T}                one CTA per tile
+// In one CTA per region these were a chain of small products between barriers
+// (tensor pipe 22% busy); the two wide ones now fill the chip.  4,096 regions of
+// about 64 rows and 64 knots with 6 ancestors: 2.09 -> 1.5 ms.
+struct FactArgs {
+    int m, keep;
+    long q0;      // first region of the launch in the level's list (post_order)
+    double* scr;  // scratch of region q0: Y [r x n], S [n x n], R^{-1} [n x n]
+    long per;
+};
+
+template <int TS>
+__global__ void __launch_bounds__(Tile<TS>::NT, Tile<TS>::CTAS) k_fact_y(DevTree<double> t, FactArgs a, int nt, int nc) {
+    extern __shared__ __align__(16) unsigned char la_dyn_smem[];
+    using TT = Tile<TS>;
+    typename TT::Smem& sm = *reinterpret_cast<typename TT::Smem*>(la_dyn_smem);
+    const int r = t.r, m = a.m;
+    const long mr1 = (long)(m + 1) * r;
+    const long q = blockIdx.x / (nt * nc);
+    const int s = (int)(blockIdx.x - q * (nt * nc)), r0 = s / nc * TS, c0 = s % nc * TS;
+    const long i = t.lstart[m] + t.post_order[t.lstart[m] + a.q0 + q];
+    const long lo = t.sub_lo[i];
+    const int n = (int)(t.sub_hi[i] - lo);
+    if (c0 >= n || skipped(t, i)) return;
+    const int M = min(TS, r - r0), N = min(TS, n - c0);
+    const double* F = (m == t.M - 2 ? t.Bhat : t.Fbuf[(m + 1) & 1]) + lo * mr1;
+    const bool vec = r % 2 == 0;
+    typename TT::Acc acc;
+    TT::zero(acc);
+    // the factor's inverse is lower triangular: rows up to r0 + M - 1
+    TT::template product<false, true>(acc, sm, t.Pinv + i * (long)r * r + r0, r, M, F + (long)c0 * mr1 + (long)m * r, mr1, N,
+                                      r0 + M, vec && M % 2 == 0, vec && (r0 + M) % 2 == 0);
+    TT::store(acc, 1.0, a.scr + q * a.per + r0 + (long)c0 * r, r, M, N);
+}
+
+__global__ void __launch_bounds__(kThreads, 2) k_fact_factor(DevTree<double> t, FactArgs a) {
+    LaSmem<double>& sm = la_smem<double>();
+    const int r = t.r, m = a.m;
+    const long q = blockIdx.x;
+    const long i = t.lstart[m] + t.post_order[t.lstart[m] + a.q0 + q];
+    if (skipped(t, i)) return;
+    const long lo = t.sub_lo[i];
+    const int n = (int)(t.sub_hi[i] - lo);
+    if (n == 0) {
+        if (threadIdx.x == 0) t.dpost[i] = 0.0;
+        return;
+    }
+    double* Y = a.scr + q * a.per;
+    double* S = Y + (long)r * n;
+    double* X = S + (long)n * n;
+    gemm<double, true, false>(n, n, r, 1.0, Y, r, Y, r, 0.0, S, n, sm);
+    for (int e = threadIdx.x; e < n; e += kThreads) S[e + (long)e * n] += 1.0;
+    __syncthreads();
+    double ld = 0.0;
+    const int info = potrf_lower<double>(n, S, n, sm, &ld, X, n);
+    // f' = R^{-1} f
+    const double* f = (m == t.M - 2 ? t.yt : t.fbuf[(m + 1) & 1]) + lo;
+    double* fp = m > 0 ? t.fbuf[m & 1] + lo : t.wsd;  // level 0 has one region
+    trmv_lower_inv<double>(n, X, n, fp, f);
+    double part = 0.0;
+    for (int e = threadIdx.x; e < n; e += kThreads) part += f[e] * f[e] - fp[e] * fp[e];
+    const double dd = cta_sum(part, sm);
+    if (threadIdx.x == 0) {
+        t.dpost[i] = ld - dd;
+        if (info) report_error(t.err, i);
+    }
+}
+
+template <int TS>
+__global__ void __launch_bounds__(Tile<TS>::NT, Tile<TS>::CTAS) k_fact_out(DevTree<double> t, FactArgs a, int nx, int nc) {
+    extern __shared__ __align__(16) unsigned char la_dyn_smem[];
+    using TT = Tile<TS>;
+    typename TT::Smem& sm = *reinterpret_cast<typename TT::Smem*>(la_dyn_smem);
+    const int r = t.r, m = a.m;
+    const long mr = (long)m * r, mr1 = mr + r;
+    const long q = blockIdx.x / (nx * nc);
+    const int s = (int)(blockIdx.x - q * (nx * nc)), x0 = s / nc * TS, c0 = s % nc * TS;
+    const long i = t.lstart[m] + t.post_order[t.lstart[m] + a.q0 + q];
+    const long lo = t.sub_lo[i];
+    const int n = (int)(t.sub_hi[i] - lo);
+    if (c0 >= n || skipped(t, i)) return;
+    const int M = (int)min((long)TS, mr - x0), N = min(TS, n - c0);
+    const double* F = (m == t.M - 2 ? t.Bhat : t.Fbuf[(m + 1) & 1]) + lo * mr1;
+    const double* X = a.scr + q * a.per + (long)r * n + (long)n * n;
+    const bool vec = r % 2 == 0;
+    typename TT::Acc acc;
+    TT::zero(acc);
+    // R^{-1} is lower triangular: its rows c0 .. c0 + N - 1 end at column c0 + N - 1
+    TT::template product<false, false>(acc, sm, F + x0, mr1, M, X + c0, n, N, c0 + N, vec && M % 2 == 0,
+                                       n % 2 == 0 && vec);
+    TT::store(acc, 1.0, t.Fbuf[m & 1] + lo * mr + x0 + (long)c0 * mr, mr, M, N);
+}
+
+// ---------------------------------------------------------------------------
 // launcher
 // ---------------------------------------------------------------------------
 template <int TS>
-static int launch_dense(const DevTree<double>& t, int m, bool keep, cudaStream_t st) {
+static int launch_dense(const DevTree<double>& t, int m, long elems, bool keep, cudaStream_t st) {
     const int nt = (t.r + TS - 1) / TS, nt2 = nt * nt;
     const size_t sb = sizeof(typename Tile<TS>::Smem);
-    DenseArgs a{m, keep ? 1 : 0, 0, t.cbuf, dense_scratch(m, t.r)};
-    const long most = t.cbuf_elems / a.per;  // regions whose scratch fits at once
+    DenseArgs a{m, keep ? 1 : 0, 0, 0, t.cbuf, dense_scratch(m, t.r)};
+    const long most = elems / a.per;  // regions whose scratch fits at once
     int launches = 0;
     for (a.q0 = 0; a.q0 < t.n_dense[m]; a.q0 += most) {
         const long n = t.n_dense[m] - a.q0 < most ? t.n_dense[m] - a.q0 : most;
@@ -403,36 +508,84 @@ static int launch_dense(const DevTree<double>& t, int m, bool keep, cudaStream_t
     return launches;
 }
 
-int launch_posterior_level(const DevTree<double>& t, int m, int grid, bool keep, cudaStream_t st, const Fork& fk) {
-    const long nf = level_count(t.J, m) - t.n_dense[m] - (m == t.M - 2 && !keep ? t.n_fused : 0);
+template <int TS>
+static int launch_factored(const DevTree<double>& t, int m, long nf, double* scr, long elems, bool keep, cudaStream_t st) {
+    const size_t sb = sizeof(typename Tile<TS>::Smem);
+    const int nt = (t.r + TS - 1) / TS, nc = (t.tf + TS - 1) / TS, nx = (int)(((long)m * t.r + TS - 1) / TS);
+    const long per = fact_scratch(m, t.r, t.tf, keep);
+    const long most = elems / per;
+    int launches = 0;
+    for (long k0 = 0; k0 < nf; k0 += most) {
+        const long n = nf - k0 < most ? nf - k0 : most;
+        const FactArgs a{m, keep ? 1 : 0, t.n_dense[m] + k0, scr, per};
+        k_fact_y<TS><<<(unsigned)(n * nt * nc), Tile<TS>::NT, sb, st>>>(t, a, nt, nc);
+        k_fact_factor<<<(unsigned)n, kThreads, sizeof(LaSmem<double>), st>>>(t, a);
+        launches += 2;
+        if (m > 0) {
+            k_fact_out<TS><<<(unsigned)(n * nx * nc), Tile<TS>::NT, sb, st>>>(t, a, nx, nc);
+            ++launches;
+        }
+        if (!keep) continue;
+        // predictive factors: L~ L~^T = L L^T + F_m^T F_m, v = L~^{-1} F_m^T f, G = L~^{-1} F_m^T F_{0..m-1}
+        const DenseArgs d{m, 1, 1, a.q0, scr, per};
+        k_dense_gather<TS><<<(unsigned)(n * (m + 1) * nt * nt), Tile<TS>::NT, sb, st>>>(t, d, nt);
+        k_dense_factor<<<(unsigned)n, kThreads, sizeof(LaSmem<double>), st>>>(t, d);
+        launches += 2;
+        if (m == 0) continue;
+        if (t.r <= 128) k_dense_solve<TS><<<(unsigned)(n * m * nt * nt), Tile<TS>::NT, sb, st>>>(t, d, nt);
+        else k_dense_solve_any<<<(unsigned)n, kThreads, sizeof(LaSmem<double>), st>>>(t, d);
+        ++launches;
+    }
+    return launches;
+}
+
+template <int TS>
+static int launch_level(const DevTree<double>& t, int m, long nf, int grid, bool keep, cudaStream_t st, const Fork& fk) {
     int launches = 0;
     // factored regions beside the dense ones (both need only the level below)
     const bool both = nf > 0 && t.n_dense[m] > 0;
+    const bool tiles = t.tf <= 128;
+    cudaStream_t sf = both ? fk.side : st;
+    long elems_f = tiles ? t.cbuf_elems : 0;
     if (both) {
         cudaEventRecord(fk.fork, st);
         cudaStreamWaitEvent(fk.side, fk.fork, 0);
-    }
-    if (t.n_dense[m] > 0)
-        launches += t.r <= 16 ? launch_dense<16>(t, m, keep, st)
-                              : (t.r <= 32 ? launch_dense<32>(t, m, keep, st) : launch_dense<64>(t, m, keep, st));
-    if (nf > 0) {
-        cudaStream_t sf = both ? fk.side : st;
-        k_posterior_factored<<<(unsigned)(nf < grid ? nf : grid), kThreads, sizeof(LaSmem<double>), sf>>>(t, m,
-                                                                                                     keep ? 1 : 0);
-        ++launches;
-        if (both) {
-            cudaEventRecord(fk.join, sf);
-            cudaStreamWaitEvent(st, fk.join, 0);
+        if (tiles) {  // the scratch in two: half each, or what one region needs
+            const long need = fact_scratch(m, t.r, t.tf, keep);
+            elems_f = std::max(need, std::min(t.cbuf_elems / 2, nf * need)) & ~1L;
         }
     }
+    const long elems_d = both ? (t.cbuf_elems - elems_f) & ~1L : t.cbuf_elems;
+    if (t.n_dense[m] > 0) launches += launch_dense<TS>(t, m, elems_d, keep, st);
+    if (nf > 0) {
+        if (tiles) {
+            launches += launch_factored<TS>(t, m, nf, t.cbuf + (both ? elems_d : 0), elems_f, keep, sf);
+        } else {
+            k_posterior_factored<<<(unsigned)(nf < grid ? nf : grid), kThreads, sizeof(LaSmem<double>), sf>>>(
+                t, m, keep ? 1 : 0);
+            ++launches;
+        }
+    }
+    if (both) {
+        cudaEventRecord(fk.join, sf);
+        cudaStreamWaitEvent(st, fk.join, 0);
+    }
     return launches;
+}
+
+int launch_posterior_level(const DevTree<double>& t, int m, int grid, bool keep, cudaStream_t st, const Fork& fk) {
+    const long nf = level_count(t.J, m) - t.n_dense[m] - (m == t.M - 2 && !keep ? t.n_fused : 0);
+    if (t.r <= 16) return launch_level<16>(t, m, nf, grid, keep, st, fk);
+    if (t.r <= 32) return launch_level<32>(t, m, nf, grid, keep, st, fk);
+    return launch_level<64>(t, m, nf, grid, keep, st, fk);
 }
 
 template <int TS>
 static cudaError_t prepare_dense() {
     const int bytes = (int)sizeof(typename Tile<TS>::Smem);
     cudaError_t e = cudaSuccess;
-    for (const void* fn : {(const void*)k_dense_gather<TS>, (const void*)k_dense_solve<TS>, (const void*)k_dense_out<TS>})
+    for (const void* fn : {(const void*)k_dense_gather<TS>, (const void*)k_dense_solve<TS>, (const void*)k_dense_out<TS>,
+                           (const void*)k_fact_y<TS>, (const void*)k_fact_out<TS>})
         if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     return e;
 }
@@ -441,7 +594,8 @@ cudaError_t prepare_posterior() {
     cudaError_t e = prepare_dense<16>();
     if (e == cudaSuccess) e = prepare_dense<32>();
     if (e == cudaSuccess) e = prepare_dense<64>();
-    for (const void* fn : {(const void*)k_posterior_factored, (const void*)k_dense_factor, (const void*)k_dense_solve_any})
+    for (const void* fn : {(const void*)k_posterior_factored, (const void*)k_dense_factor, (const void*)k_dense_solve_any,
+                           (const void*)k_fact_factor})
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LaSmem<double>));
     return e;
