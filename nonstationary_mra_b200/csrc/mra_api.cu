@@ -553,10 +553,10 @@ mra_status setup_tree(mra_ctx* c, DevTree<T>& t, const HostTree& h, const PointS
             f_sz[m & 1] = std::max(f_sz[m & 1], (size_t)c->n_obs);
         }
     }
-    t.ws_stride = post_part ? (long)r * c->tf + 2L * c->tf * c->tf + 64 : 64;
+    // factored steps of more than 128 rows (smaller ones use the covariance buffer)
+    t.ws_stride = post_part && c->tf > 128 ? (long)r * c->tf + 2L * c->tf * c->tf + 64 : 64;
     // prior: V of one conditioning step (r x r)
     if (prior_part) t.ws_stride = std::max(t.ws_stride, rr + 64);
-    if (post_part && c->tf <= 128) t.ws_stride = 64;  // the factored steps use the scratch of the covariance buffer
     t.wsd_stride = post_part ? (long)c->tf + 64 : 64;
     if (!post_part) {
         for (int p = 0; p < 2; ++p) aout_sz[p] = wout_sz[p] = F_sz[p] = f_sz[p] = 1;

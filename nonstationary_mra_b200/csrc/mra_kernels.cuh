@@ -237,7 +237,8 @@ inline long dense_scratch(int m, int r) { return ((2L * m + 1) * r * r + 1) & ~1
 // of one factored region (tf rows at most): Y, S and R^{-1}; with `keep` also a dense region's
 inline long fact_scratch(int m, int r, int tf, bool keep) {
     const long n = (long)r * tf + 2L * tf * tf, d = keep ? dense_scratch(m, r) : 0;
-    return ((n > d ? n : d) + 1) & ~1L;
+    const long e = n > d ? n : d;
+    return e > 2 ? (e + 1) & ~1L : 2;
 }
 template <typename T>
 void launch_predict(const Geom& g, const DevTree<T>& t, int grid, cudaStream_t st);

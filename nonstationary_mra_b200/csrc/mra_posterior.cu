@@ -518,10 +518,11 @@ static int launch_factored(const DevTree<double>& t, int m, long nf, double* scr
     for (long k0 = 0; k0 < nf; k0 += most) {
         const long n = nf - k0 < most ? nf - k0 : most;
         const FactArgs a{m, keep ? 1 : 0, t.n_dense[m] + k0, scr, per};
-        k_fact_y<TS><<<(unsigned)(n * nt * nc), Tile<TS>::NT, sb, st>>>(t, a, nt, nc);
+        // (MRA_FACTORED_MAX = 0 leaves only regions without rows)
+        if (nc > 0) k_fact_y<TS><<<(unsigned)(n * nt * nc), Tile<TS>::NT, sb, st>>>(t, a, nt, nc);
         k_fact_factor<<<(unsigned)n, kThreads, sizeof(LaSmem<double>), st>>>(t, a);
         launches += 2;
-        if (m > 0) {
+        if (m > 0 && nc > 0) {
             k_fact_out<TS><<<(unsigned)(n * nx * nc), Tile<TS>::NT, sb, st>>>(t, a, nx, nc);
             ++launches;
         }
