@@ -13,7 +13,7 @@
 // forward product and column-wise in the backward one, both free of bank conflicts.  The passes are
 // chains of dependent sums of fixed order, a few tiles at most in flight, so what
 // counts is how many of them run side by side: with one thread per hidden unit
-// and 16 samples each the training pass of 160 samples took 42 us, now 19, and the
+// and 16 samples each a training step of 160 samples took 48 us, now 12, and the
 // gradients of 64 samples 55 us, now 9 (4-sample tiles); every sum keeps its order,
 // so the results are bitwise the same.
 #include <cuda_bf16.h>
@@ -36,8 +36,6 @@ constexpr int SQ = 4;      // samples per tile of a small prediction
 constexpr int NT = 4 * H;  // threads of a pass
 constexpr int MAXD = 64;   // largest input width
 constexpr long MAXN = 65536;
-
-enum Mode { TRAIN = 0, PREDICT_GRAD = 1 };
 
 struct Layout {
     long W1, b1, W2, b2, w3, b3, P;
@@ -78,16 +76,16 @@ __device__ __forceinline__ void cp_async_all() { asm volatile("cp.async.wait_all
 
 constexpr int WS = H + 2;  // row stride of W2 and of W1 transposed: consecutive rows fall on different banks
 
-size_t smem_bytes(int mode, int D, int ns) {
+size_t smem_bytes(int D, int ns) {
     return (size_t)H * WS * sizeof(__nv_bfloat16)        // W2 (row-major)
            + (((size_t)D * WS * sizeof(__nv_bfloat16) + 15) & ~(size_t)15)  // W1 transposed [d][h]
            + (size_t)ns * MAXD * sizeof(float)           // x tile
-           + (mode == TRAIN ? 4 : 3) * (size_t)ns * H * sizeof(float)  // a1, g_z2, g_z1 tiles; a2
-           + (size_t)ns * 6 * sizeof(float);             // y partial sums per warp, g_y, errors
+           + 3 * (size_t)ns * H * sizeof(float)          // a1, g_z2, g_z1 tiles
+           + (size_t)ns * 4 * sizeof(float);             // y partial sums per warp
 }
 
 // ST: samples per tile; thread (h, sg) handles hidden unit h of samples sg ST/4 ...
-template <int MODE, int ST>
+template <int ST>
 __global__ void __launch_bounds__(NT, 1) k_mlp_pass(MlpArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int PT = ST / 4;
@@ -100,9 +98,6 @@ __global__ void __launch_bounds__(NT, 1) k_mlp_pass(MlpArgs a) {
     float* gzs = a1s + ST * H;
     float* g1s = gzs + ST * H;
     float* red = g1s + ST * H;
-    float* gys = red + ST * 4;
-    float* es = gys + ST;
-    float* a2s = es + ST;  // TRAIN only
 
 #pragma unroll
     for (int q = 0; q < H * H / 2 / NT; ++q) {
@@ -131,25 +126,10 @@ __global__ void __launch_bounds__(NT, 1) k_mlp_pass(MlpArgs a) {
     }
     const float b1h = a.master[a.b1 + h], b2h = a.master[a.b2 + h], b3 = a.master[a.b3];
     const float w3h = __bfloat162float(a.w3b[h]);
-    float db1 = 0.f, db2 = 0.f, dw3 = 0.f, db3 = 0.f, lsum = 0.f;
-    // TRAIN: dW2[32 sg + q][h] and dW1[sg + 4 q][h]
-    float dW2[MODE == TRAIN ? H / 4 : 1], dW1[MODE == TRAIN ? MAXD / 4 : 1];
-    if (MODE == TRAIN) {
-#pragma unroll
-        for (int q = 0; q < H / 4; ++q) dW2[q] = 0.f;
-#pragma unroll
-        for (int q = 0; q < MAXD / 4; ++q) dW1[q] = 0.f;
-    }
-
     const long ntiles = (a.N + ST - 1) / ST;
     for (long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const long s0 = tile * ST;
         const int ns = (int)min((long)ST, a.N - s0);
-        float tgt[MODE == TRAIN ? PT : 1];
-        if (MODE == TRAIN) {
-#pragma unroll
-            for (int j = 0; j < PT; ++j) tgt[j] = sg * PT + j < ns ? a.T[s0 + sg * PT + j] : 0.f;
-        }
         cp_async_all();
         __syncthreads();
         // layer 1
@@ -195,54 +175,12 @@ __global__ void __launch_bounds__(NT, 1) k_mlp_pass(MlpArgs a) {
         for (int j = 0; j < PT; ++j) {
             const int s = sg * PT + j;
             const float y = b3 + ((red[s * 4 + 0] + red[s * 4 + 1]) + (red[s * 4 + 2] + red[s * 4 + 3]));
-            float gy;
-            if (MODE == TRAIN) {
-                const float e = s < ns ? y - tgt[j] : 0.f;
-                gy = 2.f * e / (float)a.N;
-                if (h == 0) es[s] = e;
-            } else {
-                gy = s < ns ? 1.f : 0.f;
-                if (h == 0 && s < ns) a.Y[s0 + s] = y;
-            }
+            const float gy = s < ns ? 1.f : 0.f;
+            if (h == 0 && s < ns) a.Y[s0 + s] = y;
             const float sg2 = sigm(z2[j]);
             gzs[s * H + h] = gy * w3h * (sg2 * (1.f + z2[j] * (1.f - sg2)));
-            if (MODE == TRAIN) {
-                a2s[s * H + h] = z2[j] * sg2;
-                if (h == 0) gys[s] = gy;
-            }
         }
         __syncthreads();
-        if constexpr (MODE == TRAIN) {
-            float a1h[ST];
-#pragma unroll
-            for (int s = 0; s < ST; ++s) a1h[s] = a1s[s * H + h];
-#pragma unroll
-            for (int q = 0; q < H / 4; q += 4) {
-                float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-                for (int s = 0; s < ST; ++s) {
-                    const float4 gz = *reinterpret_cast<const float4*>(gzs + s * H + 32 * sg + q);
-                    acc[0] = fmaf(gz.x, a1h[s], acc[0]);
-                    acc[1] = fmaf(gz.y, a1h[s], acc[1]);
-                    acc[2] = fmaf(gz.z, a1h[s], acc[2]);
-                    acc[3] = fmaf(gz.w, a1h[s], acc[3]);
-                }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) dW2[q + u] += acc[u];
-            }
-            if (sg == 0) {
-#pragma unroll
-                for (int s = 0; s < ST; ++s) dw3 = fmaf(gys[s], a2s[s * H + h], dw3);
-            } else if (sg == 1) {
-#pragma unroll
-                for (int s = 0; s < ST; ++s) db2 += gzs[s * H + h];
-            } else if (sg == 3 && h == 0) {
-                for (int s = 0; s < ST; ++s) {
-                    lsum += es[s] * es[s];
-                    db3 += gys[s];
-                }
-            }
-        }
         // through W2 and the first activation
         float gz1[PT];
 #pragma unroll
@@ -268,24 +206,7 @@ __global__ void __launch_bounds__(NT, 1) k_mlp_pass(MlpArgs a) {
             g1s[(sg * PT + j) * H + h] = gz1[j];
         }
         __syncthreads();
-        if constexpr (MODE == TRAIN) {
-            float g1h[ST];
-#pragma unroll
-            for (int s = 0; s < ST; ++s) g1h[s] = g1s[s * H + h];
-            if (sg == 2) {
-#pragma unroll
-                for (int s = 0; s < ST; ++s) db1 += g1h[s];
-            }
-#pragma unroll
-            for (int q = 0; q < MAXD / 4; ++q) {
-                const int d = sg + 4 * q;
-                if (d >= D) break;
-                float acc = 0.f;
-#pragma unroll
-                for (int s = 0; s < ST; ++s) acc = fmaf(g1h[s], xs[s * MAXD + d], acc);
-                dW1[q] += acc;
-            }
-        } else {
+        {
             // d y / d x: sum over hidden units of W1[h][d] g_z1[h]
             for (int e = tid; e < ST * D; e += NT) {
                 int s = e / D, d = e % D;
@@ -298,16 +219,213 @@ __global__ void __launch_bounds__(NT, 1) k_mlp_pass(MlpArgs a) {
         __syncthreads();
         if (tile + gridDim.x < ntiles) load_x(tile + gridDim.x);
     }
-    if constexpr (MODE == TRAIN) {
-        float* out = a.partial + (long)blockIdx.x * (a.P + 1);
+}
+
+// ---------------------------------------------------------------------------
+// training pass
+// ---------------------------------------------------------------------------
+// A cluster of four CTAs takes a tile of 16 samples: each CTA runs the forward and
+// backward chains of four of them, one sample and hidden unit per thread, writes
+// what the weight gradients need (a1, g_z2, a2, g_z1, x, g_y) to all four, and then
+// sums a quarter of the weights' gradients over the 16 samples.  The chains are
+// latency: with them spread over four CTAs, and the launches overlapped, a step of 160
+// samples takes 12 us instead of 23 with one CTA per tile, and the order of every sum
+// is the same.
+// Launched with programmatic serialization: the inputs, which no step changes, load
+// while the previous step's Adam kernel runs.
+struct TrainSmem {
+    __nv_bfloat16 W2[H * WS];   // row-major
+    __nv_bfloat16 W1t[MAXD * WS];
+    float x[S * MAXD], a1[S * H], gz[S * H], a2[S * H], g1[S * H];
+    float red[S / 4 * 4], gy[S], err[S];
+};
+
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+// v to the same shared address in each CTA of the cluster
+__device__ __forceinline__ void store_all(float* p, float v) {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        unsigned q;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(q) : "r"(a), "r"(r));
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(q), "f"(v) : "memory");
+    }
+}
+
+__global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(NT, 1) k_mlp_train(MlpArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    TrainSmem& sm = *reinterpret_cast<TrainSmem*>(smem);
+    constexpr int SC = S / 4;  // samples of this CTA, one per thread group
+    const int D = a.D, cr = (int)cluster_rank();
+    const int tid = threadIdx.x, h = tid & (H - 1), sg = tid >> 7, warp = (tid >> 5) & 3, lane = tid & 31;
+    const int smp = cr * SC + sg;  // this thread's sample of the tile
+    const long ntiles = (a.N + S - 1) / S, n_cl = gridDim.x / 4;
+    // the tile's inputs: all 16 samples (the gradients of W1 read them)
+    auto load_x = [&](long tile) {
+        for (int d = lane; d < D; d += 32)
+            for (int s = tid >> 5; s < S; s += NT / 32) {
+                const long i = tile * S + s;
+                if (i < a.N) cp_async4(sm.x + s * MAXD + d, a.X + i * D + d);
+                else sm.x[s * MAXD + d] = 0.f;
+            }
+    };
+    const long tile0 = blockIdx.x / 4;
+    load_x(tile0);
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");  // the weights of the previous step
+#pragma unroll
+    for (int q = 0; q < H * H / 2 / NT; ++q) {
+        const int e = tid + q * NT;
+        cp_async4(reinterpret_cast<unsigned*>(sm.W2) + (e >> 6) * (WS / 2) + (e & 63),
+                  reinterpret_cast<const unsigned*>(a.W2b) + e);
+    }
+    {
+        __nv_bfloat16 v[MAXD / 4];
 #pragma unroll
         for (int q = 0; q < MAXD / 4; ++q)
-            if (sg + 4 * q < D) out[a.W1 + (long)h * D + sg + 4 * q] = dW1[q];
+            if (sg + 4 * q < D) v[q] = a.W1b[h * D + sg + 4 * q];
 #pragma unroll
-        for (int q = 0; q < H / 4; ++q) out[a.W2 + (long)(32 * sg + q) * H + h] = dW2[q];
-        if (sg == 0) out[a.w3 + h] = dw3;
-        if (sg == 1) out[a.b2 + h] = db2;
-        if (sg == 2) out[a.b1 + h] = db1;
+        for (int q = 0; q < MAXD / 4; ++q)
+            if (sg + 4 * q < D) sm.W1t[(sg + 4 * q) * WS + h] = v[q];
+    }
+    const float b1h = a.master[a.b1 + h], b2h = a.master[a.b2 + h], b3 = a.master[a.b3];
+    const float w3h = __bfloat162float(a.w3b[h]);
+    float db = 0.f, db3 = 0.f, lsum = 0.f;  // db: of b1 (sg 2), b2 (sg 1) or w3 (sg 0), on the CTA of that rank
+    // dW2[32 cr + 8 sg + q][h], dW1[4 (4 q + sg) + cr][h]
+    float dW2[H / 16], dW1[MAXD / 16];
+#pragma unroll
+    for (int q = 0; q < H / 16; ++q) dW2[q] = 0.f;
+#pragma unroll
+    for (int q = 0; q < MAXD / 16; ++q) dW1[q] = 0.f;
+
+    cluster_sync();  // every CTA of the cluster runs before any writes to it
+    for (long tile = tile0; tile < ntiles; tile += n_cl) {
+        const long s0 = tile * S;
+        const bool valid = s0 + smp < a.N;
+        const float tgt = valid ? a.T[s0 + smp] : 0.f;
+        cp_async_all();
+        __syncthreads();
+        // layer 1
+        float z1 = b1h;
+#pragma unroll 4
+        for (int d = 0; d < D; ++d) z1 = fmaf(__bfloat162float(sm.W1t[d * WS + h]), sm.x[smp * MAXD + d], z1);
+        const float s1 = sigm(z1), a1 = z1 * s1;
+        store_all(sm.a1 + smp * H + h, a1);
+        __syncthreads();
+        // layer 2 and the output
+        float z2 = b2h;
+        const __nv_bfloat162* w2r = reinterpret_cast<const __nv_bfloat162*>(sm.W2 + h * WS);
+        const float4* ar = reinterpret_cast<const float4*>(sm.a1 + smp * H);
+#pragma unroll 8
+        for (int q = 0; q < H / 4; ++q) {
+            const float2 w0 = __bfloat1622float2(w2r[2 * q]), w1 = __bfloat1622float2(w2r[2 * q + 1]);
+            const float4 x = ar[q];
+            z2 = fmaf(w0.x, x.x, z2);
+            z2 = fmaf(w0.y, x.y, z2);
+            z2 = fmaf(w1.x, x.z, z2);
+            z2 = fmaf(w1.y, x.w, z2);
+        }
+        const float s2 = sigm(z2), a2 = z2 * s2;
+        {
+            float p = w3h * a2;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
+            if (lane == 0) sm.red[sg * 4 + warp] = p;
+        }
+        __syncthreads();
+        // output error and the backward step through the output layer
+        const float y = b3 + ((sm.red[sg * 4 + 0] + sm.red[sg * 4 + 1]) + (sm.red[sg * 4 + 2] + sm.red[sg * 4 + 3]));
+        const float e = valid ? y - tgt : 0.f;
+        const float gy = 2.f * e / (float)a.N;
+        store_all(sm.gz + smp * H + h, gy * w3h * (s2 * (1.f + z2 * (1.f - s2))));
+        store_all(sm.a2 + smp * H + h, a2);
+        if (h == 0) {
+            store_all(sm.gy + smp, gy);
+            store_all(sm.err + smp, e);
+        }
+        __syncthreads();
+        // through W2 and the first activation
+        float gz1 = 0.f;
+#pragma unroll 8
+        for (int o = 0; o < H; o += 4) {
+            const float4 gz = *reinterpret_cast<const float4*>(sm.gz + smp * H + o);
+            gz1 = fmaf(__bfloat162float(sm.W2[(o + 0) * WS + h]), gz.x, gz1);
+            gz1 = fmaf(__bfloat162float(sm.W2[(o + 1) * WS + h]), gz.y, gz1);
+            gz1 = fmaf(__bfloat162float(sm.W2[(o + 2) * WS + h]), gz.z, gz1);
+            gz1 = fmaf(__bfloat162float(sm.W2[(o + 3) * WS + h]), gz.w, gz1);
+        }
+        gz1 *= s1 * (1.f + z1 * (1.f - s1));
+        store_all(sm.g1 + smp * H + h, gz1);
+        cluster_sync();  // the 16 samples of the tile are in every CTA
+        {
+            float v[S];
+#pragma unroll
+            for (int s = 0; s < S; ++s) v[s] = sm.a1[s * H + h];
+#pragma unroll
+            for (int q = 0; q < H / 16; q += 4) {
+                float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int s = 0; s < S; ++s) {
+                    const float4 gz = *reinterpret_cast<const float4*>(sm.gz + s * H + 32 * cr + 8 * sg + q);
+                    acc[0] = fmaf(gz.x, v[s], acc[0]);
+                    acc[1] = fmaf(gz.y, v[s], acc[1]);
+                    acc[2] = fmaf(gz.z, v[s], acc[2]);
+                    acc[3] = fmaf(gz.w, v[s], acc[3]);
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) dW2[q + u] += acc[u];
+            }
+#pragma unroll
+            for (int s = 0; s < S; ++s) v[s] = sm.g1[s * H + h];
+#pragma unroll
+            for (int q = 0; q < MAXD / 16; ++q) {
+                const int d = 4 * (4 * q + sg) + cr;
+                if (d >= D) break;
+                float acc = 0.f;
+#pragma unroll
+                for (int s = 0; s < S; ++s) acc = fmaf(v[s], sm.x[s * MAXD + d], acc);
+                dW1[q] += acc;
+            }
+            if (sg == cr) {
+                if (sg == 0) {
+#pragma unroll
+                    for (int s = 0; s < S; ++s) db = fmaf(sm.gy[s], sm.a2[s * H + h], db);
+                } else if (sg == 1) {
+#pragma unroll
+                    for (int s = 0; s < S; ++s) db += sm.gz[s * H + h];
+                } else if (sg == 2) {
+#pragma unroll
+                    for (int s = 0; s < S; ++s) db += v[s];
+                } else if (h == 0) {
+                    for (int s = 0; s < S; ++s) {
+                        lsum += sm.err[s] * sm.err[s];
+                        db3 += sm.gy[s];
+                    }
+                }
+            }
+        }
+        cluster_sync();  // no CTA's tile is overwritten, and none exits, while another may write to it
+        if (tile + n_cl < ntiles) load_x(tile + n_cl);
+    }
+    float* out = a.partial + tile0 * (a.P + 1);
+#pragma unroll
+    for (int q = 0; q < MAXD / 16; ++q) {
+        const int d = 4 * (4 * q + sg) + cr;
+        if (d < D) out[a.W1 + (long)h * D + d] = dW1[q];
+    }
+#pragma unroll
+    for (int q = 0; q < H / 16; ++q) out[a.W2 + (long)(32 * cr + 8 * sg + q) * H + h] = dW2[q];
+    if (sg == cr) {
+        if (sg == 0) out[a.w3 + h] = db;
+        if (sg == 1) out[a.b2 + h] = db;
+        if (sg == 2) out[a.b1 + h] = db;
         if (sg == 3 && h == 0) {
             out[a.b3] = db3;
             out[a.P] = lsum;
@@ -323,6 +441,8 @@ __global__ void k_mlp_reduce_adam(long P, int nblk, const float* __restrict__ pa
                                   __nv_bfloat16* W2b, __nv_bfloat16* w3b, long oW2, long ob2, long ow3, long ob3,
                                   long ob1, float lr, float bc1, float bc2) {
     long p = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");  // the pass's sums
     if (p > P) return;
     float g = 0.f;
 #pragma unroll 8
@@ -654,12 +774,29 @@ MlpArgs args_of(const mra_mlp* n, long N, const float* X) {
     return a;
 }
 
+// A launch that may start while the stream's previous kernel ends: the kernel itself
+// waits for it (griddepcontrol.wait) before it touches what that kernel writes.
+template <typename... P, typename... A>
+cudaError_t launch_serial(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, P(args)...);
+}
+
 mra_status launch_train_pass(mra_mlp* n) {
     if (n->N <= 0) return mfail(MRA_ERR_STATE, "mra_mlp: no training data (mra_mlp_set_data)");
     MlpArgs a = args_of(n, n->N, n->X);
     long ntiles = (n->N + S - 1) / S;
     n->grid_train = (int)std::min<long>(ntiles, n->sms);
-    k_mlp_pass<TRAIN, S><<<n->grid_train, NT, smem_bytes(TRAIN, n->D, S), n->stream>>>(a);
+    MCU(launch_serial(k_mlp_train, dim3(4 * n->grid_train), dim3(NT), sizeof(TrainSmem), n->stream, a));
     MCU(cudaGetLastError());
     return MRA_OK;
 }
@@ -673,9 +810,9 @@ mra_status launch_reduce(mra_mlp* n, float* grad_out, float* loss_out, float lr)
         bc2 = 1.f - std::pow(0.999f, (float)n->t);
     }
     long blocks = (L.P + 1 + 255) / 256;
-    k_mlp_reduce_adam<<<(unsigned)blocks, 256, 0, n->stream>>>(L.P, n->grid_train, n->partial, grad_out, loss_out,
-                                                                n->master, n->m, n->v, n->W1b, n->W2b, n->w3b, L.W2,
-                                                                L.b2, L.w3, L.b3, L.b1, lr, bc1, bc2);
+    MCU(launch_serial(k_mlp_reduce_adam, dim3((unsigned)blocks), dim3(256), 0, n->stream, L.P, n->grid_train,
+                      (const float*)n->partial, grad_out, loss_out, n->master, n->m, n->v, n->W1b, n->W2b, n->w3b, L.W2,
+                      L.b2, L.w3, L.b3, L.b1, lr, bc1, bc2));
     MCU(cudaGetLastError());
     return MRA_OK;
 }
@@ -733,14 +870,13 @@ mra_status mra_mlp_create(int32_t n_in, int32_t hidden, uint64_t seed, mra_mlp**
     MALLOC(n->loss, sizeof(float));
 #undef MALLOC
     {
-        cudaError_t e = cudaFuncSetAttribute(k_mlp_pass<TRAIN, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem_bytes(TRAIN, n_in, S));
+        cudaError_t e = cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)sizeof(TrainSmem));
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_mlp_pass<PREDICT_GRAD, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem_bytes(PREDICT_GRAD, n_in, S));
+            e = cudaFuncSetAttribute(k_mlp_pass<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(n_in, S));
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_mlp_pass<PREDICT_GRAD, SQ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem_bytes(PREDICT_GRAD, n_in, SQ));
+            e = cudaFuncSetAttribute(k_mlp_pass<SQ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)smem_bytes(n_in, SQ));
         if (e != cudaSuccess) return fail_free(mfail(MRA_ERR_CUDA, std::string("mra_mlp: smem attribute: ") + cudaGetErrorString(e)));
     }
     {
@@ -874,10 +1010,10 @@ mra_status mra_mlp_predict(mra_mlp* n, const float* x, int64_t N, float* y, floa
         // few samples: small tiles over many CTAs (the pass is latency); many: more work per weight load
         if (N <= (long)SQ * 2 * n->sms) {
             const int grid = (int)((N + SQ - 1) / SQ);
-            k_mlp_pass<PREDICT_GRAD, SQ><<<grid, NT, smem_bytes(PREDICT_GRAD, n->D, SQ), n->stream>>>(a);
+            k_mlp_pass<SQ><<<grid, NT, smem_bytes(n->D, SQ), n->stream>>>(a);
         } else {
             const int grid = (int)std::min<long>((N + S - 1) / S, (long)n->sms);
-            k_mlp_pass<PREDICT_GRAD, S><<<grid, NT, smem_bytes(PREDICT_GRAD, n->D, S), n->stream>>>(a);
+            k_mlp_pass<S><<<grid, NT, smem_bytes(n->D, S), n->stream>>>(a);
         }
     } else {
         // values only: the 128 x 128 layer on the tensor cores (tcgen05), 128 samples per tile
