@@ -60,7 +60,7 @@ struct mra_ctx {
     cudaStream_t stream = nullptr;
     cudaStream_t side = nullptr;           // heavy finest regions, beside the small ones
     cudaEvent_t fork = nullptr, join = nullptr;
-    std::vector<int> heavy_blocks;         // 64-wide block columns of each heavy finest region, largest first
+    std::vector<int> heavy_n;              // observations of each heavy finest region, largest first
     cudaEvent_t ev[8]{};
     cudaEvent_t tev[2 * MRA_MAX_TIMED]{};  // start/stop of every launch
     // start/stop of each covariance-block launch of the prior levels, and the
@@ -331,7 +331,7 @@ mra_status run_eval(mra_ctx* c, bool predict) {
     const long np_all = c->n_int * c->r + c->n_obs + c->n_pred;
     const long rr = (long)c->r * c->r;
     int i = 0, launched = 0;
-    const Fork fk{c->side, c->fork, c->join, c->heavy_blocks.data()};
+    const Fork fk{c->side, c->fork, c->join, c->heavy_n.data()};
     c->timed_plan.clear();
     CovTiming cov{c->cev, mra_ctx::kMaxCovTimed, 0, capturing, false};
     for (size_t pi = 0; pi < c->plan.size(); ++pi) {
@@ -895,7 +895,7 @@ mra_status mra_create(const mra_structure* s, const mra_model* m, int32_t precis
     // finest level, small regions: a sibling group whose children hold at most
     // kChildMax observations each and kGroupMax together is one item (FP64), any
     // other region of at most kFinTile is its own; by tile class, most expensive
-    // first.  FP64 regions beyond that are factored tile by tile.  The posterior of
+    // first.  Regions beyond that are factored tile by tile.  The posterior of
     // a factored group taken whole comes with it (FP64 path).
     std::vector<int8_t> fused(cnt2, 0);
     {
@@ -922,7 +922,7 @@ mra_status mra_create(const mra_structure* s, const mra_model* m, int32_t precis
             for (long k = clo; k < chi; ++k) {
                 const double n = (double)h.nfin[k];
                 if (n == 0) continue;
-                if (fp64 && n > kFinTile) heavy.push_back({0, n, (int64_t)k});
+                if (n > kFinTile) heavy.push_back({0, n, (int64_t)k});
                 else items.push_back({tile_class((long)n), n * n * (n + 2.0 * L * r) + 64.0 * n * L * r, (int64_t)(cnt2 + k)});
             }
         }
@@ -936,7 +936,7 @@ mra_status mra_create(const mra_structure* s, const mra_model* m, int32_t precis
         for (size_t q = 0; q < heavy.size(); ++q) {
             h.heavy.push_back(heavy[q].v);
             const int nb = (int)((h.nfin[heavy[q].v] + kFinTile - 1) / kFinTile);
-            c->heavy_blocks.push_back(nb);
+            c->heavy_n.push_back((int)h.nfin[heavy[q].v]);
             for (int bi = 0; bi < nb; ++bi)
                 for (int bj = 0; bj <= bi; ++bj) h.heavy_tiles.push_back({(int32_t)q, (uint16_t)bi, (uint16_t)bj});
         }

@@ -331,6 +331,214 @@ __global__ void __launch_bounds__(kThreads, 2) k_heavy_panel(DevTree<double> t, 
     TT::store(acc, 1.0, W, ldw, ni, nj);
 }
 
+// ---------------------------------------------------------------------------
+// finest regions of more than 64 observations, FP32 storage
+// ---------------------------------------------------------------------------
+// potrf_blocked<float> and trsm_right_lower_trans<float> of a region spread over
+// the chip: per 16-wide panel, every element goes through the same operations in
+// the same order as in one CTA (FP64 diagonal block and panel solves, one rounded
+// FP32 update per panel), so the results are bitwise the same.  Two launches per
+// panel b:
+//   k_heavy32_panel   L's diagonal block b and the rows below it (each CTA factors
+//                     the 16 x 16 block for itself); V's update by panel b - 1
+//   k_heavy32_update  Sigma's lower tiles minus panel b's products; V's columns of
+//                     panel b; the factored diagonal block into place
+// A clustered 65,536-point evaluation spent 6.3 of 11 ms in one CTA's largest
+// region (394 observations); it takes 6.9 ms now.
+struct Heavy32 {
+    float* S;    // Sigma, n x n
+    float* V;    // B^ rows: Lr x n, ld Lr
+    float* D;    // 16 x 16 diagonal block of the current panel, factored (column-major)
+    double* ld;  // running log-determinant
+    long c;
+    int n;
+};
+__device__ __forceinline__ Heavy32 heavy32(const DevTree<float>& t, int h) {
+    Heavy32 r;
+    r.c = t.heavy[h];
+    const long o0 = t.obs_off[r.c];
+    r.n = (int)(t.obs_off[r.c + 1] - o0);
+    r.S = t.Lsig + t.lsig_off[r.c];
+    r.V = t.Bhat + o0 * (long)t.L * t.r;
+    r.D = reinterpret_cast<float*>(t.heavy_inv + (long)h * 64 * 64);
+    r.ld = t.heavy_inv + (long)h * 64 * 64 + 128;
+    return r;
+}
+
+__global__ void __launch_bounds__(kThreads, 2) k_heavy32_sigma(Geom g, DevTree<float> t) {
+    LaSmem<float>& sm = la_smem<float>();
+    const long Lr = (long)t.L * t.r;
+    const HeavyTile ht = t.heavy_tiles[blockIdx.x];
+    const Heavy32 r = heavy32(t, ht.h);
+    const long o0 = t.obs_off[r.c];
+    const int i0 = 64 * ht.bi, j0 = 64 * ht.bj;
+    const int ni = min(64, r.n - i0), nj = min(64, r.n - j0);
+    float* S = r.S + i0 + (long)j0 * r.n;
+    fill_cov<float>(g, t.pts, t.obs0 + o0 + i0, ni, t.obs0 + o0 + j0, nj, ht.bi == ht.bj, S, r.n, sm);
+    __syncthreads();
+    gemm<float, true, false>(ni, nj, (int)Lr, -1.f, t.Ufin + (o0 + i0) * Lr, Lr, t.Ufin + (o0 + j0) * Lr, Lr, 1.f, S, r.n,
+                             sm);
+}
+
+// tasks per region: cs row chunks of 256, then xt x ct tiles of V
+__global__ void __launch_bounds__(kThreads, 2) k_heavy32_panel(DevTree<float> t, int b, int cs, int ct, int tasks) {
+    LaSmem<float>& sm = la_smem<float>();
+    const int tid = threadIdx.x;
+    const Heavy32 r = heavy32(t, blockIdx.x / tasks);
+    int task = blockIdx.x % tasks;
+    const int n = r.n, b0 = 16 * b, nb = min(NB, n - b0), rest = n - b0 - nb;
+    const long lda = n;
+    if (task >= cs) {  // V(:, b0..) -= V(:, panel b - 1) L(b0.., panel b - 1)^T
+        task -= cs;
+        const long Lr = (long)t.L * t.r, x0 = 64L * (task / ct);
+        const int c0 = b0 + 64 * (task % ct), p0 = b0 - NB;
+        if (c0 >= n) return;
+        gemm<float, false, true>((int)min(64L, Lr - x0), min(64, n - c0), NB, -1.f, r.V + x0 + p0 * Lr, Lr,
+                                 r.S + c0 + p0 * lda, lda, 1.f, r.V + x0 + c0 * Lr, Lr, sm);
+        return;
+    }
+    if (task > 0 && 256 * task >= rest) return;
+    for (int e = tid; e < nb * nb; e += kThreads) {
+        int i = e % nb, j = e / nb;
+        sm.D[i][j] = (double)r.S[(b0 + i) + (long)(b0 + j) * lda];
+    }
+    if (tid == 0) sm.flag = 0;
+    __syncthreads();
+    if (tid < 32) {
+        const int lane = tid;
+        for (int k = 0; k < nb; ++k) {
+            if (lane == 0) {
+                double d = sm.D[k][k];
+                if (!(d > 0.0) && sm.flag == 0) sm.flag = b0 + k + 1;
+                double sq = sqrt(d);
+                sm.D[k][k] = sq;
+                sm.inv[k] = 1.0 / sq;
+            }
+            __syncwarp();
+            if (lane > k && lane < nb) sm.D[lane][k] *= sm.inv[k];
+            __syncwarp();
+            if (lane > k && lane < nb) {
+                const double lik = sm.D[lane][k];
+                for (int j = k + 1; j <= lane; ++j) sm.D[lane][j] -= lik * sm.D[j][k];
+            }
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+    if (task == 0) {
+        for (int e = tid; e < nb * nb; e += kThreads) {
+            int i = e % nb, j = e / nb;
+            r.D[e] = j <= i ? (float)sm.D[i][j] : 0.f;
+        }
+        if (tid == 0) {
+            double ld = b == 0 ? 0.0 : *r.ld;
+            for (int k = 0; k < nb; ++k) ld += 2.0 * log(sm.D[k][k]);
+            *r.ld = ld;
+            if (sm.flag) report_error(t.err, t.n_int + r.c);
+        }
+    }
+    for (int row = 256 * task + tid; row < min(rest, 256 * (task + 1)); row += kThreads) {
+        double x[NB];
+        float* p = r.S + (b0 + nb + row) + (long)b0 * lda;
+#pragma unroll
+        for (int i = 0; i < NB; ++i) x[i] = i < nb ? (double)p[(long)i * lda] : 0.0;
+#pragma unroll
+        for (int i = 0; i < NB; ++i) {
+            if (i < nb) {
+                double s = x[i];
+#pragma unroll
+                for (int k = 0; k < i; ++k) s -= sm.D[i][k] * x[k];
+                x[i] = s * sm.inv[i];
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < NB; ++i)
+            if (i < nb) p[(long)i * lda] = (float)x[i];
+    }
+}
+
+// tasks per region: cv row chunks of V, then the lower tiles of the trailing matrix
+__global__ void __launch_bounds__(kThreads, 2) k_heavy32_update(DevTree<float> t, int b, int cv, int tasks) {
+    LaSmem<float>& sm = la_smem<float>();
+    const int tid = threadIdx.x;
+    const Heavy32 r = heavy32(t, blockIdx.x / tasks);
+    int task = blockIdx.x % tasks;
+    const int n = r.n, b0 = 16 * b, nb = min(NB, n - b0), rest = n - b0 - nb;
+    const long lda = n;
+    if (task >= cv) {
+        task -= cv;
+        int ti = 0;
+        while ((ti + 1) * (ti + 2) / 2 <= task) ++ti;
+        const int tj = task - ti * (ti + 1) / 2;
+        if (64 * ti >= rest) return;
+        const float* P = r.S + (b0 + nb) + (long)b0 * lda;
+        gemm<float, false, true>(min(64, rest - 64 * ti), min(64, rest - 64 * tj), nb, -1.f, P + 64 * ti, lda, P + 64 * tj,
+                                 lda, 1.f, r.S + (b0 + nb + 64 * ti) + (long)(b0 + nb + 64 * tj) * lda, lda, sm);
+        return;
+    }
+    if (task == 0)
+        for (int e = tid; e < nb * nb; e += kThreads) r.S[(b0 + e % nb) + (long)(b0 + e / nb) * lda] = r.D[e];
+    for (int e = tid; e < nb * nb; e += kThreads) sm.D[e % nb][e / nb] = (double)r.D[e];
+    __syncthreads();
+    if (tid < nb) sm.inv[tid] = 1.0 / sm.D[tid][tid];
+    __syncthreads();
+    const long Lr = (long)t.L * t.r;
+    for (long row = 256L * task + tid; row < min(Lr, 256L * (task + 1)); row += kThreads) {
+        double x[NB];
+        float* p = r.V + row + (long)b0 * Lr;
+#pragma unroll
+        for (int i = 0; i < NB; ++i) x[i] = i < nb ? (double)p[(long)i * Lr] : 0.0;
+#pragma unroll
+        for (int i = 0; i < NB; ++i) {
+            if (i < nb) {
+                double s = x[i];
+#pragma unroll
+                for (int k = 0; k < i; ++k) s -= sm.D[i][k] * x[k];
+                x[i] = s * sm.inv[i];
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < NB; ++i)
+            if (i < nb) p[(long)i * Lr] = (float)x[i];
+    }
+}
+
+__global__ void __launch_bounds__(kThreads, 2) k_heavy32_terms(DevTree<float> t) {
+    LaSmem<float>& sm = la_smem<float>();
+    const Heavy32 r = heavy32(t, blockIdx.x);
+    const long o0 = t.obs_off[r.c];
+    double* ytc = t.yt + o0;
+    for (int e = threadIdx.x; e < r.n; e += kThreads) ytc[e] = t.y[o0 + e];
+    __syncthreads();
+    trsv_lower_f64<float>(r.n, r.S, r.n, ytc);
+    double part = 0.0;
+    for (int e = threadIdx.x; e < r.n; e += kThreads) part += ytc[e] * ytc[e];
+    const double yy = cta_sum(part, sm);
+    if (threadIdx.x == 0) t.dchild[r.c] = yy + *r.ld;
+}
+
+static int launch_heavy32(const Geom& g, const DevTree<float>& t, const Fork& fk) {
+    const size_t sb = sizeof(LaSmem<float>);
+    cudaStream_t st = fk.side;
+    const long Lr = (long)t.L * t.r;
+    const int nmax = fk.heavy_n[0], xt = (int)((Lr + 63) / 64), cv = (int)((Lr + 255) / 256);
+    k_heavy32_sigma<<<(unsigned)t.n_heavy_tiles, kThreads, sb, st>>>(g, t);
+    int launches = 2;
+    long act = t.n_heavy;
+    for (int b = 0; 16 * b < nmax; ++b) {
+        while (act > 0 && fk.heavy_n[act - 1] <= 16 * b) --act;
+        const int rest = nmax - 16 * b - 16 > 0 ? nmax - 16 * b - 16 : 0;
+        const int cs = rest > 256 ? (rest + 255) / 256 : 1, ct = b > 0 ? (nmax - 16 * b + 63) / 64 : 0;
+        const int tasks = cs + xt * ct;
+        k_heavy32_panel<<<(unsigned)(act * tasks), kThreads, sb, st>>>(t, b, cs, ct > 0 ? ct : 1, tasks);
+        const int tt = (rest + 63) / 64, tasks2 = cv + tt * (tt + 1) / 2;
+        k_heavy32_update<<<(unsigned)(act * tasks2), kThreads, sb, st>>>(t, b, cv, tasks2);
+        launches += 2;
+    }
+    k_heavy32_terms<<<(unsigned)t.n_heavy, kThreads, sb, st>>>(t);
+    return launches;
+}
+
 // dfin of each sibling group: the sum of its children's terms, in order (the
 // slots of regions without observations, and of all but the first of a group
 // processed together, stay zero).
@@ -380,11 +588,13 @@ int launch_finest(const Geom& g, const DevTree<T>& t, int grid, bool keep, cudaS
         }
         launches += 2;
     }
-    if constexpr (sizeof(T) == 8) {
-        if (t.n_heavy > 0) {
-            // the heavy regions' chain of block columns beside the small regions
-            cudaEventRecord(fk.fork, st);
-            cudaStreamWaitEvent(fk.side, fk.fork, 0);
+    if (t.n_heavy > 0) {
+        // the heavy regions' chain of block columns beside the small regions
+        cudaEventRecord(fk.fork, st);
+        cudaStreamWaitEvent(fk.side, fk.fork, 0);
+        if constexpr (sizeof(T) == 4) {
+            launches += launch_heavy32(g, t, fk);
+        } else {
             const int LT = (int)(((long)t.L * t.r + 63) / 64);
             const size_t sb = sizeof(Tile<64>::Smem);
             with_cov_kind(cov_kind(g, true), [&](auto k) {
@@ -392,18 +602,18 @@ int launch_finest(const Geom& g, const DevTree<T>& t, int grid, bool keep, cudaS
             });
             k_heavy_sigma<<<(unsigned)t.n_heavy_tiles, kThreads, sb, fk.side>>>(t);
             launches += 2;
-            const int nb = fk.heavy_blocks[0];
+            const int nb = (fk.heavy_n[0] + 63) / 64;
             long act = t.n_heavy;
             for (int k = 0; k < nb; ++k) {
-                while (act > 0 && fk.heavy_blocks[act - 1] <= k) --act;
+                while (act > 0 && fk.heavy_n[act - 1] <= 64 * k) --act;
                 const int tiles = k == 0 ? 1 : nb - k + LT;
                 k_heavy_column<<<(unsigned)(act * tiles), kThreads, sb, fk.side>>>(t, k, tiles);
                 const int below = nb - k - 1 + LT;
                 k_heavy_panel<<<(unsigned)(act * below), kThreads, sb, fk.side>>>(t, k, below);
                 launches += 2;
             }
-            cudaEventRecord(fk.join, fk.side);
         }
+        cudaEventRecord(fk.join, fk.side);
     }
     if constexpr (sizeof(T) == 8) {
         launches += launch_finest_small(g, t, keep, st);
@@ -412,8 +622,7 @@ int launch_finest(const Geom& g, const DevTree<T>& t, int grid, bool keep, cudaS
                                st>>>(g, t);
         ++launches;
     }
-    if constexpr (sizeof(T) == 8)
-        if (t.n_heavy > 0) cudaStreamWaitEvent(st, fk.join, 0);
+    if (t.n_heavy > 0) cudaStreamWaitEvent(st, fk.join, 0);
     const long cnt2 = level_count(t.J, t.M - 2);
     k_finest_terms<T><<<(unsigned)((cnt2 + 255) / 256), 256, 0, st>>>(t);
     return launches + 1;
@@ -433,6 +642,10 @@ cudaError_t prepare_finest() {
     set((const void*)k_finest_condition_any<double>, sizeof(LaSmem<double>));
     set((const void*)k_finest_condition_any<float>, sizeof(LaSmem<float>));
     set((const void*)k_finest_regions_f32, sizeof(LaSmem<float>));
+    set((const void*)k_heavy32_sigma, sizeof(LaSmem<float>));
+    set((const void*)k_heavy32_panel, sizeof(LaSmem<float>));
+    set((const void*)k_heavy32_update, sizeof(LaSmem<float>));
+    set((const void*)k_heavy32_terms, sizeof(LaSmem<float>));
     set((const void*)k_heavy_sigma, sizeof(Tile<64>::Smem));
     set((const void*)k_heavy_column, sizeof(Tile<64>::Smem));
     set((const void*)k_heavy_panel, sizeof(Tile<64>::Smem));

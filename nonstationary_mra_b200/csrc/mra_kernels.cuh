@@ -204,12 +204,11 @@ template <typename T>
 int launch_prior_level(const Geom& g, const DevTree<T>& t, int m, int grid, cudaStream_t st, CovTiming* tm = nullptr);
 // Stream and events (timing disabled) for work beside the main stream's (heavy
 // finest regions beside small ones, factored regions beside dense ones), and the
-// number of 64-wide block columns of each heavy
-// region (host memory, largest first).
+// number of observations of each heavy region (host memory, largest first).
 struct Fork {
     cudaStream_t side;
     cudaEvent_t fork, join;
-    const int* heavy_blocks;
+    const int* heavy_n;
 };
 // The finest level (without the level M-2 posterior); returns the number of kernels launched.
 template <typename T>
