@@ -532,7 +532,13 @@ mra_status setup_tree(mra_ctx* c, DevTree<T>& t, const HostTree& h, const PointS
     t.n_heavy_tiles = (long)h.heavy_tiles.size();
     t.heavy_inv = sh.heavy_inv;
     // sizes of the level-parity buffers
-    for (int m = 0; m < kMaxLevels; ++m) t.n_dense[m] = 0;
+    for (int m = 0; m < kMaxLevels; ++m) {
+        t.n_dense[m] = t.n_mid[m] = 0;
+        if (m > M - 2) continue;
+        const long s0 = level_start(J, m), cnt = level_count(J, m);
+        for (long q = 0; q < cnt; ++q)
+            t.n_mid[m] += h.factored[s0 + q] && h.sub_hi[s0 + q] - h.sub_lo[s0 + q] > 64;
+    }
     t.n_dense[0] = h.factored[0] ? 0 : 1;
     size_t aout_sz[2] = {1, 1}, wout_sz[2] = {1, 1}, F_sz[2] = {1, 1}, f_sz[2] = {1, 1};
     for (int m = 1; m <= M - 2; ++m) {

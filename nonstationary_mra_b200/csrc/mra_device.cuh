@@ -718,88 +718,6 @@ __device__ inline void gemm_f64(int M, int N, int K, double alpha, const double*
     __syncthreads();
 }
 
-// 16-byte asynchronous global -> shared copy through L2 only (not L1); both
-// addresses 16-byte aligned.
-__device__ __forceinline__ void cp_async16(double* dst, const double* src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
-}
-
-// gemm_f64 for whole tiles (M % 64 == 0, N % (16 NW) == 0, K % 32 == 0) with
-// 16-byte aligned operand rows (aligned A and B, even lda and ldb): the same
-// tiles, the same shared-memory layout and the same per-element K order, hence
-// bitwise the same results, with the operands staged in pairs of elements by
-// 16-byte copies through L2 only -- half the copy instructions and no L1
-// allocation.
-template <bool TA, bool TB, int NW>
-__device__ inline void gemm_f64_wide(int M, int N, int K, double alpha, const double* A, long lda, const double* B,
-                                     long ldb, double beta, double* C, long ldc, LaSmem<double>& sm,
-                                     const double* Cin, long ldcin) {
-    constexpr int W = 16 * NW;
-    constexpr int WM = 8 / NW;
-    constexpr int QA = 64 * TK64 / 2 / kThreads;  // A pairs per thread per slab (4)
-    constexpr int QB = W * TK64 / 2 / kThreads;   // B pairs per thread per slab (NW)
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const int wm = (w % WM) * 8 * NW, wn = (w / WM) * 16;
-    for (int m0 = 0; m0 < M; m0 += 64) {
-        for (int n0 = 0; n0 < N; n0 += W) {
-            AccD<NW> acc;
-#pragma unroll
-            for (int i = 0; i < NW; ++i)
-#pragma unroll
-                for (int j = 0; j < 2; ++j) acc.v[i][j][0] = acc.v[i][j][1] = 0.0;
-            auto issue = [&](int k0, int stage) {
-                double* sA = sm.A[stage];
-                double* sB = sm.B[stage];
-#pragma unroll
-                for (int q = 0; q < QA; ++q) {
-                    const int e = tid + q * kThreads;
-                    // TA: pair (i, k..k+1) of A[k + i lda]; else pair (i..i+1, k) of A[i + k lda]
-                    const int i = TA ? e / (TK64 / 2) : 2 * (e % 32), k = TA ? 2 * (e % (TK64 / 2)) : e / 32;
-                    const double* src = TA ? A + (k0 + k) + (long)(m0 + i) * lda : A + (m0 + i) + (long)(k0 + k) * lda;
-                    cp_async16(sA + (TA ? i * KS64 + k : k * RS64 + i), src);
-                }
-#pragma unroll
-                for (int q = 0; q < QB; ++q) {
-                    const int e = tid + q * kThreads;
-                    // TB: pair (k, j..j+1) of B[j + k ldb]; else pair (k..k+1, j) of B[k + j ldb]
-                    const int j = TB ? 2 * (e % (W / 2)) : e / (TK64 / 2), k = TB ? e / (W / 2) : 2 * (e % (TK64 / 2));
-                    const double* src = TB ? B + (n0 + j) + (long)(k0 + k) * ldb : B + (k0 + k) + (long)(n0 + j) * ldb;
-                    cp_async16(sB + (TB ? k * RS64 + j : j * KS64 + k), src);
-                }
-                cp_async_commit();
-            };
-            issue(0, 0);
-            int stage = 0;
-            for (int k0 = 0; k0 < K; k0 += TK64, stage ^= 1) {
-                if (k0 + TK64 < K) {
-                    issue(k0 + TK64, stage ^ 1);
-                    cp_async_wait<1>();
-                } else {
-                    cp_async_wait<0>();
-                }
-                __syncthreads();
-                warp_step_f64<TA, TB, NW>(acc, sm.A[stage], sm.B[stage], wm, wn, lane);
-                __syncthreads();
-            }
-            const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-            for (int i = 0; i < NW; ++i)
-#pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    const int r = m0 + wm + 8 * i + g, c = n0 + wn + 8 * j + 2 * t;
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        double* p = C + r + (long)(c + h) * ldc;
-                        const double* q = Cin ? Cin + r + (long)(c + h) * ldcin : p;
-                        *p = beta == 0.0 ? alpha * acc.v[i][j][h] : alpha * acc.v[i][j][h] + beta * *q;
-                    }
-                }
-        }
-    }
-    __syncthreads();
-}
-
 // ---- FP32 storage (mixed path): 3xTF32 products, 64 x 64 tiles, K slabs of 16
 struct AccF {
     float v[2][2][4];  // 2 (m16) x 2 (n8) fragments of m16n8
@@ -1024,25 +942,6 @@ __device__ inline void trsm_right_lower_trans(int rows, int n, const T* L, long 
             gemm<T, false, true>(rows, n - b0 - nb, nb, (T)-1, B + (long)b0 * ldb, ldb, L + (b0 + nb) + (long)b0 * ldl,
                                  ldl, (T)1, B + (long)(b0 + nb) * ldb, ldb, sm);
     }
-}
-
-// gemm with the operand staging of gemm_f64_wide where the product qualifies
-// (FP64, whole tiles, 16-byte aligned rows), else gemm; the results are bitwise
-// the same either way.
-template <typename T, bool TA, bool TB>
-__device__ inline void gemm_wide(int M, int N, int K, T alpha, const T* A, long lda, const T* B, long ldb, T beta,
-                                 T* C, long ldc, LaSmem<T>& sm, const T* Cin = nullptr, long ldcin = 0) {
-    if constexpr (sizeof(T) == 8) {
-        const int nw = c_gemm_nw[N <= 16 ? 0 : (N <= 32 ? 1 : 2)];
-        if (M > 0 && K > 0 && M % 64 == 0 && N % (16 * nw) == 0 && K % TK64 == 0 && lda % 2 == 0 && ldb % 2 == 0 &&
-            (((unsigned long)A | (unsigned long)B) & 15ul) == 0) {
-            if (nw == 1) gemm_f64_wide<TA, TB, 1>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, sm, Cin, ldcin);
-            else if (nw == 2) gemm_f64_wide<TA, TB, 2>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, sm, Cin, ldcin);
-            else gemm_f64_wide<TA, TB, 4>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, sm, Cin, ldcin);
-            return;
-        }
-    }
-    gemm<T, TA, TB>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, sm, Cin, ldcin);
 }
 
 // Solves L x = b for one right-hand side entirely in FP64 (the vectors that feed
@@ -1373,6 +1272,117 @@ __device__ inline int potrf_mid(int n, double* A, long lda, LaSmem<double>& sm, 
     __syncthreads();
     if (threadIdx.x == 0 && logdet) *logdet = ld1 + ld2;
     return info1 ? info1 : (info2 ? info2 + 64 : 0);
+}
+
+// The scheme of potrf_core for 64 < n <= 128 with the inverse, by 256 threads, one
+// CTA per SM: L and X = L^{-1} share one array, X transposed above the diagonal
+// blocks (its own diagonal blocks beside it), so that block column k holds X's block
+// row k in the rows above and L's panel below, and one form of tile update,
+//   C(p, q) -= panel(p) panel(q)^T,  q > k, p <= k (X) or p >= q (L),
+// serves both.  A launch of one 100 x 100 factorization 70 -> 46 us against potrf_mid's
+// two factorizations with products through memory between them.
+constexpr int SLD2 = 132;
+struct Potrf128Smem {
+    double S[128 * SLD2];
+    double XD[16][64];  // diagonal blocks of X, column-major
+    double red[kThreads / 32];
+    int flag;
+};
+
+static __device__ __noinline__ int potrf_128(int n, double* A, long lda, double* logdet, double* inv, long ldinv) {
+    extern __shared__ __align__(16) unsigned char la_dyn_smem[];
+    Potrf128Smem& sm = *reinterpret_cast<Potrf128Smem*>(la_dyn_smem);
+    double* S = sm.S;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int g = lane >> 2, t = lane & 3;
+    const int nbk = (n + 7) >> 3, N = nbk << 3;
+    {
+        const int i = tid & 127;
+        for (int j0 = tid >> 7; j0 < N; j0 += 16) {  // eight loads in flight
+            double v[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int j = j0 + 2 * q;
+                v[q] = (i < n && j <= i && j < n) ? A[i + (long)j * lda] : (i == j ? 1.0 : 0.0);
+            }
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+                if (i < N && j0 + 2 * q < N) S[i + (j0 + 2 * q) * SLD2] = v[q];
+        }
+    }
+    __syncthreads();
+    int bad = 0;
+    for (int k = 0; k < nbk; ++k) {
+        const int k0 = k << 3;
+        const int row = k0 + tid, c = tid - 128;
+        const bool prow = tid < 128 && row < N, pcol = tid >= 128 && c < k0;
+        double* base = (tid < 128 ? S + row : S + c) + k0 * SLD2;  // a row of L's panel, or of X's block row transposed
+        double l[36], x[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j <= i; ++j) l[i * (i + 1) / 2 + j] = S[(k0 + i) + (k0 + j) * SLD2];
+        const int e = c - k0;  // column of X's diagonal block
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x[j] = prow || pcol ? base[j * SLD2] : (tid >= 128 && e == j ? 1.0 : 0.0);
+        __syncthreads();  // the block is read before its rows are rewritten
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const double d = l[j * (j + 1) / 2 + j];
+            if (!(d > 0.0) && bad == 0 && k0 + j < n) bad = k0 + j + 1;
+            const double r = rsqrt(d);
+#pragma unroll
+            for (int i = j + 1; i < 8; ++i) l[i * (i + 1) / 2 + j] *= r;
+            x[j] *= r;
+#pragma unroll
+            for (int i = j + 1; i < 8; ++i) {
+#pragma unroll
+                for (int q = j + 1; q <= i; ++q)
+                    l[i * (i + 1) / 2 + q] = fma(-l[i * (i + 1) / 2 + j], l[q * (q + 1) / 2 + j], l[i * (i + 1) / 2 + q]);
+                x[i] = fma(-l[i * (i + 1) / 2 + j], x[j], x[i]);
+            }
+        }
+        if (prow || pcol) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) base[j * SLD2] = tid < 128 && j > tid ? 0.0 : x[j];
+        } else if (tid >= 128 && e >= 0 && e < 8) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) sm.XD[k][j + 8 * e] = x[j];
+        }
+        __syncthreads();
+        for (int q = k + 1 + w; q < nbk; q += kThreads / 32) {
+            const double* P = S + (k0 + t) * SLD2 + g;  // panel(p): rows 8 p + g
+            const double b0 = P[8 * q], b1 = P[8 * q + 4 * SLD2];
+            double* C = S + g + (8 * q + 2 * t) * SLD2;
+            auto tile = [&](int p, double a0, double a1) {
+                double acc[2] = {-C[8 * p], -C[8 * p + SLD2]};
+                mma_f64(acc, a0, b0);
+                mma_f64(acc, a1, b1);
+                C[8 * p] = -acc[0];
+                C[8 * p + SLD2] = -acc[1];
+            };
+#pragma unroll 4
+            for (int p = 0; p < k; ++p) tile(p, P[8 * p], P[8 * p + 4 * SLD2]);
+            tile(k, sm.XD[k][t + 8 * g], sm.XD[k][t + 4 + 8 * g]);
+#pragma unroll 4
+            for (int p = q; p < nbk; ++p) tile(p, P[8 * p], P[8 * p + 4 * SLD2]);
+        }
+        __syncthreads();
+    }
+    double part = tid < n ? log(S[tid + tid * SLD2]) : 0.0;
+    for (int o = 16; o > 0; o >>= 1) part += __shfl_down_sync(0xffffffffu, part, o);
+    if (lane == 0) sm.red[w] = part;
+    if (tid == 0) sm.flag = bad;
+    for (int j = w; j < n; j += kThreads / 32)
+        for (int i = lane; i < n; i += 32) {
+            A[i + (long)j * lda] = i >= j ? S[i + j * SLD2] : 0.0;
+            inv[i + (long)j * ldinv] = i < j ? 0.0 : ((i >> 3) == (j >> 3) ? sm.XD[i >> 3][(i & 7) + 8 * (j & 7)] : S[j + i * SLD2]);
+        }
+    __syncthreads();
+    if (tid == 0 && logdet) *logdet = 2.0 * ((sm.red[0] + sm.red[1]) + (sm.red[2] + sm.red[3]));
+    const int flag = sm.flag;
+    __syncthreads();
+    return flag;
 }
 
 // In-place lower Cholesky (see potrf_blocked); FP64 matrices up to 64 go

@@ -98,10 +98,10 @@ __global__ void __launch_bounds__(kCondThreads, CondSmem<RC>::CTAS) k_finest_con
     }
 }
 
-// The same through the general products: FP32 storage, or r > 64.
+// The same through 64-row tiles (FP64, r > 64) or the general products (FP32 storage).
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 2) k_finest_condition_any(DevTree<T> t) {
-    LaSmem<T>& sm = la_smem<T>();
+    extern __shared__ __align__(16) unsigned char la_dyn_smem[];
     const int r = t.r, L = t.L, m = t.M - 2;
     const long rr = (long)r * r, Lr = (long)L * r;
     const FinChunk ch = t.chunks[blockIdx.x];
@@ -110,8 +110,14 @@ __global__ void __launch_bounds__(kThreads, 2) k_finest_condition_any(DevTree<T>
     auto step = [&](long a, int j, const T* Ua, long d, int n) {
         T* V = t.Bhat + (ch.lo + d) * Lr + (long)j * r;
         T* U = t.Ufin + (ch.lo + d) * Lr;
-        if (j > 0) gemm<T, true, false>(r, n, j * r, (T)-1, Ua, (long)j * r, U, Lr, (T)1, V, Lr, sm);
-        gemm<T, false, false>(r, n, r, (T)1, t.Pinv + a * rr, r, V, Lr, (T)0, U + (long)j * r, Lr, sm);
+        if constexpr (sizeof(T) == 8) {
+            cond_tiles(*reinterpret_cast<Tile<64>::Smem*>(la_dyn_smem), r, Ua, j * r, U, Lr, n, t.Pinv + a * rr, V, Lr, V, Lr,
+                       U + (long)j * r);
+        } else {
+            LaSmem<T>& sm = la_smem<T>();
+            if (j > 0) gemm<T, true, false>(r, n, j * r, (T)-1, Ua, (long)j * r, U, Lr, (T)1, V, Lr, sm);
+            gemm<T, false, false>(r, n, r, (T)1, t.Pinv + a * rr, r, V, Lr, (T)0, U + (long)j * r, Lr, sm);
+        }
     };
     const long g0 = m > 0 ? unit * t.J : 0, g1 = m > 0 ? g0 + t.J : 1;
     const long s2 = t.lstart[m];
@@ -582,7 +588,7 @@ int launch_finest(const Geom& g, const DevTree<T>& t, int grid, bool keep, cudaS
             if (t.r <= 16) launch_condition<16>(t, st);
             else if (t.r <= 32) launch_condition<32>(t, st);
             else if (t.r <= 64) launch_condition<64>(t, st);
-            else k_finest_condition_any<T><<<(unsigned)t.n_chunks, kThreads, sizeof(LaSmem<T>), st>>>(t);
+            else k_finest_condition_any<T><<<(unsigned)t.n_chunks, kThreads, sizeof(Tile<64>::Smem), st>>>(t);
         } else {
             k_finest_condition_any<T><<<(unsigned)t.n_chunks, kThreads, sizeof(LaSmem<T>), st>>>(t);
         }
@@ -639,7 +645,7 @@ cudaError_t prepare_finest() {
     set((const void*)k_finest_condition<32, false>, sizeof(CondSmem<32>));
     set((const void*)k_finest_condition<64, true>, sizeof(CondSmem<64>));
     set((const void*)k_finest_condition<64, false>, sizeof(CondSmem<64>));
-    set((const void*)k_finest_condition_any<double>, sizeof(LaSmem<double>));
+    set((const void*)k_finest_condition_any<double>, sizeof(Tile<64>::Smem));
     set((const void*)k_finest_condition_any<float>, sizeof(LaSmem<float>));
     set((const void*)k_finest_regions_f32, sizeof(LaSmem<float>));
     set((const void*)k_heavy32_sigma, sizeof(LaSmem<float>));

@@ -59,6 +59,7 @@ struct DevTree {
     const int64_t* post_order; // [n_int] per level m, at level_start(m): the level's regions (local index), its
                                // n_dense[m] dense ones first, each kind most expensive step first
     long n_dense[kMaxLevels];
+    long n_mid[kMaxLevels];    // of its factored ones, those of more than 64 rows (they come first)
     long n_fused;              // last factored regions of level M-2 in post_order whose posterior (outside
                                // prediction) comes with their finest group
     const int8_t* factored;    // [n_int] 1: the region's posterior output is kept as F, f

@@ -273,7 +273,9 @@ __global__ void __launch_bounds__(Tile<TS>::NT, Tile<TS>::CTAS) k_dense_gather(D
 }
 
 // L~ in place of L L^T + A_(m,m), its inverse (r <= 128), v = L~^{-1} w_m (w_m in vpost).
-__global__ void __launch_bounds__(kThreads, 2) k_dense_factor(DevTree<double> t, DenseArgs a) {
+// MID: 64 < r <= 128, on Potrf128Smem.
+template <bool MID>
+__global__ void __launch_bounds__(kThreads, MID ? 1 : 2) k_dense_factor(DevTree<double> t, DenseArgs a) {
     LaSmem<double>& sm = la_smem<double>();
     const int r = t.r;
     const long q = blockIdx.x;
@@ -282,7 +284,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_dense_factor(DevTree<double> t,
     double* Lt = t.Lpost + i * (long)r * r;
     double* X = r <= 128 ? dense_inv(t, a, q, i) : nullptr;
     double ld = 0.0;
-    const int info = potrf_lower<double>(r, Lt, r, sm, &ld, X, r);
+    const int info = MID ? potrf_128(r, Lt, r, &ld, X, r) : potrf_lower<double>(r, Lt, r, sm, &ld, X, r);
     double* v = t.vpost + i * r;
     if (X) trmv_lower_inv<double>(r, X, r, v, v);
     else trsv_lower_f64<double>(r, Lt, r, v);
@@ -426,7 +428,10 @@ __global__ void __launch_bounds__(Tile<TS>::NT, Tile<TS>::CTAS) k_fact_y(DevTree
     TT::store(acc, 1.0, a.scr + q * a.per + r0 + (long)c0 * r, r, M, N);
 }
 
-__global__ void __launch_bounds__(kThreads, 2) k_fact_factor(DevTree<double> t, FactArgs a) {
+// MID: regions of 65 to 128 rows, on Potrf128Smem (the level's list starts with the
+// largest); otherwise the others.
+template <bool MID>
+__global__ void __launch_bounds__(kThreads, MID ? 1 : 2) k_fact_factor(DevTree<double> t, FactArgs a) {
     LaSmem<double>& sm = la_smem<double>();
     const int r = t.r, m = a.m;
     const long q = blockIdx.x;
@@ -434,6 +439,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_fact_factor(DevTree<double> t, 
     if (skipped(t, i)) return;
     const long lo = t.sub_lo[i];
     const int n = (int)(t.sub_hi[i] - lo);
+    if (MID != (n > 64)) return;
     if (n == 0) {
         if (threadIdx.x == 0) t.dpost[i] = 0.0;
         return;
@@ -445,7 +451,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_fact_factor(DevTree<double> t, 
     for (int e = threadIdx.x; e < n; e += kThreads) S[e + (long)e * n] += 1.0;
     __syncthreads();
     double ld = 0.0;
-    const int info = potrf_lower<double>(n, S, n, sm, &ld, X, n);
+    const int info = MID ? potrf_128(n, S, n, &ld, X, n) : potrf_small(n, S, n, sm, &ld, X, n);
     // f' = R^{-1} f
     const double* f = (m == t.M - 2 ? t.yt : t.fbuf[(m + 1) & 1]) + lo;
     double* fp = m > 0 ? t.fbuf[m & 1] + lo : t.wsd;  // level 0 has one region
@@ -487,6 +493,11 @@ __global__ void __launch_bounds__(Tile<TS>::NT, Tile<TS>::CTAS) k_fact_out(DevTr
 // ---------------------------------------------------------------------------
 // launcher
 // ---------------------------------------------------------------------------
+static void launch_dense_factor(const DevTree<double>& t, const DenseArgs& a, long n, cudaStream_t st) {
+    if (t.r > 64 && t.r <= 128) k_dense_factor<true><<<(unsigned)n, kThreads, sizeof(Potrf128Smem), st>>>(t, a);
+    else k_dense_factor<false><<<(unsigned)n, kThreads, sizeof(LaSmem<double>), st>>>(t, a);
+}
+
 template <int TS>
 static int launch_dense(const DevTree<double>& t, int m, long elems, bool keep, cudaStream_t st) {
     const int nt = (t.r + TS - 1) / TS, nt2 = nt * nt;
@@ -497,7 +508,7 @@ static int launch_dense(const DevTree<double>& t, int m, long elems, bool keep, 
     for (a.q0 = 0; a.q0 < t.n_dense[m]; a.q0 += most) {
         const long n = t.n_dense[m] - a.q0 < most ? t.n_dense[m] - a.q0 : most;
         k_dense_gather<TS><<<(unsigned)(n * n_slices(m + 1) * nt2), Tile<TS>::NT, sb, st>>>(t, a, nt);
-        k_dense_factor<<<(unsigned)n, kThreads, sizeof(LaSmem<double>), st>>>(t, a);
+        launch_dense_factor(t, a, n, st);
         launches += 2;
         if (m == 0) continue;
         if (t.r <= 128) k_dense_solve<TS><<<(unsigned)(n * m * nt2), Tile<TS>::NT, sb, st>>>(t, a, nt);
@@ -520,7 +531,13 @@ static int launch_factored(const DevTree<double>& t, int m, long nf, double* scr
         const FactArgs a{m, keep ? 1 : 0, t.n_dense[m] + k0, scr, per};
         // (MRA_FACTORED_MAX = 0 leaves only regions without rows)
         if (nc > 0) k_fact_y<TS><<<(unsigned)(n * nt * nc), Tile<TS>::NT, sb, st>>>(t, a, nt, nc);
-        k_fact_factor<<<(unsigned)n, kThreads, sizeof(LaSmem<double>), st>>>(t, a);
+        // the list is by cost, and so by rows: the first n_mid regions hold more than 64
+        const long mid = t.n_mid[m] - k0 < n ? t.n_mid[m] - k0 : n;
+        if (mid > 0) {
+            k_fact_factor<true><<<(unsigned)mid, kThreads, sizeof(Potrf128Smem), st>>>(t, a);
+            ++launches;
+        }
+        k_fact_factor<false><<<(unsigned)n, kThreads, sizeof(LaSmem<double>), st>>>(t, a);
         launches += 2;
         if (m > 0 && nc > 0) {
             k_fact_out<TS><<<(unsigned)(n * nx * nc), Tile<TS>::NT, sb, st>>>(t, a, nx, nc);
@@ -530,7 +547,7 @@ static int launch_factored(const DevTree<double>& t, int m, long nf, double* scr
         // predictive factors: L~ L~^T = L L^T + F_m^T F_m, v = L~^{-1} F_m^T f, G = L~^{-1} F_m^T F_{0..m-1}
         const DenseArgs d{m, 1, 1, a.q0, scr, per};
         k_dense_gather<TS><<<(unsigned)(n * (m + 1) * nt * nt), Tile<TS>::NT, sb, st>>>(t, d, nt);
-        k_dense_factor<<<(unsigned)n, kThreads, sizeof(LaSmem<double>), st>>>(t, d);
+        launch_dense_factor(t, d, n, st);
         launches += 2;
         if (m == 0) continue;
         if (t.r <= 128) k_dense_solve<TS><<<(unsigned)(n * m * nt * nt), Tile<TS>::NT, sb, st>>>(t, d, nt);
@@ -595,10 +612,13 @@ cudaError_t prepare_posterior() {
     cudaError_t e = prepare_dense<16>();
     if (e == cudaSuccess) e = prepare_dense<32>();
     if (e == cudaSuccess) e = prepare_dense<64>();
-    for (const void* fn : {(const void*)k_posterior_factored, (const void*)k_dense_factor, (const void*)k_dense_solve_any,
-                           (const void*)k_fact_factor})
+    for (const void* fn : {(const void*)k_posterior_factored, (const void*)k_dense_factor<false>,
+                           (const void*)k_dense_solve_any, (const void*)k_fact_factor<false>})
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LaSmem<double>));
+    for (const void* fn : {(const void*)k_dense_factor<true>, (const void*)k_fact_factor<true>})
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Potrf128Smem));
     return e;
 }
 

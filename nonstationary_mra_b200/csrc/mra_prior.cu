@@ -1,6 +1,7 @@
 // Prior of the interior levels (class_approximation.cpp:46-50,84-169): per level,
 // the covariance blocks of its regions in one launch, then the regions.
 #include "mra_cond.cuh"
+#include "mra_tile.cuh"
 
 namespace mra {
 
@@ -142,10 +143,71 @@ __global__ void __launch_bounds__(kCondThreads, CondSmem<RC>::CTAS)
     }
 }
 
-// FP32 storage, or r > 64: one CTA per region through the general products.
-template <typename T>
-__global__ void __launch_bounds__(kThreads, 2) k_prior_level(Geom g, DevTree<T> t, int m, long loc0, long nloc,
-                                                            const T* __restrict__ C) {
+// r > 64 (FP64): a region's columns condition on the ancestors in runs of CW columns,
+// one CTA each, so that the top levels' few regions still spread over the chip; then
+// K_i's lower tiles; then the factors (levels of 1 to 64 regions of 100 knots: 120 to
+// 380 us each with one CTA per region doing all of it, 50 to 230 now).
+__global__ void __launch_bounds__(kThreads, 2) k_prior_columns(DevTree<double> t, int m, long loc0, long nloc, int CW,
+                                                               const double* __restrict__ C) {
+    extern __shared__ __align__(16) unsigned char la_dyn_smem[];
+    Tile<64>::Smem& sm = *reinterpret_cast<Tile<64>::Smem*>(la_dyn_smem);
+    const int r = t.r, nc = (r + CW - 1) / CW;
+    const long rr = (long)r * r, mr = (long)m * r;
+    double* V = t.ws + blockIdx.x * t.ws_stride;  // r x CW
+    for (long b = blockIdx.x; b < nloc * nc; b += gridDim.x) {
+        const long q = b / nc;
+        const int c0 = (int)(b - q * nc) * CW, N = min(CW, r - c0);
+        if (skipped(t, t.lstart[m] + loc0 + q)) continue;
+        const double* Cq = C + cov_slot(q, 0, m, 1) * rr;
+        double* Ui = t.U + t.u_off[m] + (loc0 + q) * mr * r + (long)c0 * mr;
+        for (int j = 0; j < m; ++j) {
+            const long a = ancestor(t, m, loc0 + q, j);
+            cond_tiles(sm, r, t.U + t.u_off[j] + (a - t.lstart[j]) * (long)j * rr, j * r, Ui, mr, N, t.Pinv + a * rr,
+                       Cq + j * rr + (long)c0 * r, r, V, r, Ui + (long)j * r);
+        }
+    }
+}
+
+// K_i = C_i - U_i^T U_i, lower tiles, into the factor's storage.
+__global__ void __launch_bounds__(kThreads, 2) k_prior_self(DevTree<double> t, int m, long loc0, int nt,
+                                                            const double* __restrict__ C) {
+    extern __shared__ __align__(16) unsigned char la_dyn_smem[];
+    using TT = Tile<64>;
+    TT::Smem& sm = *reinterpret_cast<TT::Smem*>(la_dyn_smem);
+    const int r = t.r, tiles = nt * (nt + 1) / 2;
+    const long rr = (long)r * r, mr = (long)m * r;
+    const long q = blockIdx.x / tiles;
+    int s = (int)(blockIdx.x - q * tiles), ti = 0;
+    while (s > ti) s -= ++ti;
+    const long i = t.lstart[m] + loc0 + q;
+    if (skipped(t, i)) return;
+    const int r0 = 64 * ti, c0 = 64 * s, M = min(64, r - r0), N = min(64, r - c0);
+    const double* Ui = t.U + t.u_off[m] + (loc0 + q) * mr * r;
+    const bool vec = r % 2 == 0;
+    TT::Acc acc;
+    TT::zero(acc);
+    TT::add(acc, -1.0, C + cov_slot(q, m, m, 1) * rr + r0 + (long)c0 * r, r, M, N);
+    TT::product<true, true>(acc, sm, Ui + r0 * mr, mr, M, Ui + c0 * mr, mr, N, (int)mr, vec, vec);
+    TT::store(acc, -1.0, t.Lprior + i * rr + r0 + (long)c0 * r, r, M, N);
+}
+
+// r > 128: blocked factorization, the inverse by triangular solves.
+__global__ void __launch_bounds__(kThreads, 2) k_prior_factor_any(DevTree<double> t, int m, long loc0) {
+    LaSmem<double>& sm = la_smem<double>();
+    const long i = t.lstart[m] + loc0 + blockIdx.x, rr = (long)t.r * t.r;
+    if (skipped(t, i)) return;
+    double ld = 0.0;
+    const int info = potrf_lower<double>(t.r, t.Lprior + i * rr, t.r, sm, &ld, t.Pinv + i * rr, t.r);
+    if (threadIdx.x == 0) {
+        t.ldprior[i] = ld;
+        if (info) report_error(t.err, i);
+    }
+}
+
+// FP32 storage: one CTA per region through the general products.
+__global__ void __launch_bounds__(kThreads, 2) k_prior_level_f32(DevTree<float> t, int m, long loc0, long nloc,
+                                                                 const float* __restrict__ C) {
+    using T = float;
     LaSmem<T>& sm = la_smem<T>();
     const int r = t.r;
     const long rr = (long)r * r;
@@ -175,7 +237,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_prior_level(Geom g, DevTree<T> 
             if (threadIdx.x == 0) prefetch_l2(Cj + rr, rr * sizeof(T));
             if (j > 0) {
                 const T* Ua = t.U + t.u_off[j] + (a - level_start(t.J, j)) * (long)j * rr;
-                gemm_wide<T, true, false>(r, r, j * r, (T)-1, Ua, (long)j * r, Ui, mr, (T)1, V, r, sm, Cj, r);
+                gemm<T, true, false>(r, r, j * r, (T)-1, Ua, (long)j * r, Ui, mr, (T)1, V, r, sm, Cj, r);
                 Vj = V;
             }
             // U_{i,j} = L_a^{-1} V as a product with the stored inverse
@@ -190,6 +252,18 @@ __global__ void __launch_bounds__(kThreads, 2) k_prior_level(Geom g, DevTree<T> 
             t.ldprior[i] = ld;
             if (info) report_error(t.err, i);
         }
+    }
+}
+
+// The factors of a level's regions, 64 < r <= 128.
+__global__ void __launch_bounds__(kThreads, 1) k_prior_factor(DevTree<double> t, int m, long loc0) {
+    const long i = t.lstart[m] + loc0 + blockIdx.x, rr = (long)t.r * t.r;
+    if (skipped(t, i)) return;
+    double ld = 0.0;
+    const int info = potrf_128(t.r, t.Lprior + i * rr, t.r, &ld, t.Pinv + i * rr, t.r);
+    if (threadIdx.x == 0) {
+        t.ldprior[i] = ld;
+        if (info) report_error(t.err, i);
     }
 }
 
@@ -224,18 +298,28 @@ int launch_prior_level(const Geom& g, const DevTree<T>& t, int m, int grid, cuda
         if (timed) mark(tm->ev[2 * tm->used]);
         launch_cov_level<T>(g, t, m, loc0, n, SB, (unsigned)(nb < cov_grid ? nb : cov_grid), st);
         if (timed) mark(tm->ev[2 * tm->used++ + 1]);
-        bool fused = false;
-        if constexpr (sizeof(T) == 8) {
-            if ((fused = t.r <= 64)) {
-                const unsigned runs = (unsigned)((n + SB - 1) / SB);
-                if (t.r <= 16) launch_fused<16>(t, m, loc0, n, SB, runs, st);
-                else if (t.r <= 32) launch_fused<32>(t, m, loc0, n, SB, runs, st);
-                else launch_fused<64>(t, m, loc0, n, SB, runs, st);
+        if constexpr (sizeof(T) == 4) {
+            k_prior_level_f32<<<(unsigned)(n < grid ? n : grid), kThreads, sizeof(LaSmem<T>), st>>>(t, m, loc0, n, t.cbuf);
+        } else if (t.r <= 64) {
+            const unsigned runs = (unsigned)((n + SB - 1) / SB);
+            if (t.r <= 16) launch_fused<16>(t, m, loc0, n, SB, runs, st);
+            else if (t.r <= 32) launch_fused<32>(t, m, loc0, n, SB, runs, st);
+            else launch_fused<64>(t, m, loc0, n, SB, runs, st);
+        } else {
+            const size_t sb = sizeof(Tile<64>::Smem);
+            if (m > 0) {
+                int CW = 64;  // narrower runs while there are fewer than CTAs
+                while (CW > 16 && n * ((t.r + CW - 1) / CW) < grid) CW /= 2;
+                const long items = n * ((t.r + CW - 1) / CW);
+                k_prior_columns<<<(unsigned)(items < grid ? items : grid), kThreads, sb, st>>>(t, m, loc0, n, CW, t.cbuf);
+                ++launches;
             }
+            const int nt = (t.r + 63) / 64;
+            k_prior_self<<<(unsigned)(n * (nt * (nt + 1) / 2)), kThreads, sb, st>>>(t, m, loc0, nt, t.cbuf);
+            if (t.r <= 128) k_prior_factor<<<(unsigned)n, kThreads, sizeof(Potrf128Smem), st>>>(t, m, loc0);
+            else k_prior_factor_any<<<(unsigned)n, kThreads, sizeof(LaSmem<double>), st>>>(t, m, loc0);
+            ++launches;
         }
-        if (!fused)
-            k_prior_level<T><<<(unsigned)(n < grid ? n : grid), kThreads, sizeof(LaSmem<T>), st>>>(g, t, m, loc0, n,
-                                                                                                    t.cbuf);
         launches += 2;
     }
     return launches;
@@ -246,8 +330,11 @@ cudaError_t prepare_prior() {
     auto set = [&](const void* fn, size_t bytes) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     };
-    set((const void*)k_prior_level<double>, sizeof(LaSmem<double>));
-    set((const void*)k_prior_level<float>, sizeof(LaSmem<float>));
+    set((const void*)k_prior_factor, sizeof(Potrf128Smem));
+    set((const void*)k_prior_columns, sizeof(Tile<64>::Smem));
+    set((const void*)k_prior_self, sizeof(Tile<64>::Smem));
+    set((const void*)k_prior_factor_any, sizeof(LaSmem<double>));
+    set((const void*)k_prior_level_f32, sizeof(LaSmem<float>));
     set((const void*)k_prior_fused<16, true>, sizeof(CondSmem<16>));
     set((const void*)k_prior_fused<16, false>, sizeof(CondSmem<16>));
     set((const void*)k_prior_fused<32, true>, sizeof(CondSmem<32>));

@@ -56,21 +56,24 @@ __device__ __forceinline__ void small_product(int n8, double* C, const double* A
     }
 }
 
-// C(S_c, S_c) of the regions of every group (one warp per region), into Lsig.
+// C(S_c, S_c) of the small regions, into Lsig: wpr warps per region (8 where regions
+// are few: 256 regions of 40 to 64 observations took 60 us with one).
 template <int KIND>
-__global__ void __launch_bounds__(256) k_cov_group(Geom g, DevTree<double> t) {
+__global__ void __launch_bounds__(256) k_cov_group(Geom g, DevTree<double> t, int wpr) {
     const int lane = threadIdx.x & 31;
-    const long nw = (long)gridDim.x * (blockDim.x / 32);
+    const long gw = (long)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+    const long nw = (long)gridDim.x * (blockDim.x / 32) / wpr;
+    const int part = (int)(gw % wpr);
     using F = CovForm<KIND>;
     const double hs = g.dist_scale * (F::NU == 3 ? 1.7320508075688772 : 1.0);
     const double ihs2 = 1.0 / (hs * hs), ih2 = 0.5 * ihs2;
     const PointSet& P = t.pts;
-    for (long c = (long)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); c < t.n_fin; c += nw) {
+    for (long c = gw / wpr; c < t.n_fin; c += nw) {
         const long o0 = t.obs_off[c];
         const int n = (int)(t.obs_off[c + 1] - o0);
         if (n == 0 || n > kFinTile || skipped(t, (long)t.fin_anc[c * t.L + t.L - 1])) continue;
         double* S = t.Lsig + t.lsig_off[c];
-        for (int e = lane; e < n * n; e += 32) {
+        for (int e = 32 * part + lane; e < n * n; e += 32 * wpr) {
             const int i = e % n, j = e / n;
             const long ia = t.obs0 + o0 + i, ib = t.obs0 + o0 + j;
             const double sa = P.s2[ia], ba = P.beta[ia], bb = P.beta[ib];
@@ -411,9 +414,11 @@ static void launch_class(const DevTree<double>& t, const int64_t* items, long n,
 
 int launch_finest_small(const Geom& g, const DevTree<double>& t, bool keep, cudaStream_t st) {
     if (t.n_fin_items == 0) return 0;
-    const long blocks = (t.n_fin + 7) / 8;
+    int wpr = 8;
+    while (wpr > 1 && t.n_fin * wpr > 148L * 64) wpr /= 2;
+    const long blocks = (t.n_fin * wpr + 7) / 8;
     const unsigned grid = (unsigned)(blocks < 148L * 32 ? blocks : 148L * 32);
-    with_cov_kind(cov_kind(g, true), [&](auto k) { k_cov_group<decltype(k)::value><<<grid, 256, 0, st>>>(g, t); });
+    with_cov_kind(cov_kind(g, true), [&](auto k) { k_cov_group<decltype(k)::value><<<grid, 256, 0, st>>>(g, t, wpr); });
     // largest class first
     const long n64 = t.n_fin_class[0], n32 = t.n_fin_class[1], n16 = t.n_fin_class[2];
     launch_class<64>(t, t.fin_items, n64, keep, st);

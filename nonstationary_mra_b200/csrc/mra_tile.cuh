@@ -146,4 +146,35 @@ struct Tile {
     }
 };
 
+// One conditioning step through 64-row tiles (r > 64), one CTA of 256 threads for a
+// set of at most 64 columns:
+//   V = C - Ua^T Us  (Ua: K x r, ld K; Us: K x N, ld ldu),  U = P V.
+// V (ld ldv) is global memory; r even: pair copies.  Ends with a barrier.
+__device__ __forceinline__ void cond_tiles(Tile<64>::Smem& sm, int r, const double* Ua, int K, const double* Us, long ldu,
+                                           int N, const double* P, const double* C, long ldc, double* V, long ldv,
+                                           double* U) {
+    using TT = Tile<64>;
+    const bool vec = r % 2 == 0;
+    if (K > 0 || V != C) {
+        for (int r0 = 0; r0 < r; r0 += 64) {
+            const int M = min(64, r - r0);
+            TT::Acc acc;
+            TT::zero(acc);
+            TT::add(acc, -1.0, C + r0, ldc, M, N);
+            TT::product<true, true>(acc, sm, Ua + (long)r0 * K, K, M, Us, ldu, N, K, vec, vec);
+            TT::store(acc, -1.0, V + r0, ldv, M, N);
+        }
+        __syncthreads();
+    }
+    for (int r0 = 0; r0 < r; r0 += 64) {
+        const int M = min(64, r - r0);
+        TT::Acc acc;
+        TT::zero(acc);
+        // the inverse is lower triangular: rows up to r0 + M - 1
+        TT::product<false, true>(acc, sm, P + r0, r, M, V, ldv, N, r0 + M, vec, vec && M % 2 == 0);
+        TT::store(acc, 1.0, U + r0, ldu, M, N);
+    }
+    __syncthreads();
+}
+
 }  // namespace mra
