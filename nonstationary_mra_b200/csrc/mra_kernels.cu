@@ -54,7 +54,7 @@ __device__ __forceinline__ double field_value(const Geom& g, const FieldParams& 
 __device__ __forceinline__ void store_field(int f, long i, double v, double* s2, double* beta, double* t2, double* ss) {
     if (f == 0) {
         s2[i] = v;
-        ss[i] = sqrt(v);
+        ss[i] = sqrt(fabs(v));  // the products sigma_a sigma_b are of one sign, that of the scale
     } else {
         (f == 1 ? beta : t2)[i] = v;
     }
