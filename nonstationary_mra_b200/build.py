@@ -19,7 +19,7 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libmra_b200.so")
 
-CU_SOURCES = ["mra_kernels.cu", "mra_prior.cu", "mra_finest.cu", "mra_small.cu", "mra_posterior.cu", "mra_api.cu", "mra_static.cu", "mra_mlp.cu", "mra_opt.cpp"]
+CU_SOURCES = ["mra_kernels.cu", "mra_prior.cu", "mra_finest.cu", "mra_small.cu", "mra_posterior.cu", "mra_predict.cu", "mra_api.cu", "mra_static.cu", "mra_mlp.cu", "mra_opt.cpp"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

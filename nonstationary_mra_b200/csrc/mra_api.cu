@@ -218,8 +218,9 @@ struct HostTree {
     std::vector<int64_t> nfin, npred, obs_off, pred_off, fin_anc, pred_order, lsig_off, pc_off;
     std::vector<int64_t> child_lo, child_hi, fin_items, heavy, sub_lo, sub_hi, dslot, post_order;
     std::vector<int8_t> factored;
-    long fin_class[3] = {0, 0, 0}, n_fused = 0;
-    std::vector<FinChunk> chunks;
+    long fin_class[3] = {0, 0, 0}, n_fused = 0, n_pvec = 0;
+    std::vector<FinChunk> chunks, pchunks, pitems;
+    std::vector<int64_t> pglo, pghi;
     std::vector<HeavyTile> heavy_tiles;
 };
 
@@ -415,8 +416,12 @@ mra_status run_eval(mra_ctx* c, bool predict) {
             launch_predict<float>(c->geom, tf, c->grid, st);
             launched += 3;
         } else {
-            launch_predict<double>(c->geom, td, c->grid, st);
-            launched += 1;
+            if (td.n_pchunks > 0) {
+                launched += launch_predict_chunks(c->geom, td, st);
+            } else {
+                launch_predict<double>(c->geom, td, c->grid, st);
+                launched += 1;
+            }
         }
         CU(record(c->tev[2 * i + 1], st, capturing));
         ++i;
@@ -495,7 +500,7 @@ mra_status finish_eval(mra_ctx* c) {
 // Shared FP64 vectors and bookkeeping used by both trees.
 struct Shared {
     double *yt, *ldprior, *vpost, *dpost, *dchild, *dfin, *heavy_inv, *mean, *var;
-    const FinChunk* chunks;
+    const FinChunk *chunks, *pchunks, *pitems;
     const HeavyTile* heavy_tiles;
     int *queue, *err;
     int8_t* factored;
@@ -526,6 +531,13 @@ mra_status setup_tree(mra_ctx* c, DevTree<T>& t, const HostTree& h, const PointS
     t.n_fused = h.n_fused;
     t.heavy = idx[13];
     t.n_heavy = (long)h.heavy.size();
+    t.pglo = idx[14];
+    t.pghi = idx[15];
+    t.pitems = sh.pitems;
+    t.n_pitems = (long)h.pitems.size();
+    t.n_pvec = h.n_pvec;
+    t.pchunks = sh.pchunks;
+    t.n_pchunks = (long)h.pchunks.size();
     t.chunks = sh.chunks;
     t.n_chunks = (long)h.chunks.size();
     t.heavy_tiles = sh.heavy_tiles;
@@ -877,26 +889,48 @@ mra_status mra_create(const mra_structure* s, const mra_model* m, int32_t precis
             return fa != fb ? fa < fb : cost[a] > cost[b];
         });
     }
-    // finest level, conditioning: runs of at most 64 observations below one
+    // Conditioning: runs of at most 64 observations (or prediction points) below one
     // level M-3 region (the root when M = 2).  Every run walks the same chain of
-    // products whatever its width, so wider runs cost less per observation; they
-    // are narrowed only while there are fewer runs than two per SM.
-    {
-        const long n_units = M >= 3 ? level_count(J, M - 3) : 1;
-        const long lvl3 = M >= 3 ? level_start(J, M - 3) : 0;
-        long width = 64;
-        auto build = [&]() {
-            h.chunks.clear();
+    // products whatever its width, so wider runs cost less per point; they are
+    // narrowed only while there are fewer runs than two per SM.
+    const long n_units = M >= 3 ? level_count(J, M - 3) : 1, per_unit = cnt2 / n_units;
+    auto make_chunks = [&](std::vector<FinChunk>& out, const int64_t* glo, const int64_t* ghi) {
+        for (long width = 64;; width /= 2) {
+            out.clear();
             for (long u = 0; u < n_units; ++u) {
-                const long lo = h.sub_lo[lvl3 + u], nu = h.sub_hi[lvl3 + u] - lo;
-                if (nu <= 0) continue;
-                const long k = (nu + width - 1) / width;             // runs of this region, of equal size
-                const long w = (((nu + k - 1) / k) + 7) & ~7L;       // in whole fragments of 8
+                long lo = -1, hi = -1;
+                for (long gl = u * per_unit; gl < (u + 1) * per_unit; ++gl)
+                    if (ghi[gl] > glo[gl]) {
+                        if (lo < 0) lo = glo[gl];
+                        hi = ghi[gl];
+                    }
+                const long nu = hi - lo;
+                if (lo < 0) continue;
+                const long k = (nu + width - 1) / width;        // runs of this region, of equal size
+                const long w = (((nu + k - 1) / k) + 7) & ~7L;  // in whole fragments of 8
                 for (long o = 0; o < nu; o += w)
-                    h.chunks.push_back({(int64_t)(lo + o), (int32_t)std::min(w, nu - o), (int32_t)u});
+                    out.push_back({(int64_t)(lo + o), (int32_t)std::min(w, nu - o), (int32_t)u});
             }
-        };
-        for (build(); width > 16 && (long)h.chunks.size() < 2L * c->sms; build()) width /= 2;
+            if (width <= 16 || (long)out.size() >= 2L * c->sms) break;
+        }
+    };
+    make_chunks(h.chunks, h.sub_lo.data() + lvl2, h.sub_hi.data() + lvl2);
+    if (c->have_pred && r <= 64 && precision == MRA_PRECISION_FP64) {
+        h.pglo.resize(cnt2);
+        h.pghi.resize(cnt2);
+        for (long q = 0; q < cnt2; ++q) {
+            h.pglo[q] = h.pred_off[h.child_lo[q]];
+            h.pghi[q] = h.pred_off[h.child_hi[q]];
+        }
+        make_chunks(h.pchunks, h.pglo.data(), h.pghi.data());
+        for (long k = 0; k < n_fin; ++k)
+            for (long p = 0; p < h.npred[k]; p += 64)
+                h.pitems.push_back({(int64_t)(h.pred_off[k] + p), (int32_t)std::min(64L, (long)h.npred[k] - p), (int32_t)k});
+        std::stable_sort(h.pitems.begin(), h.pitems.end(), [&](const FinChunk& a, const FinChunk& b) {
+            const bool va = a.n <= kPredVector, vb = b.n <= kPredVector;
+            return va != vb ? va : (double)a.n * h.nfin[a.unit] > (double)b.n * h.nfin[b.unit];
+        });
+        while (h.n_pvec < (long)h.pitems.size() && h.pitems[h.n_pvec].n <= kPredVector) ++h.n_pvec;
     }
     // finest level, small regions: a sibling group whose children hold at most
     // kChildMax observations each and kGroupMax together is one item (FP64), any
@@ -969,11 +1003,11 @@ mra_status mra_create(const mra_structure* s, const mra_model* m, int32_t precis
     if (ce) return bail(fail(MRA_ERR_OOM, "device allocation failed: fields"));
     double* y = c->alloc<double>(n_obs, &ce);
     if (ce) return bail(fail(MRA_ERR_OOM, "device allocation failed: y"));
-    const std::vector<int64_t>* tabs[14] = {&h.obs_off, &h.pred_off, &h.fin_anc, &h.pred_order, &h.lsig_off,
+    const std::vector<int64_t>* tabs[16] = {&h.obs_off, &h.pred_off, &h.fin_anc, &h.pred_order, &h.lsig_off,
                                             &h.pc_off, &h.child_lo, &h.child_hi, &h.fin_items, &h.sub_lo, &h.sub_hi,
-                                            &h.dslot, &h.post_order, &h.heavy};
-    int64_t* idx[14];
-    for (int q = 0; q < 14; ++q) {
+                                            &h.dslot, &h.post_order, &h.heavy, &h.pglo, &h.pghi};
+    int64_t* idx[16];
+    for (int q = 0; q < 16; ++q) {
         idx[q] = c->alloc<int64_t>(tabs[q]->size(), &ce);
         if (ce) return bail(fail(MRA_ERR_OOM, "device allocation failed: index tables"));
         mra_status u = upload(idx[q], tabs[q]->data(), tabs[q]->size() * sizeof(int64_t), c->stream);
@@ -1016,9 +1050,11 @@ mra_status mra_create(const mra_structure* s, const mra_model* m, int32_t precis
     if (!ce) sh.dchild = c->alloc<double>(n_fin, &ce);
     if (!ce) sh.dfin = c->alloc<double>(cnt2, &ce);
     if (!ce) sh.heavy_inv = c->alloc<double>(h.heavy.size() * 64 * 64, &ce);
-    FinChunk* chunks = nullptr;
+    FinChunk *chunks = nullptr, *pchunks = nullptr, *pitems = nullptr;
     HeavyTile* heavy_tiles = nullptr;
     if (!ce) sh.chunks = chunks = c->alloc<FinChunk>(h.chunks.size(), &ce);
+    if (!ce) sh.pchunks = pchunks = c->alloc<FinChunk>(h.pchunks.size(), &ce);
+    if (!ce) sh.pitems = pitems = c->alloc<FinChunk>(h.pitems.size(), &ce);
     if (!ce) sh.heavy_tiles = heavy_tiles = c->alloc<HeavyTile>(h.heavy_tiles.size(), &ce);
     if (!ce) sh.mean = c->alloc<double>(n_pred, &ce);
     if (!ce) sh.var = c->alloc<double>(n_pred, &ce);
@@ -1029,6 +1065,8 @@ mra_status mra_create(const mra_structure* s, const mra_model* m, int32_t precis
     {
         mra_status u = upload(sh.factored, h.factored.data(), n_int * sizeof(int8_t), c->stream);
         if (!u) u = upload(chunks, h.chunks.data(), h.chunks.size() * sizeof(FinChunk), c->stream);
+        if (!u) u = upload(pchunks, h.pchunks.data(), h.pchunks.size() * sizeof(FinChunk), c->stream);
+        if (!u) u = upload(pitems, h.pitems.data(), h.pitems.size() * sizeof(FinChunk), c->stream);
         if (!u) u = upload(heavy_tiles, h.heavy_tiles.data(), h.heavy_tiles.size() * sizeof(HeavyTile), c->stream);
         if (u) return bail(u);
         CU(cudaMemsetAsync(sh.dpost, 0, n_int * sizeof(double), c->stream));

@@ -9,10 +9,11 @@
 // these steps inside took 2.43 of the 2.61 ms of an 8,192-point evaluation,
 // 16 CTAs in flight, and 79 of 93 ms of a 262,144-point clustered prediction,
 // one CTA finishing the largest regions):
-//   k_cov_finest            C(Q_{a_j}, S) of every ancestor level, into B^
-//   k_finest_condition*     V_j and U_j of a chunk of at most 64 observations:
+//   k_cov_set               C(Q_{a_j}, S) of every ancestor level, into B^
+//   k_condition_set         V_j and U_j of a chunk of at most 64 observations:
 //                           every observation conditions on its own, so the
 //                           chunks are as many as the chip needs
+//                           (k_finest_condition_any: r > 64 and FP32 storage)
 //   (mra_small.cu)          Sigma, L_Sigma, y~, B^ of finest regions of at most 64
 //                           observations, sibling groups of small ones together
 //                           with their parent's posterior
@@ -27,35 +28,36 @@ namespace mra {
 // ---------------------------------------------------------------------------
 // covariance of the observations with their ancestors' knots
 // ---------------------------------------------------------------------------
+// (CondSet: the observations, or the prediction points, of every sub-tree in chunks.)
 // Task (chunk, j): block C(Q_{a_j}, S_chunk), r x n, into row block j of B^.  The
 // deepest ancestor (level M-2) differs between the sibling groups of a chunk.
 // Issue-bound like k_cov_level: its own launch keeps 4 CTAs per SM busy.
 template <typename T, int KIND>
-__global__ void __launch_bounds__(kCovThreads, 4) k_cov_finest(Geom g, DevTree<T> t) {
+__global__ void __launch_bounds__(kCovThreads, 4) k_cov_set(Geom g, DevTree<T> t, CondSetT<T> set) {
     constexpr int CH = sizeof(T) == 8 ? kCovChunk : 96;  // FP32: the chunk of fill_cov, and so its compiled code
     __shared__ __align__(16) double stage[7 * CH];
     const int r = t.r, L = t.L, m = t.M - 2;
     const long Lr = (long)L * r;
-    const long ntask = t.n_chunks * L;
+    const long ntask = set.n * L;
     for (long b = blockIdx.x; b < ntask; b += gridDim.x) {
         const long q = (unsigned)b / (unsigned)L;  // at most 2^31 tasks
         const int j = (int)(b - q * L);
-        const FinChunk ch = t.chunks[q];
+        const FinChunk ch = set.chunks[q];
         const long unit = ch.unit;  // local index at level M-3 (0 when M == 2)
         if (skipped(t, chunk_region(t, unit))) continue;
         if (j < m) {
             const long a = ancestor(t, m - 1, unit, j);
-            cov_block<T, KIND, CH>(g, t.pts, a * r, r, t.obs0 + ch.lo, ch.n, false, t.Bhat + ch.lo * Lr + (long)j * r, Lr,
+            cov_block<T, KIND, CH>(g, t.pts, a * r, r, set.pt0 + ch.lo, ch.n, false, set.V + ch.lo * Lr + (long)j * r, Lr,
                                stage);
         } else {
             const long g0 = m > 0 ? unit * t.J : 0, g1 = m > 0 ? g0 + t.J : 1;
             const long s2 = t.lstart[m];
             for (long gl = g0; gl < g1; ++gl) {
-                const long glo = t.sub_lo[s2 + gl], ghi = t.sub_hi[s2 + gl];
+                const long glo = set.glo[gl], ghi = set.ghi[gl];
                 const long lo = glo > ch.lo ? glo : ch.lo, hi = ghi < ch.lo + ch.n ? ghi : ch.lo + ch.n;
                 if (lo >= hi) continue;
-                cov_block<T, KIND, CH>(g, t.pts, (s2 + gl) * r, r, t.obs0 + lo, (int)(hi - lo), false,
-                                   t.Bhat + lo * Lr + (long)m * r, Lr, stage);
+                cov_block<T, KIND, CH>(g, t.pts, (s2 + gl) * r, r, set.pt0 + lo, (int)(hi - lo), false,
+                                   set.V + lo * Lr + (long)m * r, Lr, stage);
             }
         }
     }
@@ -66,16 +68,16 @@ __global__ void __launch_bounds__(kCovThreads, 4) k_cov_finest(Geom g, DevTree<T
 // ---------------------------------------------------------------------------
 // FP64, r <= RC <= 64 (mra_cond.cuh): one CTA per chunk.
 template <int RC, bool EVEN>
-__global__ void __launch_bounds__(kCondThreads, CondSmem<RC>::CTAS) k_finest_condition(DevTree<double> t) {
+__global__ void __launch_bounds__(kCondThreads, CondSmem<RC>::CTAS) k_condition_set(DevTree<double> t, CondSet set) {
     extern __shared__ __align__(16) unsigned char la_dyn_smem[];
     const int r = t.r, L = t.L, m = t.M - 2;
     const long rr = (long)r * r, Lr = (long)L * r;
-    const FinChunk ch = t.chunks[blockIdx.x];
+    const FinChunk ch = set.chunks[blockIdx.x];
     const long unit = ch.unit;
     if (skipped(t, chunk_region(t, unit))) return;
     Cond<RC, EVEN> cond(*reinterpret_cast<CondSmem<RC>*>(la_dyn_smem), r);
-    double* V = t.Bhat + ch.lo * Lr;
-    double* U = t.Ufin + ch.lo * Lr;
+    double* V = set.V + ch.lo * Lr;
+    double* U = set.U + ch.lo * Lr;
     // levels 0..M-3, then level M-2 per sibling group of the chunk; one call of
     // step, whose code then stays in the instruction cache
     const int ng = m > 0 ? t.J : 1;
@@ -87,8 +89,8 @@ __global__ void __launch_bounds__(kCondThreads, CondSmem<RC>::CTAS) k_finest_con
             a = ancestor(t, m - 1, unit, j);
         } else {
             a = s2 + g0 + (s - m);
-            if (t.sub_lo[a] > lo) lo = t.sub_lo[a];
-            if (t.sub_hi[a] < hi) hi = t.sub_hi[a];
+            if (set.glo[a - s2] > lo) lo = set.glo[a - s2];
+            if (set.ghi[a - s2] < hi) hi = set.ghi[a - s2];
             if (lo >= hi) continue;
         }
         const long d = (lo - ch.lo) * Lr;
@@ -562,34 +564,46 @@ __global__ void k_finest_terms(DevTree<T> t) {
 // launchers
 // ---------------------------------------------------------------------------
 template <typename T>
-static void launch_cov_finest(const Geom& g, const DevTree<T>& t, cudaStream_t st) {
-    const long tasks = t.n_chunks * t.L;
+static void launch_cov_set(const Geom& g, const DevTree<T>& t, const CondSetT<T>& s, cudaStream_t st) {
+    const long tasks = s.n * t.L;
     const unsigned grid = (unsigned)(tasks < 148L * 32 ? tasks : 148L * 32);
     if constexpr (sizeof(T) == 8)
         with_cov_kind(cov_kind(g, true),
-                      [&](auto k) { k_cov_finest<T, decltype(k)::value><<<grid, kCovThreads, 0, st>>>(g, t); });
+                      [&](auto k) { k_cov_set<T, decltype(k)::value><<<grid, kCovThreads, 0, st>>>(g, t, s); });
     else
-        k_cov_finest<T, 0><<<grid, kCovThreads, 0, st>>>(g, t);
+        k_cov_set<T, 0><<<grid, kCovThreads, 0, st>>>(g, t, s);
 }
 
 template <int RC>
-static void launch_condition(const DevTree<double>& t, cudaStream_t st) {
-    const unsigned grid = (unsigned)t.n_chunks;
-    if (t.r % 2 == 0) k_finest_condition<RC, true><<<grid, kCondThreads, sizeof(CondSmem<RC>), st>>>(t);
-    else k_finest_condition<RC, false><<<grid, kCondThreads, sizeof(CondSmem<RC>), st>>>(t);
+static void launch_condition(const DevTree<double>& t, const CondSet& s, cudaStream_t st) {
+    const unsigned grid = (unsigned)s.n;
+    if (t.r % 2 == 0) k_condition_set<RC, true><<<grid, kCondThreads, sizeof(CondSmem<RC>), st>>>(t, s);
+    else k_condition_set<RC, false><<<grid, kCondThreads, sizeof(CondSmem<RC>), st>>>(t, s);
+}
+
+int launch_condition_set(const Geom& g, const DevTree<double>& t, const CondSet& s, cudaStream_t st) {
+    launch_cov_set<double>(g, t, s, st);
+    if (t.r <= 16) launch_condition<16>(t, s, st);
+    else if (t.r <= 32) launch_condition<32>(t, s, st);
+    else launch_condition<64>(t, s, st);
+    return 2;
 }
 
 template <typename T>
 int launch_finest(const Geom& g, const DevTree<T>& t, int grid, bool keep, cudaStream_t st, const Fork& fk) {
     int launches = 0;
     if (t.n_chunks > 0) {
-        launch_cov_finest<T>(g, t, st);
+        const CondSetT<T> s{t.chunks, t.n_chunks, t.obs0, t.Bhat, t.Ufin, t.sub_lo + t.lstart[t.M - 2],
+                            t.sub_hi + t.lstart[t.M - 2]};
         if constexpr (sizeof(T) == 8) {
-            if (t.r <= 16) launch_condition<16>(t, st);
-            else if (t.r <= 32) launch_condition<32>(t, st);
-            else if (t.r <= 64) launch_condition<64>(t, st);
-            else k_finest_condition_any<T><<<(unsigned)t.n_chunks, kThreads, sizeof(Tile<64>::Smem), st>>>(t);
+            if (t.r <= 64) {
+                launch_condition_set(g, t, s, st);
+            } else {
+                launch_cov_set<T>(g, t, s, st);
+                k_finest_condition_any<T><<<(unsigned)t.n_chunks, kThreads, sizeof(Tile<64>::Smem), st>>>(t);
+            }
         } else {
+            launch_cov_set<T>(g, t, s, st);
             k_finest_condition_any<T><<<(unsigned)t.n_chunks, kThreads, sizeof(LaSmem<T>), st>>>(t);
         }
         launches += 2;
@@ -639,12 +653,12 @@ cudaError_t prepare_finest() {
     auto set = [&](const void* fn, size_t bytes) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     };
-    set((const void*)k_finest_condition<16, true>, sizeof(CondSmem<16>));
-    set((const void*)k_finest_condition<16, false>, sizeof(CondSmem<16>));
-    set((const void*)k_finest_condition<32, true>, sizeof(CondSmem<32>));
-    set((const void*)k_finest_condition<32, false>, sizeof(CondSmem<32>));
-    set((const void*)k_finest_condition<64, true>, sizeof(CondSmem<64>));
-    set((const void*)k_finest_condition<64, false>, sizeof(CondSmem<64>));
+    set((const void*)k_condition_set<16, true>, sizeof(CondSmem<16>));
+    set((const void*)k_condition_set<16, false>, sizeof(CondSmem<16>));
+    set((const void*)k_condition_set<32, true>, sizeof(CondSmem<32>));
+    set((const void*)k_condition_set<32, false>, sizeof(CondSmem<32>));
+    set((const void*)k_condition_set<64, true>, sizeof(CondSmem<64>));
+    set((const void*)k_condition_set<64, false>, sizeof(CondSmem<64>));
     set((const void*)k_finest_condition_any<double>, sizeof(Tile<64>::Smem));
     set((const void*)k_finest_condition_any<float>, sizeof(LaSmem<float>));
     set((const void*)k_finest_regions_f32, sizeof(LaSmem<float>));

@@ -13,8 +13,9 @@
 //   (mra_posterior.cu)  posterior, levels M-2..0 (...-posterior-inference.cpp:14-265,
 //                       class_approximation.cpp:186-306)
 //   k_reduce            deterministic sum of the per-region terms
-//   k_predict           prediction, one CTA per level M-2 region (its finest
-//                       children's predictions together)
+//   (mra_predict.cu)    prediction; k_predict for FP32 storage and r > 64, one CTA
+//                       per level M-2 region (its finest children's predictions
+//                       together)
 //                       (...-prior.cpp:271-392, class_approximation-predict.cpp:105-189)
 #include "mra_kernels.cuh"
 
@@ -369,6 +370,7 @@ cudaError_t prepare_kernels() {
     cudaError_t e = prepare_type<double>();
     if (e == cudaSuccess) e = prepare_type<float>();
     if (e == cudaSuccess) e = prepare_prior();
+    if (e == cudaSuccess) e = prepare_predict();
     if (e == cudaSuccess) e = prepare_posterior();
     return e == cudaSuccess ? prepare_finest() : e;
 }

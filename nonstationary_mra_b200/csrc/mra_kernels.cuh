@@ -62,6 +62,13 @@ struct DevTree {
     long n_mid[kMaxLevels];    // of its factored ones, those of more than 64 rows (they come first)
     long n_fused;              // last factored regions of level M-2 in post_order whose posterior (outside
                                // prediction) comes with their finest group
+    const FinChunk* pchunks;   // [n_pchunks] runs of prediction points conditioned together (FP64, r <= 64)
+    long n_pchunks;
+    const int64_t* pglo;       // [J^(M-2)] first prediction point of each level M-2 region
+    const int64_t* pghi;       // one past the last
+    const FinChunk* pitems;    // [n_pitems] runs of prediction points of one finest region: the n_pvec of at most
+                               // kPredVector points first, most expensive first
+    long n_pitems, n_pvec;
     const int8_t* factored;    // [n_int] 1: the region's posterior output is kept as F, f
     const int8_t* active;      // [n_int] sub-tree sharding: 0 = the region belongs to another rank's
                                // sub-tree and is skipped; nullptr: every region is computed
@@ -111,6 +118,24 @@ struct DevTree {
     int* err;                  // [0]: status, [1]: region (low), [2]: region (high)
 };
 
+// Points conditioned on their ancestors: observations (V: B^, U: Ufin) or prediction
+// points (V: Bt, U: P), L r entries per point.
+template <typename T>
+struct CondSetT {
+    const FinChunk* chunks;
+    long n;
+    long pt0;             // first point in the joint point arrays
+    T* V;
+    T* U;
+    const int64_t* glo;   // [J^(M-2)] points of each level M-2 region: first
+    const int64_t* ghi;   // and one past the last
+};
+using CondSet = CondSetT<double>;
+
+// Prediction points of a finest region handled as vectors, four per pass over its blocks; more go
+// through tile products.  65,536 observations, 16 points per region, vectors / tiles: 1.11 / 0.94 ms
+// with 64 observations per region, 2.26 / 2.48 with 16; 10 points: 1.55 / 1.73 with 16.
+constexpr int kPredVector = 12;
 constexpr int kQueuePost = 4;
 constexpr int kQueueCounters = kQueuePost + kMaxLevels;
 
@@ -217,6 +242,11 @@ int launch_finest(const Geom& g, const DevTree<T>& t, int grid, bool keep, cudaS
 // its small regions (FP64), with the posterior of groups taken whole unless `keep`
 int launch_finest_small(const Geom& g, const DevTree<double>& t, bool keep, cudaStream_t st);
 cudaError_t prepare_finest_small();
+// covariance with the ancestors and conditioning of a set (r <= 64)
+int launch_condition_set(const Geom& g, const DevTree<double>& t, const CondSet& s, cudaStream_t st);
+// prediction in chunks (FP64, r <= 64); returns the number of kernels launched
+int launch_predict_chunks(const Geom& g, const DevTree<double>& t, cudaStream_t st);
+cudaError_t prepare_predict();
 cudaError_t prepare_finest();
 cudaError_t set_gemm_tiles_finest(const int nw[3]);
 // One posterior level (FP64): its dense regions in chunks whose scratch fits
