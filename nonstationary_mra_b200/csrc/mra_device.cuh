@@ -260,11 +260,14 @@ __device__ __forceinline__ double rsqrt_seeded(double x) {
 
 // One nonstationary straight-line entry from per-point quantities (sqrt(s1 s2)
 // pre(x) matern(h), x = 2 b1 b2 / (b1^2 + b2^2), h = scale sqrt(2 d^2 / (b1^2 + b2^2))):
-// with g = b^2 / (2 scale^2) per point and b = g1 + g2, h = sqrt(d^2 / b) and x =
-// b1 b2 / (scale^2 b).  q = 1/sqrt(d^2 b) gives h = d^2 q and 1/b = h q, refined by
-// one Newton step.  Row point (pc, ga, ca = sqrt(s1) b1 / scale^2 for PREF 1; ssa,
-// ba_h = b1 / scale^2 for PREF 0), column point (q*, gq, ssbq = sqrt(s2) b2; ssq,
-// bq).  NU: 1 exponential, 3 Matern 3/2; PREF: 0 prefactor x^1.5, 1 prefactor x;
+// with g = b^2 / 2 per point and b = g1 + g2, h = scale sqrt(d^2 / b) and x = b1 b2 /
+// b.  q = 1/sqrt(d^2 b) gives sqrt(d^2 / b) = d^2 q and 1/b = d^2 q^2, refined by one
+// Newton step.  (With the scale inside g and b1, and sqrt(s) per point, an entry takes
+// two products less, but blocks of chordal distances are 3.7e-16 (Matern 1/2) and 4.0e-16
+// (3/2) from the exact values in norm; 3.2e-16 and 3.5e-16 so, at 61 us instead of 59 for
+// 4001 x 3003 entries.)  Row point
+// (pc, ga, ca = sqrt(s1) b1 for PREF 1; sa = s1, ba for PREF 0), column point (q*, gq,
+// ssbq = sqrt(s2) b2; sq = s2, bq).  NU: 1 exponential, 3 Matern 3/2; PREF: 0 prefactor x^1.5, 1 prefactor x;
 // PLANAR: no third coordinate.  SAFE = false sets `bad` where an argument is out of
 // rsqrt_seeded's range (coincident points, extreme scales, NaN) and the caller takes
 // the SAFE form: tested once per batch of entries, so that the entries' dependent
@@ -272,8 +275,8 @@ __device__ __forceinline__ double rsqrt_seeded(double x) {
 // takes 109).
 template <int NU, int PREF, bool PLANAR, bool SAFE>
 __device__ __forceinline__ double cov_fast_entry(double pc0, double pc1, double pc2, double ga, double ca,
-                                                 double ssa, double ba_h, double qx, double qy, double qz, double gq,
-                                                 double ssbq, double ssq, double bq, bool& bad) {
+                                                 double sa, double ba, double qx, double qy, double qz, double gq,
+                                                 double ssbq, double sq, double bq, double scale, bool& bad) {
     const double dx = qx - pc0, dy = qy - pc1;
     double d2 = dy * dy;
     if (!PLANAR) {
@@ -294,13 +297,15 @@ __device__ __forceinline__ double cov_fast_entry(double pc0, double pc1, double 
         w = h * q;
         w = fma(w, fma(-b, w, 1.0), w);
     }
+    h *= scale;
+    if (NU == 3) h *= 1.7320508075688772;  // the product of the two constants is rounded once for all entries
     const double em = exp_neg(h);
     const double m = NU == 3 ? fma(h, em, em) : em;
     if (PREF == 1) return (ca * ssbq) * w * m;
-    const double x = ba_h * bq * w;
-    if (!SAFE) bad = bad || !rsqrt_ok(x);
-    const double sx = SAFE ? sqrt(x) : x * rsqrt_seeded(x);
-    return (ssa * ssq) * (x * sx) * m;
+    const double x = ba * bq * w, y = sa * sq * x;  // sqrt(s1 s2) x^1.5 = x sqrt(s1 s2 x)
+    if (!SAFE) bad = bad || !rsqrt_ok(y);
+    const double sy = SAFE ? sqrt(y) : y * rsqrt_seeded(y);
+    return x * sy * m;
 }
 
 // One row point against the staged column points q_begin, q_begin + q_step,
@@ -310,17 +315,17 @@ __device__ __noinline__ void fill_row_fast(const double* __restrict__ sx, const 
                                            const double* __restrict__ sz, const double* __restrict__ ss,
                                            const double* __restrict__ sb, const double* __restrict__ sg,
                                            const double* __restrict__ ssb, double pc0, double pc1, double pc2,
-                                           double ssa, double ba, double ga, double ihs2, int q_begin, int q_end,
+                                           double sa, double ba, double ga, double scale, int q_begin, int q_end,
                                            int q_step, int qoff, T* __restrict__ ob, long ld) {
-    const double ca = ssa * ba * ihs2, ba_h = ba * ihs2;
+    const double ca = sa * ba;  // PREF 1: sa is sqrt(s1)
     for (int q = q_begin; q < q_end; q += 4 * q_step) {
         double v[4];
         bool bad = false;
         auto entry = [&](int k, auto safe) {
             const int e = q + k * q_step < q_end ? q + k * q_step : q;
             v[k] = cov_fast_entry<NU, PREF, false, decltype(safe)::value>(
-                pc0, pc1, pc2, ga, ca, ssa, ba_h, sx[e], sy[e], sz[e], sg[e], PREF == 1 ? ssb[e] : 0.0,
-                PREF == 1 ? 0.0 : ss[e], PREF == 1 ? 0.0 : sb[e], bad);
+                pc0, pc1, pc2, ga, ca, sa, ba, sx[e], sy[e], sz[e], sg[e], PREF == 1 ? ssb[e] : 0.0,
+                PREF == 1 ? 0.0 : ss[e], PREF == 1 ? 0.0 : sb[e], scale, bad);
         };
 #pragma unroll
         for (int k = 0; k < 4; ++k) entry(k, std::false_type());
@@ -336,7 +341,7 @@ __device__ __noinline__ void fill_row_fast(const double* __restrict__ sx, const 
 
 // out[t + q*ld] = C(A_{a0+t}, B_{b0+q}), t < na, q < nb.  When `self` the
 // diagonal (t == q) is sigma^2 + tau^2 (evaluate_covariance.cpp:103,307).
-// The column points (coordinates, sqrt(sigma^2), beta and two products) are staged in
+// The column points (coordinates, sigma^2 or its root, beta and two products) are staged in
 // shared memory in chunks, each thread keeps one row point in registers and
 // walks columns strided by the number of row groups (consecutive threads
 // write consecutive rows).  The straight-line nonstationary FP64 case with
@@ -358,7 +363,7 @@ __device__ __noinline__ void fill_cov_staged(const Geom& g, const PointSet& P, c
     double* sz = sy + CH;
     double* ss = sz + CH;
     double* sb = ss + CH;
-    double* sg = sb + CH;   // FP64 fast path only: beta^2 / (2 scale^2) and sqrt(sigma^2) beta
+    double* sg = sb + CH;   // FP64 fast path only: beta^2 / 2 and sqrt(sigma^2) beta
     double* ssb = sg + CH;  // (7 CH doubles fit the FP64 tile buffers)
     const int tid = threadIdx.x, nt = blockDim.x;
     const int R = nblk * na;  // all rows of all blocks
@@ -368,8 +373,6 @@ __device__ __noinline__ void fill_cov_staged(const Geom& g, const PointSet& P, c
     const int tr = tid % rows, tq = tid / rows;
     const int nu = g.nu_x2, pk = g.pref_kind;
     const bool fast = sizeof(T) == 8 && g.nonstat && g.distance != 1 && pk != 2;
-    const double hs = g.dist_scale * (nu == 3 ? 1.7320508075688772 : 1.0);
-    const double ihs2 = 1.0 / (hs * hs), ih2 = 0.5 * ihs2;
     for (int q0 = 0; q0 < nb; q0 += CH) {
         const int qn = nb - q0 < CH ? nb - q0 : CH;
         __syncthreads();
@@ -378,11 +381,11 @@ __device__ __noinline__ void fill_cov_staged(const Geom& g, const PointSet& P, c
             sx[e] = P.c0[ib];
             sy[e] = P.c1[ib];
             sz[e] = P.c2[ib];
-            ss[e] = fast ? P.ss[ib] : P.s2[ib];
+            ss[e] = fast && pk == 1 ? P.ss[ib] : P.s2[ib];
             const double bb = P.beta[ib];
             sb[e] = bb;
             if (fast) {
-                sg[e] = bb * bb * ih2;
+                sg[e] = 0.5 * (bb * bb);
                 ssb[e] = ss[e] * bb;
             }
         }
@@ -395,18 +398,18 @@ __device__ __noinline__ void fill_cov_staged(const Geom& g, const PointSet& P, c
                 T* ob = out + kb * blk + t;
                 const double pc0 = P.c0[ia], pc1 = P.c1[ia], pc2 = P.c2[ia];
                 const double sa = P.s2[ia], ba = P.beta[ia];
-                const double ssa = P.ss[ia], ga = ba * ba * ih2;
+                const double ssa = pk == 1 ? P.ss[ia] : sa, ga = 0.5 * (ba * ba);
                 if (nu == 3 && pk == 1)
-                    fill_row_fast<T, 3, 1>(sx, sy, sz, ss, sb, sg, ssb, pc0, pc1, pc2, ssa, ba, ga, ihs2, tq, qn, cols,
+                    fill_row_fast<T, 3, 1>(sx, sy, sz, ss, sb, sg, ssb, pc0, pc1, pc2, ssa, ba, ga, g.dist_scale, tq, qn, cols,
                                            q0, ob, ld);
                 else if (nu == 3)
-                    fill_row_fast<T, 3, 0>(sx, sy, sz, ss, sb, sg, ssb, pc0, pc1, pc2, ssa, ba, ga, ihs2, tq, qn, cols,
+                    fill_row_fast<T, 3, 0>(sx, sy, sz, ss, sb, sg, ssb, pc0, pc1, pc2, ssa, ba, ga, g.dist_scale, tq, qn, cols,
                                            q0, ob, ld);
                 else if (pk == 1)
-                    fill_row_fast<T, 1, 1>(sx, sy, sz, ss, sb, sg, ssb, pc0, pc1, pc2, ssa, ba, ga, ihs2, tq, qn, cols,
+                    fill_row_fast<T, 1, 1>(sx, sy, sz, ss, sb, sg, ssb, pc0, pc1, pc2, ssa, ba, ga, g.dist_scale, tq, qn, cols,
                                            q0, ob, ld);
                 else
-                    fill_row_fast<T, 1, 0>(sx, sy, sz, ss, sb, sg, ssb, pc0, pc1, pc2, ssa, ba, ga, ihs2, tq, qn, cols,
+                    fill_row_fast<T, 1, 0>(sx, sy, sz, ss, sb, sg, ssb, pc0, pc1, pc2, ssa, ba, ga, g.dist_scale, tq, qn, cols,
                                            q0, ob, ld);
                 // the diagonal of a self block, whose entry this thread has just written
                 if (self && kb == 0) {
@@ -456,12 +459,11 @@ constexpr int kCovChunk = 64;  // column points staged per chunk (7 x 64 doubles
 
 // The straight-line nonstationary FP64 block: two row points per thread with their
 // parameters in registers, the column points staged in chunks as pairs (x, y), (z,
-// g), (sqrt(s2) b or sqrt(s2), b), which both rows read.
+// g), (sqrt(s2) b or s2, b), which both rows read.
 // self: row t is the point of column t + doff.
 template <typename T, int NU, int PREF, bool PLANAR>
 __device__ __forceinline__ void cov_block_fast(const PointSet& P, long a0, int nr, long b0, int nc, bool self, int doff,
-                                               T* __restrict__ out, long ld, double ih2, double ihs2,
-                                               double* stage) {
+                                               T* __restrict__ out, long ld, double scale, double* stage) {
     double2* sxy = reinterpret_cast<double2*>(stage);
     double2* szg = sxy + kCovChunk;
     double2* s45 = szg + kCovChunk;
@@ -476,16 +478,16 @@ __device__ __forceinline__ void cov_block_fast(const PointSet& P, long a0, int n
         __syncthreads();
         for (int e = tid; e < qn; e += nt) {
             const long ib = b0 + q0 + e;
-            const double bb = P.beta[ib], ssq = P.ss[ib];
+            const double bb = P.beta[ib], sq = PREF == 1 ? P.ss[ib] : P.s2[ib];
             sxy[e] = make_double2(P.c0[ib], P.c1[ib]);
-            szg[e] = make_double2(PLANAR ? 0.0 : P.c2[ib], bb * bb * ih2);
-            s45[e] = make_double2(PREF == 1 ? ssq * bb : ssq, bb);
+            szg[e] = make_double2(PLANAR ? 0.0 : P.c2[ib], 0.5 * (bb * bb));
+            s45[e] = make_double2(PREF == 1 ? sq * bb : sq, bb);
         }
         __syncthreads();
         if (!worker) continue;
         for (int t = tr; t < half; t += rows) {
             const bool two = t + half < nr;
-            double pc0[2], pc1[2], pc2[2], ga[2], ca[2], ssa[2], bh[2], diag[2];
+            double pc0[2], pc1[2], pc2[2], ga[2], ca[2], sa[2], bt[2], diag[2];
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
                 const long ia = a0 + t + (k && two ? half : 0);
@@ -493,10 +495,10 @@ __device__ __forceinline__ void cov_block_fast(const PointSet& P, long a0, int n
                 pc0[k] = P.c0[ia];
                 pc1[k] = P.c1[ia];
                 pc2[k] = PLANAR ? 0.0 : P.c2[ia];
-                ssa[k] = P.ss[ia];
-                ga[k] = ba * ba * ih2;
-                bh[k] = ba * ihs2;
-                ca[k] = ssa[k] * bh[k];
+                sa[k] = PREF == 1 ? P.ss[ia] : P.s2[ia];
+                ga[k] = 0.5 * (ba * ba);
+                bt[k] = ba;
+                ca[k] = sa[k] * ba;
                 diag[k] = self ? P.s2[ia] + P.t2[ia] : 0.0;
             }
             T* ob = out + t + (long)(q0 + tc) * ld;
@@ -510,8 +512,8 @@ __device__ __forceinline__ void cov_block_fast(const PointSet& P, long a0, int n
                     const double2 xy = sxy[c], zg = szg[c], r45 = s45[c];
                     bool b1 = false;
                     v[e] = cov_fast_entry<NU, PREF, PLANAR, decltype(safe)::value>(
-                        pc0[k], pc1[k], pc2[k], ga[k], ca[k], ssa[k], bh[k], xy.x, xy.y, zg.x, zg.y, r45.x, r45.x, r45.y,
-                        b1);
+                        pc0[k], pc1[k], pc2[k], ga[k], ca[k], sa[k], bt[k], xy.x, xy.y, zg.x, zg.y, r45.x, r45.x, r45.y,
+                        scale, b1);
                     bad = bad || (b1 && !(self && t + k * half + doff == q0 + c));  // the diagonal is replaced below
                 };
 #pragma unroll
@@ -551,9 +553,7 @@ __device__ __forceinline__ void cov_block(const Geom& g, const PointSet& P, long
         fill_cov_staged<T, CH>(g, P, &a0, 1, nr, b0, nc, self, out, ld, 0, stage);
     } else {
         using F = CovForm<KIND>;
-        const double hs = g.dist_scale * (F::NU == 3 ? 1.7320508075688772 : 1.0);
-        const double ihs2 = 1.0 / (hs * hs), ih2 = 0.5 * ihs2;
-        cov_block_fast<T, F::NU, F::PREF, F::PLANAR>(P, a0, nr, b0, nc, self, 0, out, ld, ih2, ihs2, stage);
+        cov_block_fast<T, F::NU, F::PREF, F::PLANAR>(P, a0, nr, b0, nc, self, 0, out, ld, g.dist_scale, stage);
     }
 }
 

@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_sample(DevTree<T> t, const doub
 // evaluate_*covariance blocks (layout out[i1*n2 + i2])
 // ---------------------------------------------------------------------------
 // Straight-line nonstationary forms: tiles of RT rows x CT columns by the blocks of
-// mra_device.cuh (4001 x 3003 entries: 54 us, 1.8 TB/s of results; by the
+// mra_device.cuh (4001 x 3003 entries: 61 us a call, 1.6 TB/s of results; by the
 // entry-per-thread kernel below about 130).
 template <int KIND>
 __global__ void __launch_bounds__(kCovThreads, 4) k_cov_tiles(Geom g, PointSet P, long a0, int na, long b0, int nb,
@@ -264,10 +264,8 @@ __global__ void __launch_bounds__(kCovThreads, 4) k_cov_tiles(Geom g, PointSet P
     const int t0 = blockIdx.x * RT, q0 = blockIdx.y * CT;
     const int nr = min(RT, na - t0), nc = min(CT, nb - q0);
     using F = CovForm<KIND>;
-    const double hs = g.dist_scale * (F::NU == 3 ? 1.7320508075688772 : 1.0);
-    const double ihs2 = 1.0 / (hs * hs), ih2 = 0.5 * ihs2;
     cov_block_fast<double, F::NU, F::PREF, F::PLANAR>(P, a0 + t0, nr, b0 + q0, nc, self != 0, t0 - q0,
-                                                      out + t0 + (long)q0 * na, na, ih2, ihs2, stage);
+                                                      out + t0 + (long)q0 * na, na, g.dist_scale, stage);
 }
 
 __global__ void k_cov_block(Geom g, PointSet P, long a0, int na, long b0, int nb, int self, double* out) {

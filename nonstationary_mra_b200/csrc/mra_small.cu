@@ -65,8 +65,6 @@ __global__ void __launch_bounds__(256) k_cov_group(Geom g, DevTree<double> t, in
     const long nw = (long)gridDim.x * (blockDim.x / 32) / wpr;
     const int part = (int)(gw % wpr);
     using F = CovForm<KIND>;
-    const double hs = g.dist_scale * (F::NU == 3 ? 1.7320508075688772 : 1.0);
-    const double ihs2 = 1.0 / (hs * hs), ih2 = 0.5 * ihs2;
     const PointSet& P = t.pts;
     for (long c = gw / wpr; c < t.n_fin; c += nw) {
         const long o0 = t.obs_off[c];
@@ -83,12 +81,12 @@ __global__ void __launch_bounds__(256) k_cov_group(Geom g, DevTree<double> t, in
             } else if constexpr (KIND == 0) {
                 v = cov_entry(g, P.pt(ia), sa, ba, P.pt(ib), P.s2[ib], bb);
             } else {
-                const double ssa = P.ss[ia], ssb = P.ss[ib];
+                const double ra = F::PREF ? P.ss[ia] : sa, rb = F::PREF ? P.ss[ib] : P.s2[ib];
                 auto entry = [&](auto safe) {
                     bool bad = false;
                     v = cov_fast_entry<F::NU, F::PREF, F::PLANAR, decltype(safe)::value>(
-                        P.c0[ia], P.c1[ia], P.c2[ia], ba * ba * ih2, ssa * ba * ihs2, ssa, ba * ihs2, P.c0[ib],
-                        P.c1[ib], P.c2[ib], bb * bb * ih2, ssb * bb, ssb, bb, bad);
+                        P.c0[ia], P.c1[ia], P.c2[ia], 0.5 * (ba * ba), ra * ba, ra, ba, P.c0[ib],
+                        P.c1[ib], P.c2[ib], 0.5 * (bb * bb), rb * bb, rb, bb, g.dist_scale, bad);
                     return bad;
                 };
                 if (entry(std::false_type())) entry(std::true_type());
