@@ -825,7 +825,7 @@ def main():
 
     # roofline of the dominant stage of one evaluation.  A prior level is two
     # kernels: its covariance-block launches (k_cov_level: covariance entries,
-    # reported as bytes written) and its region launches (k_prior_level: the
+    # reported as bytes written) and its region launches (k_prior_fused: the
     # stage's products and factorizations, all of its algorithmic FLOPs); the
     # roofline is the region launches' own, the stage figure is kept beside it.
     launches = stats["launches"]
@@ -899,7 +899,7 @@ def main():
                    "stage_ms": {k: stats[k] for k in ("ms_fields", "ms_prior", "ms_finest", "ms_posterior")},
                    "other_precision": other},
         "roofline": {"bound": "tensor",
-                     "kernel": (f"k_prior_level (level {dom['level']}: the level's region launches, "
+                     "kernel": (f"k_prior_fused (level {dom['level']}: the level's region launches, "
                                 f"{kernel_ms:.2f} ms)") if split else f"{dom['kernel']}(level {dom['level']})",
                      "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                      "frac": achieved / peak if peak else None, "traffic": traffic,

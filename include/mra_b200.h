@@ -115,7 +115,7 @@ typedef struct {
 typedef enum {
     MRA_KERNEL_FIELDS = 0,         /* sigma^2 / beta / tau^2 at every point          */
     MRA_KERNEL_PRIOR_LEVEL = 1,    /* prior of one interior level (timed_level = m)  */
-    MRA_KERNEL_FINEST = 2,         /* finest level + level M-2 posterior, per sibling group */
+    MRA_KERNEL_FINEST = 2,         /* finest level (FP64: with the level M-2 posterior) */
     MRA_KERNEL_POSTERIOR_LEVEL = 3,/* posterior of one interior level                */
     MRA_KERNEL_REDUCE = 4,         /* final log-likelihood sum                       */
     MRA_KERNEL_PREDICT = 5,        /* prediction                                     */
@@ -234,14 +234,15 @@ mra_status mra_timer_stop(mra_ctx* ctx, double* ms);
  * device-wide synchronisation of cudaMalloc/cudaFree on every call.  Inputs and
  * output are the caller's DEVICE buffers: p1_dev [3][n1] and p2_dev [3][n2]
  * coordinates, out_dev n1*n2 doubles (n1*n1 when self != 0; p2_dev/n2 ignored).
- * The model's basis tables and theta are read from host memory as elsewhere,
- * with cudaMemcpyAsync on `stream` (a cudaStream_t; NULL = the legacy default
- * stream): theta always goes through a pageable buffer of the call, and a copy
- * from pageable memory waits for the stream's earlier work before it starts.
- * Basis tables or weights in pinned (page-locked) host memory are copied
- * asynchronously instead, so they must stay unchanged until the stream has
- * passed this call.  The kernels are queued on `stream`; the call does not wait
- * for them.
+ * The model's basis tables and theta are read from host memory as elsewhere.  Up
+ * to 108 basis functions over the three fields travel with the launch, by value,
+ * and the call only queues kernels on `stream` (a cudaStream_t; NULL = the legacy
+ * default stream).  Larger tables are copied with cudaMemcpyAsync on `stream`:
+ * theta then goes through a pageable buffer of the call, and a copy from pageable
+ * memory waits for the stream's earlier work before it starts; tables or weights
+ * in pinned (page-locked) host memory are copied asynchronously instead, so they
+ * must stay unchanged until the stream has passed this call.  The call does not
+ * wait for its kernels.
  *
  * Scratch lives in one fixed array in device global memory, held by every GPU
  * that loads the library until the process exits; limits: n1 + n2 <=

@@ -196,12 +196,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_predict(Geom g, DevTree<T> t) {
         for (int j = L - 1; j >= 0; --j) {
             const long a = anc[j];
             T* KcB = Bt + (long)j * r;
-            if (t.Lpinv) {
-                // L~_a^{-1} KcB in place (one row tile, r <= 64)
-                gemm<T, false, false>(r, np, r, (T)1, t.Lpinv + a * rr, r, KcB, Lr, (T)0, KcB, Lr, sm);
-            } else {
-                trsm_left_lower<T>(r, np, t.Lpost + a * rr, r, KcB, Lr, sm);
-            }
+            trsm_left_lower<T>(r, np, t.Lpost + a * rr, r, KcB, Lr, sm);
             if (j > 0) {
                 const T* Ga = t.G + t.u_off[j] + (a - level_start(t.J, j)) * (long)j * rr;
                 gemm<T, true, false>(j * r, np, r, (T)-1, Ga, r, KcB, Lr, (T)1, Bt, Lr, sm);
