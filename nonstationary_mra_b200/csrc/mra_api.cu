@@ -380,7 +380,9 @@ mra_status run_eval(mra_ctx* c, bool predict) {
                     } else {
                         launched += launch_finest<double>(c->geom, td, c->grid, predict || !td.fuse_post, st, fk);
                         if (td.fuse_post) {
-                            launched += launch_posterior_level(td, c->M - 2, c->grid, predict, st, fk);
+                            const int k = launch_posterior_level(td, c->M - 2, c->grid, predict, st, fk);
+                            if (k < 0) return fail(MRA_ERR_STATE, "posterior scratch too small");
+                            launched += k;
                         }
                     }
                 }
@@ -396,9 +398,12 @@ mra_status run_eval(mra_ctx* c, bool predict) {
                     launched += 1;
                 }
                 break;
-            case MRA_KERNEL_POSTERIOR_LEVEL:
-                launched += launch_posterior_level(td, l.level, c->grid, predict, st, fk);
+            case MRA_KERNEL_POSTERIOR_LEVEL: {
+                const int k = launch_posterior_level(td, l.level, c->grid, predict, st, fk);
+                if (k < 0) return fail(MRA_ERR_STATE, "posterior scratch too small");
+                launched += k;
                 break;
+            }
             case MRA_KERNEL_REDUCE:
                 launch_reduce<double>(td, c->d_result, st);
                 launched += 1;

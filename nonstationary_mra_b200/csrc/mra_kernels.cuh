@@ -250,7 +250,8 @@ cudaError_t prepare_predict();
 cudaError_t prepare_finest();
 cudaError_t set_gemm_tiles_finest(const int nw[3]);
 // One posterior level (FP64): its dense regions in chunks whose scratch fits
-// t.cbuf, its factored ones beside them; returns the number of kernels launched.
+// t.cbuf, its factored ones beside them; returns the number of kernels launched, or -1
+// (nothing launched) if the scratch does not hold one region of each kind.
 int launch_posterior_level(const DevTree<double>& t, int m, int grid, bool keep, cudaStream_t st, const Fork& fk);
 cudaError_t prepare_prior();
 cudaError_t set_gemm_tiles_prior(const int nw[3]);

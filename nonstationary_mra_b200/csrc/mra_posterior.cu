@@ -564,16 +564,21 @@ static int launch_level(const DevTree<double>& t, int m, long nf, int grid, bool
     const bool both = nf > 0 && t.n_dense[m] > 0;
     const bool tiles = t.tf <= 128;
     cudaStream_t sf = both ? fk.side : st;
-    long elems_f = tiles ? t.cbuf_elems : 0;
+    const long need_d = dense_scratch(m, t.r), need_f = fact_scratch(m, t.r, t.tf, keep);
+    long elems_f = tiles ? t.cbuf_elems : 0, elems_d = t.cbuf_elems;
+    if (both && tiles) {
+        // the scratch in two: half each, or what one factored region needs, but never less for the dense ones than
+        // one of them needs (the buffer holds one of each at least)
+        elems_f = std::max(need_f, std::min(t.cbuf_elems / 2, nf * need_f));
+        elems_f = std::min(elems_f, t.cbuf_elems - need_d) & ~1L;
+        elems_d = (t.cbuf_elems - elems_f) & ~1L;
+    }
+    // every loop below takes at least one region per turn
+    if ((t.n_dense[m] > 0 && elems_d < need_d) || (nf > 0 && tiles && elems_f < need_f)) return -1;
     if (both) {
         cudaEventRecord(fk.fork, st);
         cudaStreamWaitEvent(fk.side, fk.fork, 0);
-        if (tiles) {  // the scratch in two: half each, or what one region needs
-            const long need = fact_scratch(m, t.r, t.tf, keep);
-            elems_f = std::max(need, std::min(t.cbuf_elems / 2, nf * need)) & ~1L;
-        }
     }
-    const long elems_d = both ? (t.cbuf_elems - elems_f) & ~1L : t.cbuf_elems;
     if (t.n_dense[m] > 0) launches += launch_dense<TS>(t, m, elems_d, keep, st);
     if (nf > 0) {
         if (tiles) {
