@@ -227,8 +227,10 @@ __device__ __forceinline__ unsigned hi_word(double x) { return (unsigned)__doubl
 
 // e^{-s} for s >= 0: Cody-Waite reduction s = n ln2 + r, |r| <= ln2/2; e^{-r} from
 // its Taylor polynomial of degree 13 in Horner form (truncation below 5e-18
-// relative); 2^{-n} added to the exponent field.  s is taken as at most 700.25 (the
-// result is then below 1e-303).  Within 1 ulp of exp(-s) on this range.
+// relative); 2^{-n} added to the exponent field.  Within 1 ulp of exp(-s) up to
+// s = 700; beyond it, and for a negative or undefined s (exp_neg_ok), the result is
+// e^{-700}, below 1e-303.
+__device__ __forceinline__ bool exp_neg_ok(double s) { return hi_word(s) < 0x4085E000u; }
 __device__ __forceinline__ double exp_neg(double s) {
     s = __hiloint2double((int)min(hi_word(s), 0x4085E000u), __double2loint(s));
     const double t = fma(s, c_exp[0], c_exp[1]);
@@ -272,8 +274,9 @@ __device__ __forceinline__ double rsqrt_seeded(double x) {
 // rsqrt_seeded's range (coincident points, extreme scales, NaN) and the caller takes
 // the SAFE form: tested once per batch of entries, so that the entries' dependent
 // chains interleave (a branch in each entry serialised them, 125 us where this form
-// takes 109).
-template <int NU, int PREF, bool PLANAR, bool SAFE>
+// takes 109).  TAIL: so do exponents beyond exp_neg's range, for blocks whose entries
+// are a result by themselves; inside an evaluation e^{-700} serves for what lies beyond.
+template <int NU, int PREF, bool PLANAR, bool SAFE, bool TAIL = false>
 __device__ __forceinline__ double cov_fast_entry(double pc0, double pc1, double pc2, double ga, double ca,
                                                  double sa, double ba, double qx, double qy, double qz, double gq,
                                                  double ssbq, double sq, double bq, double scale, bool& bad) {
@@ -299,7 +302,8 @@ __device__ __forceinline__ double cov_fast_entry(double pc0, double pc1, double 
     }
     h *= scale;
     if (NU == 3) h *= 1.7320508075688772;  // the product of the two constants is rounded once for all entries
-    const double em = exp_neg(h);
+    if (TAIL && !SAFE) bad = bad || !exp_neg_ok(h);
+    const double em = SAFE ? exp(-h) : exp_neg(h);
     const double m = NU == 3 ? fma(h, em, em) : em;
     if (PREF == 1) return (ca * ssbq) * w * m;
     const double x = ba * bq * w, y = sa * sq * x;  // sqrt(s1 s2) x^1.5 = x sqrt(s1 s2 x)
@@ -461,7 +465,7 @@ constexpr int kCovChunk = 64;  // column points staged per chunk (7 x 64 doubles
 // parameters in registers, the column points staged in chunks as pairs (x, y), (z,
 // g), (sqrt(s2) b or s2, b), which both rows read.
 // self: row t is the point of column t + doff.
-template <typename T, int NU, int PREF, bool PLANAR>
+template <typename T, int NU, int PREF, bool PLANAR, bool TAIL = false>
 __device__ __forceinline__ void cov_block_fast(const PointSet& P, long a0, int nr, long b0, int nc, bool self, int doff,
                                                T* __restrict__ out, long ld, double scale, double* stage) {
     double2* sxy = reinterpret_cast<double2*>(stage);
@@ -511,7 +515,7 @@ __device__ __forceinline__ void cov_block_fast(const PointSet& P, long a0, int n
                     const int k = e & 1, c = e < 2 ? q : qb;
                     const double2 xy = sxy[c], zg = szg[c], r45 = s45[c];
                     bool b1 = false;
-                    v[e] = cov_fast_entry<NU, PREF, PLANAR, decltype(safe)::value>(
+                    v[e] = cov_fast_entry<NU, PREF, PLANAR, decltype(safe)::value, TAIL>(
                         pc0[k], pc1[k], pc2[k], ga[k], ca[k], sa[k], bt[k], xy.x, xy.y, zg.x, zg.y, r45.x, r45.x, r45.y,
                         scale, b1);
                     bad = bad || (b1 && !(self && t + k * half + doff == q0 + c));  // the diagonal is replaced below

@@ -1,0 +1,49 @@
+"""Covariance blocks at the ends of their range, against the oracle: scaled distances
+where the exponential becomes denormal and then zero, infinite and undefined coordinates.
+
+Tolerance: an argument of at most 745 with a relative error of a few roundings gives an
+entry with 745 * 8 * 1.1e-16 < 1e-12 relative error.  A denormal exponential may be off by
+its last digit, 5e-324 (the device's e^-745 is 0), which sigma^2 (1 + s) multiplies:
+1.3 * 747 * 5e-324 < 5e-321, and as much for the rounding of the product."""
+import itertools
+
+import numpy as np
+import pytest
+
+from nonstationary_mra_b200 import api
+from nonstationary_mra_b200.model import Field, Model
+
+from test_gpu_covariance import CHORDAL, PLANAR, RTOL, THETA, expected, static_block
+
+pytestmark = pytest.mark.gpu
+
+FORMS = list(itertools.product((CHORDAL, PLANAR), (1, 3), (1.0, 1.5)))
+
+
+def plain_model(distance, nu_x2, pref, dist_scale=1.0):
+    """Constant fields (no basis functions): sigma^2 = 1.3, beta = 0.5, tau^2 = 0.1."""
+    fields = [Field(np.log(v), np.zeros((3, 0)), np.zeros(0)) for v in (1.3, 0.5, 0.1)]
+    return Model(nonstationary=True, distance=distance, nu_x2=nu_x2, prefactor_exp=pref, dist_scale=dist_scale,
+                 basis_len=0.4, fields=fields)
+
+
+def line(x):
+    return np.vstack([x, np.zeros((2, len(x)))])
+
+
+@pytest.mark.parametrize("form", FORMS, ids=lambda f: f"d{f[0]}nu{f[1]}p{f[2]}")
+def test_block_tail_and_undefined(form):
+    distance, nu, pref = form
+    md = plain_model(*form)
+    # exponents (sqrt(3) d / 0.5 or d / 0.5) of 0, 1, 60, ... infinity, and an undefined coordinate
+    h = np.array([0.0, 1.0, 60.0, 699.0, 699.9, 700.0, 700.0004, 701.0, 708.0, 709.0, 720.0, 744.0, 746.0, 800.0, 1e4, 1e9,
+                  1e160, np.inf, np.nan])
+    p1, p2 = line(0.5 * h / (np.sqrt(3.0) if nu == 3 else 1.0)), line(np.array([0.0, 0.25]))
+    th = dict(THETA, sill=1.0, range=1.0, nugget=0.0)
+    with np.errstate(all="ignore"):
+        ref = expected(md, p1, p2)
+        ref_self = expected(md, p1)
+    for out, want in ((api.eval_covariance(md, th, p1, p2), ref), (static_block(md, p1, p2), ref),
+                      (api.eval_covariance(md, th, p1), ref_self)):
+        assert np.array_equal(np.isnan(out), np.isnan(want))
+        np.testing.assert_allclose(out, want, rtol=RTOL, atol=1e-320)
