@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(kCovThreads, 4) k_cov_tiles(Geom g, PointSet P
     const int t0 = blockIdx.x * RT, q0 = blockIdx.y * CT;
     const int nr = min(RT, na - t0), nc = min(CT, nb - q0);
     using F = CovForm<KIND>;
-    cov_block_fast<double, F::NU, F::PREF, F::PLANAR, true>(P, a0 + t0, nr, b0 + q0, nc, self != 0, t0 - q0,
+    cov_block_fast<double, F::NU, F::PREF, true>(P, a0 + t0, nr, b0 + q0, nc, self != 0, t0 - q0,
                                                       out + t0 + (long)q0 * na, na, g.dist_scale, stage);
 }
 

@@ -13,7 +13,7 @@ import pytest
 from nonstationary_mra_b200 import api
 from nonstationary_mra_b200.model import Field, Model
 
-from test_gpu_covariance import CHORDAL, PLANAR, RTOL, THETA, expected, static_block
+from test_gpu_covariance import CHORDAL, PLANAR, RTOL, THETA, expected, model, static_block
 
 pytestmark = pytest.mark.gpu
 
@@ -47,3 +47,38 @@ def test_block_tail_and_undefined(form):
                       (api.eval_covariance(md, th, p1), ref_self)):
         assert np.array_equal(np.isnan(out), np.isnan(want))
         np.testing.assert_allclose(out, want, rtol=RTOL, atol=1e-320)
+
+
+@pytest.mark.parametrize("form", itertools.product((1, 3), (1.0, 1.5, 1.25)), ids=lambda f: f"nu{f[0]}p{f[1]}")
+def test_third_coordinate_of_planar_points(form):
+    """The straight-line distances are one formula: planar points enter it with all three
+    coordinates (zero in the third, as the readers write it), in every kernel."""
+    rng = np.random.default_rng(12)
+    md = model(rng, PLANAR, *form)
+    p1, p2 = rng.random((3, 70)) * 0.5, rng.random((3, 90)) * 0.5
+    md.fields[0].centers[2] = 0.1
+    th = dict(THETA, sill=1.0, range=1.0, nugget=0.0)
+    md.distance = CHORDAL
+    ref, ref_self = expected(md, p1, p2), expected(md, p1)
+    md.distance = PLANAR
+    np.testing.assert_allclose(api.eval_covariance(md, th, p1, p2), ref, rtol=RTOL)
+    np.testing.assert_allclose(static_block(md, p1, p2), ref, rtol=RTOL)
+    np.testing.assert_allclose(api.eval_covariance(md, th, p1), ref_self, rtol=RTOL)
+
+
+def test_third_coordinate_in_an_evaluation():
+    """The same problem on planar points as on chordal ones: bitwise, through every kernel (small
+    and heavy finest regions, prediction in vectors and in tiles)."""
+    from test_gpu_parity import random_case, run_loglik
+    st, md = random_case(44, 4, 4, 49, 2500, 300, True, 1, True)
+    rng = np.random.default_rng(3)
+    for a in (st.knots, st.obs, st.pred):
+        a[2] = 0.05 * rng.random(a.shape[1])
+    out = []
+    for md.distance in (PLANAR, CHORDAL):
+        ctx, (d, _) = run_loglik(st, md)
+        mean, var = ctx.predict()
+        out.append((d, mean, var))
+        ctx.close()
+    assert out[0][0] == out[1][0]
+    assert np.array_equal(out[0][1], out[1][1]) and np.array_equal(out[0][2], out[1][2])
