@@ -372,6 +372,7 @@ __device__ __noinline__ void fill_cov_staged(const Geom& g, const PointSet& P, c
     const int tr = tid % rows, tq = tid / rows;
     const int nu = g.nu_x2, pk = g.pref_kind;
     const bool fast = sizeof(T) == 8 && g.nonstat && g.distance != 1 && pk != 2;
+    const double scale = fabs(g.dist_scale);  // as in cov_block
     for (int q0 = 0; q0 < nb; q0 += CH) {
         const int qn = nb - q0 < CH ? nb - q0 : CH;
         __syncthreads();
@@ -399,16 +400,16 @@ __device__ __noinline__ void fill_cov_staged(const Geom& g, const PointSet& P, c
                 const double sa = P.s2[ia], ba = P.beta[ia];
                 const double ssa = pk == 1 ? P.ss[ia] : sa, ga = 0.5 * (ba * ba);
                 if (nu == 3 && pk == 1)
-                    fill_row_fast<T, 3, 1>(sx, sy, sz, ss, sb, sg, ssb, pc0, pc1, pc2, ssa, ba, ga, g.dist_scale, tq, qn, cols,
+                    fill_row_fast<T, 3, 1>(sx, sy, sz, ss, sb, sg, ssb, pc0, pc1, pc2, ssa, ba, ga, scale, tq, qn, cols,
                                            q0, ob, ld);
                 else if (nu == 3)
-                    fill_row_fast<T, 3, 0>(sx, sy, sz, ss, sb, sg, ssb, pc0, pc1, pc2, ssa, ba, ga, g.dist_scale, tq, qn, cols,
+                    fill_row_fast<T, 3, 0>(sx, sy, sz, ss, sb, sg, ssb, pc0, pc1, pc2, ssa, ba, ga, scale, tq, qn, cols,
                                            q0, ob, ld);
                 else if (pk == 1)
-                    fill_row_fast<T, 1, 1>(sx, sy, sz, ss, sb, sg, ssb, pc0, pc1, pc2, ssa, ba, ga, g.dist_scale, tq, qn, cols,
+                    fill_row_fast<T, 1, 1>(sx, sy, sz, ss, sb, sg, ssb, pc0, pc1, pc2, ssa, ba, ga, scale, tq, qn, cols,
                                            q0, ob, ld);
                 else
-                    fill_row_fast<T, 1, 0>(sx, sy, sz, ss, sb, sg, ssb, pc0, pc1, pc2, ssa, ba, ga, g.dist_scale, tq, qn, cols,
+                    fill_row_fast<T, 1, 0>(sx, sy, sz, ss, sb, sg, ssb, pc0, pc1, pc2, ssa, ba, ga, scale, tq, qn, cols,
                                            q0, ob, ld);
                 // the diagonal of a self block, whose entry this thread has just written
                 if (self && kb == 0) {
@@ -552,7 +553,8 @@ __device__ __forceinline__ void cov_block(const Geom& g, const PointSet& P, long
         fill_cov_staged<T, CH>(g, P, &a0, 1, nr, b0, nc, self, out, ld, 0, stage);
     } else {
         using F = CovForm<KIND>;
-        cov_block_fast<T, F::NU, F::PREF>(P, a0, nr, b0, nc, self, 0, out, ld, g.dist_scale, stage);
+        // an evaluation's straight-line distances take the scale's magnitude
+        cov_block_fast<T, F::NU, F::PREF>(P, a0, nr, b0, nc, self, 0, out, ld, fabs(g.dist_scale), stage);
     }
 }
 

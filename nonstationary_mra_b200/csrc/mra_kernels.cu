@@ -316,7 +316,7 @@ void launch_cov_block(const Geom& g, const PointSet& P, long a0, int na, long b0
                       cudaStream_t st) {
     long n = (long)na * nb;
     if (n <= 0) return;
-    const int kind = cov_kind(g, true);
+    const int kind = g.dist_scale >= 0 ? cov_kind(g, true) : 0;  // exp_neg takes no negative exponent
     if (kind > 0) {
         // long column runs, unless that leaves the chip short of blocks
         int RT = 256, CT = kCovChunk;

@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(256) k_cov_group(Geom g, DevTree<double> t, in
                     bool bad = false;
                     v = cov_fast_entry<F::NU, F::PREF, decltype(safe)::value>(
                         P.c0[ia], P.c1[ia], P.c2[ia], 0.5 * (ba * ba), ra * ba, ra, ba, P.c0[ib],
-                        P.c1[ib], P.c2[ib], 0.5 * (bb * bb), rb * bb, rb, bb, g.dist_scale, bad);
+                        P.c1[ib], P.c2[ib], 0.5 * (bb * bb), rb * bb, rb, bb, fabs(g.dist_scale), bad);
                     return bad;
                 };
                 if (entry(std::false_type())) entry(std::true_type());

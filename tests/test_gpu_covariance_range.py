@@ -49,7 +49,7 @@ def test_block_tail_and_undefined(form):
         np.testing.assert_allclose(out, want, rtol=RTOL, atol=1e-320)
 
 
-@pytest.mark.parametrize("form", itertools.product((1, 3), (1.0, 1.5, 1.25)), ids=lambda f: f"nu{f[0]}p{f[1]}")
+@pytest.mark.parametrize("form", list(itertools.product((1, 3), (1.0, 1.5, 1.25))), ids=lambda f: f"nu{f[0]}p{f[1]}")
 def test_third_coordinate_of_planar_points(form):
     """The straight-line distances are one formula: planar points enter it with all three
     coordinates (zero in the third, as the readers write it), in every kernel."""
@@ -79,6 +79,28 @@ def test_third_coordinate_in_an_evaluation():
         ctx, (d, _) = run_loglik(st, md)
         mean, var = ctx.predict()
         out.append((d, mean, var))
+        ctx.close()
+    assert out[0][0] == out[1][0]
+    assert np.array_equal(out[0][1], out[1][1]) and np.array_equal(out[0][2], out[1][2])
+
+
+@pytest.mark.parametrize("form", FORMS, ids=lambda f: f"d{f[0]}nu{f[1]}p{f[2]}")
+def test_negative_distance_scale(form):
+    """A block takes the scale with its sign; an evaluation's straight-line entries take its square."""
+    from test_gpu_parity import random_case, run_loglik
+    md = plain_model(*form, dist_scale=-1.5)
+    rng = np.random.default_rng(2)
+    p1, p2 = line(rng.random(70)), line(rng.random(90))
+    th = dict(THETA, sill=1.0, range=1.0, nugget=0.0)
+    ref = expected(md, p1, p2)
+    np.testing.assert_allclose(api.eval_covariance(md, th, p1, p2), ref, rtol=RTOL)
+    np.testing.assert_allclose(static_block(md, p1, p2), ref, rtol=RTOL)
+    st, md = random_case(4, 4, 3, 16, 900, 40, True, form[1], True)
+    md.distance, md.prefactor_exp = form[0], form[2]
+    out = []
+    for md.dist_scale in (1.0, -1.0):
+        ctx, (d, _) = run_loglik(st, md)
+        out.append((d, *ctx.predict()))
         ctx.close()
     assert out[0][0] == out[1][0]
     assert np.array_equal(out[0][1], out[1][1]) and np.array_equal(out[0][2], out[1][2])
