@@ -251,32 +251,40 @@ __device__ __forceinline__ double exp_neg(double s) {
 // takes the error below 2^-66: within an ulp of the exact value.  x must be in
 // [2^-100, 2^100) (rsqrt_ok), where the single-precision seed is normal.
 __device__ __forceinline__ bool rsqrt_ok(double x) { return hi_word(x) - 0x39B00000u < 0x0C800000u; }
-__device__ __forceinline__ double rsqrt_seeded(double x) {
+__device__ __forceinline__ double rsqrt_parts(double x, double& c) {  // 1/sqrt(x) = y (1 + c), y of 24 bits
     float yf;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(__double2float_rn(x)));
     const double y = (double)yf;
     const double s = x * y;  // e = 1 - x y^2 with the rounding of x y taken back: the distance enters an exponential
     const double e = fma(-fma(x, y, -s), y, fma(-s, y, 1.0));
-    return fma(y * e, fma(0.375, e, 0.5), y);
+    c = e * fma(0.375, e, 0.5);
+    return y;
+}
+__device__ __forceinline__ double rsqrt_seeded(double x) {
+    double c;
+    const double y = rsqrt_parts(x, c);
+    return fma(y, c, y);
+}
+// a / sqrt(x) from the parts, without rounding 1/sqrt(x) first: lo is the rest that hi + lo rounds
+__device__ __forceinline__ double times_parts(double a, double y, double c, double& lo) {
+    const double hi = a * y;
+    lo = fma(hi, c, fma(a, y, -hi));
+    return hi;
 }
 
 // One nonstationary straight-line entry from per-point quantities (sqrt(s1 s2)
 // pre(x) matern(h), x = 2 b1 b2 / (b1^2 + b2^2), h = scale sqrt(2 d^2 / (b1^2 + b2^2))):
 // with g = b^2 / 2 per point and b = g1 + g2, h = scale sqrt(d^2 / b) and x = b1 b2 /
 // b.  q = 1/sqrt(d^2 b) gives sqrt(d^2 / b) = d^2 q and 1/b = d^2 q^2, refined by one
-// Newton step.  (With the scale inside g and b1, and sqrt(s) per point, an entry takes
-// two products less, but blocks of chordal distances are 3.7e-16 (Matern 1/2) and 4.0e-16
-// (3/2) from the exact values in norm; 3.2e-16 and 3.5e-16 so, at 61 us instead of 59 for
-// 4001 x 3003 entries.)  Row point
+// Newton step.  Row point
 // (pc, ga, ca = sqrt(s1) b1 for PREF 1; sa = s1, ba for PREF 0), column point (q*, gq,
 // ssbq = sqrt(s2) b2; sq = s2, bq).  NU: 1 exponential, 3 Matern 3/2; PREF: 0 prefactor x^1.5, 1 prefactor x;
 // SAFE = false sets `bad` where an argument is out of
 // rsqrt_seeded's range (coincident points, extreme scales, NaN) and the caller takes
 // the SAFE form: tested once per batch of entries, so that the entries' dependent
 // chains interleave (a branch in each entry serialised them, 125 us where this form
-// takes 109).  TAIL: so do exponents beyond exp_neg's range, for blocks whose entries
-// are a result by themselves; inside an evaluation e^{-700} serves for what lies beyond.
-template <int NU, int PREF, bool SAFE, bool TAIL = false>
+// takes 109).  Exponents beyond exp_neg's range give e^{-700}, which serves inside an evaluation.
+template <int NU, int PREF, bool SAFE>
 __device__ __forceinline__ double cov_fast_entry(double pc0, double pc1, double pc2, double ga, double ca,
                                                  double sa, double ba, double qx, double qy, double qz, double gq,
                                                  double ssbq, double sq, double bq, double scale, bool& bad) {
@@ -296,8 +304,7 @@ __device__ __forceinline__ double cov_fast_entry(double pc0, double pc1, double 
         w = fma(w, fma(-b, w, 1.0), w);
     }
     h *= scale;
-    if (NU == 3) h *= 1.7320508075688772;  // the product of the two constants is rounded once for all entries
-    if (TAIL && !SAFE) bad = bad || !exp_neg_ok(h);
+    if (NU == 3) h *= 1.7320508075688772;
     const double em = SAFE ? exp(-h) : exp_neg(h);
     const double m = NU == 3 ? fma(h, em, em) : em;
     if (PREF == 1) return (ca * ssbq) * w * m;
@@ -305,6 +312,64 @@ __device__ __forceinline__ double cov_fast_entry(double pc0, double pc1, double 
     if (!SAFE) bad = bad || !rsqrt_ok(y);
     const double sy = SAFE ? sqrt(y) : y * rsqrt_seeded(y);
     return x * sy * m;
+}
+
+// The same entry where the block is a result by itself, with fewer roundings: the
+// exponent is rounded once from d^2 / sqrt(d^2 b) in two parts and the scale (Matern
+// 3/2: the scale times sqrt(3), in two parts), c = sqrt(s) b once per point
+// (root_times), sqrt(s1 s2 x) once.  An exponent beyond exp_neg's range, negative or
+// undefined makes the batch `bad` too.
+// Norm of the error against extended precision, fields included, 1500 x 1300 points,
+// Matern 1/2 and 3/2, literal form (a division, two square roots, exp) / cov_fast_entry /
+// this: chordal 6.67 / 6.72 / 6.67 and 7.16 / 7.20 / 7.11 e-16, planar 3.08 / 3.23 / 3.15
+// and 3.41 / 3.52 / 3.40 e-16; against the 64-bit expression 3.08 / 3.18 / 3.10, 3.29 /
+// 3.43 / 3.37, 2.39 / 2.43 / 2.26 and 2.60 / 2.63 / 2.52 e-16.  66 us for 4001 x 3003
+// planar entries instead of 63.
+struct CovScale {
+    double scale, hi, lo;  // distance scale; hi + lo: the exponent's factor, scale or sqrt(3) scale
+};
+template <int NU, int PREF, bool SAFE>
+__device__ __forceinline__ double cov_result_entry(double pc0, double pc1, double pc2, double ga, double ca, double sa,
+                                                   double ba, double qx, double qy, double qz, double gq, double cq,
+                                                   double sq, double bq, const CovScale& k, bool& bad) {
+    const double dx = qx - pc0, dy = qy - pc1, dz = qz - pc2;
+    const double d2 = fma(dx, dx, fma(dz, dz, dy * dy));
+    const double b = ga + gq;
+    double h, w;
+    if (SAFE) {
+        w = 1.0 / b;
+        h = k.scale * sqrt(d2 * w);
+        if (NU == 3) h *= 1.7320508075688772;
+    } else {
+        const double z = d2 * b;
+        bad = bad || !rsqrt_ok(z);
+        double c, lo;
+        const double y = rsqrt_parts(z, c), s = times_parts(d2, y, c, lo);  // sqrt(d^2 / b) = s + lo
+        lo *= k.hi;
+        if (NU == 3) lo = fma(k.lo, s, lo);
+        h = fma(k.hi, s, lo);
+        bad = bad || !exp_neg_ok(h);
+        w = s * y;  // 1/b to 2^-23, then a third-order step
+        const double e = fma(-b, w, 1.0);
+        w = fma(w, fma(e, e, e), w);
+    }
+    const double em = SAFE ? exp(-h) : exp_neg(h);
+    const double m = NU == 3 ? fma(h, em, em) : em;
+    if (PREF == 1) return (ca * cq) * w * m;
+    const double x = ba * bq * w, v = sa * sq * x;
+    if (SAFE) return x * sqrt(v) * m;
+    bad = bad || !rsqrt_ok(v);
+    double c, lo;
+    const double y = rsqrt_parts(v, c), r = times_parts(v, y, c, lo);
+    return x * (r + lo) * m;
+}
+// sqrt(|s|) b
+__device__ __forceinline__ double root_times(double s, double b) {
+    s = fabs(s);
+    if (!rsqrt_ok(s)) return sqrt(s) * b;
+    double c, lo;
+    const double y = rsqrt_parts(s, c), r = times_parts(s, y, c, lo);
+    return fma(r, b, lo * b);
 }
 
 // One row point against the staged column points q_begin, q_begin + q_step,
@@ -461,9 +526,10 @@ constexpr int kCovChunk = 64;  // column points staged per chunk (7 x 64 doubles
 // parameters in registers, the column points staged in chunks as pairs (x, y), (z,
 // g), (sqrt(s2) b or s2, b), which both rows read.
 // self: row t is the point of column t + doff.
-template <typename T, int NU, int PREF, bool TAIL = false>
+// RESULT: the entries are a result by themselves (cov_result_entry).
+template <typename T, int NU, int PREF, bool RESULT = false>
 __device__ __forceinline__ void cov_block_fast(const PointSet& P, long a0, int nr, long b0, int nc, bool self, int doff,
-                                               T* __restrict__ out, long ld, double scale, double* stage) {
+                                               T* __restrict__ out, long ld, const CovScale& scale, double* stage) {
     double2* sxy = reinterpret_cast<double2*>(stage);
     double2* szg = sxy + kCovChunk;
     double2* s45 = szg + kCovChunk;
@@ -478,10 +544,10 @@ __device__ __forceinline__ void cov_block_fast(const PointSet& P, long a0, int n
         __syncthreads();
         for (int e = tid; e < qn; e += nt) {
             const long ib = b0 + q0 + e;
-            const double bb = P.beta[ib], sq = PREF == 1 ? P.ss[ib] : P.s2[ib];
+            const double bb = P.beta[ib], sq = PREF == 1 && !RESULT ? P.ss[ib] : P.s2[ib];
             sxy[e] = make_double2(P.c0[ib], P.c1[ib]);
             szg[e] = make_double2(P.c2[ib], 0.5 * (bb * bb));
-            s45[e] = make_double2(PREF == 1 ? sq * bb : sq, bb);
+            s45[e] = make_double2(PREF == 1 ? (RESULT ? root_times(sq, bb) : sq * bb) : sq, bb);
         }
         __syncthreads();
         if (!worker) continue;
@@ -495,10 +561,10 @@ __device__ __forceinline__ void cov_block_fast(const PointSet& P, long a0, int n
                 pc0[k] = P.c0[ia];
                 pc1[k] = P.c1[ia];
                 pc2[k] = P.c2[ia];
-                sa[k] = PREF == 1 ? P.ss[ia] : P.s2[ia];
+                sa[k] = PREF == 1 && !RESULT ? P.ss[ia] : P.s2[ia];
                 ga[k] = 0.5 * (ba * ba);
                 bt[k] = ba;
-                ca[k] = sa[k] * ba;
+                ca[k] = PREF == 1 && RESULT ? root_times(sa[k], ba) : sa[k] * ba;
                 diag[k] = self ? P.s2[ia] + P.t2[ia] : 0.0;
             }
             T* ob = out + t + (long)(q0 + tc) * ld;
@@ -511,9 +577,14 @@ __device__ __forceinline__ void cov_block_fast(const PointSet& P, long a0, int n
                     const int k = e & 1, c = e < 2 ? q : qb;
                     const double2 xy = sxy[c], zg = szg[c], r45 = s45[c];
                     bool b1 = false;
-                    v[e] = cov_fast_entry<NU, PREF, decltype(safe)::value, TAIL>(
-                        pc0[k], pc1[k], pc2[k], ga[k], ca[k], sa[k], bt[k], xy.x, xy.y, zg.x, zg.y, r45.x, r45.x, r45.y,
-                        scale, b1);
+                    if constexpr (RESULT)
+                        v[e] = cov_result_entry<NU, PREF, decltype(safe)::value>(
+                            pc0[k], pc1[k], pc2[k], ga[k], ca[k], sa[k], bt[k], xy.x, xy.y, zg.x, zg.y, r45.x, r45.x,
+                            r45.y, scale, b1);
+                    else
+                        v[e] = cov_fast_entry<NU, PREF, decltype(safe)::value>(
+                            pc0[k], pc1[k], pc2[k], ga[k], ca[k], sa[k], bt[k], xy.x, xy.y, zg.x, zg.y, r45.x, r45.x,
+                            r45.y, scale.scale, b1);
                     bad = bad || (b1 && !(self && t + k * half + doff == q0 + c));  // the diagonal is replaced below
                 };
 #pragma unroll
@@ -554,7 +625,8 @@ __device__ __forceinline__ void cov_block(const Geom& g, const PointSet& P, long
     } else {
         using F = CovForm<KIND>;
         // an evaluation's straight-line distances take the scale's magnitude
-        cov_block_fast<T, F::NU, F::PREF>(P, a0, nr, b0, nc, self, 0, out, ld, fabs(g.dist_scale), stage);
+        cov_block_fast<T, F::NU, F::PREF>(P, a0, nr, b0, nc, self, 0, out, ld, CovScale{fabs(g.dist_scale), 0.0, 0.0},
+                                          stage);
     }
 }
 

@@ -250,17 +250,17 @@ __global__ void __launch_bounds__(kThreads, 2) k_sample(DevTree<T> t, const doub
 // evaluate_*covariance blocks (layout out[i1*n2 + i2])
 // ---------------------------------------------------------------------------
 // Straight-line nonstationary forms: tiles of RT rows x CT columns by the blocks of
-// mra_device.cuh (4001 x 3003 entries: 61 us a call, 1.6 TB/s of results; by the
-// entry-per-thread kernel below about 130).
+// mra_device.cuh (4001 x 3003 planar entries: 66 to 68 us a call, 1.4 TB/s of results; by the
+// entry-per-thread kernel below 142 to 144).
 template <int KIND>
-__global__ void __launch_bounds__(kCovThreads, 4) k_cov_tiles(Geom g, PointSet P, long a0, int na, long b0, int nb,
+__global__ void __launch_bounds__(kCovThreads, 4) k_cov_tiles(CovScale scale, PointSet P, long a0, int na, long b0, int nb,
                                                               int self, int RT, int CT, double* out) {
     __shared__ __align__(16) double stage[7 * kCovChunk];
     const int t0 = blockIdx.x * RT, q0 = blockIdx.y * CT;
     const int nr = min(RT, na - t0), nc = min(CT, nb - q0);
     using F = CovForm<KIND>;
     cov_block_fast<double, F::NU, F::PREF, true>(P, a0 + t0, nr, b0 + q0, nc, self != 0, t0 - q0,
-                                                      out + t0 + (long)q0 * na, na, g.dist_scale, stage);
+                                                      out + t0 + (long)q0 * na, na, scale, stage);
 }
 
 __global__ void k_cov_block(Geom g, PointSet P, long a0, int na, long b0, int nb, int self, double* out) {
@@ -324,9 +324,12 @@ void launch_cov_block(const Geom& g, const PointSet& P, long a0, int na, long b0
         const long gy = (nb + CT - 1) / CT;
         if (gy <= 65535) {
             const dim3 grid((unsigned)((na + RT - 1) / RT), (unsigned)gy);
+            // the product with the rounded root that matern() multiplies by, itself not rounded
+            const long double f = (g.nu_x2 == 3 ? (long double)1.7320508075688772 : 1.0L) * g.dist_scale;
+            const CovScale scale{g.dist_scale, (double)f, (double)(f - (double)f)};
             with_cov_kind(kind, [&](auto k) {
                 if constexpr (decltype(k)::value > 0)
-                    k_cov_tiles<decltype(k)::value><<<grid, kCovThreads, 0, st>>>(g, P, a0, na, b0, nb, self ? 1 : 0, RT,
+                    k_cov_tiles<decltype(k)::value><<<grid, kCovThreads, 0, st>>>(scale, P, a0, na, b0, nb, self ? 1 : 0, RT,
                                                                                   CT, out);
             });
             return;
