@@ -10,6 +10,7 @@ import itertools
 import numpy as np
 import pytest
 
+import mra_oracle as oracle
 from nonstationary_mra_b200 import api
 from nonstationary_mra_b200.model import Field, Model
 
@@ -104,3 +105,41 @@ def test_negative_distance_scale(form):
         ctx.close()
     assert out[0][0] == out[1][0]
     assert np.array_equal(out[0][1], out[1][1]) and np.array_equal(out[0][2], out[1][2])
+
+
+@pytest.mark.parametrize("nu", [1, 3])
+@pytest.mark.parametrize("distance,pref,dist_scale", [(CHORDAL, 1.5, 6371.0), (PLANAR, 1.0, 1.0)])
+def test_block_error_against_extended_precision(distance, pref, dist_scale, nu):
+    """From the library's own fields, a block is no further from its value in extended precision
+    than the literal expression evaluated in 64 bits (norm over 2 million entries; counting the
+    roundings of both gives 0.88 to 0.96 of the literal form's error)."""
+    L = np.longdouble
+    rng = np.random.default_rng(20)
+    if distance == CHORDAL:
+        def draw(n):
+            lon, lat = np.radians(-120 + 40 * rng.random(n)), np.radians(25 + 25 * rng.random(n))
+            return np.stack([np.cos(lat) * np.cos(lon), np.cos(lat) * np.sin(lon), np.sin(lat)])
+    else:
+        def draw(n):
+            return np.vstack([rng.random((2, n)), np.zeros((1, n))])
+    centers = [draw(9) for _ in range(3)]
+    fields = [Field(a, c, 0.3 * rng.standard_normal(9))
+              for a, c in zip((0.1, np.log(300.0 if distance == CHORDAL else 0.1), -3.0), centers)]
+    md = Model(nonstationary=True, distance=distance, nu_x2=nu, prefactor_exp=pref, dist_scale=dist_scale, basis_len=0.25,
+               fields=fields)
+    p1, p2 = draw(1500), draw(1300)
+    th = dict(THETA, sill=1.0, range=1.0, nugget=0.0)
+    f1, f2 = api.eval_fields(md, th, p1), api.eval_fields(md, th, p2)
+    omd = oracle.Model(nonstationary=True, distance=distance, nu_x2=nu, prefactor_exp=pref, dist_scale=dist_scale,
+                       basis=md.basis, basis_len=md.basis_len, fields=[])
+    literal = oracle.cross_cov(omd, p1, f1, p2, f2)
+    d2 = sum((p1[c].astype(L)[:, None] - p2[c].astype(L)[None, :]) ** 2 for c in range(3))
+    (s1, b1, _), (s2, b2, _) = f1.astype(L), f2.astype(L)
+    bms = (b1[:, None] ** 2 + b2[None, :] ** 2) / 2
+    h = L(dist_scale) * np.sqrt(d2 / bms) * (np.sqrt(L(3)) if nu == 3 else 1)
+    exact = np.sqrt(s1[:, None] * s2[None, :]) * (b1[:, None] * b2[None, :] / bms) ** L(pref) * np.exp(-h)
+    if nu == 3:
+        exact *= 1 + h
+    norm = lambda out: float(np.sqrt(((out - exact) ** 2).sum() / (exact ** 2).sum()))
+    for out in (static_block(md, p1, p2), api.eval_covariance(md, th, p1, p2)):
+        assert norm(out) <= norm(literal), (norm(out), norm(literal))
