@@ -14,7 +14,7 @@ import mra_oracle as oracle
 from nonstationary_mra_b200 import api
 from nonstationary_mra_b200.model import Field, Model
 
-from test_gpu_covariance import CHORDAL, PLANAR, RTOL, THETA, expected, model, static_block
+from test_gpu_covariance import CHORDAL, PLANAR, RTOL, THETA, expected, model, points, static_block
 
 pytestmark = pytest.mark.gpu
 
@@ -143,3 +143,14 @@ def test_block_error_against_extended_precision(distance, pref, dist_scale, nu):
     norm = lambda out: float(np.sqrt(((out - exact) ** 2).sum() / (exact ** 2).sum()))
     for out in (static_block(md, p1, p2), api.eval_covariance(md, th, p1, p2)):
         assert norm(out) <= norm(literal), (norm(out), norm(literal))
+
+
+@pytest.mark.parametrize("form", FORMS, ids=lambda f: f"d{f[0]}nu{f[1]}p{f[2]}")
+def test_negative_sill_scale_of_every_form(form):
+    """sqrt(sigma_a^2 sigma_b^2) of two negative values: its square root once, or a root per point."""
+    rng = np.random.default_rng(8)
+    md = model(rng, *form)
+    p1, p2 = points(rng, form[0], 75), points(rng, form[0], 20)
+    ref = expected(md, p1, p2)
+    np.testing.assert_allclose(static_block(md, p1, p2, -1.0), ref, rtol=RTOL)
+    np.testing.assert_allclose(api.eval_covariance(md, dict(THETA, sill_scale=-1.0), p1, p2), ref, rtol=RTOL)
