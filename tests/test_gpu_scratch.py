@@ -7,7 +7,7 @@ import pytest
 import mra_oracle as oracle
 from nonstationary_mra_b200 import partition, synth
 
-from test_gpu_parity import run_loglik, to_oracle
+from test_gpu_parity import random_case, run_loglik, to_oracle
 
 pytestmark = pytest.mark.gpu
 
@@ -42,3 +42,30 @@ def test_dense_region_needs_most_of_the_scratch(J, M, limit, per_quadrant, monke
     ctx.capture_graph()
     assert ctx.loglik()[0] == d
     ctx.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_levels_in_chunks(precision, monkeypatch):
+    """A covariance buffer of about a third of what the deepest level asks for (the least that a
+    context takes is one region per resident CTA): its prior regions, and its dense and its
+    factored posterior regions, which share the buffer, run in chunks.  A region's steps do not
+    depend on the chunk, so the results are bitwise the same."""
+    J, M, r = 4, 7, 16
+    st, md = random_case(50, J, M, r, 33000, 2000, False, 1, True)   # about 2 r observations per level M-2 region
+    parent = np.asarray(st.finest_parent)
+    per_region = np.bincount(parent - parent.min(), weights=np.diff(st.obs_offset))
+    assert (per_region > 2 * r).sum() > 200 and (per_region <= 2 * r).sum() > 200
+    out = []
+    for mb in (None, "1"):
+        if mb:
+            monkeypatch.setenv("MRA_COV_BUF_MB", mb)
+        ctx, (d, _) = run_loglik(st, md, precision=precision)
+        launches = [ctx.stats()["kernel_launches"]]
+        mean, var = ctx.predict()
+        launches.append(ctx.stats()["kernel_launches"])
+        out.append((d, mean, var, launches))
+        ctx.close()
+    assert out[0][0] == out[1][0]
+    assert np.array_equal(out[0][1], out[1][1]) and np.array_equal(out[0][2], out[1][2])
+    # the prior's level in four chunks and the posterior's kinds of region in two at least
+    assert all(b >= a + 6 + 4 for a, b in zip(out[0][3], out[1][3])), (out[0][3], out[1][3])
