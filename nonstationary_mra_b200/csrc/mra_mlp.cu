@@ -825,6 +825,49 @@ mra_status sync_bf16(mra_mlp* n) {
     return MRA_OK;
 }
 
+// Queues a prediction's copies and kernels.
+mra_status enqueue_predict(mra_mlp* n, const float* x, long N, float* y, float* dydx, int* tc_err) {
+    MlpArgs a = args_of(n, N, n->Xq);
+    a.Y = n->Yq;
+    a.G = n->Gq;
+    if (dydx) {
+        MCU(cudaMemcpyAsync(n->Xq, x, (size_t)N * n->D * sizeof(float), cudaMemcpyHostToDevice, n->stream));
+        // few samples: small tiles over many CTAs (the pass is latency); many: more work per weight load
+        if (N <= (long)SQ * 2 * n->sms) {
+            const int grid = (int)((N + SQ - 1) / SQ);
+            k_mlp_pass<SQ><<<grid, NT, smem_bytes(n->D, SQ), n->stream>>>(a);
+        } else {
+            const int grid = (int)std::min<long>((N + S - 1) / S, (long)n->sms);
+            k_mlp_pass<S><<<grid, NT, smem_bytes(n->D, S), n->stream>>>(a);
+        }
+    } else {
+        // values only: the 128 x 128 layer on the tensor cores (tcgen05), 128 samples per tile
+        MCU(cudaMemsetAsync(n->tc_err, 0, sizeof(int), n->stream));
+        // The inputs are copied in runs of one tile per SM on a stream of their own, each run's kernel after its
+        // copy: the copies (some 260 us for 65,536 samples of 19 from pageable memory) hide all kernels but the last.
+        const long run = (long)TC_M * n->sms;
+        for (long i0 = 0; i0 < N; i0 += run) {
+            const long k = std::min(run, N - i0);
+            cudaStream_t cs = N > run ? n->copy : n->stream;
+            MCU(cudaMemcpyAsync(n->Xq + i0 * n->D, x + i0 * n->D, (size_t)k * n->D * sizeof(float),
+                                cudaMemcpyHostToDevice, cs));
+            if (N > run) {
+                MCU(cudaEventRecord(n->copied, n->copy));
+                MCU(cudaStreamWaitEvent(n->stream, n->copied, 0));
+            }
+            a.N = k;
+            a.X = n->Xq + i0 * n->D;
+            a.Y = n->Yq + i0;
+            k_mlp_forward_tc<<<(int)((k + TC_M - 1) / TC_M), TC_T, sizeof(TcSmem), n->stream>>>(a, n->tc_err);
+        }
+    }
+    MCU(cudaGetLastError());
+    MCU(cudaMemcpyAsync(y, n->Yq, (size_t)N * sizeof(float), cudaMemcpyDeviceToHost, n->stream));
+    if (dydx) MCU(cudaMemcpyAsync(dydx, n->Gq, (size_t)N * n->D * sizeof(float), cudaMemcpyDeviceToHost, n->stream));
+    if (!dydx) MCU(cudaMemcpyAsync(tc_err, n->tc_err, sizeof(int), cudaMemcpyDeviceToHost, n->stream));
+    return MRA_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -1002,45 +1045,13 @@ mra_status mra_mlp_predict(mra_mlp* n, const float* x, int64_t N, float* y, floa
         MCU(cudaMalloc((void**)&n->Gq, (size_t)MAXN * n->D * sizeof(float)));
     }
     if (!n->tc_err) MCU(cudaMalloc((void**)&n->tc_err, sizeof(int)));
-    MlpArgs a = args_of(n, N, n->Xq);
-    a.Y = n->Yq;
-    a.G = n->Gq;
-    if (dydx) {
-        MCU(cudaMemcpyAsync(n->Xq, x, (size_t)N * n->D * sizeof(float), cudaMemcpyHostToDevice, n->stream));
-        // few samples: small tiles over many CTAs (the pass is latency); many: more work per weight load
-        if (N <= (long)SQ * 2 * n->sms) {
-            const int grid = (int)((N + SQ - 1) / SQ);
-            k_mlp_pass<SQ><<<grid, NT, smem_bytes(n->D, SQ), n->stream>>>(a);
-        } else {
-            const int grid = (int)std::min<long>((N + S - 1) / S, (long)n->sms);
-            k_mlp_pass<S><<<grid, NT, smem_bytes(n->D, S), n->stream>>>(a);
-        }
-    } else {
-        // values only: the 128 x 128 layer on the tensor cores (tcgen05), 128 samples per tile
-        MCU(cudaMemsetAsync(n->tc_err, 0, sizeof(int), n->stream));
-        // The inputs are copied in runs of one tile per SM on a stream of their own, each run's kernel after its
-        // copy: the copies (some 260 us for 65,536 samples of 19 from pageable memory) hide all kernels but the last.
-        const long run = (long)TC_M * n->sms;
-        for (long i0 = 0; i0 < N; i0 += run) {
-            const long k = std::min(run, N - i0);
-            cudaStream_t cs = N > run ? n->copy : n->stream;
-            MCU(cudaMemcpyAsync(n->Xq + i0 * n->D, x + i0 * n->D, (size_t)k * n->D * sizeof(float),
-                                cudaMemcpyHostToDevice, cs));
-            if (N > run) {
-                MCU(cudaEventRecord(n->copied, n->copy));
-                MCU(cudaStreamWaitEvent(n->stream, n->copied, 0));
-            }
-            a.N = k;
-            a.X = n->Xq + i0 * n->D;
-            a.Y = n->Yq + i0;
-            k_mlp_forward_tc<<<(int)((k + TC_M - 1) / TC_M), TC_T, sizeof(TcSmem), n->stream>>>(a, n->tc_err);
-        }
-    }
-    MCU(cudaGetLastError());
-    MCU(cudaMemcpyAsync(y, n->Yq, (size_t)N * sizeof(float), cudaMemcpyDeviceToHost, n->stream));
-    if (dydx) MCU(cudaMemcpyAsync(dydx, n->Gq, (size_t)N * n->D * sizeof(float), cudaMemcpyDeviceToHost, n->stream));
     int tc_err = 0;
-    if (!dydx) MCU(cudaMemcpyAsync(&tc_err, n->tc_err, sizeof(int), cudaMemcpyDeviceToHost, n->stream));
+    const mra_status s = enqueue_predict(n, x, N, y, dydx, &tc_err);
+    if (s != MRA_OK) {  // what was queued on either stream still uses the caller's arrays
+        cudaStreamSynchronize(n->copy);
+        cudaStreamSynchronize(n->stream);
+        return s;
+    }
     MCU(cudaStreamSynchronize(n->stream));
     if (tc_err) return mfail(MRA_ERR_TIMEOUT, "mra_mlp_predict: the tensor-core product did not complete in time");
     return MRA_OK;
