@@ -479,7 +479,7 @@ __global__ void k_mlp_sync_bf16(long P, const float* master, __nv_bfloat16* W1b,
 
 // ---------------------------------------------------------------------------
 // Forward pass on the 5th-generation tensor cores (prediction without input
-// gradients).  One CTA of 512 threads takes tiles of 128 samples (sample s = TMEM
+// gradients).  One CTA of 512 threads takes a tile of 128 samples (sample s = TMEM
 // lane s), four threads per sample, each a quarter of the hidden units:
 //   layer 1 (n_in x 128, small) on the FP32 cores, exactly as k_mlp_pass;
 //   layer 2 (128 x 128 x 128) as tcgen05.mma kind::tf32 with the product in
@@ -488,8 +488,9 @@ __global__ void k_mlp_sync_bf16(long P, const float* master, __nv_bfloat16* W1b,
 //     hi W2^T + lo W2^T is FP32-accurate (the remainder's own truncation to TF32
 //     costs at most 2^-21 |a1|);
 //   the output layer on the FP32 cores from the product read back by tcgen05.ld.
-// The FP32 parts (layer 1 and 256 SiLUs per sample) set the time: 65,536 samples
-// took 140 us with one thread per sample, 50 us now.
+// The FP32 parts (layer 1 and 256 SiLUs per sample) set the time: 65,536 samples in one
+// launch took 140 us with one thread per sample and 50 with four (mra_mlp_predict
+// launches them in runs of a tile per SM, behind their input copies).
 // Operands sit in shared memory in the canonical K-major layout without
 // swizzle: 8-row x 16-byte core matrices, the two core matrices of one MMA's K
 // slice 128 bytes apart (leading byte offset), consecutive 8-row groups 4096
@@ -509,7 +510,6 @@ struct TcSmem {
     float b1[H], b2[H], w3[H];
     unsigned long long bar;                  // MMA completion
     unsigned tmem_base;
-    int abort;
 };
 
 // element (row, k) of a 128-row, 128-deep K-major tile of 4-byte elements
@@ -573,25 +573,26 @@ __device__ __forceinline__ void fma2(float* z, float2 a, float2 b) {
     z[1] = c.y;
 }
 
-// y = MLP(x) for a.N samples (a.Y); *err = 1 if a bounded wait gave up.
+// y = MLP(x) for a.N samples (a.Y), one tile per CTA; *err = 1 if a bounded wait gave up.
 __global__ void __launch_bounds__(TC_T, 1) k_mlp_forward_tc(MlpArgs a, int* err) {
     extern __shared__ __align__(1024) unsigned char tc_raw[];
     TcSmem& sm = *reinterpret_cast<TcSmem*>(tc_raw);
     const int tid = threadIdx.x, warp = tid >> 5, D = a.D;
     const int smp = tid & (TC_M - 1), hq = tid / TC_M;  // sample of the tile, quarter of the hidden units
     const int XD = D | 1;
-    auto load_x = [&](long tile) {
-        const long left = a.N - tile * TC_M;
+    const long s0 = (long)blockIdx.x * TC_M;
+    const bool valid = s0 + smp < a.N;
+    {
+        const long left = a.N - s0;
         const int n = (int)(left < TC_M ? left : TC_M) * D;
-        const float* X = a.X + tile * TC_M * D;
+        const float* X = a.X + s0 * D;
         for (int e = tid; e < TC_M * D; e += TC_T) {
             const int q = e / D;
             float* dst = sm.Alo + e + q * (XD - D);
             if (e < n) cp_async4(dst, X + e);
             else *dst = 0.f;
         }
-    };
-    load_x(blockIdx.x);
+    }
     {
         uint4 v[4];
 #pragma unroll
@@ -621,7 +622,6 @@ __global__ void __launch_bounds__(TC_T, 1) k_mlp_forward_tc(MlpArgs a, int* err)
         sm.w3[h] = __bfloat162float(a.w3b[h]);
     }
     if (tid == 0) {
-        sm.abort = 0;
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(tc_smem(&sm.bar)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
@@ -638,83 +638,71 @@ __global__ void __launch_bounds__(TC_T, 1) k_mlp_forward_tc(MlpArgs a, int* err)
     const unsigned tmem = sm.tmem_base;
     const unsigned lane_addr = tmem + ((unsigned)((warp & 3) * 32) << 16) + (unsigned)(32 * hq);
     const float b3 = a.master[a.b3];
-    const long ntiles = (a.N + TC_M - 1) / TC_M;
-    unsigned parity = 0;
-    for (long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const long s0 = tile * TC_M;
-        const bool valid = s0 + smp < a.N;
-        const float* xs = sm.Alo;
-        cp_async_all();
-        __syncthreads();
-        // layer 1 on the FP32 cores, in k_mlp_pass's order: z1 = b1 + sum_d W1[h][d] x[d]
-        float z[H / 4];
+    const float* xs = sm.Alo;
+    cp_async_all();
+    __syncthreads();
+    // layer 1 on the FP32 cores, in k_mlp_pass's order: z1 = b1 + sum_d W1[h][d] x[d]
+    float z[H / 4];
 #pragma unroll
-        for (int h = 0; h < H / 4; ++h) z[h] = sm.b1[32 * hq + h];
-        for (int d = 0; d < D; ++d) {
-            const float xd = xs[smp * XD + d];
-            const float2 x2 = make_float2(xd, xd);
-            const float4* wr = reinterpret_cast<const float4*>(sm.W1t + d * H + 32 * hq);
+    for (int h = 0; h < H / 4; ++h) z[h] = sm.b1[32 * hq + h];
+    for (int d = 0; d < D; ++d) {
+        const float xd = xs[smp * XD + d];
+        const float2 x2 = make_float2(xd, xd);
+        const float4* wr = reinterpret_cast<const float4*>(sm.W1t + d * H + 32 * hq);
 #pragma unroll
-            for (int q = 0; q < H / 16; ++q) {
-                const float4 w = wr[q];
-                fma2(z + 4 * q, make_float2(w.x, w.y), x2);
-                fma2(z + 4 * q + 2, make_float2(w.z, w.w), x2);
-            }
+        for (int q = 0; q < H / 16; ++q) {
+            const float4 w = wr[q];
+            fma2(z + 4 * q, make_float2(w.x, w.y), x2);
+            fma2(z + 4 * q + 2, make_float2(w.z, w.w), x2);
         }
-        __syncthreads();  // the inputs have been read
+    }
+    __syncthreads();  // the inputs have been read
 #pragma unroll
-        for (int h = 0; h < H / 4; h += 4) {
-            float4 hi, lo;
-            float* ph = &hi.x;
-            float* pl = &lo.x;
+    for (int h = 0; h < H / 4; h += 4) {
+        float4 hi, lo;
+        float* ph = &hi.x;
+        float* pl = &lo.x;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float a1 = z[h + e] * sigm(z[h + e]);
-                ph[e] = __uint_as_float(__float_as_uint(a1) & 0xffffe000u);  // exact in TF32
-                pl[e] = a1 - ph[e];
-            }
-            const int at = tc_idx(smp, 32 * hq + h);  // four consecutive k of one core-matrix row
-            *reinterpret_cast<float4*>(sm.Ahi + at) = hi;
-            *reinterpret_cast<float4*>(sm.Alo + at) = lo;
+        for (int e = 0; e < 4; ++e) {
+            const float a1 = z[h + e] * sigm(z[h + e]);
+            ph[e] = __uint_as_float(__float_as_uint(a1) & 0xffffe000u);  // exact in TF32
+            pl[e] = a1 - ph[e];
         }
-        // the tile's operands, written by every thread, become visible to the tensor core
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        tc_fence_before();
-        __syncthreads();
-        if (tid == 0) {
-            tc_fence_after();
-            const unsigned ahi = tc_smem(sm.Ahi), alo = tc_smem(sm.Alo), bw = tc_smem(sm.W2f);
-            for (int k = 0; k < H / 8; ++k) {
-                const unsigned off = (unsigned)k * 2u * TC_LBO;  // K slice k: core matrices 2k, 2k+1
-                tc_mma(tmem, tc_desc(ahi + off), tc_desc(bw + off), k > 0);
-                tc_mma(tmem, tc_desc(alo + off), tc_desc(bw + off), true);
-            }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                             tc_smem(&sm.bar))
-                         : "memory");
-        }
-        bool done = false;
-        for (long it = 0; it < kTcSpin && !done; ++it) done = tc_try_wait(&sm.bar, parity);
-        parity ^= 1u;
-        if (__syncthreads_or(done ? 0 : 1)) {
-            if (tid == 0) atomicExch(err, 1);
-            break;
-        }
+        const int at = tc_idx(smp, 32 * hq + h);  // four consecutive k of one core-matrix row
+        *reinterpret_cast<float4*>(sm.Ahi + at) = hi;
+        *reinterpret_cast<float4*>(sm.Alo + at) = lo;
+    }
+    // the tile's operands, written by every thread, become visible to the tensor core
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    tc_fence_before();
+    __syncthreads();
+    if (tid == 0) {
         tc_fence_after();
-        // the operands are free: the next tile's inputs arrive during the output layer
-        if (tile + gridDim.x < ntiles) load_x(tile + gridDim.x);
-        {
-            float v[32], y = 0.f;
-            tc_ld32(lane_addr, v);
-            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-#pragma unroll
-            for (int q = 0; q < 32; ++q) {
-                const float z2 = v[q] + sm.b2[32 * hq + q];
-                y = fmaf(sm.w3[32 * hq + q], z2 * sigm(z2), y);
-            }
-            sm.Ahi[hq * TC_M + smp] = y;  // the product is complete: its operands are free
+        const unsigned ahi = tc_smem(sm.Ahi), alo = tc_smem(sm.Alo), bw = tc_smem(sm.W2f);
+        for (int k = 0; k < H / 8; ++k) {
+            const unsigned off = (unsigned)k * 2u * TC_LBO;  // K slice k: core matrices 2k, 2k+1
+            tc_mma(tmem, tc_desc(ahi + off), tc_desc(bw + off), k > 0);
+            tc_mma(tmem, tc_desc(alo + off), tc_desc(bw + off), true);
         }
-        // every thread's reads of the product precede the next tile's MMAs into it
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
+                         tc_smem(&sm.bar))
+                     : "memory");
+    }
+    bool done = false;
+    for (long it = 0; it < kTcSpin && !done; ++it) done = tc_try_wait(&sm.bar, 0);
+    if (__syncthreads_or(done ? 0 : 1)) {
+        if (tid == 0) atomicExch(err, 1);
+    } else {
+        tc_fence_after();
+        float v[32], y = 0.f;
+        tc_ld32(lane_addr, v);
+        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+        for (int q = 0; q < 32; ++q) {
+            const float z2 = v[q] + sm.b2[32 * hq + q];
+            y = fmaf(sm.w3[32 * hq + q], z2 * sigm(z2), y);
+        }
+        sm.Ahi[hq * TC_M + smp] = y;  // the product is complete: its operands are free
         tc_fence_before();
         __syncthreads();
         if (hq == 0 && valid)
