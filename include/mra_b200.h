@@ -205,8 +205,10 @@ mra_status mra_eval_covariance(const mra_model* m, const mra_theta* theta, const
 mra_status mra_eval_fields(const mra_model* m, const mra_theta* theta, const double* p, uint64_t n,
                            double* out);
 
-/* Autotuner of the FP64 products' tile shapes.  No counterpart in the
- * reference.  Times `evals` log-likelihood evaluations of this context (after
+/* Autotuner of the tile shapes of the general FP64 products: the products
+ * inside factored posterior steps, prediction from finest regions of many
+ * points or with r > 64, factors of more than 128 rows (the other stages run on
+ * tiles of fixed shape).  No counterpart in the reference.  Times `evals` log-likelihood evaluations of this context (after
  * one warm-up) for each candidate CTA tile width per product-width bucket
  * (products at most 16, at most 32, and more than 32 columns wide; widths of
  * 16, 32 or 64 columns over 64 rows) and keeps the fastest for the device.

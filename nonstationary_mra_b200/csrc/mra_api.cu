@@ -1443,9 +1443,6 @@ mra_status mra_autotune(mra_ctx* c, int32_t evals, int32_t* choice_out, double* 
     int ib = 0;
     for (int k = 0; k < nc; ++k) {
         CU(set_gemm_tiles(cand[k]));
-        CU(set_gemm_tiles_prior(cand[k]));
-        CU(set_gemm_tiles_finest(cand[k]));
-        CU(set_gemm_tiles_posterior(cand[k]));
         double d, ll, ms = 0.0;
         mra_status st = mra_loglik(c, &d, &ll);  // warm-up with this choice
         if (st != MRA_OK) return st;
@@ -1460,9 +1457,6 @@ mra_status mra_autotune(mra_ctx* c, int32_t evals, int32_t* choice_out, double* 
         if (ms < best) best = ms, ib = k;
     }
     CU(set_gemm_tiles(cand[ib]));
-    CU(set_gemm_tiles_prior(cand[ib]));
-    CU(set_gemm_tiles_finest(cand[ib]));
-    CU(set_gemm_tiles_posterior(cand[ib]));
     if (choice_out)
         for (int b = 0; b < 3; ++b) choice_out[b] = cand[ib][b];
     if (ms_out) *ms_out = best / evals;

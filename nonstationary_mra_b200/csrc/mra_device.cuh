@@ -912,7 +912,8 @@ __device__ inline void gemm_f32(int M, int N, int K, float alpha, const float* A
 // any leading dimensions; A and B in global memory.  beta == 0 never reads C.
 // Ends with a barrier.
 // FP64 tile width (NW) per product-width bucket (N <= 16, N <= 32, wider),
-// chosen per device by the autotuner (mra_autotune); {1, 2, 4} by default.
+// chosen per device by the autotuner (mra_autotune); {1, 2, 4} by default.  Every
+// file that includes this holds its own copy (set_gemm_tiles sets them all).
 // The choice changes only how output tiles are spread over warps: every
 // element is accumulated by one thread in the same K order, so results are
 // bitwise the same whatever the choice.

@@ -675,8 +675,6 @@ cudaError_t prepare_finest() {
     return e;
 }
 
-cudaError_t set_gemm_tiles_finest(const int nw[3]) { return cudaMemcpyToSymbol(c_gemm_nw, nw, 3 * sizeof(int)); }
-
 template int launch_finest<double>(const Geom&, const DevTree<double>&, int, bool, cudaStream_t, const Fork&);
 template int launch_finest<float>(const Geom&, const DevTree<float>&, int, bool, cudaStream_t, const Fork&);
 

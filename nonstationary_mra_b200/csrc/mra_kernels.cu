@@ -360,7 +360,13 @@ static cudaError_t prepare_type() {
     return e;
 }
 
-cudaError_t set_gemm_tiles(const int nw[3]) { return cudaMemcpyToSymbol(c_gemm_nw, nw, 3 * sizeof(int)); }
+// every file with FP64 products holds its own copy of the widths
+cudaError_t set_gemm_tiles(const int nw[3]) {
+    cudaError_t e = cudaMemcpyToSymbol(c_gemm_nw, nw, 3 * sizeof(int));
+    for (auto set : {set_gemm_tiles_prior, set_gemm_tiles_posterior, set_gemm_tiles_predict})
+        if (e == cudaSuccess) e = set(nw);
+    return e;
+}
 
 cudaError_t prepare_kernels() {
     cudaError_t e = prepare_type<double>();

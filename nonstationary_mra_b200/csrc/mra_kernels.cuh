@@ -247,8 +247,8 @@ int launch_condition_set(const Geom& g, const DevTree<double>& t, const CondSet&
 // prediction in chunks (FP64, r <= 64); returns the number of kernels launched
 int launch_predict_chunks(const Geom& g, const DevTree<double>& t, cudaStream_t st);
 cudaError_t prepare_predict();
+cudaError_t set_gemm_tiles_predict(const int nw[3]);
 cudaError_t prepare_finest();
-cudaError_t set_gemm_tiles_finest(const int nw[3]);
 // One posterior level (FP64): its dense regions in chunks whose scratch fits
 // t.cbuf, its factored ones beside them; returns the number of kernels launched, or -1
 // (nothing launched) if the scratch does not hold one region of each kind.

@@ -419,4 +419,6 @@ cudaError_t prepare_predict() {
     return e;
 }
 
+cudaError_t set_gemm_tiles_predict(const int nw[3]) { return cudaMemcpyToSymbol(c_gemm_nw, nw, 3 * sizeof(int)); }
+
 }  // namespace mra
