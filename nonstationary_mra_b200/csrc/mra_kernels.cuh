@@ -135,6 +135,8 @@ using CondSet = CondSetT<double>;
 // Prediction points of a finest region handled as vectors, four per pass over its blocks; more go
 // through tile products.  65,536 observations, 16 points per region, vectors / tiles: 1.11 / 0.94 ms
 // with 64 observations per region, 2.26 / 2.48 with 16; 10 points: 1.55 / 1.73 with 16.
+// The crossing lies lower where a region holds more observations (its blocks are read
+// once per four points); the line is taken for the usual 16.
 constexpr int kPredVector = 12;
 constexpr int kQueuePost = 4;
 constexpr int kQueueCounters = kQueuePost + kMaxLevels;

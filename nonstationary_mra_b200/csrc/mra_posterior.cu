@@ -16,9 +16,11 @@
 // regions use the reference's dense r x r slices.  Prediction mode also forms
 // L~, v and G of factored regions from (F, f).
 //
-// A level's factored regions (k_fact_*; beyond 128 rows one CTA each from a queue,
-// k_posterior_factored) and its dense ones run tile by tile, in launches split by
-// what is independent.  Dense:
+// A level's dense regions and, where the context keeps at most 128 rows in factored
+// form (MRA_FACTORED_MAX; 2r by default, so r <= 64), its factored ones run tile by
+// tile, in launches split by what is independent (k_dense_*, k_fact_*).  With a larger
+// limit all factored regions, whatever their rows, take one CTA each from a queue
+// (k_posterior_factored).  Dense:
 //   k_dense_gather   slices (j, k) of the summed children contributions, and
 //                    L L^T + A_(m,m): one CTA per tile of a slice
 //   k_dense_factor   L~ with its inverse, v, the log-lik term: one CTA per region
@@ -36,7 +38,7 @@
 namespace mra {
 
 // ---------------------------------------------------------------------------
-// factored regions of more than 128 rows (MRA_FACTORED_MAX above 128)
+// factored regions of a context that keeps more than 128 rows in factored form
 // ---------------------------------------------------------------------------
 // The products of the posterior steps go through a separate function: the
 // steps keep many values live across their products, and inlined there the
@@ -389,7 +391,7 @@ __global__ void __launch_bounds__(Tile<TS>::NT, Tile<TS>::CTAS) k_dense_out(DevT
 }
 
 // ---------------------------------------------------------------------------
-// factored regions of at most 128 rows, in tiles
+// factored regions of a context that keeps at most 128 rows in factored form, in tiles
 // ---------------------------------------------------------------------------
 // k_fact_y       Y = L^{-1} F_m^T                      one CTA per tile
 // k_fact_factor  R R^T = I + Y^T Y with R^{-1}, f'     one CTA per region
