@@ -324,7 +324,7 @@ __device__ __forceinline__ double cov_fast_entry(double pc0, double pc1, double 
 // this: chordal 6.67 / 6.72 / 6.67 and 7.16 / 7.20 / 7.11 e-16, planar 3.08 / 3.23 / 3.15
 // and 3.41 / 3.52 / 3.40 e-16; against the 64-bit expression 3.08 / 3.18 / 3.10, 3.29 /
 // 3.43 / 3.37, 2.39 / 2.43 / 2.26 and 2.60 / 2.63 / 2.52 e-16.  66 us for 4001 x 3003
-// planar entries instead of 63.
+// planar entries instead of 63, with k_cov_tiles at four CTAs per SM.
 struct CovScale {
     double scale, hi, lo;  // distance scale; hi + lo: the exponent's factor, scale or sqrt(3) scale
 };

@@ -250,10 +250,11 @@ __global__ void __launch_bounds__(kThreads, 2) k_sample(DevTree<T> t, const doub
 // evaluate_*covariance blocks (layout out[i1*n2 + i2])
 // ---------------------------------------------------------------------------
 // Straight-line nonstationary forms: tiles of RT rows x CT columns by the blocks of
-// mra_device.cuh (4001 x 3003 planar entries: 66 to 68 us a call, 1.4 TB/s of results; by the
-// entry-per-thread kernel below 142 to 144).
+// mra_device.cuh (4001 x 3003 planar entries: 62 to 64 us a call, 1.5 TB/s of results; by the
+// entry-per-thread kernel below 142 to 144).  Two CTAs per SM, whose 128 registers hold the
+// entry without spills: 3 take 64 and 66 us, 4 take 66 and 68.
 template <int KIND>
-__global__ void __launch_bounds__(kCovThreads, 4) k_cov_tiles(CovScale scale, PointSet P, long a0, int na, long b0, int nb,
+__global__ void __launch_bounds__(kCovThreads, 2) k_cov_tiles(CovScale scale, PointSet P, long a0, int na, long b0, int nb,
                                                               int self, int RT, int CT, double* out) {
     __shared__ __align__(16) double stage[7 * kCovChunk];
     const int t0 = blockIdx.x * RT, q0 = blockIdx.y * CT;
