@@ -41,6 +41,12 @@ struct Pt {
     double c0, c1, c2;
 };
 
+// Models whose FP64 entries take the short forms: nonstationary, straight-line distance, prefactor
+// exponent 1.5 or 1 (and a scale that is a number: exp_neg passes no undefined exponent on).
+__host__ __device__ __forceinline__ bool fast_form(const Geom& g) {
+    return g.nonstat && g.distance != 1 && g.pref_kind != 2 && g.dist_scale == g.dist_scale;
+}
+
 __device__ __forceinline__ double point_distance(const Geom& g, const Pt& a, const Pt& b) {
     if (g.distance == 1) {
         // great_circle_dist, evaluate_covariance.cpp:9-25
@@ -436,7 +442,7 @@ __device__ __noinline__ void fill_cov_staged(const Geom& g, const PointSet& P, c
     const bool worker = tid < rows * cols;
     const int tr = tid % rows, tq = tid / rows;
     const int nu = g.nu_x2, pk = g.pref_kind;
-    const bool fast = sizeof(T) == 8 && g.nonstat && g.distance != 1 && pk != 2;
+    const bool fast = sizeof(T) == 8 && fast_form(g);
     const double scale = fabs(g.dist_scale);  // as in cov_block
     for (int q0 = 0; q0 < nb; q0 += CH) {
         const int qn = nb - q0 < CH ? nb - q0 : CH;
@@ -631,7 +637,7 @@ __device__ __forceinline__ void cov_block(const Geom& g, const PointSet& P, long
 }
 
 inline int cov_kind(const Geom& g, bool fp64) {
-    if (!(fp64 && g.nonstat && g.distance != 1 && g.pref_kind != 2)) return 0;
+    if (!fp64 || !fast_form(g)) return 0;
     return g.nu_x2 == 3 ? (g.pref_kind == 1 ? 1 : 2) : (g.pref_kind == 1 ? 3 : 4);
 }
 

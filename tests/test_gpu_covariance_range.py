@@ -154,3 +154,14 @@ def test_negative_sill_scale_of_every_form(form):
     ref = expected(md, p1, p2)
     np.testing.assert_allclose(static_block(md, p1, p2, -1.0), ref, rtol=RTOL)
     np.testing.assert_allclose(api.eval_covariance(md, dict(THETA, sill_scale=-1.0), p1, p2), ref, rtol=RTOL)
+
+
+@pytest.mark.parametrize("form", FORMS, ids=lambda f: f"d{f[0]}nu{f[1]}p{f[2]}")
+def test_undefined_distance_scale(form):
+    """An undefined scale makes the entries undefined: an error status, not a finite log-likelihood."""
+    from nonstationary_mra_b200.capi import MRAError
+    from test_gpu_parity import random_case, run_loglik
+    st, md = random_case(4, 4, 3, 16, 900, 40, False, form[1], True)
+    md.distance, md.prefactor_exp, md.dist_scale = form[0], form[2], float("nan")
+    with pytest.raises(MRAError, match="NOT_SPD"):
+        run_loglik(st, md)
